@@ -330,6 +330,9 @@ lf2_status lf2_create(lf2_ctx** out, int device, const int n[3], const double bo
   ok = ok && cudaMallocHost(&c->h_flags, sizeof(uint32_t)) == cudaSuccess;
   ok = ok && cudaMallocHost(&c->h_i64, sizeof(int64_t) * 4) == cudaSuccess;
   ok = ok && cudaMalloc(&c->work, sizeof(int)) == cudaSuccess;
+  ok = ok && cudaMalloc(&c->part_item, sizeof(int4) * (PART_ITEMS + PART_TILES)) == cudaSuccess;
+  ok = ok && cudaMalloc(&c->part_head, sizeof(int32_t) * 3) == cudaSuccess;
+  ok = ok && cudaMalloc(&c->part_tile, sizeof(uint64_t*) * PART_TILES) == cudaSuccess;
   ok = ok && cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess;
   if (ok) {
     ok = cudaMemsetAsync(c->count, 0, sizeof(int32_t) * nb, c->stream) == cudaSuccess &&
@@ -385,6 +388,9 @@ lf2_status lf2_destroy(lf2_ctx* c)
   cudaFree(c->ovf_count);
   cudaFree(c->ovf_state);
   cudaFree(c->spill);
+  cudaFree(c->part_item);
+  cudaFree(c->part_head);
+  cudaFree(c->part_tile);
   cudaFree(c->stencil_partial);
   cudaFree(c->pm_acc);
   fft_release(c);

@@ -38,6 +38,7 @@
 //                           the rounding of unordered FP32 additions.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 
@@ -57,6 +58,11 @@ namespace {
 #define LF2_DEP_THREADS 256
 #endif
 constexpr int DEP_THREADS = LF2_DEP_THREADS;
+
+// Fewest particles of a part of a split brick.
+#ifndef LF2_PART_MIN
+#define LF2_PART_MIN 1024
+#endif
 
 // Components of the field of a kind.
 template <int KIND>
@@ -83,17 +89,18 @@ struct Pass {
   // threads per CTA: a tile above 100 KB leaves room for one CTA per SM, so
   // it gets twice the warps
   static constexpr int THREADS = smem() > 100 * 1024 ? 2 * DEP_THREADS : DEP_THREADS;
+  // CTAs per SM that the registers leave room for: those whose tiles fit
+  static constexpr int CTAS = smem() > 100 * 1024 ? 1 : smem() > 50 * 1024 ? 3 : 5;
 };
 
 __device__ __forceinline__ float sel(int b, float up, float dn) { return b ? up : dn; }
 
 // ------------------------------------------------------------- tile pass
 template <int KIND, int PASS, int ACC>
-__global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS) k_deposit(StoreView v, DepositParams dp,
-                                                         float* __restrict__ out,
-                                                         uint64_t* __restrict__ spill,
-                                                         const uint32_t* __restrict__ vmax_bits,
-                                                         uint32_t* flags, const uint32_t* gate)
+__global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PASS, ACC>::CTAS)
+    k_deposit(StoreView v, DepositParams dp, float* __restrict__ out, uint64_t* __restrict__ spill,
+              const uint32_t* __restrict__ vmax_bits, uint32_t* flags, const uint32_t* gate,
+              PartView pv)
 {
   // gate: run only when the word is set (the redo of a fused deposit)
   if (gate && *gate == 0u) return;
@@ -105,16 +112,22 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS) k_deposit(Stor
   constexpr int T = P::THREADS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
 
+  __shared__ unsigned s_mass;
+
   const Geom& g = v.g;
-  const int64_t b = blockIdx.x;
+  Part part;
+  if (!part_take(pv, g.nbricks, v.count, v.cap, part)) return;
+  const int64_t b = part.b;
   int bx, by, bz;
   brick_coords(g, b, bx, by, bz);
   const int ex = brick_extent(g.n[0], bx), ey = brick_extent(g.n[1], by),
             ez = brick_extent(g.n[2], bz);
   const int x0 = bx * BRICK, y0 = by * BRICK, z0 = bz * BRICK;
-  const int64_t base = v.seg_start[b];
-  const int cnt = LF2_BRICK_COUNT(v, b);
-  TileRef<TILE3> tr{smem_raw, FIXED && cnt <= split_max<SIGNED>(dp.has_mass != 0)};
+  const int64_t base = v.seg_start[b] + part.first;
+  const int cnt = part.cnt;
+  const int mass_bound =
+      FIXED && dp.has_mass ? part_mass_bound(v.a.mass, (uint32_t)base, cnt, dp.inv_unit, &s_mass) : 1;
+  TileRef<TILE3> tr{smem_raw, FIXED && cnt <= split_max<SIGNED>(mass_bound)};
   // fixed point: velocity quantum and conversion scale for this field
   int vexp = 0;
   if (FIXED && KIND != 0) vexp = vexp_of(*vmax_bits);
@@ -322,6 +335,10 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS) k_deposit(Stor
     else particles(std::false_type{}, std::false_type{});
   }
   __syncthreads();
+  if (uint64_t* scratch = part_tile(pv)) {  // k_part_finish sums the parts and writes the vertices
+    part_store<ACC, SIGNED, NC, TILE3>(scratch, tr);
+    return;
+  }
 
   // Flush: interior vertices to the field, shell vertices to the shell store
   // (8-byte slots: the integer sum, hi and lo, or the plain float).  Two
@@ -386,6 +403,58 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS) k_deposit(Stor
             make_float2(facc[(size_t)j * 2 * TILE3 + t], facc[(size_t)j * 2 * TILE3 + TILE3 + t]);
       } else {
         reinterpret_cast<float*>(sp)[(size_t)c * SHELL + f] = facc[(size_t)j * TILE3 + t];
+      }
+    }
+  }
+}
+
+// The vertices of the split bricks, from the sums of their parts: to the
+// field and the shell store as the tile pass writes them.
+constexpr int FINISH_CHUNK = 512;  // vertices per unit of work
+
+template <int KIND, int PASS, int ACC>
+__global__ void __launch_bounds__(FINISH_CHUNK) k_part_finish(Geom g, PartView pv, float fixed_scale,
+                                                     float* __restrict__ out,
+                                                     uint64_t* __restrict__ spill,
+                                                     const uint32_t* __restrict__ vmax_bits,
+                                                     uint32_t* flags, const uint32_t* gate)
+{
+  if (gate && *gate == 0u) return;
+  using P = Pass<KIND, PASS, ACC>;
+  constexpr int C = Comps<KIND>::value;
+  constexpr int CHUNKS = (TILE3 + FINISH_CHUNK - 1) / FINISH_CHUNK;
+  const int units = pv.head[2] * CHUNKS;
+  if ((int)blockIdx.x >= units) return;
+  const int vexp = ACC == ACC_FIXED && KIND != 0 ? vexp_of(*vmax_bits) : 0;
+  const float conv = ldexpf(fixed_scale, (KIND == 1 ? vexp : 2 * vexp) - (KIND != 0 ? 16 : 0));
+  for (int w = blockIdx.x; w < units; w += gridDim.x) {
+    const int4 sp = pv.split[w / CHUNKS];
+    const int t = (w % CHUNKS) * FINISH_CHUNK + threadIdx.x;
+    int bx, by, bz;
+    brick_coords(g, sp.x, bx, by, bz);
+    const int ex = brick_extent(g.n[0], bx), ey = brick_extent(g.n[1], by),
+              ez = brick_extent(g.n[2], bz);
+    const int i = t % TILE, j = (t / TILE) % TILE, k = t / (TILE * TILE);
+    if (t >= TILE3 || i > ex || j > ey || k > ez) continue;
+    const bool inner = i >= 1 && i < ex && j >= 1 && j < ey && k >= 1 && k < ez;
+    const int64_t site = inner ? site_index(g, bx * BRICK + i, by * BRICK + j, bz * BRICK + k) : 0;
+    const int si = inner ? 0
+                         : shell_index(i == ex ? BRICK : i, j == ey ? BRICK : j, k == ez ? BRICK : k);
+    uint64_t* shell = spill + (size_t)sp.x * C * SHELL;
+#pragma unroll
+    for (int jc = 0; jc < P::NC; jc++) {
+      const int c = P::comp(jc);
+      const PartSum s = part_sum<ACC>(pv, sp, jc * TILE3 + t);
+      if (inner) {
+        if (KIND == 0 && s.q < 0) set_flag(flags, ERR_FIXED_OVERFLOW);
+        out[(size_t)c * g.nsites + site] =
+            ACC == ACC_FIXED ? __fmul_rn(__ll2float_rn(s.q), conv) : __fadd_rn(s.hi, s.lo);
+      } else if (ACC == ACC_FIXED) {
+        shell[(size_t)c * SHELL + si] = (uint64_t)s.q;
+      } else if (ACC == ACC_COMP) {
+        reinterpret_cast<float2*>(shell)[(size_t)c * SHELL + si] = make_float2(s.hi, s.lo);
+      } else {
+        reinterpret_cast<float*>(shell)[(size_t)c * SHELL + si] = s.hi;
       }
     }
   }
@@ -575,8 +644,66 @@ __global__ void __launch_bounds__(256) k_vmax(StoreView v, uint32_t* vmax_bits, 
   if ((threadIdx.x & 31) == 0 && m) atomicMax(vmax_bits, m);
 }
 
+// Scratch tiles of `slots` 8-byte values, `tiles` to a bank.
+struct Banks {
+  uint64_t* bank[7];
+  int tiles, slots;
+};
+
+// Items of the bricks above `first` particles: a brick above `split` makes
+// ceil(count / P) parts, the others one.  Where the parts would need more
+// tiles than there are, P and split double until they do not; where the items
+// would not fit, `first` does.  One CTA.
+__global__ void __launch_bounds__(1024) k_part_plan(int64_t nb, const int32_t* __restrict__ count,
+                                                    const int32_t* __restrict__ cap, int P0, int split0,
+                                                    int first0, int max_items, Banks banks, int4* item,
+                                                    int4* split_list, int32_t* head, uint64_t** tile)
+{
+  __shared__ unsigned long long s_tiles, s_items;
+  __shared__ int s_tile, s_item, s_split;
+  const int max_tiles = min(7 * banks.tiles, PART_TILES);
+  long long P = P0, split = split0, first = first0;
+  for (;;) {
+    if (threadIdx.x == 0) s_tiles = s_items = 0ull, s_tile = s_item = s_split = 0;
+    __syncthreads();
+    unsigned long long tiles = 0, items = 0;
+    for (int64_t b = threadIdx.x; b < nb; b += blockDim.x) {
+      const long long c = min(count[b], cap[b]);
+      if (c > split) tiles += (unsigned long long)((c + P - 1) / P);
+      else if (c > first) items++;
+    }
+    if (tiles) atomicAdd(&s_tiles, tiles);
+    if (items) atomicAdd(&s_items, items);
+    __syncthreads();
+    const bool fewer_tiles = s_tiles > (unsigned long long)max_tiles;
+    const bool fewer_items = s_items + s_tiles > (unsigned long long)max_items;
+    if (!fewer_tiles && !fewer_items) break;
+    if (fewer_tiles || first == split) P *= 2, split *= 2;
+    if (fewer_items) first *= 2;
+    first = min(first, split);
+    __syncthreads();
+  }
+  for (int64_t b = threadIdx.x; b < nb; b += blockDim.x) {
+    const long long c = min(count[b], cap[b]);
+    if (c <= first) continue;
+    const int parts = c > split ? (int)((c + P - 1) / P) : 1;
+    const int i0 = atomicAdd(&s_item, parts), t0 = parts > 1 ? atomicAdd(&s_tile, parts) : 0;
+    for (int k = 0; k < parts; k++) item[i0 + k] = make_int4((int)b, k, parts, t0);
+    if (parts > 1) split_list[atomicAdd(&s_split, 1)] = make_int4((int)b, parts, t0, 0);
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < s_tile; t += blockDim.x)
+    tile[t] = banks.bank[t / banks.tiles] + (size_t)(t % banks.tiles) * banks.slots;
+  if (threadIdx.x == 0) {
+    head[0] = s_item;
+    head[1] = (int)min(first, (long long)INT32_MAX);
+    head[2] = s_split;
+  }
+}
+
 template <int KIND, int PASS, int ACC>
-cudaError_t tile_pass(lf2_ctx* c, float* out, const DepositParams& dp, const uint32_t* gate)
+cudaError_t tile_pass(lf2_ctx* c, float* out, const DepositParams& dp, const uint32_t* gate,
+                      const PartView& pv)
 {
   using P = Pass<KIND, PASS, ACC>;
   const size_t smem = P::smem();
@@ -584,8 +711,12 @@ cudaError_t tile_pass(lf2_ctx* c, float* out, const DepositParams& dp, const uin
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   c->launches += 1;
-  k_deposit<KIND, PASS, ACC><<<(unsigned)c->g.nbricks, P::THREADS, smem, c->stream>>>(
-      view(c), dp, out, c->spill, c->vmax_bits, c->flags, gate);
+  k_deposit<KIND, PASS, ACC><<<(unsigned)(c->g.nbricks + pv.max_items), P::THREADS, smem, c->stream>>>(
+      view(c), dp, out, c->spill, c->vmax_bits, c->flags, gate, pv);
+  if (!pv.max_items) return cudaGetLastError();
+  c->launches += 1;
+  k_part_finish<KIND, PASS, ACC><<<4 * c->num_sms, FINISH_CHUNK, 0, c->stream>>>(
+      c->g, pv, dp.fixed_scale, out, c->spill, c->vmax_bits, c->flags, gate);
   return cudaGetLastError();
 }
 
@@ -594,13 +725,19 @@ cudaError_t run(lf2_ctx* c, float* out, const DepositParams& dp, int stage, cons
 {
   const unsigned nb = (unsigned)c->g.nbricks;
   if (stage == 0) {
+    using P = Pass<KIND, 0, ACC>;
+    PartView pv;
+    const cudaError_t ep = launch_part_plan(
+        c, P::smem(), P::THREADS, (size_t)P::NC * TILE3,
+        ACC == ACC_FIXED ? split_max<KIND != 0>(c->has_mass ? 2 : 1) : 0, &pv);
+    if (ep != cudaSuccess) return ep;
     if (ACC == ACC_FIXED && KIND != 0) {
       cudaError_t e = launch_vmax(c);
       if (e != cudaSuccess) return e;
     }
-    cudaError_t e = tile_pass<KIND, 0, ACC>(c, out, dp, gate);
+    cudaError_t e = tile_pass<KIND, 0, ACC>(c, out, dp, gate, pv);
     if constexpr (KIND == 2 && ACC != ACC_PLAIN) {
-      if (e == cudaSuccess) e = tile_pass<KIND, 1, ACC>(c, out, dp, gate);
+      if (e == cudaSuccess) e = tile_pass<KIND, 1, ACC>(c, out, dp, gate, pv);
     }
     return e;
   }
@@ -619,6 +756,46 @@ cudaError_t run_mode(lf2_ctx* c, float* out, const DepositParams& dp, int stage,
 }
 
 }  // namespace
+
+// What is heavy depends on the chip's share of the particles per CTA that runs
+// at once (`share`).  A brick is an item, taken first, above a quarter of the
+// share (a brick that starts last then ends with the others) and three times
+// the mean count (an even distribution has no items).  It is split above 3/2 P
+// with P half the share, so that no CTA is left with more than that, but parts
+// hold at least LF2_PART_MIN particles: each clears and writes its tile.
+// `cap` bounds what a split fixed-point tile sums.  The scratch tiles lie in
+// the repack scratch (c->alt), which nothing uses between the rebins.
+cudaError_t launch_part_plan(lf2_ctx* c, size_t smem, int threads, size_t tile_slots, int cap,
+                             PartView* pv)
+{
+  *pv = PartView{};
+  if (c->np == 0) return cudaSuccess;
+  const int per_sm = std::max(1, std::min((int)(227 * 1024 / (smem + 1024)), 2048 / threads));
+  const int64_t share = c->np / ((int64_t)c->num_sms * per_sm);
+  if (cap <= 0) cap = 1 << 28;
+  const int64_t P = std::min<int64_t>(std::max<int64_t>(share / 2, LF2_PART_MIN), cap - cap / 16);
+  const int64_t split = std::min<int64_t>(P + P / 2, cap);
+  const int64_t first = std::min(split, std::max(share / 4, 3 * (c->np / c->g.nbricks)));
+  // np particles make at most 3/2 np / P parts and np / first items
+  const int64_t most = std::min<int64_t>(PART_ITEMS, c->np * 3 / (2 * P) + c->np / first);
+  if (most == 0) return cudaSuccess;
+  const Banks banks{{reinterpret_cast<uint64_t*>(c->alt.key), reinterpret_cast<uint64_t*>(c->alt.ox),
+                     reinterpret_cast<uint64_t*>(c->alt.oy), reinterpret_cast<uint64_t*>(c->alt.oz),
+                     reinterpret_cast<uint64_t*>(c->alt.vx), reinterpret_cast<uint64_t*>(c->alt.vy),
+                     reinterpret_cast<uint64_t*>(c->alt.vz)},
+                    (int)std::min<int64_t>(c->capacity / 2 / (int64_t)tile_slots, PART_TILES),
+                    (int)tile_slots};
+  pv->item = c->part_item;
+  pv->split = c->part_item + PART_ITEMS;
+  pv->head = c->part_head;
+  pv->tile = c->part_tile;
+  pv->max_items = (int)most;
+  c->launches += 1;
+  k_part_plan<<<1, 1024, 0, c->stream>>>(c->g.nbricks, c->count, c->cap, (int)P, (int)split,
+                                         (int)first, (int)most, banks, c->part_item,
+                                         c->part_item + PART_ITEMS, c->part_head, c->part_tile);
+  return cudaGetLastError();
+}
 
 // Shell-store slots (8 bytes each) a deposit of `comps` components needs.
 size_t deposit_spill_slots(const lf2_ctx* c, int comps)

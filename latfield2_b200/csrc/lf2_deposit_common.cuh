@@ -25,13 +25,14 @@ enum : int {
 // update is a native 32-bit shared-memory reduction; the sum is
 // lo + hi * 2^16, hi read as unsigned (scalar, q >= 0) or as signed (momentum
 // and stress).  Neither partial sum may wrap: per particle and vertex
-// |q| <= 2^32 * M with M = 1 for a global mass and M = 64 with per-particle
-// masses (relative mass < 64), so the split is exact for bricks of at most
-// split_max particles; larger bricks use 64-bit shared atomics.
+// |q| <= 2^32 * M with M = 1 for a global mass and otherwise the largest
+// relative mass of the particles summed, rounded up (mass_q keeps it below
+// 64), so the split is exact for up to split_max(M) particles; more use
+// 64-bit shared atomics, which compile to compare-and-swap loops.
 template <bool SIGNED>
-__host__ __device__ inline int split_max(bool has_mass)
+__host__ __device__ inline int split_max(int mass_bound)
 {
-  return SIGNED ? (has_mass ? 511 : 32767) : (has_mass ? 1023 : 65535);
+  return (SIGNED ? 32767 : 65535) / mass_bound;
 }
 
 // A tile of N vertices per component in shared memory: component j occupies
@@ -109,7 +110,7 @@ __device__ __forceinline__ void add_float(TileRef<N> tr, int j, int t, float w)
 // (every carry out of the 32-bit add, seen in the value the atomic returns,
 // goes to hi) and hi = the sum of (q >> 32) plus those carries, so the
 // vertex sum is hi 2^32 + lo exactly while hi stays within int32: bricks of
-// at most 32767 particles (511 with per-particle masses), split_max<true>.
+// at most split_max<true> particles.
 template <bool SPLIT, int N>
 __device__ __forceinline__ void add_fixed48_t(unsigned char* smem, int j, int t, long long q)
 {
@@ -260,6 +261,120 @@ __host__ __device__ inline int vexp_of(uint32_t bits)
   if (bits == 0u) return 0;
   const int e = (int)((bits >> 23) & 0xffu) - 126;
   return e < -96 ? -96 : e;
+}
+
+// --------------------------------------------------- parts of heavy bricks
+// A brick that holds far more particles than the others would keep one CTA
+// busy long after the rest of the chip is done.  k_part_plan lists the heavy
+// bricks (lf2_deposit.cu says which) as items that the first CTAs of a tile
+// pass take, the heaviest of them split into parts of equal particle counts.
+// A part's CTA writes its whole tile to the scratch; a finishing kernel sums
+// the parts of each split brick in part order and writes the brick's vertices
+// as the tile pass does for a brick in one part.
+struct PartView {
+  const int4* item;       // brick, part, parts of the brick, tile of part 0
+  const int4* split;      // brick, parts, tile of part 0
+  const int32_t* head;    // items, largest count that is not an item, split bricks
+  uint64_t* const* tile;  // scratch tiles, NC * N 8-byte slots each
+  int max_items;          // what the plan may list
+};
+
+// One unit of work of a tile pass: particles [first, first + cnt) of a brick.
+struct Part {
+  int64_t b;
+  int first, cnt;
+};
+
+// The unit of this CTA in a grid of nbricks + max_items: the items, then the
+// bricks in their order; false where there is none or the brick is an item.
+__device__ __forceinline__ bool part_take(const PartView& pv, int64_t nbricks, const int32_t* count,
+                                          const int32_t* cap, Part& p)
+{
+  const int i = (int)blockIdx.x, items = pv.max_items ? pv.head[0] : 0;
+  p.first = 0;
+  if (i >= items) {
+    p.b = i - items;
+    if (p.b >= nbricks) return false;
+    p.cnt = min(count[p.b], cap[p.b]);
+    return !pv.max_items || p.cnt <= pv.head[1];
+  }
+  const int4 w = pv.item[i];
+  p.b = w.x;
+  const int64_t n = min(count[p.b], cap[p.b]);
+  p.first = (int)(n * w.y / w.z);
+  p.cnt = (int)(n * (w.y + 1) / w.z) - p.first;
+  return true;
+}
+
+// The scratch tile of this CTA's unit when that is a part of a split brick
+// (read again here, so that the particle loop keeps no register for it).
+__device__ __forceinline__ uint64_t* part_tile(const PartView& pv)
+{
+  if (!pv.max_items || (int)blockIdx.x >= pv.head[0]) return nullptr;
+  const int4 w = pv.item[blockIdx.x];
+  return w.z > 1 ? pv.tile[w.w + w.y] : nullptr;
+}
+
+// A part's tile to the scratch: 8-byte values, component j of vertex t at
+// j * N + t (the integer sum, the hi/lo pair or the float).
+template <int ACC, bool SIGNED, int NC, int N>
+__device__ __forceinline__ void part_store(uint64_t* dst, const TileRef<N>& tr)
+{
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(tr.smem);
+  for (int t = threadIdx.x; t < N; t += blockDim.x) {
+#pragma unroll
+    for (int j = 0; j < NC; j++) {
+      uint64_t q;
+      if (ACC == ACC_FIXED)
+        q = (uint64_t)tile_fixed<SIGNED>(tr, j, t);
+      else if (ACC == ACC_COMP)
+        q = (uint64_t)w[(size_t)j * 2 * N + t] | ((uint64_t)w[(size_t)j * 2 * N + N + t] << 32);
+      else
+        q = w[(size_t)j * N + t];
+      dst[(size_t)j * N + t] = q;
+    }
+  }
+}
+
+// Vertex sum over a split brick's parts, in part order: the integer, or the
+// hi and lo words (lo 0 in the plain mode).
+struct PartSum {
+  long long q;
+  float hi, lo;
+};
+
+template <int ACC>
+__device__ __forceinline__ PartSum part_sum(const PartView& pv, const int4& sp, int at)
+{
+  PartSum r{0, 0.0f, 0.0f};
+#pragma unroll 4
+  for (int k = 0; k < sp.y; k++) {
+    const uint64_t v = __ldg(pv.tile[sp.z + k] + at);
+    if (ACC == ACC_FIXED)
+      r.q += (long long)v;
+    else if (ACC == ACC_COMP)
+      comp_acc(r.hi, r.lo, __uint_as_float((uint32_t)v), __uint_as_float((uint32_t)(v >> 32)));
+    else
+      r.hi = __fadd_rn(r.hi, __uint_as_float((uint32_t)v));
+  }
+  return r;
+}
+
+// Largest relative mass of the part's particles, clamped as mass_q clamps it
+// and rounded up to a whole number (at least 1): the factor by which a
+// contribution can exceed a global-mass particle's.
+__device__ __forceinline__ int part_mass_bound(const float* mass, uint32_t p0, int cnt,
+                                               float inv_unit, unsigned* s_max)
+{
+  if (threadIdx.x == 0) *s_max = 0u;
+  __syncthreads();
+  float m = 0.0f;
+  for (int i = threadIdx.x; i < cnt; i += blockDim.x)
+    m = fmaxf(m, fminf(fmaxf(__fmul_rn(mass[p0 + (uint32_t)i], inv_unit), 0.0f), 63.0f));
+  const unsigned w = __reduce_max_sync(0xffffffffu, __float_as_uint(m));  // non-negative floats
+  if ((threadIdx.x & 31) == 0 && w) atomicMax(s_max, w);
+  __syncthreads();
+  return max(1, (int)ceilf(__uint_as_float(*s_max)));
 }
 
 }  // namespace lf2

@@ -118,20 +118,22 @@ __device__ __forceinline__ int tile_at(int t0, int t1, int t2) { return t0 + FT 
 template <int PASS>
 __global__ void __launch_bounds__(FULL_THREADS)
     k_deposit_full(StoreView v, DepositParams dp, float* __restrict__ out,
-                   float* __restrict__ outer)
+                   float* __restrict__ outer, PartView pv)
 {
   constexpr int CT = FullPass<PASS>::total;
   extern __shared__ __align__(16) float tile[];
 
   const Geom& g = v.g;
-  const int64_t b = blockIdx.x;
+  Part part;
+  if (!part_take(pv, g.nbricks, v.count, v.cap, part)) return;
+  const int64_t b = part.b;
   int bx, by, bz;
   brick_coords(g, b, bx, by, bz);
   const int e[3] = {brick_extent(g.n[0], bx), brick_extent(g.n[1], by),
                     brick_extent(g.n[2], bz)};
   const int x0 = bx * BRICK, y0 = by * BRICK, z0 = bz * BRICK;
-  const int64_t base = v.seg_start[b];
-  const int cnt = LF2_BRICK_COUNT(v, b);
+  const int64_t base = v.seg_start[b] + part.first;
+  const int cnt = part.cnt;
 
   for (int t = threadIdx.x; t < 3 * FT3; t += blockDim.x) tile[t] = 0.0f;
   __syncthreads();
@@ -217,6 +219,11 @@ __global__ void __launch_bounds__(FULL_THREADS)
     }
   }
   __syncthreads();
+  if (uint64_t* scratch = part_tile(pv)) {  // k_part_finish_full sums the parts and writes the vertices
+    part_store<ACC_PLAIN, true, 3, FT3>(
+        scratch, TileRef<FT3>{reinterpret_cast<unsigned char*>(tile), false});
+    return;
+  }
 
   float* os = outer + (size_t)b * CT * FOUTER;
   for (int t = threadIdx.x; t < FT3; t += blockDim.x) {
@@ -328,22 +335,27 @@ template <int PASS, int ACC>
 __global__ void __launch_bounds__(FULL2_THREADS)
     k_deposit_full2(StoreView v, DepositParams dp, float* __restrict__ out,
                     uint64_t* __restrict__ store, const uint32_t* __restrict__ vmax_bits,
-                    uint32_t* flags)
+                    uint32_t* flags, PartView pv)
 {
   constexpr int CT = FullPass<PASS>::total;
   constexpr bool FIXED = ACC == ACC_FIXED;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ unsigned s_mass;
 
   const Geom& g = v.g;
-  const int64_t b = blockIdx.x;
+  Part part;
+  if (!part_take(pv, g.nbricks, v.count, v.cap, part)) return;
+  const int64_t b = part.b;
   int bx, by, bz;
   brick_coords(g, b, bx, by, bz);
   const int e[3] = {brick_extent(g.n[0], bx), brick_extent(g.n[1], by),
                     brick_extent(g.n[2], bz)};
   const int x0 = bx * BRICK, y0 = by * BRICK, z0 = bz * BRICK;
-  const int64_t base = v.seg_start[b];
-  const int cnt = LF2_BRICK_COUNT(v, b);
-  TileRef<FT3> tr{smem_raw, FIXED && cnt <= split_max<true>(dp.has_mass != 0)};
+  const int64_t base = v.seg_start[b] + part.first;
+  const int cnt = part.cnt;
+  const int mass_bound =
+      FIXED && dp.has_mass ? part_mass_bound(v.a.mass, (uint32_t)base, cnt, dp.inv_unit, &s_mass) : 1;
+  TileRef<FT3> tr{smem_raw, FIXED && cnt <= split_max<true>(mass_bound)};
   int vexp = 0;
   if (FIXED) vexp = vexp_of(*vmax_bits);
   const float vscale = vel_scale(vexp);
@@ -515,6 +527,10 @@ __global__ void __launch_bounds__(FULL2_THREADS)
     else particles(std::false_type{}, std::false_type{});
   }
   __syncthreads();
+  if (uint64_t* scratch = part_tile(pv)) {
+    part_store<ACC, true, 3, FT3>(scratch, tr);
+    return;
+  }
 
   // Flush: private vertices (every tile coordinate in [2, e-1]) to the field,
   // the thick shell to the store.
@@ -538,6 +554,62 @@ __global__ void __launch_bounds__(FULL2_THREADS)
         if (priv) out[(size_t)c * g.nsites + site] = __fadd_rn(hi, lo);
         else reinterpret_cast<float2*>(st)[(size_t)c * FSHELL + si] = make_float2(hi, lo);
       }
+    }
+  }
+}
+
+// The vertices of the split bricks, from the sums of their parts, as the
+// tile pass of the mode writes them (`store`: the outer layer of the plain
+// mode, the thick shell of the others).
+constexpr int FINISH_CHUNK = 512;  // vertices per unit of work
+
+template <int PASS, int ACC>
+__global__ void __launch_bounds__(FINISH_CHUNK)
+    k_part_finish_full(Geom g, PartView pv, float fixed_scale, float* __restrict__ out,
+                       uint64_t* __restrict__ store, const uint32_t* __restrict__ vmax_bits)
+{
+  constexpr int CT = FullPass<PASS>::total;
+  constexpr int CHUNKS = (FT3 + FINISH_CHUNK - 1) / FINISH_CHUNK;
+  const int units = pv.head[2] * CHUNKS;
+  if ((int)blockIdx.x >= units) return;
+  const int vexp = ACC == ACC_FIXED ? vexp_of(*vmax_bits) : 0;
+  const float conv = ldexpf(fixed_scale, (PASS == 0 ? vexp : 2 * vexp) - 16);
+  for (int w = blockIdx.x; w < units; w += gridDim.x) {
+    const int4 sp = pv.split[w / CHUNKS];
+    const int t = (w % CHUNKS) * FINISH_CHUNK + threadIdx.x;
+    int bc[3];
+    brick_coords(g, sp.x, bc[0], bc[1], bc[2]);
+    const int e[3] = {brick_extent(g.n[0], bc[0]), brick_extent(g.n[1], bc[1]),
+                      brick_extent(g.n[2], bc[2])};
+    const int u[3] = {t % FT, (t / FT) % FT, t / (FT * FT)};
+    if (t >= FT3 || u[0] > e[0] + 1 || u[1] > e[1] + 1 || u[2] > e[2] + 1) continue;
+    // vertices that go to the field: the brick's own (plain), or those that
+    // no other brick reaches
+    bool to_field = true;
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+      to_field &= ACC == ACC_PLAIN ? u[d] >= 1 && u[d] <= e[d] : u[d] >= 2 && u[d] < e[d];
+    const int64_t site = to_field ? site_index(g, bc[0] * BRICK + u[0] - 1, bc[1] * BRICK + u[1] - 1,
+                                               bc[2] * BRICK + u[2] - 1)
+                                  : 0;
+    int si = 0;
+    if (!to_field)
+      si = ACC == ACC_PLAIN ? outer_index(u[0] == e[0] + 1 ? FT - 1 : u[0], u[1] == e[1] + 1 ? FT - 1 : u[1],
+                                          u[2] == e[2] + 1 ? FT - 1 : u[2])
+                            : thick_index(canon(u[0], e[0]), canon(u[1], e[1]), canon(u[2], e[2]));
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      const int c = FullPass<PASS>::comp(j);
+      const PartSum s = part_sum<ACC>(pv, sp, j * FT3 + t);
+      if (to_field)
+        out[(size_t)c * g.nsites + site] =
+            ACC == ACC_FIXED ? __fmul_rn(__ll2float_rn(s.q), conv) : __fadd_rn(s.hi, s.lo);
+      else if (ACC == ACC_PLAIN)
+        reinterpret_cast<float*>(store)[((size_t)sp.x * CT + c) * FOUTER + si] = s.hi;
+      else if (ACC == ACC_FIXED)
+        store[((size_t)sp.x * CT + c) * FSHELL + si] = (uint64_t)s.q;
+      else
+        reinterpret_cast<float2*>(store)[((size_t)sp.x * CT + c) * FSHELL + si] = make_float2(s.hi, s.lo);
     }
   }
 }
@@ -634,17 +706,30 @@ __global__ void __launch_bounds__(256, 4)
   }
 }
 
+constexpr size_t FULL_SMEM = (size_t)3 * FT3 * sizeof(float), FULL2_SMEM = 2 * FULL_SMEM;
+
 template <int PASS, int ACC>
-cudaError_t tile_pass2(lf2_ctx* c, float* out, const DepositParams& dp)
+cudaError_t finish(lf2_ctx* c, float* out, const DepositParams& dp, const PartView& pv)
 {
-  const size_t smem = (size_t)3 * 2 * FT3 * sizeof(float);
+  if (!pv.max_items) return cudaGetLastError();
+  c->launches += 1;
+  k_part_finish_full<PASS, ACC><<<4 * c->num_sms, FINISH_CHUNK, 0, c->stream>>>(
+      c->g, pv, dp.fixed_scale, out, c->spill, c->vmax_bits);
+  return cudaGetLastError();
+}
+
+template <int PASS, int ACC>
+cudaError_t tile_pass2(lf2_ctx* c, float* out, const DepositParams& dp, const PartView& pv)
+{
+  constexpr size_t smem = FULL2_SMEM;
   cudaError_t e = cudaFuncSetAttribute(k_deposit_full2<PASS, ACC>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   c->launches += 1;
-  k_deposit_full2<PASS, ACC><<<(unsigned)c->g.nbricks, FULL2_THREADS, smem, c->stream>>>(
-      view(c), dp, out, c->spill, c->vmax_bits, c->flags);
-  return cudaGetLastError();
+  k_deposit_full2<PASS, ACC>
+      <<<(unsigned)(c->g.nbricks + pv.max_items), FULL2_THREADS, smem, c->stream>>>(
+          view(c), dp, out, c->spill, c->vmax_bits, c->flags, pv);
+  return finish<PASS, ACC>(c, out, dp, pv);
 }
 
 template <int ACC>
@@ -652,12 +737,15 @@ cudaError_t run2(lf2_ctx* c, int kind, float* out, const DepositParams& dp, int 
 {
   const unsigned nb = (unsigned)c->g.nbricks;
   if (stage == 0) {
-    cudaError_t e = cudaSuccess;
+    PartView pv;
+    cudaError_t e = launch_part_plan(c, FULL2_SMEM, FULL2_THREADS, (size_t)3 * FT3,
+                                     ACC == ACC_FIXED ? split_max<true>(c->has_mass ? 2 : 1) : 0, &pv);
+    if (e != cudaSuccess) return e;
     if (ACC == ACC_FIXED) e = launch_vmax(c);
     if (e != cudaSuccess) return e;
-    if (kind == 3) return tile_pass2<0, ACC>(c, out, dp);
-    e = tile_pass2<1, ACC>(c, out, dp);
-    return e != cudaSuccess ? e : tile_pass2<2, ACC>(c, out, dp);
+    if (kind == 3) return tile_pass2<0, ACC>(c, out, dp, pv);
+    e = tile_pass2<1, ACC>(c, out, dp, pv);
+    return e != cudaSuccess ? e : tile_pass2<2, ACC>(c, out, dp, pv);
   }
   c->launches += 1;
   if (kind == 3)
@@ -668,16 +756,16 @@ cudaError_t run2(lf2_ctx* c, int kind, float* out, const DepositParams& dp, int 
 }
 
 template <int PASS>
-cudaError_t tile_pass(lf2_ctx* c, float* out, const DepositParams& dp)
+cudaError_t tile_pass(lf2_ctx* c, float* out, const DepositParams& dp, const PartView& pv)
 {
-  const size_t smem = (size_t)3 * FT3 * sizeof(float);
+  constexpr size_t smem = FULL_SMEM;
   cudaError_t e = cudaFuncSetAttribute(k_deposit_full<PASS>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   c->launches += 1;
-  k_deposit_full<PASS><<<(unsigned)c->g.nbricks, FULL_THREADS, smem, c->stream>>>(
-      view(c), dp, out, reinterpret_cast<float*>(c->spill));
-  return cudaGetLastError();
+  k_deposit_full<PASS><<<(unsigned)(c->g.nbricks + pv.max_items), FULL_THREADS, smem, c->stream>>>(
+      view(c), dp, out, reinterpret_cast<float*>(c->spill), pv);
+  return finish<PASS, ACC_PLAIN>(c, out, dp, pv);
 }
 
 }  // namespace
@@ -697,9 +785,12 @@ cudaError_t launch_deposit_full(lf2_ctx* c, int kind, float* out, int stage)
   const unsigned nb = (unsigned)c->g.nbricks;
   float* outer = reinterpret_cast<float*>(c->spill);
   if (stage == 0) {
-    if (kind == 3) return tile_pass<0>(c, out, dp);
-    cudaError_t e = tile_pass<1>(c, out, dp);
-    return e != cudaSuccess ? e : tile_pass<2>(c, out, dp);
+    PartView pv;
+    cudaError_t e = launch_part_plan(c, FULL_SMEM, FULL_THREADS, (size_t)3 * FT3, 0, &pv);
+    if (e != cudaSuccess) return e;
+    if (kind == 3) return tile_pass<0>(c, out, dp, pv);
+    e = tile_pass<1>(c, out, dp, pv);
+    return e != cudaSuccess ? e : tile_pass<2>(c, out, dp, pv);
   }
   c->launches += 1;
   if (kind == 3)

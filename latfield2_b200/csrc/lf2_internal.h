@@ -42,6 +42,9 @@ struct DepositParams {
   int has_mass;
 };
 
+// Bounds of a plan of heavy bricks: scratch tiles (parts) and items.
+constexpr int PART_TILES = 4096, PART_ITEMS = 8192;
+
 struct MoveParams {
   float dtk;   // kick: dtau
   float dtn;   // drift: dtau / res (cell units per velocity unit)
@@ -98,6 +101,10 @@ struct lf2_ctx {
   float* stencil_partial = nullptr;  // per-CTA partial sums of the stencil weight gradient
   unsigned long long* pm_acc = nullptr; // chain's fixed-point deposit: [nsites] sums + max mass word
   size_t spill_slots = 0;
+  // parts of heavy bricks (deposit tile passes, lf2_deposit_common.cuh)
+  int4* part_item = nullptr;         // [PART_ITEMS] items, [PART_TILES] split bricks
+  int32_t* part_head = nullptr;      // device [3]: items, largest count that is not one, split bricks
+  uint64_t** part_tile = nullptr;    // device [PART_TILES]: the scratch tiles
   double* h_stats = nullptr;         // pinned [8]
   uint32_t* h_flags = nullptr;       // pinned
   int64_t* h_i64 = nullptr;          // pinned [4]
@@ -180,6 +187,13 @@ cudaError_t launch_deposit(lf2_ctx* c, int kind, float* out, int stage,
 // largest |v_i| of the store into c->vmax_bits (fixed-point momentum/stress)
 cudaError_t launch_vmax(lf2_ctx* c);
 DepositParams deposit_params(const lf2_ctx* c);
+// The plan of heavy bricks for a tile pass of `smem` bytes and `threads`
+// threads per CTA, tiles of tile_slots 8-byte values and at most `cap`
+// particles summed in one split tile (0: no such bound); enqueues the plan
+// kernel and fills *pv.
+struct PartView;
+cudaError_t launch_part_plan(lf2_ctx* c, size_t smem, int threads, size_t tile_slots, int cap,
+                             PartView* pv);
 
 // lf2_exchange.cu (slab decomposition): particles with cell z outside
 // [zlo, zhi] counted (below, above, more than one plane outside: 3 counters)

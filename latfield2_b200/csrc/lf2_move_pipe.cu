@@ -1001,7 +1001,7 @@ cudaError_t launch_move_pipe(lf2_ctx* c, const float* F, MoveParams mp, float* r
     d.rim = c->spill;
     d.scale = (float)(std::ldexp(1.0, -32) * c->m_unit / vol);
     d.inv_unit = (float)(1.0 / c->m_unit);
-    d.split_max = split_max<false>(c->has_mass);
+    d.split_max = split_max<false>(c->has_mass ? 64 : 1);
   }
   using Kern = decltype(&k_move_pipe<LF2_PIPE_WARPS, false, false, false>);
   const Kern kerns[2][4] = {

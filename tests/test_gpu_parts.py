@@ -1,0 +1,86 @@
+"""Deposits of bricks that are split over several CTAs (parts of heavy
+bricks): bricks one particle below and above the threshold, a brick of
+tens of parts beside empty ones, on a lattice of whole bricks and on a ragged
+one.  The fixed-point fields are bit-exact against the oracle; the FP32 modes
+are within the tolerances of test_gpu_precision.py (1e-6 compensated, 1e-5 of
+the field maximum for unordered FP32 sums)."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from tests.helpers import precision, small_case
+from tests.test_gpu_precision import KINDS, _ctx, _deposit, _fp64
+
+pytestmark = pytest.mark.gpu
+
+
+def _in_brick(n, brick, count, seed):
+    """`count` particles anywhere in the cells of one brick."""
+    rng = np.random.default_rng(seed)
+    ext = [min(16, n[d] - 16 * brick[d]) for d in range(3)]
+    xyz = [16 * brick[d] + rng.integers(0, ext[d], count) for d in range(3)]
+    cell = (xyz[0] + n[0] * (xyz[1] + n[1] * xyz[2])).astype(np.int32)
+    off = (rng.random((count, 3)) * (1 - 2.0 ** -23)).astype(np.float32)
+    vel = (0.2 * rng.standard_normal((count, 3))).astype(np.float32)
+    return cell, off, vel
+
+
+def _case(name):
+    # fewer than 512 * 1024 particles: parts of 1024, bricks above 1536 split
+    if name == "edges":
+        n = (64, 32, 48)
+        bits = [_in_brick(n, (0, 0, 0), 1536, 1), _in_brick(n, (3, 1, 2), 1537, 2),
+                _in_brick(n, (1, 1, 1), 2049, 3), _in_brick(n, (2, 0, 1), 1, 4)]
+    else:
+        n = (33, 17, 24)
+        bits = [_in_brick(n, (1, 0, 0), 30011, 5), _in_brick(n, (2, 1, 1), 4000, 6),
+                small_case(n, 500, seed=7, vel_sigma=0.2)]
+    return (n,) + tuple(np.concatenate([b[k] for b in bits]) for k in range(3))
+
+
+@pytest.mark.parametrize("name", ["edges", "ragged"])
+@pytest.mark.parametrize("kind", [0, 1, 2, 3, 4])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_split_bricks(cuda, name, kind, mode):
+    n, cell, off, vel = _case(name)
+    gm = 1.0 / cell.shape[0]
+    got = _deposit(n, mode, kind, cell, off, vel, gm)
+    ref, mag = _fp64(n, kind, cell, off, vel, gm)
+    for c in range(ref.shape[0]):
+        p = precision(got[c], ref[c], mag[c])
+        assert p["norm_max"] <= (1e-5 if mode == 2 else 1e-6), (c, p)
+        assert mode == 2 or p["cell_max"] <= 1e-6, (c, p)
+    if mode == 1 and kind:
+        acc, e = O.state_deposit_fixed_kind(kind, n, cell, off, vel)
+        np.testing.assert_array_equal(got, O.fixed_kind_to_f32(acc, kind, e, gm, 1.0 / n[0]))
+    elif mode == 1:
+        scale = np.float32(2.0 ** -32 * gm / (1.0 / n[0]) ** 3)
+        np.testing.assert_array_equal(got.reshape(-1),
+                                      O.fixed_to_f32(O.state_deposit_fixed(n, cell, off), scale))
+
+
+@pytest.mark.parametrize("spread", [0.1, 30.0])
+@pytest.mark.parametrize("kind", [0, 1, 2, 3, 4])
+def test_split_bricks_with_individual_masses(cuda, kind, spread):
+    """Masses up to 1.1 or about 20 of their mean: the bound on the particles
+    that two 32-bit words sum exactly follows the largest mass of the part."""
+    n, cell, off, vel = _case("ragged")
+    npart = cell.shape[0]
+    u = np.random.default_rng(9).random(npart)
+    m = ((1.0 + (spread * (2 * u - 1) if spread < 1 else spread * (u > 0.97))) / npart).astype(np.float32)
+    unit = float(np.sum(m.astype(np.float64)) / npart)
+    mrel = (m * np.float32(1.0 / unit)).astype(np.float32)
+    ctx = _ctx(n, 1)
+    ctx.set_particles(cell, off, vel, mass=m)
+    name, comps = ("deposit_scalar", 1) if kind == 0 else KINDS[kind][:2]
+    f = ctx.field(comps)
+    getattr(ctx, name)(f)
+    got = f.export_internal()
+    if kind == 0:
+        scale = np.float32(2.0 ** -32 * unit / (1.0 / n[0]) ** 3)
+        want = O.fixed_to_f32(O.state_deposit_fixed(n, cell, off, mrel=mrel), scale).reshape(got.shape)
+    else:
+        acc, e = O.state_deposit_fixed_kind(kind, n, cell, off, vel, mrel=mrel)
+        want = O.fixed_kind_to_f32(acc, kind, e, unit, 1.0 / n[0])
+    np.testing.assert_array_equal(got, want)
+    ctx.close()
