@@ -332,7 +332,7 @@ lf2_status lf2_create(lf2_ctx** out, int device, const int n[3], const double bo
   ok = ok && cudaMalloc(&c->work, sizeof(int)) == cudaSuccess;
   ok = ok && cudaMalloc(&c->part_item, sizeof(int4) * (PART_ITEMS + PART_TILES)) == cudaSuccess;
   ok = ok && cudaMalloc(&c->part_head, sizeof(int32_t) * 3) == cudaSuccess;
-  ok = ok && cudaMalloc(&c->part_tile, sizeof(uint64_t*) * PART_TILES) == cudaSuccess;
+  ok = ok && cudaMalloc(&c->part_mark, (size_t)nb) == cudaSuccess;
   ok = ok && cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess;
   if (ok) {
     ok = cudaMemsetAsync(c->count, 0, sizeof(int32_t) * nb, c->stream) == cudaSuccess &&
@@ -390,7 +390,7 @@ lf2_status lf2_destroy(lf2_ctx* c)
   cudaFree(c->spill);
   cudaFree(c->part_item);
   cudaFree(c->part_head);
-  cudaFree(c->part_tile);
+  cudaFree(c->part_mark);
   cudaFree(c->stencil_partial);
   cudaFree(c->pm_acc);
   fft_release(c);

@@ -45,11 +45,6 @@
 #include "lf2_deposit_common.cuh"
 #include "lf2_internal.h"
 
-// Owned face vertices per thread and trip of the one-component fix-up.
-#ifndef FIX_V
-#define FIX_V 2
-#endif
-
 namespace lf2 {
 
 namespace {
@@ -58,10 +53,17 @@ namespace {
 #define LF2_DEP_THREADS 256
 #endif
 constexpr int DEP_THREADS = LF2_DEP_THREADS;
+// ... and of a tile that leaves room for one CTA per SM
+#ifndef LF2_DEP_BIG
+#define LF2_DEP_BIG 1024
+#endif
+#ifndef LF2_DEP_BIG_ITEMS
+#define LF2_DEP_BIG_ITEMS 2
+#endif
 
 // Fewest particles of a part of a split brick.
 #ifndef LF2_PART_MIN
-#define LF2_PART_MIN 1024
+#define LF2_PART_MIN 4096
 #endif
 
 // Components of the field of a kind.
@@ -88,7 +90,8 @@ struct Pass {
   static constexpr size_t smem() { return (size_t)NC * WORDS * TILE3 * 4; }
   // threads per CTA: a tile above 100 KB leaves room for one CTA per SM, so
   // it gets twice the warps
-  static constexpr int THREADS = smem() > 100 * 1024 ? 2 * DEP_THREADS : DEP_THREADS;
+  static constexpr int THREADS = smem() > 100 * 1024 ? LF2_DEP_BIG : DEP_THREADS;
+  static constexpr int ITEMS = smem() > 100 * 1024 ? LF2_DEP_BIG_ITEMS : 4;  // particles in flight per thread
   // CTAs per SM that the registers leave room for: those whose tiles fit
   static constexpr int CTAS = smem() > 100 * 1024 ? 1 : smem() > 50 * 1024 ? 3 : 5;
 };
@@ -112,7 +115,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
   constexpr int T = P::THREADS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
 
-  __shared__ unsigned s_mass;
+  __shared__ unsigned s_max[2];
 
   const Geom& g = v.g;
   Part part;
@@ -126,8 +129,16 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
   const int64_t base = v.seg_start[b] + part.first;
   const int cnt = part.cnt;
   const int mass_bound =
-      FIXED && dp.has_mass ? part_mass_bound(v.a.mass, (uint32_t)base, cnt, dp.inv_unit, &s_mass) : 1;
-  TileRef<TILE3> tr{smem_raw, FIXED && cnt <= split_max<SIGNED>(mass_bound)};
+      FIXED && dp.has_mass ? part_mass_bound(v.a.mass, (uint32_t)base, cnt, dp.inv_unit, s_max) : 1;
+  CompUnit cu{0, false};
+  if (ACC == ACC_COMP)
+    cu = comp_unit<KIND>(dp.has_mass ? v.a.mass : nullptr, dp.inv_vol, dp.mf, v.a.vx, v.a.vy, v.a.vz,
+                         (uint32_t)base, cnt, s_max);
+  // two integer words per vertex, or the sums that hold anything
+  const bool ints = FIXED ? cnt <= split_max<SIGNED>(mass_bound) : cu.ok;
+  TileRef<TILE3> tr{smem_raw, ints};
+  // unit of the FP32 terms that the integer sums take (add_comp_int)
+  const float unit = ACC == ACC_COMP && ints ? ldexpf(1.0f, 16 - cu.e) : 1.0f;
   // fixed point: velocity quantum and conversion scale for this field
   int vexp = 0;
   if (FIXED && KIND != 0) vexp = vexp_of(*vmax_bits);
@@ -146,7 +157,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
 
   // The particle loop, instantiated for the split fixed-point tile (or not)
   // and for per-particle masses (or a global mass), chosen once per CTA.
-  constexpr int ITEMS = 4;  // particles in flight per thread
+  constexpr int ITEMS = P::ITEMS;
   auto particles = [&](auto split_c, auto hm_c) {
     constexpr bool SPLIT = decltype(split_c)::value;
     constexpr bool HM = decltype(hm_c)::value;
@@ -187,7 +198,6 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
           const uint32_t qx[2] = {(1u << 31) - ux, ux};
           const uint32_t qy[2] = {(1u << 31) - uy, uy};
           const uint32_t qz[2] = {(1u << 31) - uz, uz};
-          constexpr uint32_t ONE = 1u << 31;
           if (KIND == 0) {
             const uint64_t pxy[4] = {(uint64_t)qx[0] * qy[0], (uint64_t)qx[0] * qy[1],
                                      (uint64_t)qx[1] * qy[0], (uint64_t)qx[1] * qy[1]};
@@ -214,9 +224,9 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
                 const int a = (k >> 1) & 1, bb = k & 1;
                 uint64_t w;
                 int t;
-                if (c == 0) w = fixed_corner(ONE, qy[a], qz[bb]), t = t0 + a * TY + bb * TZ;
-                else if (c == 1) w = fixed_corner(qx[a], ONE, qz[bb]), t = t0 + a + bb * TZ;
-                else w = fixed_corner(qx[a], qy[bb], ONE), t = t0 + a + bb * TY;
+                if (c == 0) w = fixed_edge(qy[a], qz[bb]), t = t0 + a * TY + bb * TZ;
+                else if (c == 1) w = fixed_edge(qx[a], qz[bb]), t = t0 + a + bb * TZ;
+                else w = fixed_edge(qx[a], qy[bb]), t = t0 + a + bb * TY;
                 add_fixed48_t<SPLIT, TILE3>(smem_raw, c, t, mass_sign48_t<HM>(mul_wv48(w, vq), mq, neg));
               }
             }
@@ -262,32 +272,33 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
         const float gx = __fsub_rn(1.0f, fx[j]), gy = __fsub_rn(1.0f, fy[j]),
                     gz = __fsub_rn(1.0f, fz[j]);
         const float ox = fx[j], oy = fy[j], oz = fz[j];
-        const float mf = HM ? __fmul_rn(m[j], dp.inv_vol) : dp.mf;
+        float mf = HM ? __fmul_rn(m[j], dp.inv_vol) : dp.mf;
+        if (ACC == ACC_COMP && SPLIT) mf = __fmul_rn(mf, unit);
         if (KIND == 0) {
   #pragma unroll
           for (int k = 0; k < 8; k++) {
             const int cx = (k >> 2) & 1, cy = (k >> 1) & 1, cz = k & 1;
             const float w = __fmul_rn(
                 __fmul_rn(__fmul_rn(sel(cx, ox, gx), sel(cy, oy, gy)), sel(cz, oz, gz)), mf);
-            add_float<ACC>(tr, 0, t0 + cx + cy * TY + cz * TZ, w);
+            add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0 + cx + cy * TY + cz * TZ, w);
           }
         } else if (KIND == 1) {
           // projections.hpp:501-544: component i is NGP along i, CIC across.
           const float vxm = __fmul_rn(mf, vx[j]);
           const float vym = __fmul_rn(mf, vy[j]);
           const float vzm = __fmul_rn(mf, vz[j]);
-          add_float<ACC>(tr, 0, t0, __fmul_rn(__fmul_rn(vxm, gy), gz));
-          add_float<ACC>(tr, 0, t0 + TY, __fmul_rn(__fmul_rn(vxm, oy), gz));
-          add_float<ACC>(tr, 0, t0 + TZ, __fmul_rn(__fmul_rn(vxm, gy), oz));
-          add_float<ACC>(tr, 0, t0 + TY + TZ, __fmul_rn(__fmul_rn(vxm, oy), oz));
-          add_float<ACC>(tr, 1, t0, __fmul_rn(__fmul_rn(vym, gx), gz));
-          add_float<ACC>(tr, 1, t0 + 1, __fmul_rn(__fmul_rn(vym, ox), gz));
-          add_float<ACC>(tr, 1, t0 + TZ, __fmul_rn(__fmul_rn(vym, gx), oz));
-          add_float<ACC>(tr, 1, t0 + 1 + TZ, __fmul_rn(__fmul_rn(vym, ox), oz));
-          add_float<ACC>(tr, 2, t0, __fmul_rn(__fmul_rn(vzm, gx), gy));
-          add_float<ACC>(tr, 2, t0 + 1, __fmul_rn(__fmul_rn(vzm, ox), gy));
-          add_float<ACC>(tr, 2, t0 + TY, __fmul_rn(__fmul_rn(vzm, gx), oy));
-          add_float<ACC>(tr, 2, t0 + 1 + TY, __fmul_rn(__fmul_rn(vzm, ox), oy));
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0, __fmul_rn(__fmul_rn(vxm, gy), gz));
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0 + TY, __fmul_rn(__fmul_rn(vxm, oy), gz));
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0 + TZ, __fmul_rn(__fmul_rn(vxm, gy), oz));
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0 + TY + TZ, __fmul_rn(__fmul_rn(vxm, oy), oz));
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 1, t0, __fmul_rn(__fmul_rn(vym, gx), gz));
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 1, t0 + 1, __fmul_rn(__fmul_rn(vym, ox), gz));
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 1, t0 + TZ, __fmul_rn(__fmul_rn(vym, gx), oz));
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 1, t0 + 1 + TZ, __fmul_rn(__fmul_rn(vym, ox), oz));
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 2, t0, __fmul_rn(__fmul_rn(vzm, gx), gy));
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 2, t0 + 1, __fmul_rn(__fmul_rn(vzm, ox), gy));
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 2, t0 + TY, __fmul_rn(__fmul_rn(vzm, gx), oy));
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 2, t0 + 1 + TY, __fmul_rn(__fmul_rn(vzm, ox), oy));
         } else {
           // projections.hpp:786-843: T_ii at the 8 vertices, T_ij on plaquettes.
           const float vv[3] = {vx[j], vy[j], vz[j]};
@@ -305,7 +316,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
                 const int cx = (k >> 2) & 1, cy = (k >> 1) & 1, cz = k & 1;
                 const float w = __fmul_rn(
                     __fmul_rn(__fmul_rn(mv2, sel(cx, ox, gx)), sel(cy, oy, gy)), sel(cz, oz, gz));
-                add_float<ACC>(tr, jd, t0 + cx + cy * TY + cz * TZ, w);
+                add_float<ACC, SPLIT, TILE3>(smem_raw, jd, t0 + cx + cy * TY + cz * TZ, w);
               }
             }
           }
@@ -315,19 +326,19 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
             const float m01 = __fmul_rn(__fmul_rn(mf, vv[0]), vv[1]);
             const float m02 = __fmul_rn(__fmul_rn(mf, vv[0]), vv[2]);
             const float m12 = __fmul_rn(__fmul_rn(mf, vv[1]), vv[2]);
-            add_float<ACC>(tr, j01, t0, __fmul_rn(m01, gz));
-            add_float<ACC>(tr, j01, t0 + TZ, __fmul_rn(m01, oz));
-            add_float<ACC>(tr, j02, t0, __fmul_rn(m02, gy));
-            add_float<ACC>(tr, j02, t0 + TY, __fmul_rn(m02, oy));
-            add_float<ACC>(tr, j12, t0, __fmul_rn(m12, gx));
-            add_float<ACC>(tr, j12, t0 + 1, __fmul_rn(m12, ox));
+            add_float<ACC, SPLIT, TILE3>(smem_raw, j01, t0, __fmul_rn(m01, gz));
+            add_float<ACC, SPLIT, TILE3>(smem_raw, j01, t0 + TZ, __fmul_rn(m01, oz));
+            add_float<ACC, SPLIT, TILE3>(smem_raw, j02, t0, __fmul_rn(m02, gy));
+            add_float<ACC, SPLIT, TILE3>(smem_raw, j02, t0 + TY, __fmul_rn(m02, oy));
+            add_float<ACC, SPLIT, TILE3>(smem_raw, j12, t0, __fmul_rn(m12, gx));
+            add_float<ACC, SPLIT, TILE3>(smem_raw, j12, t0 + 1, __fmul_rn(m12, ox));
           }
         }
       }
     }
   };
   const bool hm_rt = dp.has_mass != 0;
-  if (FIXED && tr.split) {
+  if (ACC != ACC_PLAIN && tr.split) {
     if (hm_rt) particles(std::true_type{}, std::true_type{});
     else particles(std::true_type{}, std::false_type{});
   } else {
@@ -335,8 +346,8 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
     else particles(std::false_type{}, std::false_type{});
   }
   __syncthreads();
-  if (uint64_t* scratch = part_tile(pv)) {  // k_part_finish sums the parts and writes the vertices
-    part_store<ACC, SIGNED, NC, TILE3>(scratch, tr);
+  if (uint64_t* scratch = part_tile(pv, P::NC * TILE3)) {  // k_part_finish sums the parts and writes the vertices
+    part_store<ACC, SIGNED, NC, TILE3>(scratch, tr, cu.e);
     return;
   }
 
@@ -363,8 +374,8 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
         if (!SIGNED && q < 0) set_flag(flags, ERR_FIXED_OVERFLOW);
         out[(size_t)c * g.nsites + s] = __fmul_rn(__ll2float_rn(q), conv);
       } else if (ACC == ACC_COMP) {
-        out[(size_t)c * g.nsites + s] =
-            __fadd_rn(facc[(size_t)j * 2 * TILE3 + t], facc[(size_t)j * 2 * TILE3 + TILE3 + t]);
+        const float2 p = comp_pair(tr, j, t, cu.e);
+        out[(size_t)c * g.nsites + s] = __fadd_rn(p.x, p.y);
       } else {
         out[(size_t)c * g.nsites + s] = facc[(size_t)j * TILE3 + t];
       }
@@ -399,8 +410,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
       if (FIXED) {
         sp[(size_t)c * SHELL + f] = (uint64_t)tile_fixed<SIGNED>(tr, j, t);
       } else if (ACC == ACC_COMP) {
-        reinterpret_cast<float2*>(sp)[(size_t)c * SHELL + f] =
-            make_float2(facc[(size_t)j * 2 * TILE3 + t], facc[(size_t)j * 2 * TILE3 + TILE3 + t]);
+        reinterpret_cast<float2*>(sp)[(size_t)c * SHELL + f] = comp_pair(tr, j, t, cu.e);
       } else {
         reinterpret_cast<float*>(sp)[(size_t)c * SHELL + f] = facc[(size_t)j * TILE3 + t];
       }
@@ -423,7 +433,7 @@ __global__ void __launch_bounds__(FINISH_CHUNK) k_part_finish(Geom g, PartView p
   using P = Pass<KIND, PASS, ACC>;
   constexpr int C = Comps<KIND>::value;
   constexpr int CHUNKS = (TILE3 + FINISH_CHUNK - 1) / FINISH_CHUNK;
-  const int units = pv.head[2] * CHUNKS;
+  const int units = pv.head[1] * CHUNKS;
   if ((int)blockIdx.x >= units) return;
   const int vexp = ACC == ACC_FIXED && KIND != 0 ? vexp_of(*vmax_bits) : 0;
   const float conv = ldexpf(fixed_scale, (KIND == 1 ? vexp : 2 * vexp) - (KIND != 0 ? 16 : 0));
@@ -444,7 +454,7 @@ __global__ void __launch_bounds__(FINISH_CHUNK) k_part_finish(Geom g, PartView p
 #pragma unroll
     for (int jc = 0; jc < P::NC; jc++) {
       const int c = P::comp(jc);
-      const PartSum s = part_sum<ACC>(pv, sp, jc * TILE3 + t);
+      const PartSum s = part_sum<ACC>(pv, sp, P::NC * TILE3, jc * TILE3 + t);
       if (inner) {
         if (KIND == 0 && s.q < 0) set_flag(flags, ERR_FIXED_OVERFLOW);
         out[(size_t)c * g.nsites + site] =
@@ -466,238 +476,184 @@ __global__ void __launch_bounds__(FINISH_CHUNK) k_part_finish(Geom g, PartView p
 // neighbour brick across S at tile coordinate BRICK in those dims.  The sum
 // runs in that fixed order: exact integers (fixed point), a compensated FP32
 // sum of the hi and lo words, or plain FP32 additions.
+//
+// The pass is bound by the latency of its scattered reads.  675 of the 721
+// vertices lie inside one of the three faces and have one neighbour: thread
+// t < 225 takes vertex t of each face, so that all its reads (two per face
+// and component, at fixed offsets from one another) are in flight together;
+// the other threads take one edge vertex each (3 neighbours) or the corner
+// (7), so that no thread waits for memory twice.
+template <int ACC>
+struct ShellSum {
+  long long q = 0;
+  float s = 0.0f, c = 0.0f;
+  __device__ __forceinline__ void add(uint64_t v)
+  {
+    if (ACC == ACC_FIXED)
+      q += (long long)v;
+    else if (ACC == ACC_COMP)
+      comp_acc(s, c, __uint_as_float((uint32_t)v), __uint_as_float((uint32_t)(v >> 32)));
+    else
+      s = __fadd_rn(s, __uint_as_float((uint32_t)v));
+  }
+  __device__ __forceinline__ float value(float conv) const
+  {
+    return ACC == ACC_FIXED ? __fmul_rn(__ll2float_rn(q), conv) : ACC == ACC_COMP ? __fadd_rn(s, c) : s;
+  }
+};
+
+constexpr int FIX_FACE = (BRICK - 1) * (BRICK - 1), FIX_EDGE = 3 * (BRICK - 1);
+constexpr int FIX_THREADS = (FIX_FACE + FIX_EDGE + 1 + 31) & ~31;
+
 template <int KIND, int ACC>
-__global__ void k_fixup(Geom g, const uint64_t* __restrict__ spill, float fixed_scale,
-                        const uint32_t* __restrict__ vmax_bits, float* __restrict__ out,
-                        uint32_t* flags, const uint32_t* gate)
+__global__ void __launch_bounds__(FIX_THREADS)
+    k_fixup(Geom g, const uint64_t* __restrict__ spill, float fixed_scale,
+            const uint32_t* __restrict__ vmax_bits, float* __restrict__ out, uint32_t* flags,
+            const uint32_t* gate)
 {
   if (gate && *gate == 0u) return;
-  constexpr int C = Comps<KIND>::value;
-  constexpr bool SIGNED = KIND != 0;
+  constexpr int CT = Comps<KIND>::value, C = CT < 3 ? CT : 3;  // of the field, of this CTA
+  const int c0 = C * blockIdx.y;
   const int64_t b = blockIdx.x;
   int bx, by, bz;
   brick_coords(g, b, bx, by, bz);
-  const int ex = brick_extent(g.n[0], bx), ey = brick_extent(g.n[1], by),
-            ez = brick_extent(g.n[2], bz);
-  const int x0 = bx * BRICK, y0 = by * BRICK, z0 = bz * BRICK;
-  const int bxm = bx ? bx - 1 : g.nb[0] - 1;
-  const int bym = by ? by - 1 : g.nb[1] - 1;
-  const int bzm = bz ? bz - 1 : g.nb[2] - 1;
-  // the brick itself (s = 0) and its lower neighbours across every subset s
-  // of the dims (bit 0: x, 1: y, 2: z)
-  __shared__ uint32_t nbr[8];
-  if (threadIdx.x < 8) {
-    const int s = threadIdx.x;
-    nbr[s] = (uint32_t)((s & 1) ? bxm : bx) +
-             (uint32_t)g.nb[0] * ((uint32_t)((s & 2) ? bym : by) + (uint32_t)g.nb[1] * ((s & 4) ? bzm : bz));
-  }
-  __syncthreads();
+  const int e[3] = {brick_extent(g.n[0], bx), brick_extent(g.n[1], by), brick_extent(g.n[2], bz)};
+  // index of the lower neighbour across a dim, minus the brick's own
+  const int64_t nb0 = g.nb[0], nb01 = nb0 * g.nb[1];
+  const int64_t lower[3] = {bx ? -1 : nb0 - 1, by ? -nb0 : nb01 - nb0,
+                            bz ? -nb01 : (int64_t)g.nbricks - nb01};
   float conv = 0.0f;
   if (ACC == ACC_FIXED) {
     const int vexp = KIND != 0 ? vexp_of(*vmax_bits) : 0;
     conv = ldexpf(fixed_scale, KIND == 0 ? 0 : (KIND == 1 ? vexp : 2 * vexp) - 16);
   }
-  const int nface = ey * ez + (ex - 1) * ez + (ex - 1) * (ey - 1);
-  // owned face vertex number f -> tile coordinates
-  auto face_vertex = [&](int f, int& i, int& j, int& k) {
-    if (f < ey * ez) {  // x face: i = 0
-      i = 0;
-      j = f % ey;
-      k = f / ey;
-    } else if (f < ey * ez + (ex - 1) * ez) {  // y face: j = 0, i >= 1
-      const int r = f - ey * ez;
-      j = 0;
-      i = 1 + r % (ex - 1);
-      k = r / (ex - 1);
-    } else {  // z face: k = 0, i, j >= 1
-      const int r = f - ey * ez - (ex - 1) * ez;
-      k = 0;
-      i = 1 + r % (ex - 1);
-      j = 1 + r / (ex - 1);
-    }
+  const int64_t site0 = site_index(g, bx * BRICK, by * BRICK, bz * BRICK);
+  const int64_t step[3] = {1, g.n[0], (int64_t)g.n[0] * g.n[1]};
+  // shell value `si` of component c0 + c of brick nb (a brick's region is
+  // SHELL 8-byte slots per component; the plain mode fills the first CT *
+  // SHELL floats)
+  auto read = [&](int64_t nb, int c, int si) -> uint64_t {
+    const uint64_t* sp = spill + (size_t)nb * (CT * SHELL);
+    const int at = (c0 + c) * SHELL + si;
+    return ACC == ACC_PLAIN ? (uint64_t)__float_as_uint(__ldg(reinterpret_cast<const float*>(sp) + at))
+                            : __ldg(sp + at);
   };
-  if constexpr (C == 1) {
-    // One component: FIX_V vertices per thread, all their shell reads issued
-    // before any is used (the pass is bound by the latency of these
-    // scattered reads; at 512^3, 2 per thread: 0.261 ms, 3: 0.287 ms, 4:
-    // 0.345 ms).  Subset s of a vertex's zero coordinates is read
-    // when (s & zmask) == s; the sum runs over s in ascending order.
-    constexpr int FV = FIX_V;
-    const float* spf = reinterpret_cast<const float*>(spill);
-    for (int f0 = threadIdx.x; f0 < nface; f0 += FV * blockDim.x) {
-      int vi[FV], vj[FV], vk[FV], zm[FV];
-      bool on[FV];
+  auto put = [&](int64_t site, int c, const ShellSum<ACC>& r) {
+    if (ACC == ACC_FIXED && KIND == 0 && r.q < 0) set_flag(flags, ERR_FIXED_OVERFLOW);
+    out[(c0 + c) * g.nsites + site] = r.value(conv);
+  };
+  if (threadIdx.x < FIX_FACE) {
+    constexpr int I = BRICK - 1;
+    const int u = 1 + threadIdx.x % I, w = 1 + threadIdx.x / I;
+    // face d: coordinate 0 in dim d, (u, w) in the others; its own shell slot
+    // and the lower neighbour's (shell_index at 0 and at BRICK)
+    const int own[3] = {w * TILE + u, 2 * TILE * TILE + w * I + (u - 1),
+                        2 * TILE * TILE + 2 * I * TILE + (w - 1) * I + (u - 1)};
+    constexpr int up[3] = {TILE * TILE, I * TILE, I * I};
+    constexpr int du[3] = {1, 0, 0}, dw[3] = {2, 2, 1};
+    uint64_t r[3][C][2];
+    bool on[3];
 #pragma unroll
-      for (int h = 0; h < FV; h++) {
-        const int f = f0 + h * blockDim.x;
-        on[h] = f < nface;
-        vi[h] = vj[h] = vk[h] = 0;
-        if (on[h]) face_vertex(f, vi[h], vj[h], vk[h]);
-        zm[h] = on[h] ? (vi[h] == 0 ? 1 : 0) | (vj[h] == 0 ? 2 : 0) | (vk[h] == 0 ? 4 : 0) : 0;
-      }
-      long long q[FV];
-      float fs[FV], fc[FV];
+    for (int d = 0; d < 3; d++) {
+      on[d] = u < e[du[d]] && w < e[dw[d]];
 #pragma unroll
-      for (int h = 0; h < FV; h++) q[h] = 0, fs[h] = 0.0f, fc[h] = 0.0f;
-      auto read = [&](int h, int s) -> uint64_t {
-        const int si = shell_index((s & 1) ? BRICK : vi[h], (s & 2) ? BRICK : vj[h], (s & 4) ? BRICK : vk[h]);
-        // a brick's shell region is SHELL 8-byte slots; the plain mode
-        // fills its first SHELL floats
-        const size_t at = (size_t)nbr[s] * SHELL;
-        return ACC == ACC_PLAIN ? (uint64_t)__float_as_uint(spf[2 * at + si]) : spill[at + si];
-      };
-#pragma unroll
-      for (int s = 0; s < 8; s++) {
-        uint64_t r[FV];
-#pragma unroll
-        for (int h = 0; h < FV; h++) r[h] = on[h] && (s & zm[h]) == s ? read(h, s) : 0ull;
-#pragma unroll
-        for (int h = 0; h < FV; h++) {
-          if (!(on[h] && (s & zm[h]) == s)) continue;
-          if (ACC == ACC_FIXED)
-            q[h] += (long long)r[h];
-          else if (ACC == ACC_COMP)
-            comp_acc(fs[h], fc[h], __uint_as_float((uint32_t)r[h]), __uint_as_float((uint32_t)(r[h] >> 32)));
-          else
-            fs[h] = __fadd_rn(fs[h], __uint_as_float((uint32_t)r[h]));
-        }
-      }
-#pragma unroll
-      for (int h = 0; h < FV; h++) {
-        if (!on[h]) continue;
-        const int64_t site = site_index(g, x0 + vi[h], y0 + vj[h], z0 + vk[h]);
-        if (ACC == ACC_FIXED) {
-          if (!SIGNED && q[h] < 0) set_flag(flags, ERR_FIXED_OVERFLOW);
-          out[site] = __fmul_rn(__ll2float_rn(q[h]), conv);
-        } else {
-          out[site] = ACC == ACC_COMP ? __fadd_rn(fs[h], fc[h]) : fs[h];
-        }
+      for (int c = 0; c < C; c++) {
+        r[d][c][0] = on[d] ? read(b, c, own[d]) : 0;
+        r[d][c][1] = on[d] ? read(b + lower[d], c, own[d] + up[d]) : 0;
       }
     }
-  } else {
-    for (int f = threadIdx.x; f < nface; f += blockDim.x) {
-      int i, j, k;
-      face_vertex(f, i, j, k);
-      const int zmask = (i == 0 ? 1 : 0) | (j == 0 ? 2 : 0) | (k == 0 ? 4 : 0);
-      long long qs[C];
-      float fs[C], fc[C];
-  #pragma unroll
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      if (!on[d]) continue;
+      const int64_t site = site0 + u * step[du[d]] + w * step[dw[d]];
+#pragma unroll
       for (int c = 0; c < C; c++) {
-        qs[c] = 0;
-        fs[c] = 0.0f;
-        fc[c] = 0.0f;
-      }
-      // the subsets s of zmask in ascending order (s -> (s - zmask) & zmask)
-      for (int s = 0;; s = (s - zmask) & zmask) {
-        const uint32_t nb = nbr[s];
-        const int si = shell_index((s & 1) ? BRICK : i, (s & 2) ? BRICK : j, (s & 4) ? BRICK : k);
-        const uint64_t* sp = spill + (size_t)nb * (C * SHELL);
-  #pragma unroll
-        for (int c = 0; c < C; c++) {
-          if (ACC == ACC_FIXED) {
-            qs[c] += (long long)sp[c * SHELL + si];
-          } else if (ACC == ACC_COMP) {
-            const float2 hl = reinterpret_cast<const float2*>(sp)[c * SHELL + si];
-            comp_acc(fs[c], fc[c], hl.x, hl.y);
-          } else {
-            fs[c] = __fadd_rn(fs[c], reinterpret_cast<const float*>(sp)[c * SHELL + si]);
-          }
-        }
-        if (s == zmask) break;
-      }
-      const int64_t site = site_index(g, x0 + i, y0 + j, z0 + k);
-  #pragma unroll
-      for (int c = 0; c < C; c++) {
-        if (ACC == ACC_FIXED) {
-          if (!SIGNED && qs[c] < 0) set_flag(flags, ERR_FIXED_OVERFLOW);
-          out[c * g.nsites + site] = __fmul_rn(__ll2float_rn(qs[c]), conv);
-        } else if (ACC == ACC_COMP) {
-          out[c * g.nsites + site] = __fadd_rn(fs[c], fc[c]);
-        } else {
-          out[c * g.nsites + site] = fs[c];
-        }
+        ShellSum<ACC> s;
+        s.add(r[d][c][0]);
+        s.add(r[d][c][1]);
+        put(site, c, s);
       }
     }
+  }
+  // edges: coordinate m > 0 along one dim, 0 in the others; then the corner
+  const int f = (int)threadIdx.x - FIX_FACE;
+  if (f >= 0 && f <= FIX_EDGE) {
+    const int d = f == FIX_EDGE ? 3 : f / (BRICK - 1), m = 1 + f % (BRICK - 1);
+    if (d < 3 && m >= e[d]) return;
+    const int i = d == 0 ? m : 0, j = d == 1 ? m : 0, k = d == 2 ? m : 0;
+    const int zmask = 7 & ~(d < 3 ? 1 << d : 0);
+    ShellSum<ACC> r[C];
+#pragma unroll
+    for (int s = 0; s < 8; s++) {  // the subsets of zmask in ascending order
+      if ((s & zmask) != s) continue;
+      const int64_t nb = b + ((s & 1) ? lower[0] : 0) + ((s & 2) ? lower[1] : 0) + ((s & 4) ? lower[2] : 0);
+      const int si = shell_index((s & 1) ? BRICK : i, (s & 2) ? BRICK : j, (s & 4) ? BRICK : k);
+#pragma unroll
+      for (int c = 0; c < C; c++) r[c].add(read(nb, c, si));
+    }
+    const int64_t site = site0 + i * step[0] + j * step[1] + k * step[2];
+#pragma unroll
+    for (int c = 0; c < C; c++) put(site, c, r[c]);
   }
 }
 
 // Largest |v_i| of the stored particles, as the bits of a non-negative float
 // (they order as unsigned integers); a non-finite velocity raises the flag.
-__global__ void __launch_bounds__(256) k_vmax(StoreView v, uint32_t* vmax_bits, uint32_t* flags)
+__global__ void __launch_bounds__(256) k_vmax(StoreView v, uint32_t* vmax_bits, uint32_t* flags, PartView pv)
 {
-  const int64_t b = blockIdx.x;
-  const int64_t base = v.seg_start[b];
-  const int cnt = LF2_BRICK_COUNT(v, b);
+  Part part;  // the tile passes' units, so that no CTA reads a heavy brick alone
+  if (!part_take(pv, v.g.nbricks, v.count, v.cap, part)) return;
+  // four slots per load: segments and parts start on multiples of four
+  const int64_t base = v.seg_start[part.b] + part.first;
+  const float* const comp[3] = {v.a.vx + base, v.a.vy + base, v.a.vz + base};
   uint32_t m = 0u;
-  bool bad = false;
-  for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
-    const int64_t p = base + i;
-    const uint32_t a = __float_as_uint(v.a.vx[p]) & 0x7fffffffu;
-    const uint32_t c = __float_as_uint(v.a.vy[p]) & 0x7fffffffu;
-    const uint32_t d = __float_as_uint(v.a.vz[p]) & 0x7fffffffu;
-    const uint32_t mm = max(a, max(c, d));
-    bad |= mm >= 0x7f800000u;
-    m = max(m, mm);
+#pragma unroll 4
+  for (int i = 4 * threadIdx.x; i < part.cnt; i += 4 * blockDim.x) {
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const uint4 q = __ldg(reinterpret_cast<const uint4*>(comp[d] + i));
+      m = max(m, q.x & 0x7fffffffu);
+      if (i + 1 < part.cnt) m = max(m, q.y & 0x7fffffffu);
+      if (i + 2 < part.cnt) m = max(m, q.z & 0x7fffffffu);
+      if (i + 3 < part.cnt) m = max(m, q.w & 0x7fffffffu);
+    }
   }
-  if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) set_flag(flags, ERR_NONFINITE);
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m) atomicMax(vmax_bits, m);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) != 0) return;
+  if (m >= 0x7f800000u) set_flag(flags, ERR_NONFINITE);
+  if (m > *reinterpret_cast<volatile uint32_t*>(vmax_bits)) atomicMax(vmax_bits, m);
 }
 
-// Scratch tiles of `slots` 8-byte values, `tiles` to a bank.
-struct Banks {
-  uint64_t* bank[7];
-  int tiles, slots;
-};
-
 // Items of the bricks above `first` particles: a brick above `split` makes
-// ceil(count / P) parts, the others one.  Where the parts would need more
-// tiles than there are, P and split double until they do not; where the items
-// would not fit, `first` does.  One CTA.
-__global__ void __launch_bounds__(1024) k_part_plan(int64_t nb, const int32_t* __restrict__ count,
-                                                    const int32_t* __restrict__ cap, int P0, int split0,
-                                                    int first0, int max_items, Banks banks, int4* item,
-                                                    int4* split_list, int32_t* head, uint64_t** tile)
+// ceil(count / P) parts while there are scratch tiles, the others one.  One
+// CTA (which clears the counters head[0..2]), or several after they have
+// been cleared.
+__global__ void __launch_bounds__(1024) k_part_plan(int nb, const int32_t* __restrict__ count,
+                                                    const int32_t* __restrict__ cap, int P, int split,
+                                                    int first, int max_items, int max_tiles, int4* item,
+                                                    int4* split_list, uint8_t* mark, int32_t* head)
 {
-  __shared__ unsigned long long s_tiles, s_items;
-  __shared__ int s_tile, s_item, s_split;
-  const int max_tiles = min(7 * banks.tiles, PART_TILES);
-  long long P = P0, split = split0, first = first0;
-  for (;;) {
-    if (threadIdx.x == 0) s_tiles = s_items = 0ull, s_tile = s_item = s_split = 0;
+  if (gridDim.x == 1) {
+    if (threadIdx.x < 3) head[threadIdx.x] = 0;
     __syncthreads();
-    unsigned long long tiles = 0, items = 0;
-    for (int64_t b = threadIdx.x; b < nb; b += blockDim.x) {
-      const long long c = min(count[b], cap[b]);
-      if (c > split) tiles += (unsigned long long)((c + P - 1) / P);
-      else if (c > first) items++;
+  }
+  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
+    const int c = min(count[b], cap[b]);
+    bool listed = false;
+    if (c > first) {
+      int parts = 1, t0 = 0;
+      if (c > split) {
+        parts = (int)(((unsigned)c + (unsigned)P - 1u) / (unsigned)P);
+        t0 = atomicAdd(&head[2], parts);
+        if (t0 + parts > max_tiles) parts = 1;
+      }
+      const int i0 = atomicAdd(&head[0], parts);
+      listed = i0 + parts <= max_items;
+      for (int k = 0; k < parts && i0 + k < max_items; k++)
+        item[i0 + k] = make_int4(listed ? b : -1, k, parts, t0);
+      if (listed && parts > 1) split_list[atomicAdd(&head[1], 1)] = make_int4(b, parts, t0, 0);
     }
-    if (tiles) atomicAdd(&s_tiles, tiles);
-    if (items) atomicAdd(&s_items, items);
-    __syncthreads();
-    const bool fewer_tiles = s_tiles > (unsigned long long)max_tiles;
-    const bool fewer_items = s_items + s_tiles > (unsigned long long)max_items;
-    if (!fewer_tiles && !fewer_items) break;
-    if (fewer_tiles || first == split) P *= 2, split *= 2;
-    if (fewer_items) first *= 2;
-    first = min(first, split);
-    __syncthreads();
-  }
-  for (int64_t b = threadIdx.x; b < nb; b += blockDim.x) {
-    const long long c = min(count[b], cap[b]);
-    if (c <= first) continue;
-    const int parts = c > split ? (int)((c + P - 1) / P) : 1;
-    const int i0 = atomicAdd(&s_item, parts), t0 = parts > 1 ? atomicAdd(&s_tile, parts) : 0;
-    for (int k = 0; k < parts; k++) item[i0 + k] = make_int4((int)b, k, parts, t0);
-    if (parts > 1) split_list[atomicAdd(&s_split, 1)] = make_int4((int)b, parts, t0, 0);
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < s_tile; t += blockDim.x)
-    tile[t] = banks.bank[t / banks.tiles] + (size_t)(t % banks.tiles) * banks.slots;
-  if (threadIdx.x == 0) {
-    head[0] = s_item;
-    head[1] = (int)min(first, (long long)INT32_MAX);
-    head[2] = s_split;
+    mark[b] = listed;
   }
 }
 
@@ -729,10 +685,13 @@ cudaError_t run(lf2_ctx* c, float* out, const DepositParams& dp, int stage, cons
     PartView pv;
     const cudaError_t ep = launch_part_plan(
         c, P::smem(), P::THREADS, (size_t)P::NC * TILE3,
-        ACC == ACC_FIXED ? split_max<KIND != 0>(c->has_mass ? 2 : 1) : 0, &pv);
+        ACC == ACC_FIXED  ? split_max<KIND != 0>(c->has_mass ? 2 : 1)
+        : ACC == ACC_COMP ? split_max<true>(1)
+                          : 0,
+        &pv);
     if (ep != cudaSuccess) return ep;
     if (ACC == ACC_FIXED && KIND != 0) {
-      cudaError_t e = launch_vmax(c);
+      cudaError_t e = launch_vmax(c, pv);
       if (e != cudaSuccess) return e;
     }
     cudaError_t e = tile_pass<KIND, 0, ACC>(c, out, dp, gate, pv);
@@ -742,7 +701,7 @@ cudaError_t run(lf2_ctx* c, float* out, const DepositParams& dp, int stage, cons
     return e;
   }
   c->launches += 1;
-  k_fixup<KIND, ACC><<<nb, 256, 0, c->stream>>>(c->g, c->spill, dp.fixed_scale, c->vmax_bits, out,
+  k_fixup<KIND, ACC><<<dim3(nb, KIND == 2 ? 2 : 1), FIX_THREADS, 0, c->stream>>>(c->g, c->spill, dp.fixed_scale, c->vmax_bits, out,
                                                 c->flags, gate);
   return cudaGetLastError();
 }
@@ -762,7 +721,8 @@ cudaError_t run_mode(lf2_ctx* c, float* out, const DepositParams& dp, int stage,
 // share (a brick that starts last then ends with the others) and three times
 // the mean count (an even distribution has no items).  It is split above 3/2 P
 // with P half the share, so that no CTA is left with more than that, but parts
-// hold at least LF2_PART_MIN particles: each clears and writes its tile.
+// hold at least LF2_PART_MIN particles: each clears and writes its tile (parts
+// of 1024 took 41 us for 64 uniform bricks of 4096 against 35 unsplit).
 // `cap` bounds what a split fixed-point tile sums.  The scratch tiles lie in
 // the repack scratch (c->alt), which nothing uses between the rebins.
 cudaError_t launch_part_plan(lf2_ctx* c, size_t smem, int threads, size_t tile_slots, int cap,
@@ -779,21 +739,25 @@ cudaError_t launch_part_plan(lf2_ctx* c, size_t smem, int threads, size_t tile_s
   // np particles make at most 3/2 np / P parts and np / first items
   const int64_t most = std::min<int64_t>(PART_ITEMS, c->np * 3 / (2 * P) + c->np / first);
   if (most == 0) return cudaSuccess;
-  const Banks banks{{reinterpret_cast<uint64_t*>(c->alt.key), reinterpret_cast<uint64_t*>(c->alt.ox),
-                     reinterpret_cast<uint64_t*>(c->alt.oy), reinterpret_cast<uint64_t*>(c->alt.oz),
-                     reinterpret_cast<uint64_t*>(c->alt.vx), reinterpret_cast<uint64_t*>(c->alt.vy),
-                     reinterpret_cast<uint64_t*>(c->alt.vz)},
-                    (int)std::min<int64_t>(c->capacity / 2 / (int64_t)tile_slots, PART_TILES),
-                    (int)tile_slots};
+  float* const banks[7] = {reinterpret_cast<float*>(c->alt.key), c->alt.ox, c->alt.oy, c->alt.oz,
+                           c->alt.vx, c->alt.vy, c->alt.vz};
+  for (int i = 0; i < 7; i++) pv->bank[i] = reinterpret_cast<uint64_t*>(banks[i]);
+  pv->bank_tiles = (int)std::min<int64_t>(c->capacity / 2 / (int64_t)tile_slots, PART_TILES);
   pv->item = c->part_item;
   pv->split = c->part_item + PART_ITEMS;
+  pv->mark = c->part_mark;
   pv->head = c->part_head;
-  pv->tile = c->part_tile;
   pv->max_items = (int)most;
+  const int nb = (int)c->g.nbricks;
+  if (nb > 4096) {
+    const cudaError_t e = cudaMemsetAsync(c->part_head, 0, 3 * sizeof(int32_t), c->stream);
+    if (e != cudaSuccess) return e;
+  }
   c->launches += 1;
-  k_part_plan<<<1, 1024, 0, c->stream>>>(c->g.nbricks, c->count, c->cap, (int)P, (int)split,
-                                         (int)first, (int)most, banks, c->part_item,
-                                         c->part_item + PART_ITEMS, c->part_head, c->part_tile);
+  k_part_plan<<<nb > 4096 ? (nb + 1023) / 1024 : 1, 1024, 0, c->stream>>>(
+      nb, c->count, c->cap, (int)P, (int)split, (int)first, (int)most,
+      std::min(7 * pv->bank_tiles, PART_TILES), c->part_item, c->part_item + PART_ITEMS, c->part_mark,
+      c->part_head);
   return cudaGetLastError();
 }
 
@@ -803,12 +767,13 @@ size_t deposit_spill_slots(const lf2_ctx* c, int comps)
   return (size_t)c->g.nbricks * (size_t)comps * SHELL;
 }
 
-cudaError_t launch_vmax(lf2_ctx* c)
+cudaError_t launch_vmax(lf2_ctx* c, const PartView& pv)
 {
   cudaError_t e = cudaMemsetAsync(c->vmax_bits, 0, sizeof(uint32_t), c->stream);
   if (e != cudaSuccess) return e;
   c->launches += 1;
-  k_vmax<<<(unsigned)c->g.nbricks, 256, 0, c->stream>>>(view(c), c->vmax_bits, c->flags);
+  k_vmax<<<(unsigned)(c->g.nbricks + pv.max_items), 256, 0, c->stream>>>(view(c), c->vmax_bits, c->flags,
+                                                                         pv);
   return cudaGetLastError();
 }
 

@@ -93,16 +93,6 @@ __device__ __forceinline__ void comp_acc(float& s, float& c, float h, float l)
   c = __fadd_rn(c, __fadd_rn(err, l));
 }
 
-template <int ACC, int N>
-__device__ __forceinline__ void add_float(TileRef<N> tr, int j, int t, float w)
-{
-  float* f = reinterpret_cast<float*>(tr.smem);
-  if (ACC == ACC_PLAIN) {
-    atomicAdd(&f[(size_t)j * N + t], w);
-  } else {
-    add_comp(&f[(size_t)j * 2 * N + t], &f[(size_t)j * 2 * N + N + t], w);
-  }
-}
 
 // Signed kinds (momentum and stress): contributions are in units of 2^-48
 // of a unit mass times V or V^2, |q| <= 2^48 for a global mass and 2^54 with
@@ -123,6 +113,100 @@ __device__ __forceinline__ void add_fixed48_t(unsigned char* smem, int j, int t,
   } else {
     atomicAdd(reinterpret_cast<unsigned long long*>(smem) + (size_t)j * N + t, (unsigned long long)q);
   }
+}
+
+// Compensated FP32 mode.  The terms are the FP32 products of the reference's
+// arithmetic; their sum is kept, as in the signed fixed-point kinds, as a
+// 64-bit integer in two 32-bit words, in units of 2^-48 of a power of two
+// 2^e above every |term| of the CTA's particles.  A term is added exactly
+// when it is at least 2^-24 of 2^e, and otherwise to 2^-49 of it; the sum is
+// exact.  (An FP32 shared atomic compiles to a compare-and-swap loop: the
+// TwoSum pair of add_comp takes 3.4 times the shared wavefronts of the two
+// integer words.)  add_comp stays for what the integers cannot hold: terms
+// that are not finite or out of range, and more than split_max particles.
+//
+// x: the term in units of 2^(e - 16), |x| < 2^16.  x = hi + lo 2^-32 with hi
+// the nearest integer (the sum with 1.5 * 2^23 rounds there) and lo signed.
+template <int N>
+__device__ __forceinline__ void add_comp_int(unsigned char* smem, int j, int t, float x)
+{
+  uint32_t* w = reinterpret_cast<uint32_t*>(smem) + (size_t)j * 2 * N;
+  const float h = __fadd_rn(x, 12582912.0f);
+  const int hi = __float_as_int(h) - 0x4B400000;
+  const float r = __fsub_rn(x, __fsub_rn(h, 12582912.0f));  // exact, |r| <= 1/2
+  const int lo = __float2int_rn(__fmul_rn(r, 4294967296.0f));  // 2^31 - 1 at r = 1/2
+  const uint32_t old = atomicAdd(&w[t], (uint32_t)lo);
+  const int carry = old + (uint32_t)lo < old ? 1 : 0;
+  atomicAdd(reinterpret_cast<int*>(&w[N + t]), hi + (lo >> 31) + carry);
+}
+
+// One FP32 term of either mode; SPLIT: the integer sums of the compensated one.
+template <int ACC, bool SPLIT, int N>
+__device__ __forceinline__ void add_float(unsigned char* smem, int j, int t, float w)
+{
+  float* f = reinterpret_cast<float*>(smem);
+  if (ACC == ACC_PLAIN)
+    atomicAdd(&f[(size_t)j * N + t], w);
+  else if (SPLIT)
+    add_comp_int<N>(smem, j, t, w);
+  else
+    add_comp(&f[(size_t)j * 2 * N + t], &f[(size_t)j * 2 * N + N + t], w);
+}
+
+// The unit of a CTA's terms: e with 2^(e - 1) above every |factor| (the FP32
+// rounding of a term's products stays below 2^e).  ok: the scaled factors
+// are in range.
+struct CompUnit {
+  int e;
+  bool ok;
+};
+
+// Largest |mass / volume| (mf for a global mass) and, for NV = 3, |v_i| of
+// the particles, to the power P: the bound of the factors |mf v_i v_j|.
+template <int P>
+__device__ __forceinline__ CompUnit comp_unit(const float* mass, float inv_vol, float mf,
+                                              const float* vx, const float* vy, const float* vz,
+                                              uint32_t p0, int cnt, unsigned* s_max)
+{
+  unsigned m = mass ? 0u : __float_as_uint(mf) & 0x7fffffffu, u = 0u;
+  if (mass || P > 0) {
+    if (threadIdx.x < 2) s_max[threadIdx.x] = 0u;
+    __syncthreads();
+    for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
+      const uint32_t p = p0 + (uint32_t)i;
+      if (mass) m = max(m, __float_as_uint(__fmul_rn(mass[p], inv_vol)) & 0x7fffffffu);
+      if (P > 0)
+        u = max(max(u, __float_as_uint(vx[p]) & 0x7fffffffu),
+                max(__float_as_uint(vy[p]) & 0x7fffffffu, __float_as_uint(vz[p]) & 0x7fffffffu));
+    }
+    m = __reduce_max_sync(0xffffffffu, m);  // bits of |x| order as integers, NaN above infinity
+    u = __reduce_max_sync(0xffffffffu, u);
+    if ((threadIdx.x & 31) == 0) {
+      atomicMax(&s_max[0], m);
+      if (P > 0) atomicMax(&s_max[1], u);
+    }
+    __syncthreads();
+    m = s_max[0];
+    u = s_max[1];
+  }
+  // exponents: |x| < 2^(bits - 126) for a normal number
+  const int em = (int)(m >> 23) - 126, eu = P > 0 ? (int)(u >> 23) - 126 : 0;
+  CompUnit r;
+  r.e = em + P * eu + 1;
+  r.ok = m != 0u && em >= -90 && em <= 90 && (P == 0 || (u != 0u && eu >= -40 && eu <= 40)) &&
+         cnt <= split_max<true>(1);
+  return r;
+}
+
+// hi/lo pair of a compensated vertex sum, from the integers or the floats.
+template <int N>
+__device__ __forceinline__ float2 comp_pair(const TileRef<N>& tr, int j, int t, int e)
+{
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(tr.smem) + (size_t)j * 2 * N;
+  if (!tr.split) return make_float2(__uint_as_float(w[t]), __uint_as_float(w[N + t]));
+  const long long q = (long long)(int32_t)w[N + t] * 4294967296ll + (long long)w[t];
+  const float hi = __ll2float_rn(q), lo = __ll2float_rn(q - (long long)hi);
+  return make_float2(ldexpf(hi, e - 48), ldexpf(lo, e - 48));
 }
 
 // Integer vertex sum of component j: the scalar's split (lo + hi 2^16) or
@@ -147,6 +231,12 @@ __device__ __forceinline__ uint32_t weight_q(float w) { return __float2uint_rn(w
 __device__ __forceinline__ uint32_t vel_q(float v, float vscale)
 {
   return __float2uint_rn(fabsf(v) * vscale);
+}
+
+// fixed_corner with one weight equal to 1 (2^31): (qa qb 2^31 + 2^60) >> 61.
+__device__ __forceinline__ uint64_t fixed_edge(uint32_t qa, uint32_t qb)
+{
+  return ((uint64_t)qa * qb + (1ull << 29)) >> 30;
 }
 
 // Product of two such velocities in units of 2^-31 V^2, rounded.
@@ -272,12 +362,28 @@ __host__ __device__ inline int vexp_of(uint32_t bits)
 // the parts of each split brick in part order and writes the brick's vertices
 // as the tile pass does for a brick in one part.
 struct PartView {
-  const int4* item;       // brick, part, parts of the brick, tile of part 0
+  const int4* item;       // brick (-1: none), part, parts of the brick, tile of part 0
   const int4* split;      // brick, parts, tile of part 0
-  const int32_t* head;    // items, largest count that is not an item, split bricks
-  uint64_t* const* tile;  // scratch tiles, NC * N 8-byte slots each
+  const uint8_t* mark;    // per brick: 1 when it is an item
+  const int32_t* head;    // items, split bricks
+  uint64_t* bank[7];      // scratch tiles, NC * N 8-byte slots each,
+  int bank_tiles;         // so many to a bank
   int max_items;          // what the plan may list
 };
+
+__device__ __forceinline__ uint64_t* scratch_tile(const PartView& pv, int i, int slots)
+{
+  uint64_t* p = pv.bank[0];  // (selected, so that the view stays in parameter space)
+#pragma unroll
+  for (int k = 1; k < 7; k++)
+    if (i >= k * pv.bank_tiles) p = pv.bank[k];
+  return p + (size_t)(i % pv.bank_tiles) * slots;
+}
+
+__device__ __forceinline__ int part_items(const PartView& pv)
+{
+  return pv.max_items ? min(pv.head[0], pv.max_items) : 0;
+}
 
 // One unit of work of a tile pass: particles [first, first + cnt) of a brick.
 struct Part {
@@ -290,47 +396,51 @@ struct Part {
 __device__ __forceinline__ bool part_take(const PartView& pv, int64_t nbricks, const int32_t* count,
                                           const int32_t* cap, Part& p)
 {
-  const int i = (int)blockIdx.x, items = pv.max_items ? pv.head[0] : 0;
+  const int i = (int)blockIdx.x, items = part_items(pv);
   p.first = 0;
   if (i >= items) {
     p.b = i - items;
-    if (p.b >= nbricks) return false;
+    if (p.b >= nbricks || (items && pv.mark[p.b])) return false;
     p.cnt = min(count[p.b], cap[p.b]);
-    return !pv.max_items || p.cnt <= pv.head[1];
+    return true;
   }
   const int4 w = pv.item[i];
   p.b = w.x;
+  if (w.x < 0) return false;
   const int64_t n = min(count[p.b], cap[p.b]);
-  p.first = (int)(n * w.y / w.z);
-  p.cnt = (int)(n * (w.y + 1) / w.z) - p.first;
+  p.first = (int)(n * w.y / w.z) & ~3;  // parts start on 16-byte boundaries
+  p.cnt = (w.y + 1 == w.z ? (int)n : (int)(n * (w.y + 1) / w.z) & ~3) - p.first;
   return true;
 }
 
 // The scratch tile of this CTA's unit when that is a part of a split brick
 // (read again here, so that the particle loop keeps no register for it).
-__device__ __forceinline__ uint64_t* part_tile(const PartView& pv)
+__device__ __forceinline__ uint64_t* part_tile(const PartView& pv, int slots)
 {
-  if (!pv.max_items || (int)blockIdx.x >= pv.head[0]) return nullptr;
+  if ((int)blockIdx.x >= part_items(pv)) return nullptr;
   const int4 w = pv.item[blockIdx.x];
-  return w.z > 1 ? pv.tile[w.w + w.y] : nullptr;
+  return w.z > 1 ? scratch_tile(pv, w.w + w.y, slots) : nullptr;
 }
 
 // A part's tile to the scratch: 8-byte values, component j of vertex t at
-// j * N + t (the integer sum, the hi/lo pair or the float).
+// j * N + t (the integer sum, the hi/lo pair or the float).  e: the unit of
+// the compensated mode's terms.
 template <int ACC, bool SIGNED, int NC, int N>
-__device__ __forceinline__ void part_store(uint64_t* dst, const TileRef<N>& tr)
+__device__ __forceinline__ void part_store(uint64_t* dst, const TileRef<N>& tr, int e)
 {
   const uint32_t* w = reinterpret_cast<const uint32_t*>(tr.smem);
   for (int t = threadIdx.x; t < N; t += blockDim.x) {
 #pragma unroll
     for (int j = 0; j < NC; j++) {
       uint64_t q;
-      if (ACC == ACC_FIXED)
+      if (ACC == ACC_FIXED) {
         q = (uint64_t)tile_fixed<SIGNED>(tr, j, t);
-      else if (ACC == ACC_COMP)
-        q = (uint64_t)w[(size_t)j * 2 * N + t] | ((uint64_t)w[(size_t)j * 2 * N + N + t] << 32);
-      else
+      } else if (ACC == ACC_COMP) {
+        const float2 v = comp_pair(tr, j, t, e);
+        q = (uint64_t)__float_as_uint(v.x) | ((uint64_t)__float_as_uint(v.y) << 32);
+      } else {
         q = w[(size_t)j * N + t];
+      }
       dst[(size_t)j * N + t] = q;
     }
   }
@@ -344,12 +454,12 @@ struct PartSum {
 };
 
 template <int ACC>
-__device__ __forceinline__ PartSum part_sum(const PartView& pv, const int4& sp, int at)
+__device__ __forceinline__ PartSum part_sum(const PartView& pv, const int4& sp, int slots, int at)
 {
   PartSum r{0, 0.0f, 0.0f};
 #pragma unroll 4
   for (int k = 0; k < sp.y; k++) {
-    const uint64_t v = __ldg(pv.tile[sp.z + k] + at);
+    const uint64_t v = __ldg(scratch_tile(pv, sp.z + k, slots) + at);
     if (ACC == ACC_FIXED)
       r.q += (long long)v;
     else if (ACC == ACC_COMP)

@@ -219,9 +219,9 @@ __global__ void __launch_bounds__(FULL_THREADS)
     }
   }
   __syncthreads();
-  if (uint64_t* scratch = part_tile(pv)) {  // k_part_finish_full sums the parts and writes the vertices
+  if (uint64_t* scratch = part_tile(pv, 3 * FT3)) {  // k_part_finish_full sums the parts and writes the vertices
     part_store<ACC_PLAIN, true, 3, FT3>(
-        scratch, TileRef<FT3>{reinterpret_cast<unsigned char*>(tile), false});
+        scratch, TileRef<FT3>{reinterpret_cast<unsigned char*>(tile), false}, 0);
     return;
   }
 
@@ -329,7 +329,10 @@ __global__ void __launch_bounds__(256, 4)
 // as k_deposit_full, two words per vertex (140 KB for three components, one
 // CTA per SM with 512 threads), and every vertex another brick can reach goes
 // to the thick-shell store.
-constexpr int FULL2_THREADS = 512;
+#ifndef LF2_FULL2_THREADS
+#define LF2_FULL2_THREADS 1024
+#endif
+constexpr int FULL2_THREADS = LF2_FULL2_THREADS;
 
 template <int PASS, int ACC>
 __global__ void __launch_bounds__(FULL2_THREADS)
@@ -340,7 +343,7 @@ __global__ void __launch_bounds__(FULL2_THREADS)
   constexpr int CT = FullPass<PASS>::total;
   constexpr bool FIXED = ACC == ACC_FIXED;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ unsigned s_mass;
+  __shared__ unsigned s_max[2];
 
   const Geom& g = v.g;
   Part part;
@@ -354,8 +357,13 @@ __global__ void __launch_bounds__(FULL2_THREADS)
   const int64_t base = v.seg_start[b] + part.first;
   const int cnt = part.cnt;
   const int mass_bound =
-      FIXED && dp.has_mass ? part_mass_bound(v.a.mass, (uint32_t)base, cnt, dp.inv_unit, &s_mass) : 1;
-  TileRef<FT3> tr{smem_raw, FIXED && cnt <= split_max<true>(mass_bound)};
+      FIXED && dp.has_mass ? part_mass_bound(v.a.mass, (uint32_t)base, cnt, dp.inv_unit, s_max) : 1;
+  CompUnit cu{0, false};
+  if (!FIXED)
+    cu = comp_unit<PASS == 0 ? 1 : 2>(dp.has_mass ? v.a.mass : nullptr, dp.inv_vol, dp.mf, v.a.vx, v.a.vy,
+                                      v.a.vz, (uint32_t)base, cnt, s_max);
+  TileRef<FT3> tr{smem_raw, FIXED ? cnt <= split_max<true>(mass_bound) : cu.ok};
+  const float unit = !FIXED && cu.ok ? ldexpf(1.0f, 16 - cu.e) : 1.0f;
   int vexp = 0;
   if (FIXED) vexp = vexp_of(*vmax_bits);
   const float vscale = vel_scale(vexp);
@@ -456,7 +464,8 @@ __global__ void __launch_bounds__(FULL2_THREADS)
         continue;
       }
       // compensated FP32: the arithmetic of k_deposit_full
-      const float mf = HM ? __fmul_rn(v.a.mass[p], dp.inv_vol) : dp.mf;
+      float mf = HM ? __fmul_rn(v.a.mass[p], dp.inv_vol) : dp.mf;
+      if (SPLIT) mf = __fmul_rn(mf, unit);
       float sw[3][2], tw[3][2];
   #pragma unroll
       for (int d = 0; d < 3; d++) {
@@ -482,7 +491,7 @@ __global__ void __launch_bounds__(FULL2_THREADS)
             const float w2 = c == 2 ? tw[2][b2] : sw[2][b2];
             const int t = tile_at((c == 0 ? lt[0] : ls[0]) + b0, (c == 1 ? lt[1] : ls[1]) + b1,
                                   (c == 2 ? lt[2] : ls[2]) + b2);
-            add_float<ACC>(tr, c, t, __fmul_rn(__fmul_rn(__fmul_rn(mv, w0), w1), w2));
+            add_float<ACC, SPLIT, FT3>(smem_raw, c, t, __fmul_rn(__fmul_rn(__fmul_rn(mv, w0), w1), w2));
           }
         }
       } else if (PASS == 1) {
@@ -492,7 +501,7 @@ __global__ void __launch_bounds__(FULL2_THREADS)
   #pragma unroll
           for (int k = 0; k < 8; k++) {
             const int b0 = (k >> 2) & 1, b1 = (k >> 1) & 1, b2 = k & 1;
-            add_float<ACC>(tr, i2, tile_at(ls[0] + b0, ls[1] + b1, ls[2] + b2),
+            add_float<ACC, SPLIT, FT3>(smem_raw, i2, tile_at(ls[0] + b0, ls[1] + b1, ls[2] + b2),
                            __fmul_rn(__fmul_rn(__fmul_rn(m2, sw[0][b0]), sw[1][b1]), sw[2][b2]));
           }
         }
@@ -511,7 +520,7 @@ __global__ void __launch_bounds__(FULL2_THREADS)
               w[d] = st ? tw[d][bb[d]] : sw[d][bb[d]];
               t[d] = (st ? lt[d] : ls[d]) + bb[d];
             }
-            add_float<ACC>(tr, q, tile_at(t[0], t[1], t[2]),
+            add_float<ACC, SPLIT, FT3>(smem_raw, q, tile_at(t[0], t[1], t[2]),
                            __fmul_rn(__fmul_rn(__fmul_rn(mm, w[0]), w[1]), w[2]));
           }
         }
@@ -519,7 +528,7 @@ __global__ void __launch_bounds__(FULL2_THREADS)
     }
   };
   const bool hm_rt = dp.has_mass != 0;
-  if (FIXED && tr.split) {
+  if (tr.split) {
     if (hm_rt) particles(std::true_type{}, std::true_type{});
     else particles(std::true_type{}, std::false_type{});
   } else {
@@ -527,15 +536,14 @@ __global__ void __launch_bounds__(FULL2_THREADS)
     else particles(std::false_type{}, std::false_type{});
   }
   __syncthreads();
-  if (uint64_t* scratch = part_tile(pv)) {
-    part_store<ACC, true, 3, FT3>(scratch, tr);
+  if (uint64_t* scratch = part_tile(pv, 3 * FT3)) {
+    part_store<ACC, true, 3, FT3>(scratch, tr, cu.e);
     return;
   }
 
   // Flush: private vertices (every tile coordinate in [2, e-1]) to the field,
   // the thick shell to the store.
   uint64_t* st = store + (size_t)b * CT * FSHELL;
-  const float* facc = reinterpret_cast<const float*>(smem_raw);
   for (int t = threadIdx.x; t < FT3; t += blockDim.x) {
     const int t0 = t % FT, t1 = (t / FT) % FT, t2 = t / (FT * FT);
     if (t0 > e[0] + 1 || t1 > e[1] + 1 || t2 > e[2] + 1) continue;
@@ -550,9 +558,9 @@ __global__ void __launch_bounds__(FULL2_THREADS)
         if (priv) out[(size_t)c * g.nsites + site] = __fmul_rn(__ll2float_rn(q), conv);
         else st[(size_t)c * FSHELL + si] = (uint64_t)q;
       } else {
-        const float hi = facc[(size_t)j * 2 * FT3 + t], lo = facc[(size_t)j * 2 * FT3 + FT3 + t];
-        if (priv) out[(size_t)c * g.nsites + site] = __fadd_rn(hi, lo);
-        else reinterpret_cast<float2*>(st)[(size_t)c * FSHELL + si] = make_float2(hi, lo);
+        const float2 p = comp_pair(tr, j, t, cu.e);
+        if (priv) out[(size_t)c * g.nsites + site] = __fadd_rn(p.x, p.y);
+        else reinterpret_cast<float2*>(st)[(size_t)c * FSHELL + si] = p;
       }
     }
   }
@@ -570,7 +578,7 @@ __global__ void __launch_bounds__(FINISH_CHUNK)
 {
   constexpr int CT = FullPass<PASS>::total;
   constexpr int CHUNKS = (FT3 + FINISH_CHUNK - 1) / FINISH_CHUNK;
-  const int units = pv.head[2] * CHUNKS;
+  const int units = pv.head[1] * CHUNKS;
   if ((int)blockIdx.x >= units) return;
   const int vexp = ACC == ACC_FIXED ? vexp_of(*vmax_bits) : 0;
   const float conv = ldexpf(fixed_scale, (PASS == 0 ? vexp : 2 * vexp) - 16);
@@ -600,7 +608,7 @@ __global__ void __launch_bounds__(FINISH_CHUNK)
 #pragma unroll
     for (int j = 0; j < 3; j++) {
       const int c = FullPass<PASS>::comp(j);
-      const PartSum s = part_sum<ACC>(pv, sp, j * FT3 + t);
+      const PartSum s = part_sum<ACC>(pv, sp, 3 * FT3, j * FT3 + t);
       if (to_field)
         out[(size_t)c * g.nsites + site] =
             ACC == ACC_FIXED ? __fmul_rn(__ll2float_rn(s.q), conv) : __fadd_rn(s.hi, s.lo);
@@ -619,91 +627,180 @@ __global__ void __launch_bounds__(FINISH_CHUNK)
 // to 26 neighbours that reach it, z outermost, -1 before 0 before +1 (own
 // brick included at 0, 0, 0).  Same enumeration of the boundary vertices as
 // k_fixup_full.
+//
+// Bound by the latency of its scattered reads, as k_fixup: 1176 of a full
+// brick's 1352 boundary vertices lie inside one of its six faces and have one
+// neighbour; thread t takes vertex t of each face, the reads of three faces in
+// flight together, while the threads beyond a face's 14^2 take an
+// edge or corner vertex each.  Bricks one vertex wide, whose vertices have neighbours on both
+// sides, take that general loop for every vertex.
+constexpr int FIX2_FACE = (BRICK - 2) * (BRICK - 2), FIX2_EDGE = 12 * (BRICK - 2) + 8;
+constexpr int FIX2_THREADS = (FIX2_FACE + FIX2_EDGE + 31) & ~31;
+
 template <int C, int ACC>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(FIX2_THREADS, 2)
     k_fixup_full2(Geom g, const uint64_t* __restrict__ store, float fixed_scale,
                   const uint32_t* __restrict__ vmax_bits, float* __restrict__ out)
 {
   const int64_t b = blockIdx.x;
+  const int c0 = 3 * blockIdx.y;  // three components per CTA
   int bc[3];
   brick_coords(g, b, bc[0], bc[1], bc[2]);
   const int e[3] = {brick_extent(g.n[0], bc[0]), brick_extent(g.n[1], bc[1]),
                     brick_extent(g.n[2], bc[2])};
-  const int nzp = e[2] > 1 ? 2 : 1, nyp = e[1] > 1 ? 2 : 1, nxp = e[0] > 1 ? 2 : 1;
-  const int iz = e[2] > 2 ? e[2] - 2 : 0, iy = e[1] > 2 ? e[1] - 2 : 0;
-  const int nzf = nzp * e[0] * e[1];
-  const int nyf = iz * nyp * e[0];
-  const int total = nzf + nyf + iz * iy * nxp;
-  int nbc[3][3];
+  // index of the neighbour below ([0]) and above ([1]) a dim, minus the own
+  int64_t nbr[3][2];
+  {
+    int64_t s = 1;
 #pragma unroll
-  for (int d = 0; d < 3; d++) {
-    nbc[d][0] = bc[d];
-    nbc[d][1] = wrap_add(bc[d], -1, g.nb[d]);
-    nbc[d][2] = wrap_add(bc[d], 1, g.nb[d]);
+    for (int d = 0; d < 3; d++) {
+      nbr[d][0] = (wrap_add(bc[d], -1, g.nb[d]) - bc[d]) * s;
+      nbr[d][1] = (wrap_add(bc[d], 1, g.nb[d]) - bc[d]) * s;
+      s *= g.nb[d];
+    }
   }
   float conv = 0.0f;
   if (ACC == ACC_FIXED) {
     const int vexp = vexp_of(*vmax_bits);
     conv = ldexpf(fixed_scale, (C == 3 ? vexp : 2 * vexp) - 16);
   }
-  for (int f = threadIdx.x; f < total; f += blockDim.x) {
-    int q[3];
-    if (f < nzf) {
-      q[0] = f % e[0];
-      q[1] = (f / e[0]) % e[1];
-      q[2] = f / (e[0] * e[1]) ? e[2] - 1 : 0;
-    } else if (f < nzf + nyf) {
-      const int r = f - nzf;
-      q[0] = r % e[0];
-      q[1] = (r / e[0]) % nyp ? e[1] - 1 : 0;
-      q[2] = 1 + r / (e[0] * nyp);
-    } else {
-      const int r = f - nzf - nyf;
-      q[1] = 1 + r % iy;
-      q[0] = (r / iy) % nxp ? e[0] - 1 : 0;
-      q[2] = 1 + r / (iy * nxp);
+  const int64_t site0 = site_index(g, bc[0] * BRICK, bc[1] * BRICK, bc[2] * BRICK);
+  const int64_t step[3] = {1, g.n[0], (int64_t)g.n[0] * g.n[1]};
+  auto read = [&](int64_t nb, int c, int si) {
+    return __ldg(store + ((size_t)nb * C + c0 + c) * FSHELL + si);
+  };
+  struct Sum {
+    long long q = 0;
+    float s = 0.0f, c = 0.0f;
+    __device__ __forceinline__ void add(uint64_t v)
+    {
+      if (ACC == ACC_FIXED) q += (long long)v;
+      else comp_acc(s, c, __uint_as_float((uint32_t)v), __uint_as_float((uint32_t)(v >> 32)));
     }
-    const bool lo[3] = {q[0] == 0, q[1] == 0, q[2] == 0};
-    const bool hi[3] = {q[0] == e[0] - 1, q[1] == e[1] - 1, q[2] == e[2] - 1};
-    const int64_t site = site_index(g, bc[0] * BRICK + q[0], bc[1] * BRICK + q[1],
-                                    bc[2] * BRICK + q[2]);
-    long long qs[C];
-    float fs[C], fc[C];
+    __device__ __forceinline__ float value(float conv) const
+    {
+      return ACC == ACC_FIXED ? __fmul_rn(__ll2float_rn(q), conv) : __fadd_rn(s, c);
+    }
+  };
+  // a vertex at one end (side[d]) of the dims of `ends`: the subsets of those
+  // dims across which a neighbour is read, in ascending order
+  auto corner = [&](const int (&q)[3], int ends, const int (&side)[3]) {
+    const int64_t site = site0 + q[0] * step[0] + q[1] * step[1] + q[2] * step[2];
+    const int own[3] = {canon(q[0] + 1, e[0]), canon(q[1] + 1, e[1]), canon(q[2] + 1, e[2])};
+    Sum r[3];
 #pragma unroll
-    for (int c = 0; c < C; c++) qs[c] = 0, fs[c] = 0.0f, fc[c] = 0.0f;
+    for (int s = 0; s < 8; s++) {
+      if ((s & ends) != s) continue;
+      int64_t nb = b;
+      int u[3];
 #pragma unroll
-    for (int dz = -1; dz <= 1; dz++) {
-      if ((dz < 0 && !lo[2]) || (dz > 0 && !hi[2])) continue;
+      for (int d = 0; d < 3; d++) {
+        const bool across = (s >> d) & 1;
+        nb += across ? (side[d] ? nbr[d][1] : nbr[d][0]) : 0;
+        u[d] = across ? (side[d] ? 0 : FT - 1) : own[d];
+      }
+      const int si = thick_index(u[0], u[1], u[2]);
 #pragma unroll
-      for (int dy = -1; dy <= 1; dy++) {
-        if ((dy < 0 && !lo[1]) || (dy > 0 && !hi[1])) continue;
+      for (int c = 0; c < 3; c++) r[c].add(read(nb, c, si));
+    }
 #pragma unroll
-        for (int dx = -1; dx <= 1; dx++) {
-          if ((dx < 0 && !lo[0]) || (dx > 0 && !hi[0])) continue;
-          const int64_t nb = (int64_t)nbc[0][dx < 0 ? 1 : (dx > 0 ? 2 : 0)] +
-                             (int64_t)g.nb[0] * ((int64_t)nbc[1][dy < 0 ? 1 : (dy > 0 ? 2 : 0)] +
-                                                 (int64_t)g.nb[1] * nbc[2][dz < 0 ? 1 : (dz > 0 ? 2 : 0)]);
-          const int si = thick_index(dx < 0 ? FT - 1 : (dx > 0 ? 0 : canon(q[0] + 1, e[0])),
-                                     dy < 0 ? FT - 1 : (dy > 0 ? 0 : canon(q[1] + 1, e[1])),
-                                     dz < 0 ? FT - 1 : (dz > 0 ? 0 : canon(q[2] + 1, e[2])));
-          const uint64_t* sp = store + (size_t)nb * C * FSHELL + si;
+    for (int c = 0; c < 3; c++) out[(c0 + c) * g.nsites + site] = r[c].value(conv);
+  };
+  // any owned boundary vertex, neighbours on both sides included: z outermost,
+  // below before own before above
+  auto general = [&](const int (&q)[3]) {
+    const int own[3] = {canon(q[0] + 1, e[0]), canon(q[1] + 1, e[1]), canon(q[2] + 1, e[2])};
+    const int64_t site = site0 + q[0] * step[0] + q[1] * step[1] + q[2] * step[2];
+#pragma unroll 1
+    for (int c = 0; c < 3; c++) {
+      Sum r;
+#pragma unroll 1
+      for (int s = 0; s < 27; s++) {
+        int64_t nb = b;
+        int u[3], rest[3] = {s % 3, (s / 3) % 3, s / 9};
+        bool in = true;
 #pragma unroll
-          for (int c = 0; c < C; c++) {
-            if (ACC == ACC_FIXED) {
-              qs[c] += (long long)sp[(size_t)c * FSHELL];
-            } else {
-              const float2 hl = reinterpret_cast<const float2*>(sp)[(size_t)c * FSHELL];
-              comp_acc(fs[c], fc[c], hl.x, hl.y);
-            }
-          }
+        for (int d = 0; d < 3; d++) {
+          in &= rest[d] == 1 || q[d] == (rest[d] ? e[d] - 1 : 0);
+          nb += rest[d] == 1 ? 0 : rest[d] ? nbr[d][1] : nbr[d][0];
+          u[d] = rest[d] == 1 ? own[d] : rest[d] ? 0 : FT - 1;
+        }
+        if (in) r.add(read(nb, c, thick_index(u[0], u[1], u[2])));
+      }
+      out[(c0 + c) * g.nsites + site] = r.value(conv);
+    }
+  };
+  if (e[0] < 2 || e[1] < 2 || e[2] < 2) {
+    for (int v = threadIdx.x; v < e[0] * e[1] * e[2]; v += blockDim.x) {
+      const int q[3] = {v % e[0], v / e[0] % e[1], v / (e[0] * e[1])};
+      if (q[0] == 0 || q[1] == 0 || q[2] == 0 || q[0] == e[0] - 1 || q[1] == e[1] - 1 || q[2] == e[2] - 1)
+        general(q);
+    }
+    return;
+  }
+  constexpr int I = BRICK - 2;
+  if (threadIdx.x < FIX2_FACE) {
+    const int u = 1 + threadIdx.x % I, w = 1 + threadIdx.x / I;
+#pragma unroll 1
+    for (int side = 0; side < 2; side++) {  // the faces below, then those above
+      uint64_t r[3][3][2];
+      bool on[3];
+      constexpr int du[3] = {1, 0, 0}, dw[3] = {2, 2, 1};
+      // own tile coordinate of the face, and the neighbour's that reaches it
+      const int mine = side ? FT - 2 : 1, theirs = side ? 0 : FT - 1;
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        on[d] = u < e[du[d]] - 1 && w < e[dw[d]] - 1;
+        const int so = d == 0 ? thick_index(mine, u + 1, w + 1)
+                       : d == 1 ? thick_index(u + 1, mine, w + 1) : thick_index(u + 1, w + 1, mine);
+        const int sn = d == 0 ? thick_index(theirs, u + 1, w + 1)
+                       : d == 1 ? thick_index(u + 1, theirs, w + 1) : thick_index(u + 1, w + 1, theirs);
+        const int64_t nb = b + (side ? nbr[d][1] : nbr[d][0]);
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          // the lower one is added first
+          r[d][c][0] = on[d] ? read(side ? b : nb, c, side ? so : sn) : 0;
+          r[d][c][1] = on[d] ? read(side ? nb : b, c, side ? sn : so) : 0;
+        }
+      }
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        if (!on[d]) continue;
+        const int64_t site = site0 + u * step[du[d]] + w * step[dw[d]] + (side ? (e[d] - 1) * step[d] : 0);
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          Sum s;
+          s.add(r[d][c][0]);
+          s.add(r[d][c][1]);
+          out[(c0 + c) * g.nsites + site] = s.value(conv);
         }
       }
     }
-#pragma unroll
-    for (int c = 0; c < C; c++)
-      out[c * g.nsites + site] = ACC == ACC_FIXED ? __fmul_rn(__ll2float_rn(qs[c]), conv)
-                                                  : __fadd_rn(fs[c], fc[c]);
+    return;
   }
+  // edges (two coordinates at an end, the third inside) and corners
+  const int ne[3] = {e[0] - 2, e[1] - 2, e[2] - 2};
+  const int edges = 4 * (ne[0] + ne[1] + ne[2]);
+  const int f = (int)threadIdx.x - FIX2_FACE;
+  if (f >= edges + 8) return;
+  int q[3], side[3], ends = 7;
+  if (f < edges) {
+    const int d = f < 4 * ne[0] ? 0 : f < 4 * (ne[0] + ne[1]) ? 1 : 2;
+    const int r = f - (d > 0 ? 4 * ne[0] : 0) - (d > 1 ? 4 * ne[1] : 0);
+    ends = 7 & ~(1 << d);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      side[k] = k == (d == 0 ? 1 : 0) ? r & 1 : (r >> 1) & 1;
+      q[k] = k == d ? 1 + r / 4 : side[k] ? e[k] - 1 : 0;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      side[k] = ((f - edges) >> k) & 1;
+      q[k] = side[k] ? e[k] - 1 : 0;
+    }
+  }
+  corner(q, ends, side);
 }
 
 constexpr size_t FULL_SMEM = (size_t)3 * FT3 * sizeof(float), FULL2_SMEM = 2 * FULL_SMEM;
@@ -739,9 +836,9 @@ cudaError_t run2(lf2_ctx* c, int kind, float* out, const DepositParams& dp, int 
   if (stage == 0) {
     PartView pv;
     cudaError_t e = launch_part_plan(c, FULL2_SMEM, FULL2_THREADS, (size_t)3 * FT3,
-                                     ACC == ACC_FIXED ? split_max<true>(c->has_mass ? 2 : 1) : 0, &pv);
+                                     split_max<true>(ACC == ACC_FIXED && c->has_mass ? 2 : 1), &pv);
     if (e != cudaSuccess) return e;
-    if (ACC == ACC_FIXED) e = launch_vmax(c);
+    if (ACC == ACC_FIXED) e = launch_vmax(c, pv);
     if (e != cudaSuccess) return e;
     if (kind == 3) return tile_pass2<0, ACC>(c, out, dp, pv);
     e = tile_pass2<1, ACC>(c, out, dp, pv);
@@ -749,9 +846,9 @@ cudaError_t run2(lf2_ctx* c, int kind, float* out, const DepositParams& dp, int 
   }
   c->launches += 1;
   if (kind == 3)
-    k_fixup_full2<3, ACC><<<nb, 256, 0, c->stream>>>(c->g, c->spill, dp.fixed_scale, c->vmax_bits, out);
+    k_fixup_full2<3, ACC><<<nb, FIX2_THREADS, 0, c->stream>>>(c->g, c->spill, dp.fixed_scale, c->vmax_bits, out);
   else
-    k_fixup_full2<6, ACC><<<nb, 256, 0, c->stream>>>(c->g, c->spill, dp.fixed_scale, c->vmax_bits, out);
+    k_fixup_full2<6, ACC><<<dim3(nb, 2), FIX2_THREADS, 0, c->stream>>>(c->g, c->spill, dp.fixed_scale, c->vmax_bits, out);
   return cudaGetLastError();
 }
 

@@ -103,8 +103,8 @@ struct lf2_ctx {
   size_t spill_slots = 0;
   // parts of heavy bricks (deposit tile passes, lf2_deposit_common.cuh)
   int4* part_item = nullptr;         // [PART_ITEMS] items, [PART_TILES] split bricks
-  int32_t* part_head = nullptr;      // device [3]: items, largest count that is not one, split bricks
-  uint64_t** part_tile = nullptr;    // device [PART_TILES]: the scratch tiles
+  int32_t* part_head = nullptr;      // device [3]: items, split bricks, tiles
+  uint8_t* part_mark = nullptr;      // [nbricks] 1 when the brick is an item
   double* h_stats = nullptr;         // pinned [8]
   uint32_t* h_flags = nullptr;       // pinned
   int64_t* h_i64 = nullptr;          // pinned [4]
@@ -184,8 +184,6 @@ cudaError_t launch_fixup_rim(lf2_ctx* c, float* rho);
 // stage 0: tile pass (k_deposit), stage 1: face fix-up (k_fixup)
 cudaError_t launch_deposit(lf2_ctx* c, int kind, float* out, int stage,
                            const uint32_t* gate = nullptr);
-// largest |v_i| of the store into c->vmax_bits (fixed-point momentum/stress)
-cudaError_t launch_vmax(lf2_ctx* c);
 DepositParams deposit_params(const lf2_ctx* c);
 // The plan of heavy bricks for a tile pass of `smem` bytes and `threads`
 // threads per CTA, tiles of tile_slots 8-byte values and at most `cap`
@@ -201,6 +199,8 @@ cudaError_t launch_part_plan(lf2_ctx* c, size_t smem, int threads, size_t tile_s
 cudaError_t launch_count_outside(lf2_ctx* c, int zlo, int zhi, unsigned long long* n,
                                  bool max_v = false);
 cudaError_t launch_extract_outside(lf2_ctx* c, int zlo, int zhi, int32_t* cell, float* off3,
+// largest |v_i| of the store into c->vmax_bits (fixed-point momentum/stress)
+cudaError_t launch_vmax(lf2_ctx* c, const PartView& pv);
                                    float* vel3, float* mass, int64_t* id,
                                    unsigned long long* out_count);
 cudaError_t launch_pack_movers(lf2_ctx* c, int64_t n, const int32_t* cell, const float* off3,

@@ -26,14 +26,14 @@ def _in_brick(n, brick, count, seed):
 
 
 def _case(name):
-    # fewer than 512 * 1024 particles: parts of 1024, bricks above 1536 split
+    # parts of 4096 particles: bricks above 6144 are split
     if name == "edges":
         n = (64, 32, 48)
-        bits = [_in_brick(n, (0, 0, 0), 1536, 1), _in_brick(n, (3, 1, 2), 1537, 2),
-                _in_brick(n, (1, 1, 1), 2049, 3), _in_brick(n, (2, 0, 1), 1, 4)]
+        bits = [_in_brick(n, (0, 0, 0), 6144, 1), _in_brick(n, (3, 1, 2), 6145, 2),
+                _in_brick(n, (1, 1, 1), 8193, 3), _in_brick(n, (2, 0, 1), 1, 4)]
     else:
         n = (33, 17, 24)
-        bits = [_in_brick(n, (1, 0, 0), 30011, 5), _in_brick(n, (2, 1, 1), 4000, 6),
+        bits = [_in_brick(n, (1, 0, 0), 30011, 5), _in_brick(n, (2, 1, 1), 9000, 6),
                 small_case(n, 500, seed=7, vel_sigma=0.2)]
     return (n,) + tuple(np.concatenate([b[k] for b in bits]) for k in range(3))
 
@@ -83,4 +83,51 @@ def test_split_bricks_with_individual_masses(cuda, kind, spread):
         acc, e = O.state_deposit_fixed_kind(kind, n, cell, off, vel, mrel=mrel)
         want = O.fixed_kind_to_f32(acc, kind, e, unit, 1.0 / n[0])
     np.testing.assert_array_equal(got, want)
+    ctx.close()
+
+
+def test_compensated_sums_outside_the_integer_range(cuda):
+    """Terms that the compensated mode's integers do not take (a velocity unit
+    of 1e-15 squared, masses far from 1, an infinity): the FP32 sums give the
+    scaled field, and an infinity or NaN stays at the vertices it reaches."""
+    n, cell, off, vel = _case("ragged")
+    npart = cell.shape[0]
+    gm = 1.0 / npart
+    for kind in (2, 4):
+        got = _deposit(n, 0, kind, cell, off, vel * np.float32(2.0 ** -50), gm)
+        ref, mag = _fp64(n, kind, cell, off, vel, gm)
+        for c in range(ref.shape[0]):
+            p = precision(got[c].astype(np.float64) * 2.0 ** 100, ref[c], mag[c])
+            assert p["norm_max"] <= 1e-6 and p["cell_max"] <= 1e-6, (c, p)
+    bad = vel.copy()
+    bad[7] = (np.inf, 0.5, 0.25)
+    ctx = _ctx(n, 0)
+    ctx.set_particles(cell, off, bad, global_mass=gm)
+    f = ctx.field(3)
+    ctx.deposit_vector_cic(f)
+    got = f.export_internal()
+    ref, _ = _fp64(n, 3, cell, off, vel, gm)
+    ref2, _ = _fp64(n, 3, np.delete(cell, 7), np.delete(off, 7, 0), np.delete(vel, 7, 0), gm)
+    touched = np.abs(ref - ref2) > 0
+    assert not np.isfinite(got[0][touched[0]]).any()
+    assert np.isfinite(got[0][~touched[0]]).all() and np.isfinite(got[1:]).all()
+    ctx.close()
+
+
+def test_compensated_sums_with_a_wide_range_of_masses(cuda):
+    """Masses over seven decades in one brick: each vertex to 2e-7 of its sum
+    wherever that is above 1e-9 of the largest mass's contribution, the unit
+    of the integers being 2^-48 of it."""
+    n = (20, 20, 20)
+    cell, off, vel = small_case(n, 4000, seed=23, vel_sigma=0.1)
+    m = (10.0 ** np.random.default_rng(1).uniform(-7, 0, 4000)).astype(np.float32)
+    ctx = _ctx(n, 0)
+    ctx.set_particles(cell, off, vel, mass=m)
+    f = ctx.field(1)
+    ctx.deposit_scalar(f)
+    got = f.export_internal()[0].astype(np.float64).reshape(-1)
+    ref = O.state_deposit_f64(n, cell, off, 1.0 / 20, mass=m)
+    sel = ref > 1e-9 * 8000
+    # three FP32 products and the rounding of the sum: 4 ulp of 2^-24
+    assert np.max(np.abs(got[sel] - ref[sel]) / ref[sel]) < 4 * 2.0 ** -24 + 8 * 2.0 ** -48 / 1e-9
     ctx.close()
