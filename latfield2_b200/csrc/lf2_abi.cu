@@ -315,7 +315,6 @@ lf2_status lf2_create(lf2_ctx** out, int device, const int n[3], const double bo
   ok = ok && cudaMalloc(&c->brick_maxv2, sizeof(float) * nb) == cudaSuccess;
   ok = ok && cudaMalloc(&c->brick_sums, sizeof(double) * 7 * nb) == cudaSuccess;
   ok = ok && cudaMalloc(&c->stats, sizeof(double) * 8) == cudaSuccess;
-  ok = ok && cudaMalloc(&c->mov_count, sizeof(unsigned long long)) == cudaSuccess;
   ok = ok && cudaMalloc(&c->mig, sizeof(unsigned long long) * 4) == cudaSuccess;
   ok = ok && cudaMalloc(&c->flags, sizeof(uint32_t)) == cudaSuccess;
   ok = ok && cudaMalloc(&c->vmax_bits, sizeof(uint32_t)) == cudaSuccess;
@@ -329,7 +328,10 @@ lf2_status lf2_create(lf2_ctx** out, int device, const int n[3], const double bo
   ok = ok && cudaMallocHost(&c->h_stats, sizeof(double) * 8) == cudaSuccess;
   ok = ok && cudaMallocHost(&c->h_flags, sizeof(uint32_t)) == cudaSuccess;
   ok = ok && cudaMallocHost(&c->h_i64, sizeof(int64_t) * 4) == cudaSuccess;
-  ok = ok && cudaMalloc(&c->work, sizeof(int)) == cudaSuccess;
+  ok = ok && cudaMalloc(&c->work, 2 * sizeof(int) + sizeof(unsigned long long)) == cudaSuccess;
+  c->mov_count = reinterpret_cast<unsigned long long*>(c->work + 2);
+  ok = ok && cudaMalloc(&c->move_list, sizeof(int32_t) * nb) == cudaSuccess;
+  ok = ok && cudaMalloc(&c->move_mark, (size_t)nb) == cudaSuccess;
   ok = ok && cudaMalloc(&c->part_item, sizeof(int4) * (PART_ITEMS + PART_TILES)) == cudaSuccess;
   ok = ok && cudaMalloc(&c->part_head, sizeof(int32_t) * 3) == cudaSuccess;
   ok = ok && cudaMalloc(&c->part_mark, (size_t)nb) == cudaSuccess;
@@ -375,11 +377,13 @@ lf2_status lf2_destroy(lf2_ctx* c)
   cudaFree(c->brick_maxv2);
   cudaFree(c->brick_sums);
   cudaFree(c->stats);
-  cudaFree(c->mov_count);
   cudaFree(c->mig);
   cudaFree(c->work);
   cudaFree(c->flags);
   cudaFree(c->vmax_bits);
+  cudaFree(c->move_list);
+  cudaFree(c->f_rows);
+  cudaFree(c->move_mark);
   cudaFree(c->redep);
   cudaFree(c->repack);
   cudaFree(c->diag);
@@ -983,7 +987,11 @@ lf2_status lf2_gather_kick(lf2_ctx* c, lf2_field F, double dtau, double* max_v)
   MoveParams mp{(float)dtau, 0.0f};
   {
     PhaseScope ps(c, PH_MOVE);
-    LF2_CUDA(c, launch_move(c, F->data, true, false, mp));
+    // the pipelined kernel where it takes the field (lf2_set_move_kernel(1)
+    // keeps the per-brick one)
+    LF2_CUDA(c, c->move_kernel != 1 && move_pipe_auto(c, F->data)
+                    ? launch_move_pipe(c, F->data, true, false, mp, nullptr)
+                    : launch_move(c, F->data, true, false, mp));
   }
   if (max_v) {
     LF2_CUDA(c, launch_reduce_maxv(c));
@@ -999,10 +1007,12 @@ lf2_status lf2_drift_rebin(lf2_ctx* c, double dtau)
 {
   if (!c) return LF2_ERR_ARG;
   MoveParams mp{0.0f, (float)(dtau / c->res)};
-  LF2_CUDA(c, cudaMemsetAsync(c->mov_count, 0, sizeof(unsigned long long), c->stream));
+  if (c->move_kernel == 1)  // the pipelined pass resets the counter itself
+    LF2_CUDA(c, cudaMemsetAsync(c->mov_count, 0, sizeof(unsigned long long), c->stream));
   {
     PhaseScope ps(c, PH_MOVE);
-    LF2_CUDA(c, launch_move(c, nullptr, false, true, mp));
+    LF2_CUDA(c, c->move_kernel != 1 ? launch_move_pipe(c, nullptr, false, true, mp, nullptr)
+                                    : launch_move(c, nullptr, false, true, mp));
   }
   return rebin_tail(c);
 }
@@ -1012,13 +1022,14 @@ lf2_status lf2_step(lf2_ctx* c, lf2_field F, double dtau_kick, double dtau_drift
   if (!valid_field(c, F)) return LF2_ERR_ARG;
   if (F->comps != 3) return fail(c, LF2_ERR_ARG, "the kick field needs 3 components");
   MoveParams mp{(float)dtau_kick, (float)(dtau_drift / c->res)};
-  LF2_CUDA(c, cudaMemsetAsync(c->mov_count, 0, sizeof(unsigned long long), c->stream));
   if ((c->move_kernel == 2 || c->move_kernel == 3) && !move_pipe_eligible(c, F->data))
     return fail(c, LF2_ERR_UNSUPPORTED, "pipelined move needs n0 % 4 == 0, n >= 32, aligned F");
   if (c->move_kernel == 3 && !move_dep_eligible(c, F->data))
     return fail(c, LF2_ERR_UNSUPPORTED, "the fused deposit needs the fixed-point mode and room "
                                         "for its tile");
-  const bool pipe = c->move_kernel >= 2 || (c->move_kernel == 0 && move_pipe_eligible(c, F->data));
+  const bool pipe = c->move_kernel >= 2 || (c->move_kernel == 0 && move_pipe_auto(c, F->data));
+  if (!pipe)  // the pipelined pass resets the counter itself
+    LF2_CUDA(c, cudaMemsetAsync(c->mov_count, 0, sizeof(unsigned long long), c->stream));
   // the fixed-point scalar deposit fused into the pipelined pass (automatic
   // when eligible, or kernel 3), finished by the movers' rim atomics and the
   // rim fix-up; redone by the tile pass if a mover went past the rim
@@ -1029,7 +1040,7 @@ lf2_status lf2_step(lf2_ctx* c, lf2_field F, double dtau_kick, double dtau_drift
   if (!fused) {
     {
       PhaseScope ps(c, PH_MOVE);
-      LF2_CUDA(c, pipe ? launch_move_pipe(c, F->data, mp, nullptr)
+      LF2_CUDA(c, pipe ? launch_move_pipe(c, F->data, true, true, mp, nullptr)
                        : launch_move(c, F->data, true, true, mp));
     }
     LF2_TRY(rebin_tail(c));
@@ -1040,7 +1051,7 @@ lf2_status lf2_step(lf2_ctx* c, lf2_field F, double dtau_kick, double dtau_drift
   LF2_CUDA(c, cudaMemsetAsync(c->redep, 0, sizeof(uint32_t), c->stream));
   {
     PhaseScope ps(c, PH_MOVE);
-    LF2_CUDA(c, launch_move_pipe(c, F->data, mp, rho->data));
+    LF2_CUDA(c, launch_move_pipe(c, F->data, true, true, mp, rho->data));
   }
   {
     PhaseScope ps(c, PH_FIXUP);

@@ -113,7 +113,10 @@ struct lf2_ctx {
   int num_sms = 0;
   int move_kernel = 0;               // 0 auto, 1 per-brick k_move, 2 pipelined
   int last_move_kernel = 0;          // kernel of the last kick-drift pass (1 or 2)
-  int* work = nullptr;               // device brick counter
+  int* work = nullptr;               // device [2]: brick counter, bricks of move_list; then mov_count
+  int32_t* move_list = nullptr;      // [nbricks] bricks taken first
+  uint8_t* move_mark = nullptr;      // [nbricks] 1 for those
+  float* f_rows = nullptr;           // F with rows on 16-byte boundaries (other row lengths)
   int64_t wait_cycles = 0;           // limit of its bounded waits (0: about 2 s)
   int wait_stall = 0;                // consumers first wait on a barrier nothing completes
   const float* tmap_src = nullptr;   // field the cached tensor map describes
@@ -171,12 +174,15 @@ cudaError_t launch_insert(lf2_ctx* c);
 cudaError_t launch_reduce_maxv(lf2_ctx* c);
 cudaError_t launch_maxv_to_device(lf2_ctx* c, double* dst);
 
-// lf2_move_pipe.cu (rho != nullptr: the fixed-point scalar deposit fused in;
-// its rim store is c->spill, rim_store_slots(c) slots)
+// lf2_move_pipe.cu (kick and drift, or one of them; rho != nullptr: the
+// fixed-point scalar deposit fused in; its rim store is c->spill,
+// rim_store_slots(c) slots).  A kick needs move_pipe_eligible.
 bool move_pipe_eligible(const lf2_ctx* c, const float* F);
 bool move_dep_eligible(const lf2_ctx* c, const float* F);
+bool move_pipe_auto(lf2_ctx* c, const float* F);
 size_t rim_store_slots(const lf2_ctx* c);
-cudaError_t launch_move_pipe(lf2_ctx* c, const float* F, MoveParams mp, float* rho);
+cudaError_t launch_move_pipe(lf2_ctx* c, const float* F, bool kick, bool drift, MoveParams mp,
+                             float* rho);
 cudaError_t launch_dep_movers(lf2_ctx* c);
 cudaError_t launch_fixup_rim(lf2_ctx* c, float* rho);
 

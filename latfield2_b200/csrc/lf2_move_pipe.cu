@@ -11,7 +11,8 @@
 //   * one CTA per SM: consumer warps, one producer warp (a single thread)
 //     and one patch warp;
 //   * bricks are taken from a global counter (load balance for clustered
-//     particle distributions); empty bricks cost one atomic;
+//     particle distributions), those far above the mean count first
+//     (k_move_order); empty bricks cost one atomic;
 //   * the producer loads each brick's (BRICK+1)^3 vertex tile of F with one
 //     4-D TMA copy (cp.async.bulk.tensor, box 20 x 17 x 17 x 3, rows padded to
 //     20 floats so the box width is a multiple of 16 bytes) into one of two
@@ -39,6 +40,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <mutex>
 
@@ -264,6 +266,14 @@ struct DepOut {
   int split_max;     // bricks up to this count accumulate in two 32-bit words
 };
 
+// Order of work of the bricks: head[0] is the counter, head[1] the number of
+// bricks of `list`, which come first; mark[b] tells them from the others.
+struct MoveOrder {
+  int* head;
+  const int32_t* list;
+  const uint8_t* mark;
+};
+
 // Bounded wait by lane 0 of the calling warp; the outcome is broadcast so the
 // warp stays together, and every lane then acquires the completed phase.
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, uint32_t* flags, int lane,
@@ -277,16 +287,18 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, uint32
   return ok != 0;
 }
 
-template <int WARPS, bool DEP, bool HM, bool HID>
+// KICK: gather and kick; DRIFT: drift and rebin.  The kick alone writes the
+// velocities back where they are; the drift alone loads no field tile.
+template <int WARPS, bool KICK, bool DRIFT, bool DEP, bool HM, bool HID>
 __global__ void __launch_bounds__(WARPS * 32 + 64, 1)
     k_move_pipe(const __grid_constant__ CUtensorMap tmF, StoreView v, const float* __restrict__ F,
                 MoveParams mp, PartArrays mov, unsigned long long* mov_count,
-                float* __restrict__ brick_maxv2, uint32_t* flags, int* work, int nst,
+                float* __restrict__ brick_maxv2, uint32_t* flags, MoveOrder order, int nst,
                 int stage_bytes, long long wait_limit, int stall, DepOut dep)
 {
   constexpr int CHUNK = WARPS * WSUB;            // particles per chunk buffer
   constexpr int PC_WARPS = WARPS;                // consumer warps
-  constexpr int FST = DEP ? FSTRIDE_DEP : FSTRIDE;
+  constexpr int FST = !KICK ? 0 : DEP ? FSTRIDE_DEP : FSTRIDE;
   constexpr uint32_t ALIGN = DEP ? 127 : 1023;
   extern __shared__ __align__(128) unsigned char dyn[];
   // tma_f: tile copy landed (or the end of the bricks); full_f: tile
@@ -351,12 +363,21 @@ __global__ void __launch_bounds__(WARPS * 32 + 64, 1)
       for (int f = 0; f < NF; f++)
         if (tl_busy[f]) mbar_wait(&tma_f[f], tl_par[f], flags, WAIT_CYCLES);
     };
+    // the bricks in their order of work: the listed ones, then the others
+    const int nheavy = order.head[1];
+    auto take = [&]() -> long long {
+      for (;;) {
+        const long long i = atomicAdd(&order.head[0], 1);
+        if (i < nheavy) return order.list[i];
+        if (i - nheavy >= g.nbricks || nheavy == 0 || !order.mark[i - nheavy]) return i - nheavy;
+      }
+    };
     // q0: next brick with its count and segment start loaded; q1: the index
     // after it
-    long long q0 = atomicAdd(work, 1);
+    long long q0 = take();
     int cq0 = q0 < g.nbricks ? LF2_BRICK_COUNT(v, q0) : 0;
     long long bq0 = q0 < g.nbricks ? v.seg_start[q0] : 0;
-    long long q1 = q0 < g.nbricks ? atomicAdd(work, 1) : q0;
+    long long q1 = q0 < g.nbricks ? take() : q0;
     // the next brick with particles (b = -1 after the last)
     auto next_brick = [&](long long& b, int& cnt, long long& base) {
       for (;;) {
@@ -365,7 +386,7 @@ __global__ void __launch_bounds__(WARPS * 32 + 64, 1)
         if (q0 < g.nbricks) {
           cq0 = LF2_BRICK_COUNT(v, q0);
           bq0 = v.seg_start[q0];
-          q1 = atomicAdd(work, 1);
+          q1 = take();
         }
         if (b >= g.nbricks) {
           b = -1;
@@ -391,7 +412,7 @@ __global__ void __launch_bounds__(WARPS * 32 + 64, 1)
       s_cursor[fs] = 0;
       s_done[fs] = 0;
       s_maxv2[fs] = 0u;
-      if (cnt == 0) {  // an empty brick (fused deposit): no tile to load
+      if (!KICK || cnt == 0) {  // no tile to load (cnt: an empty brick of the fused deposit)
         tl_busy[fs] = false;
         mbar_arrive(&tma_f[fs]);
         return;
@@ -494,7 +515,7 @@ __global__ void __launch_bounds__(WARPS * 32 + 64, 1)
       const int ex = brick_extent(g.n[0], bx), ey = brick_extent(g.n[1], by),
                 ez = brick_extent(g.n[2], bz);
       const bool wx = x0 + ex == g.n[0], wy = y0 + ey == g.n[1], wz = z0 + ez == g.n[2];
-      if (jb.cnt > 0 && (wx || wy || wz)) {
+      if (KICK && jb.cnt > 0 && (wx || wy || wz)) {
         float* ft = reinterpret_cast<float*>(sm + fs * FST);
         constexpr int NP = TILE * TILE, NT = 3 * NP, U = 7;  // U loads in flight per lane
         for (int t0 = lane; t0 < NT; t0 += 32 * U) {
@@ -612,26 +633,37 @@ __global__ void __launch_bounds__(WARPS * 32 + 64, 1)
       for (int j = 0; j < W_ITEMS; j++) {
         const int x = (int)(key[j] & g.mask[0]), y = (int)((key[j] >> g.shift[1]) & g.mask[1]),
                   z = (int)((key[j] >> g.shift[2]) & g.mask[2]);
-        const int t0 = (x - x0) + FX * ((y - y0) + TILE * (z - z0));
-        const float gx = __fsub_rn(1.0f, ox[j]), gy = __fsub_rn(1.0f, oy[j]),
-                    gz = __fsub_rn(1.0f, oz[j]);
-        float a0 = 0.f, a1 = 0.f, a2 = 0.f;
+        if (KICK) {
+          const int t0 = (x - x0) + FX * ((y - y0) + TILE * (z - z0));
+          const float gx = __fsub_rn(1.0f, ox[j]), gy = __fsub_rn(1.0f, oy[j]),
+                      gz = __fsub_rn(1.0f, oz[j]);
+          float a0 = 0.f, a1 = 0.f, a2 = 0.f;
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-          const int cx = (k >> 2) & 1, cy = (k >> 1) & 1, cz = k & 1;
-          const float w = __fmul_rn(__fmul_rn(sel(cx, ox[j], gx), sel(cy, oy[j], gy)),
-                                    sel(cz, oz[j], gz));
-          const int t = t0 + cx + cy * FX + cz * FX * TILE;
-          a0 = __fmaf_rn(w, ft[t], a0);
-          a1 = __fmaf_rn(w, ft[FCOMP + t], a1);
-          a2 = __fmaf_rn(w, ft[2 * FCOMP + t], a2);
+          for (int k = 0; k < 8; k++) {
+            const int cx = (k >> 2) & 1, cy = (k >> 1) & 1, cz = k & 1;
+            const float w = __fmul_rn(__fmul_rn(sel(cx, ox[j], gx), sel(cy, oy[j], gy)),
+                                      sel(cz, oz[j], gz));
+            const int t = t0 + cx + cy * FX + cz * FX * TILE;
+            a0 = __fmaf_rn(w, ft[t], a0);
+            a1 = __fmaf_rn(w, ft[FCOMP + t], a1);
+            a2 = __fmaf_rn(w, ft[2 * FCOMP + t], a2);
+          }
+          vx[j] = __fmaf_rn(mp.dtk, a0, vx[j]);
+          vy[j] = __fmaf_rn(mp.dtk, a1, vy[j]);
+          vz[j] = __fmaf_rn(mp.dtk, a2, vz[j]);
         }
-        vx[j] = __fmaf_rn(mp.dtk, a0, vx[j]);
-        vy[j] = __fmaf_rn(mp.dtk, a1, vy[j]);
-        vz[j] = __fmaf_rn(mp.dtk, a2, vz[j]);
         const float v2 = __fadd_rn(__fadd_rn(__fmul_rn(vx[j], vx[j]), __fmul_rn(vy[j], vy[j])),
                                    __fmul_rn(vz[j], vz[j]));
         maxv2 = fmaxf(maxv2, act[j] ? v2 : 0.0f);
+        if (!DRIFT) {
+          if (act[j]) {
+            const uint32_t q = base32 + (uint32_t)(c0 + i0 + j);
+            v.a.vx[q] = vx[j];
+            v.a.vy[q] = vy[j];
+            v.a.vz[q] = vz[j];
+          }
+          continue;
+        }
         // drift in cell units: o += dtn v, integer part carried into the cell
         const float px = __fmaf_rn(mp.dtn, vx[j], ox[j]), py = __fmaf_rn(mp.dtn, vy[j], oy[j]),
                     pz = __fmaf_rn(mp.dtn, vz[j], oz[j]);
@@ -660,6 +692,7 @@ __global__ void __launch_bounds__(WARPS * 32 + 64, 1)
         if (!finite && act[j]) set_flag(flags, ERR_NONFINITE);
       }
 
+      if (!DRIFT) continue;
       // stayers: lane-major order inside the warp, slots from the brick cursor
       const unsigned lt = (1u << lane) - 1u;
       unsigned sb[W_ITEMS], mb[W_ITEMS];
@@ -746,7 +779,7 @@ __global__ void __launch_bounds__(WARPS * 32 + 64, 1)
       if (atomicAdd(&s_done[fs], 1) == PC_WARPS - 1) {
         __threadfence_block();
         brick_maxv2[b] = __uint_as_float(atomicAdd(&s_maxv2[fs], 0u));
-        v.count[b] = atomicAdd(&s_cursor[fs], 0);
+        if (DRIFT) v.count[b] = atomicAdd(&s_cursor[fs], 0);
         mbar_arrive(&empty_f[fs]);  // every warp is done with this brick
       }
     }
@@ -789,6 +822,41 @@ __global__ void __launch_bounds__(WARPS * 32 + 64, 1)
       if (!warp_wait(&dep_clean, par, flags, lane, wait_limit)) return;
     }
     fk++;
+  }
+}
+
+// The order of work: bricks above `first` particles before the others, so
+// that none of them is left to one SM at the end.  One CTA (which resets the
+// counters of the pass), or several after they have been.
+__global__ void __launch_bounds__(1024) k_move_order(int nb, const int32_t* __restrict__ count,
+                                                     const int32_t* __restrict__ cap, int first,
+                                                     int32_t* list, uint8_t* mark, int* head,
+                                                     unsigned long long* mov_count)
+{
+  if (gridDim.x == 1) {
+    if (threadIdx.x == 0) {
+      head[0] = head[1] = 0;
+      *mov_count = 0ull;
+    }
+    __syncthreads();
+  }
+  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
+    const bool heavy = min(count[b], cap[b]) > first;
+    mark[b] = heavy;
+    if (heavy) list[atomicAdd(&head[1], 1)] = (int32_t)b;
+  }
+}
+
+// `rows` rows of n floats to rows of `pitch` floats, a warp per row.
+__global__ void __launch_bounds__(256) k_pad_rows(const float* __restrict__ src, float* __restrict__ dst,
+                                                  int n, int pitch, int rows)
+{
+  const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
+  for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += warps) {
+    const float* s = src + (int64_t)r * n;
+    float* d = dst + (int64_t)r * pitch;
+#pragma unroll 4
+    for (int x = lane; x < n; x += 32) d[x] = __ldg(s + x);
   }
 }
 
@@ -926,19 +994,34 @@ EncodeTiledFn encode_fn()
 constexpr int DEP_WARPS = LF2_PIPE_DEP_WARPS;  // consumer warps of the fused-deposit kernel
 constexpr int STATIC_SMEM = 256;               // the kernel's static shared memory, rounded up
 
-size_t stage_bytes_for(const lf2_ctx* c, int warps)
+// Rows of F as a tensor map takes them: on 16-byte boundaries.
+bool rows_aligned(const lf2_ctx* c, const float* F)
 {
-  return (size_t)warps * WSUB * (28 + (c->has_mass ? 4 : 0) + (c->has_id ? 8 : 0));
+  return ((uintptr_t)F & 15) == 0 && (c->g.n[0] & 3) == 0;
 }
 
-// Chunk buffers that fit beside the vertex tiles (and the deposit tile).
-int stages_for(const lf2_ctx* c, bool dep)
+int64_t padded_row(const lf2_ctx* c) { return ((int64_t)c->g.n[0] + 3) & ~3ll; }
+
+// Bytes of a chunk buffer; the kick alone carries neither masses nor IDs.
+size_t stage_bytes_for(const lf2_ctx* c, int warps, bool drift)
+{
+  return (size_t)warps * WSUB * (28 + (drift && c->has_mass ? 4 : 0) + (drift && c->has_id ? 8 : 0));
+}
+
+// Shared memory in front of the chunk buffers: the vertex tiles (none without
+// a kick) and the deposit tile, with their alignment.
+size_t fixed_bytes(bool kick, bool dep)
+{
+  return dep ? 128 + NF * (size_t)FSTRIDE_DEP + DEP_BYTES : 1024 + (kick ? NF * (size_t)FSTRIDE : 0);
+}
+
+// Chunk buffers that fit beside them.
+int stages_for(const lf2_ctx* c, bool kick, bool drift, bool dep)
 {
   int optin = 0;
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
-  const size_t sb = stage_bytes_for(c, dep ? DEP_WARPS : LF2_PIPE_WARPS);
-  const size_t fixed = dep ? 128 + NF * (size_t)FSTRIDE_DEP + DEP_BYTES + STATIC_SMEM
-                           : 1024 + NF * (size_t)FSTRIDE + 2048;
+  const size_t sb = stage_bytes_for(c, dep ? DEP_WARPS : LF2_PIPE_WARPS, drift);
+  const size_t fixed = fixed_bytes(kick, dep) + (dep ? STATIC_SMEM : 2048);
   int nst = (int)(((size_t)optin > fixed ? (size_t)optin - fixed : 0) / sb);
   return nst > MAX_STAGES ? MAX_STAGES : nst;
 }
@@ -951,7 +1034,7 @@ size_t rim_store_slots(const lf2_ctx* c) { return (size_t)c->g.nbricks * RIM; }
 // pipelined pass: the deposit tile and two chunk buffers must fit.
 bool move_dep_eligible(const lf2_ctx* c, const float* F)
 {
-  return move_pipe_eligible(c, F) && c->mode == LF2_DEPOSIT_FIXED64 && stages_for(c, true) >= 2;
+  return move_pipe_eligible(c, F) && c->mode == LF2_DEPOSIT_FIXED64 && stages_for(c, true, true, true) >= 2;
 }
 
 // Whether lf2_step's fused move can take the pipelined kernel: a 4-D tensor
@@ -959,25 +1042,60 @@ bool move_dep_eligible(const lf2_ctx* c, const float* F)
 // at least two bricks wide in every dim.
 bool move_pipe_eligible(const lf2_ctx* c, const float* F)
 {
-  if (!F || ((uintptr_t)F & 15) || (c->g.n[0] & 3)) return false;
+  if (!F || !rows_aligned(c, F)) return false;
   for (int d = 0; d < 3; d++)
     if (c->g.n[d] < 2 * BRICK) return false;
   return encode_fn() != nullptr;
 }
 
-cudaError_t launch_move_pipe(lf2_ctx* c, const float* F, MoveParams mp, float* rho)
+// Whether a kick with F takes the pipelined kernel when the choice is
+// automatic: where it is eligible, and on lattices with other row lengths (or
+// an F off the 16-byte boundary) from a copy of F with aligned rows, kept in
+// the context.  The copy moves 24 bytes per site and the pipelined kernel
+// saves the per-brick one's time per particle, so sparse stores (fewer than a
+// third of a particle per site) and contexts without room for the copy keep
+// the per-brick kernel.
+bool move_pipe_auto(lf2_ctx* c, const float* F)
+{
+  if (!F || rows_aligned(c, F)) return move_pipe_eligible(c, F);
+  for (int d = 0; d < 3; d++)
+    if (c->g.n[d] < 2 * BRICK) return false;
+  if (!encode_fn() || 3 * c->np < c->g.nsites) return false;
+  if (!c->f_rows) {
+    const size_t floats = (size_t)3 * padded_row(c) * c->g.n[1] * c->g.n[2];
+    if (cudaMalloc(&c->f_rows, floats * sizeof(float)) != cudaSuccess) {
+      cudaGetLastError();
+      c->f_rows = nullptr;
+      return false;
+    }
+  }
+  return true;
+}
+
+cudaError_t launch_move_pipe(lf2_ctx* c, const float* F, bool kick, bool drift, MoveParams mp,
+                             float* rho)
 {
   static_assert(sizeof(CUtensorMap) <= sizeof(c->tmap_bytes), "tensor map storage");
   CUtensorMap* map = reinterpret_cast<CUtensorMap*>(c->tmap_bytes);
-  if (c->tmap_src != F) {
+  // the field the tiles are copied from: F, or its rows at 16-byte strides
+  const float* src = F;
+  cuuint64_t row = (cuuint64_t)c->g.n[0];
+  if (kick && !rows_aligned(c, F)) {
+    row = (cuuint64_t)padded_row(c);
+    src = c->f_rows;
+    c->launches += 1;
+    k_pad_rows<<<c->num_sms * 8, 256, 0, c->stream>>>(F, c->f_rows, c->g.n[0], (int)row,
+                                                      3 * c->g.n[1] * c->g.n[2]);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  if (kick && c->tmap_src != src) {
     const cuuint64_t dims[4] = {(cuuint64_t)c->g.n[0], (cuuint64_t)c->g.n[1],
                                 (cuuint64_t)c->g.n[2], 3};
-    const cuuint64_t strides[3] = {(cuuint64_t)c->g.n[0] * 4,
-                                   (cuuint64_t)c->g.n[0] * c->g.n[1] * 4,
-                                   (cuuint64_t)c->g.nsites * 4};
+    const cuuint64_t strides[3] = {row * 4, row * c->g.n[1] * 4, row * c->g.n[1] * c->g.n[2] * 4};
     const cuuint32_t box[4] = {FX, TILE, TILE, 3};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
-    const CUresult r = encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(F),
+    const CUresult r = encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(src),
                                    dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -985,15 +1103,14 @@ cudaError_t launch_move_pipe(lf2_ctx* c, const float* F, MoveParams mp, float* r
       c->tmap_src = nullptr;
       return cudaErrorInvalidValue;
     }
-    c->tmap_src = F;
+    c->tmap_src = src;
   }
   const bool dep = rho != nullptr;
   const int warps = dep ? DEP_WARPS : LF2_PIPE_WARPS;
-  const size_t sb = stage_bytes_for(c, warps);
-  const int nst = stages_for(c, dep);
+  const size_t sb = stage_bytes_for(c, warps, drift);
+  const int nst = stages_for(c, kick, drift, dep);
   if (nst < 2) return cudaErrorInvalidConfiguration;
-  const size_t smem = dep ? 128 + NF * (size_t)FSTRIDE_DEP + DEP_BYTES + (size_t)nst * sb
-                          : 1024 + NF * (size_t)FSTRIDE + (size_t)nst * sb;
+  const size_t smem = fixed_bytes(kick, dep) + (size_t)nst * sb;
   DepOut d{};
   if (dep) {
     const double vol = c->res * c->res * c->res;
@@ -1003,20 +1120,46 @@ cudaError_t launch_move_pipe(lf2_ctx* c, const float* F, MoveParams mp, float* r
     d.inv_unit = (float)(1.0 / c->m_unit);
     d.split_max = split_max<false>(c->has_mass ? 64 : 1);
   }
-  using Kern = decltype(&k_move_pipe<LF2_PIPE_WARPS, false, false, false>);
-  const Kern kerns[2][4] = {
-      {k_move_pipe<LF2_PIPE_WARPS, false, false, false>, k_move_pipe<LF2_PIPE_WARPS, false, true, false>,
-       k_move_pipe<LF2_PIPE_WARPS, false, false, true>, k_move_pipe<LF2_PIPE_WARPS, false, true, true>},
-      {k_move_pipe<DEP_WARPS, true, false, false>, k_move_pipe<DEP_WARPS, true, true, false>,
-       k_move_pipe<DEP_WARPS, true, false, true>, k_move_pipe<DEP_WARPS, true, true, true>}};
-  const Kern kern = kerns[dep ? 1 : 0][(c->has_mass ? 1 : 0) + (c->has_id ? 2 : 0)];
+  constexpr int PW = LF2_PIPE_WARPS;
+  using Kern = decltype(&k_move_pipe<PW, true, true, false, false, false>);
+  const int mi = (c->has_mass ? 1 : 0) + (c->has_id ? 2 : 0);
+  const Kern fused[4] = {k_move_pipe<DEP_WARPS, true, true, true, false, false>,
+                         k_move_pipe<DEP_WARPS, true, true, true, true, false>,
+                         k_move_pipe<DEP_WARPS, true, true, true, false, true>,
+                         k_move_pipe<DEP_WARPS, true, true, true, true, true>};
+  const Kern both[4] = {k_move_pipe<PW, true, true, false, false, false>,
+                        k_move_pipe<PW, true, true, false, true, false>,
+                        k_move_pipe<PW, true, true, false, false, true>,
+                        k_move_pipe<PW, true, true, false, true, true>};
+  const Kern drifts[4] = {k_move_pipe<PW, false, true, false, false, false>,
+                          k_move_pipe<PW, false, true, false, true, false>,
+                          k_move_pipe<PW, false, true, false, false, true>,
+                          k_move_pipe<PW, false, true, false, true, true>};
+  const Kern kern = dep                ? fused[mi]
+                    : (kick && drift)  ? both[mi]
+                    : kick             ? k_move_pipe<PW, true, false, false, false, false>
+                                       : drifts[mi];
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(c->work, 0, sizeof(int), c->stream);
+  // a brick of a quarter of an SM's share of the particles still ends with
+  // the others when it starts last; three times the mean leaves an even
+  // distribution in its order
+  const int64_t share = c->np / c->num_sms;
+  const int64_t first = std::max(share / 4, 3 * (c->np / c->g.nbricks));
+  const int nb = (int)c->g.nbricks;
+  if (nb > 4096) {
+    e = cudaMemsetAsync(c->work, 0, 2 * sizeof(int) + sizeof(unsigned long long), c->stream);
+    if (e != cudaSuccess) return e;
+  }
+  c->launches += 2;
+  k_move_order<<<nb > 4096 ? (nb + 1023) / 1024 : 1, 1024, 0, c->stream>>>(
+      nb, c->count, c->cap, (int)std::min<int64_t>(first, INT32_MAX), c->move_list, c->move_mark,
+      c->work, c->mov_count);
+  e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  c->launches += 1;
   kern<<<c->num_sms, warps * 32 + 64, smem, c->stream>>>(
-      *map, view(c), F, mp, c->mov, c->mov_count, c->brick_maxv2, c->flags, c->work, nst, (int)sb,
+      *map, view(c), F, mp, c->mov, c->mov_count, c->brick_maxv2, c->flags,
+      MoveOrder{c->work, c->move_list, c->move_mark}, nst, (int)sb,
       c->wait_cycles > 0 ? (long long)c->wait_cycles : WAIT_CYCLES, c->wait_stall, d);
   return cudaGetLastError();
 }
