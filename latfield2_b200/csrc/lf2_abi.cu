@@ -302,6 +302,8 @@ lf2_status lf2_create(lf2_ctx** out, int device, const int n[3], const double bo
     shift += b;
   }
   g.nsites = nsites;
+  fast_div_set((uint32_t)n[0], g.div_m[0], g.div_s[0]);
+  fast_div_set((uint32_t)(n[0] * n[1]), g.div_m[1], g.div_s[1]);
   g.nbricks = (int64_t)g.nb[0] * g.nb[1] * g.nb[2];
   const int64_t nb = g.nbricks;
 

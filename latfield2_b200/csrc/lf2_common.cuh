@@ -48,7 +48,35 @@ struct Geom {
   uint32_t mask[3]; // bit mask of each coordinate (after shift)
   int64_t nsites;
   int64_t nbricks;
+  uint32_t div_m[2], div_s[2];  // division by n0 and by n0 n1 (fast_div)
 };
+
+// n / d for 0 <= n < 2^31 by one high multiplication: with 2^(l-1) < d <= 2^l,
+// m = ceil(2^(31+l) / d) is below 2^32 and exceeds 2^(31+l) / d by less than
+// 2^l / d, so that n m / 2^(31+l) has the quotient's integer part.  m = 0
+// stands for d = 1.
+inline void fast_div_set(uint32_t d, uint32_t& m, uint32_t& s)
+{
+  uint32_t l = 0;
+  while ((1ull << l) < d) l++;
+  m = l ? (uint32_t)(((1ull << (31 + l)) + d - 1) / d) : 0u;
+  s = l ? l - 1 : 0u;
+}
+
+__device__ __forceinline__ uint32_t fast_div(uint32_t n, uint32_t m, uint32_t s)
+{
+  return m ? __umulhi(n, m) >> s : n;
+}
+
+// Coordinates of cell c = x + n0 (y + n1 z).
+__device__ __forceinline__ void cell_xyz(const Geom& g, int32_t c, int& x, int& y, int& z)
+{
+  const uint32_t u = (uint32_t)c;
+  z = (int)fast_div(u, g.div_m[1], g.div_s[1]);
+  const uint32_t r = u - (uint32_t)z * (uint32_t)(g.n[0] * g.n[1]);
+  y = (int)fast_div(r, g.div_m[0], g.div_s[0]);
+  x = (int)(r - (uint32_t)y * (uint32_t)g.n[0]);
+}
 
 __host__ __device__ inline uint32_t pack_key(const Geom& g, int x, int y, int z)
 {

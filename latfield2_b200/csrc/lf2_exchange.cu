@@ -317,7 +317,8 @@ __global__ void k_pack_movers(Geom g, int64_t n, const int32_t* __restrict__ cel
       continue;
     }
     if (!write) continue;
-    const int x = c % g.n[0], y = (c / g.n[0]) % g.n[1], z = c / (g.n[0] * g.n[1]);
+    int x, y, z;
+    cell_xyz(g, c, x, y, z);
     mov.key[i] = pack_key(g, x, y, z);
     mov.ox[i] = ox, mov.oy[i] = oy, mov.oz[i] = oz;
     mov.vx[i] = vel3[3 * i], mov.vy[i] = vel3[3 * i + 1], mov.vz[i] = vel3[3 * i + 2];
@@ -361,7 +362,8 @@ __global__ void k_pack_records(Geom g, int64_t na, const uint32_t* __restrict__ 
     first = __shfl_sync(0xffffffffu, first, leader);
     if (!ok) continue;
     const int64_t q = (int64_t)first + __popc(bal & ((1u << lane) - 1u));
-    const int x = c % g.n[0], y = (c / g.n[0]) % g.n[1], z = c / (g.n[0] * g.n[1]);
+    int x, y, z;
+    cell_xyz(g, c, x, y, z);
     const float vx = __uint_as_float(r[4]), vy = __uint_as_float(r[5]), vz = __uint_as_float(r[6]);
     int w = 7;
     const float m = has_mass ? __uint_as_float(r[w++]) : 0.0f;

@@ -31,9 +31,7 @@ __host__ __device__ inline int32_t cap_of(int32_t count)
 __device__ inline bool decode_cell(const Geom& g, int32_t c, int& x, int& y, int& z)
 {
   if (c < 0 || (int64_t)c >= g.nsites) return false;
-  x = c % g.n[0];
-  y = (c / g.n[0]) % g.n[1];
-  z = c / (g.n[0] * g.n[1]);
+  cell_xyz(g, c, x, y, z);
   return true;
 }
 
@@ -56,6 +54,45 @@ __global__ void k_load_count(Geom g, int64_t n, const int32_t* __restrict__ cell
 }
 
 // One CTA: cap[b] = count[b] + slack (when caps != nullptr), starts = exclusive
+// The same for lattices whose brick counters fit a CTA's shared memory: a CTA
+// counts its share of the particles there and adds each brick once, so that
+// the bricks of a clump (millions of additions to one counter) do not
+// serialise on their counter's address.  At 256^3 with half of 16.8M particles
+// in 64 clumps: 78 us against 631 with the global counters.  (The scatter below
+// keeps them: it is bound by its 4-byte writes to nine arrays, and ranks formed
+// in shared memory took 1456 us against 1321 there.)
+constexpr int LOAD_THREADS = 1024;
+
+__device__ __forceinline__ void load_share(int64_t n, int64_t& i0, int64_t& i1)
+{
+  i0 = n * blockIdx.x / gridDim.x;
+  i1 = n * (blockIdx.x + 1) / gridDim.x;
+}
+
+__global__ void __launch_bounds__(LOAD_THREADS) k_load_count_sh(Geom g, int64_t n,
+                                                                const int32_t* __restrict__ cell,
+                                                                const float* __restrict__ off3,
+                                                                int32_t* count, uint32_t* flags)
+{
+  extern __shared__ int32_t h[];
+  for (int b = threadIdx.x; b < g.nbricks; b += blockDim.x) h[b] = 0;
+  __syncthreads();
+  int64_t i0, i1;
+  load_share(n, i0, i1);
+  bool bad = false;
+#pragma unroll 4
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+    int x, y, z;
+    const bool ok = decode_cell(g, cell[i], x, y, z);
+    bad |= !ok || !valid_off(off3[3 * i]) || !valid_off(off3[3 * i + 1]) || !valid_off(off3[3 * i + 2]);
+    if (ok) atomicAdd(&h[brick_of(g, x, y, z)], 1);
+  }
+  if (bad) set_flag(flags, ERR_BAD_CELL);  // the load is refused
+  __syncthreads();
+  for (int b = threadIdx.x; b < g.nbricks; b += blockDim.x)
+    if (h[b]) atomicAdd(&count[b], h[b]);
+}
+
 // scan of caps (or of counts), starts[nb] = total.
 __global__ void __launch_bounds__(1024) k_caps_scan(int64_t nb, const int32_t* __restrict__ counts,
                                                     int32_t* caps, int64_t* starts)
@@ -144,7 +181,8 @@ __global__ void k_state_to_pos(Geom g, double res, int64_t n, const int32_t* __r
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int32_t c = cell[i];
-    const int x = c % g.n[0], y = (c / g.n[0]) % g.n[1], z = c / (g.n[0] * g.n[1]);
+    int x, y, z;
+    cell_xyz(g, c, x, y, z);
     pos3[3 * i + 0] = (T)(((double)x + (double)off3[3 * i + 0]) * res);
     pos3[3 * i + 1] = (T)(((double)y + (double)off3[3 * i + 1]) * res);
     pos3[3 * i + 2] = (T)(((double)z + (double)off3[3 * i + 2]) * res);
@@ -422,9 +460,33 @@ __global__ void k_reloc_movers(Geom g, PartArrays mov, int32_t* placed,
 }
 
 __global__ void k_ovf_reset(int32_t* list, int32_t* nlist, int32_t* state)
+// Brick counters of a load in a CTA's shared memory: bytes, or 0 where they
+// do not fit (above 51,200 bricks, lattices beyond 590^3).
+static size_t load_counters(const lf2_ctx* c)
+{
+  const size_t bytes = sizeof(int32_t) * (size_t)c->g.nbricks;
+  return bytes <= 200 * 1024 ? bytes : 0;
+}
+
+// CTAs of a load: those that run at once, fewer when they would hold under 4096
+// particles.
+static unsigned load_ctas(const lf2_ctx* c, int64_t n)
+{
+  const int64_t most = (n + 4095) / 4096;
+  const int64_t all = (int64_t)c->num_sms * (load_counters(c) <= 100 * 1024 ? 2 : 1);
+  return (unsigned)(most < 1 ? 1 : most < all ? most : all);
+}
+
 {
   const int n = *nlist;
   for (int i = threadIdx.x; i < n; i += blockDim.x) state[list[i]] = 0;
+  if (const size_t sh = load_counters(c)) {
+    const cudaError_t e = cudaFuncSetAttribute(k_load_count_sh, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)sh);
+    if (e != cudaSuccess) return e;
+    k_load_count_sh<<<load_ctas(c, n), LOAD_THREADS, sh, c->stream>>>(c->g, n, cell, off3, c->count, c->flags);
+    return cudaGetLastError();
+  }
   __syncthreads();
   if (threadIdx.x == 0) *nlist = 0;
 }
