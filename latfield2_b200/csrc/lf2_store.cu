@@ -6,6 +6,7 @@
 // (LATfield2_Particles.hpp:97-103, :333, :370-373) and addParticle_global
 // (:500-540).  Loading is a counting sort over bricks: histogram, capacity
 // (count + slack) and exclusive scan, then a scatter into the segments.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "lf2_internal.h"
@@ -53,7 +54,6 @@ __global__ void k_load_count(Geom g, int64_t n, const int32_t* __restrict__ cell
   }
 }
 
-// One CTA: cap[b] = count[b] + slack (when caps != nullptr), starts = exclusive
 // The same for lattices whose brick counters fit a CTA's shared memory: a CTA
 // counts its share of the particles there and adds each brick once, so that
 // the bricks of a clump (millions of additions to one counter) do not
@@ -93,6 +93,7 @@ __global__ void __launch_bounds__(LOAD_THREADS) k_load_count_sh(Geom g, int64_t 
     if (h[b]) atomicAdd(&count[b], h[b]);
 }
 
+// One CTA: cap[b] = count[b] + slack (when caps != nullptr), starts = exclusive
 // scan of caps (or of counts), starts[nb] = total.
 __global__ void __launch_bounds__(1024) k_caps_scan(int64_t nb, const int32_t* __restrict__ counts,
                                                     int32_t* caps, int64_t* starts)
@@ -228,47 +229,15 @@ __global__ void k_cell_counts(StoreView v, int32_t* counts)
   }
 }
 
-// ------------------------------------------------------------------ repack
-// Runs only when k_insert found a brick without a free slot (*repack != 0);
-// every kernel returns at once otherwise, so the sequence can stay in the
-// step without a host round trip.
-
-__global__ void __launch_bounds__(1024) k_repack_caps(int64_t nb, const int32_t* __restrict__ count,
-                                                      int32_t* cap_alt, int64_t* start_alt,
-                                                      int64_t capacity, int32_t* repack,
-                                                      uint32_t* flags)
-{
-  if (*repack == 0) return;
-  __shared__ int64_t sh[1024];
-  const int t = threadIdx.x;
-  const int64_t per = (nb + blockDim.x - 1) / blockDim.x;
-  const int64_t lo = t * per, hi = min(nb, lo + per);
-  int64_t s = 0;
-  for (int64_t b = lo; b < hi; b++) {
-    const int32_t c = cap_alt[b] = cap_of(count[b]);
-    s += c;
-  }
-  sh[t] = s;
-  __syncthreads();
-  for (int o = 1; o < (int)blockDim.x; o <<= 1) {
-    const int64_t add = t >= o ? sh[t - o] : 0;
-    __syncthreads();
-    sh[t] += add;
-    __syncthreads();
-  }
-  int64_t run = sh[t] - s;
-  for (int64_t b = lo; b < hi; b++) {
-    start_alt[b] = run;
-    run += cap_alt[b];
-  }
-  if (t == blockDim.x - 1) {
-    start_alt[nb] = sh[t];
-    if (sh[t] > capacity) {
-      set_flag(flags, ERR_CAPACITY);
-      *repack = 0;  // cannot repack: leave the store as it is
-    }
-  }
-}
+// ------------------------------------------------- relocation and repack
+// After k_insert.  A brick that ran out of free slots there is moved on its
+// own to a fresh, larger segment carved from the relocation region (bump
+// allocation past the contiguous segments); its old slots are abandoned until
+// the next full repack.  Only when the region is exhausted is the whole store
+// repacked.  One cooperative kernel: in most steps no brick ran out and it
+// returns at once (nine kernels that each found nothing to do took 20 us of
+// a step, 25% of the smallest); otherwise its phases are separated by grid
+// barriers, without a host round trip.
 
 // One particle's arrays, read before any is written (source and destination
 // may be the same arrays, so interleaved loads and stores would wait for
@@ -330,136 +299,167 @@ __device__ inline void copy_run(const PartArrays& s, int64_t s0, const PartArray
   }
 }
 
-// The per-brick repack kernels run on a small grid (grid-stride over bricks)
-// so that returning early costs a few microseconds, not one CTA per brick.
-__global__ void k_repack_copy_out(StoreView v, PartArrays alt, const int64_t* __restrict__ start_alt,
-                                  int32_t* fill, const int32_t* repack)
+struct RebinTail {
+  StoreView v;
+  PartArrays alt, mov;
+  int64_t* seg_start;
+  int32_t* cap;
+  int64_t* start_alt;
+  int32_t* cap_alt;
+  int32_t* fill;
+  int32_t* placed;
+  const unsigned long long* mov_count;
+  const int32_t* list;  // bricks that ran out of slots
+  int32_t* nlist;
+  int32_t* state;       // 1 listed, 2 relocated
+  unsigned long long* heap_top;
+  int64_t capacity;
+  int32_t* repack;
+  uint32_t* flags;
+  unsigned long long* diag;
+};
+
+constexpr int TAIL_THREADS = 1024;
+
+// Capacities and starts of a full repack (one CTA).
+__device__ void repack_caps(const RebinTail& t, int64_t* sh)
 {
-  if (*repack == 0) return;
-  for (int64_t b = blockIdx.x; b < v.g.nbricks; b += gridDim.x) {
-    const int placed = min(v.count[b], v.cap[b]);
-    const int64_t s0 = v.seg_start[b], d0 = start_alt[b];
-    copy_run(v.a, s0, alt, d0, placed);
-    if (threadIdx.x == 0) fill[b] = placed;
+  const int64_t nb = t.v.g.nbricks, per = (nb + blockDim.x - 1) / blockDim.x;
+  const int64_t lo = threadIdx.x * per, hi = min(nb, lo + per);
+  int64_t s = 0;
+  for (int64_t b = lo; b < hi; b++) s += t.cap_alt[b] = cap_of(t.v.count[b]);
+  sh[threadIdx.x] = s;
+  __syncthreads();
+  for (int o = 1; o < (int)blockDim.x; o <<= 1) {
+    const int64_t add = (int)threadIdx.x >= o ? sh[threadIdx.x - o] : 0;
+    __syncthreads();
+    sh[threadIdx.x] += add;
+    __syncthreads();
+  }
+  int64_t run = sh[threadIdx.x] - s;
+  for (int64_t b = lo; b < hi; b++) {
+    t.start_alt[b] = run;
+    run += t.cap_alt[b];
+  }
+  if (threadIdx.x == blockDim.x - 1) {
+    t.start_alt[nb] = sh[threadIdx.x];
+    if (sh[threadIdx.x] > t.capacity) {
+      set_flag(t.flags, ERR_CAPACITY);
+      *t.repack = 0;  // cannot repack: leave the store as it is
+    }
   }
 }
 
-__global__ void k_repack_movers(Geom g, PartArrays mov, const int32_t* __restrict__ placed,
-                                const unsigned long long* __restrict__ mov_count, PartArrays alt,
-                                const int64_t* __restrict__ start_alt, int32_t* fill,
-                                const int32_t* repack)
+__global__ void __launch_bounds__(TAIL_THREADS, 1) k_rebin_tail(RebinTail t)
 {
-  if (*repack == 0) return;
-  const int64_t nm = (int64_t)*mov_count;
-  for (int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; m < nm;
-       m += (int64_t)gridDim.x * blockDim.x) {
-    if (placed[m]) continue;
-    int x, y, z;
-    unpack_key(g, mov.key[m], x, y, z);
-    const int64_t b = brick_of(g, x, y, z);
-    copy_particle(mov, m, alt, start_alt[b] + atomicAdd(&fill[b], 1));
-  }
-}
-
-__global__ void k_repack_copy_back(StoreView v, PartArrays alt, const int64_t* __restrict__ start_alt,
-                                   const int32_t* __restrict__ fill, const int32_t* repack)
-{
-  if (*repack == 0) return;
-  for (int64_t b = blockIdx.x; b < v.g.nbricks; b += gridDim.x) {
-    const int n = fill[b];
-    const int64_t d0 = start_alt[b];
-    copy_run(alt, d0, v.a, d0, n);
-    if (threadIdx.x == 0) v.count[b] = n;
-  }
-}
-
-__global__ void k_repack_finish(int64_t nb, const int64_t* __restrict__ start_alt,
-                                const int32_t* __restrict__ cap_alt, int64_t* seg_start,
-                                int32_t* cap, int32_t* repack, unsigned long long* heap_top)
-{
-  if (*repack == 0) return;
-  for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b <= nb;
-       b += (int64_t)gridDim.x * blockDim.x) {
-    seg_start[b] = start_alt[b];
-    if (b < nb) cap[b] = cap_alt[b];
-    else *heap_top = (unsigned long long)start_alt[nb];  // relocation region starts after the segments
-  }
-}
-
-__global__ void k_repack_clear(int32_t* repack, uint32_t* flags, unsigned long long* diag,
-                               const unsigned long long* movers)
-{
-  if (*repack) {
-    set_flag(flags, ERR_REPACK);
-    diag[0] += 1;
-    *repack = 0;
-  }
-  diag[1] = *movers;
-}
-
-// ----------------------------------------------------------- relocation
-// A brick that ran out of free slots in k_insert is moved on its own to a
-// fresh, larger segment carved from the relocation region (bump allocation
-// past the contiguous segments).  Its old slots are abandoned until the next
-// full repack.  Only when the region is exhausted does the whole store get
-// repacked (k_repack_*).
-
-__global__ void __launch_bounds__(1024)
-    k_reloc(StoreView v, int64_t* seg_start, int32_t* cap, const int32_t* __restrict__ list,
-                        const int32_t* __restrict__ nlist, int32_t* state, int32_t* fill,
-                        unsigned long long* heap_top, int64_t capacity, int32_t* repack,
-                        unsigned long long* diag)
-{
+  __shared__ int64_t sh[TAIL_THREADS];
   __shared__ long long s_new;
-  const int n = *nlist;
+  const int n = *t.nlist;
+  if (n == 0) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) t.diag[1] = *t.mov_count;
+    return;
+  }
+  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+  const Geom& g = t.v.g;
+  const int64_t nm = (int64_t)*t.mov_count;
+  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+
+  // full bricks into new segments
   for (int i = blockIdx.x; i < n; i += gridDim.x) {
-    const int64_t b = list[i];
-    const int32_t need = v.count[b];  // stays + every arrival that tried
-    const int32_t placed = min(need, cap[b]);
+    const int64_t b = t.list[i];
+    const int32_t need = t.v.count[b];  // stays + every arrival that tried
+    const int32_t placed = min(need, t.cap[b]);
     const int32_t ncap = cap_of(need);
     if (threadIdx.x == 0) {
-      const unsigned long long s0 = atomicAdd(heap_top, (unsigned long long)ncap);
-      s_new = (s0 + (unsigned long long)ncap <= (unsigned long long)capacity) ? (long long)s0 : -1;
-      if (s_new < 0) *repack = 1;  // region exhausted: repack everything
+      const unsigned long long s0 = atomicAdd(t.heap_top, (unsigned long long)ncap);
+      s_new = (s0 + (unsigned long long)ncap <= (unsigned long long)t.capacity) ? (long long)s0 : -1;
+      if (s_new < 0) *t.repack = 1;  // region exhausted: repack everything
     }
     __syncthreads();
     const long long d0 = s_new;
     if (d0 >= 0) {
-      const int64_t s0 = seg_start[b];
-      copy_run(v.a, s0, v.a, d0, placed);
+      const int64_t s0 = t.seg_start[b];
+      copy_run(t.v.a, s0, t.v.a, d0, placed);
       __syncthreads();
       if (threadIdx.x == 0) {
-        seg_start[b] = d0;
-        cap[b] = ncap;
-        fill[b] = placed;
-        state[b] = 2;
-        atomicAdd(&diag[2], 1ull);
+        t.seg_start[b] = d0;
+        t.cap[b] = ncap;
+        t.fill[b] = placed;
+        t.state[b] = 2;
+        atomicAdd(&t.diag[2], 1ull);
       }
     }
     __syncthreads();
   }
-}
-
-__global__ void k_reloc_movers(Geom g, PartArrays mov, int32_t* placed,
-                               const unsigned long long* __restrict__ mov_count, PartArrays dst,
-                               const int64_t* __restrict__ seg_start, const int32_t* __restrict__ state,
-                               int32_t* fill, const int32_t* __restrict__ nlist)
-{
-  if (*nlist == 0) return;
-  const int64_t nm = (int64_t)*mov_count;
-  for (int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; m < nm;
-       m += (int64_t)gridDim.x * blockDim.x) {
-    if (placed[m]) continue;
+  grid.sync();
+  // their movers that found no slot
+  for (int64_t m = i0; m < nm; m += stride) {
+    if (t.placed[m]) continue;
     int x, y, z;
-    unpack_key(g, mov.key[m], x, y, z);
+    unpack_key(g, t.mov.key[m], x, y, z);
     const int64_t b = brick_of(g, x, y, z);
-    if (state[b] != 2) continue;  // not relocated: left to the full repack
-    copy_particle(mov, m, dst, seg_start[b] + atomicAdd(&fill[b], 1));
-    placed[m] = 1;
+    if (t.state[b] != 2) continue;  // not relocated: left to the full repack
+    copy_particle(t.mov, m, t.v.a, t.seg_start[b] + atomicAdd(&t.fill[b], 1));
+    t.placed[m] = 1;
+  }
+  if (*t.repack) {  // set before the barrier
+    grid.sync();
+    if (blockIdx.x == 0) repack_caps(t, sh);
+    grid.sync();
+    if (*t.repack) {
+      for (int64_t b = blockIdx.x; b < g.nbricks; b += gridDim.x) {
+        const int placed = min(t.v.count[b], t.cap[b]);
+        copy_run(t.v.a, t.seg_start[b], t.alt, t.start_alt[b], placed);
+        if (threadIdx.x == 0) t.fill[b] = placed;
+      }
+      grid.sync();
+      for (int64_t m = i0; m < nm; m += stride) {
+        if (t.placed[m]) continue;
+        int x, y, z;
+        unpack_key(g, t.mov.key[m], x, y, z);
+        const int64_t b = brick_of(g, x, y, z);
+        copy_particle(t.mov, m, t.alt, t.start_alt[b] + atomicAdd(&t.fill[b], 1));
+      }
+      grid.sync();
+      for (int64_t b = blockIdx.x; b < g.nbricks; b += gridDim.x) {
+        copy_run(t.alt, t.start_alt[b], t.v.a, t.start_alt[b], t.fill[b]);
+        if (threadIdx.x == 0) {
+          t.v.count[b] = t.fill[b];
+          t.seg_start[b] = t.start_alt[b];
+          t.cap[b] = t.cap_alt[b];
+        }
+      }
+      if (blockIdx.x == 0 && threadIdx.x == 0) {
+        t.seg_start[g.nbricks] = t.start_alt[g.nbricks];
+        // the relocation region starts after the segments
+        *t.heap_top = (unsigned long long)t.start_alt[g.nbricks];
+      }
+    }
+  }
+  grid.sync();
+  if (blockIdx.x != 0) return;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) t.state[t.list[i]] = 0;
+  if (threadIdx.x == 0) {
+    if (*t.repack) {
+      set_flag(t.flags, ERR_REPACK);
+      t.diag[0] += 1;
+      *t.repack = 0;
+    }
+    t.diag[1] = *t.mov_count;
+    *t.nlist = 0;
   }
 }
 
-__global__ void k_ovf_reset(int32_t* list, int32_t* nlist, int32_t* state)
+inline int grid_for(int64_t n, int threads)
+{
+  int64_t g = (n + threads - 1) / threads;
+  if (g > 148 * 32) g = 148 * 32;
+  return (int)(g > 0 ? g : 1);
+}
+
+}  // namespace
+
 // Brick counters of a load in a CTA's shared memory: bytes, or 0 where they
 // do not fit (above 51,200 bricks, lattices beyond 590^3).
 static size_t load_counters(const lf2_ctx* c)
@@ -477,9 +477,9 @@ static unsigned load_ctas(const lf2_ctx* c, int64_t n)
   return (unsigned)(most < 1 ? 1 : most < all ? most : all);
 }
 
+cudaError_t launch_load_count(lf2_ctx* c, int64_t n, const int32_t* cell, const float* off3)
 {
-  const int n = *nlist;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) state[list[i]] = 0;
+  c->launches += 1;
   if (const size_t sh = load_counters(c)) {
     const cudaError_t e = cudaFuncSetAttribute(k_load_count_sh, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)sh);
@@ -487,22 +487,6 @@ static unsigned load_ctas(const lf2_ctx* c, int64_t n)
     k_load_count_sh<<<load_ctas(c, n), LOAD_THREADS, sh, c->stream>>>(c->g, n, cell, off3, c->count, c->flags);
     return cudaGetLastError();
   }
-  __syncthreads();
-  if (threadIdx.x == 0) *nlist = 0;
-}
-
-inline int grid_for(int64_t n, int threads)
-{
-  int64_t g = (n + threads - 1) / threads;
-  if (g > 148 * 32) g = 148 * 32;
-  return (int)(g > 0 ? g : 1);
-}
-
-}  // namespace
-
-cudaError_t launch_load_count(lf2_ctx* c, int64_t n, const int32_t* cell, const float* off3)
-{
-  c->launches += 1;
   k_load_count<<<grid_for(n, 256), 256, 0, c->stream>>>(c->g, n, cell, off3, c->count, c->flags);
   return cudaGetLastError();
 }
@@ -584,27 +568,19 @@ cudaError_t launch_heap_reset(lf2_ctx* c)
 
 cudaError_t launch_repack(lf2_ctx* c)
 {
-  c->launches += 9;
-  const int64_t nb = c->g.nbricks;
-  k_reloc<<<148, 1024, 0, c->stream>>>(view(c), c->seg_start, c->cap, c->ovf_list, c->ovf_count,
-                                      c->ovf_state, c->fill, c->heap_top, c->capacity, c->repack,
-                                      c->diag);
-  k_reloc_movers<<<148 * 2, 256, 0, c->stream>>>(c->g, c->mov, c->mov_placed, c->mov_count, c->cur,
-                                                 c->seg_start, c->ovf_state, c->fill, c->ovf_count);
-  k_repack_caps<<<1, 1024, 0, c->stream>>>(nb, c->count, c->cap_alt, c->seg_start_alt, c->capacity,
-                                           c->repack, c->flags);
-  const unsigned small = (unsigned)(nb < 148 * 8 ? nb : 148 * 8);
-  k_repack_copy_out<<<small, 256, 0, c->stream>>>(view(c), c->alt, c->seg_start_alt, c->fill,
-                                                  c->repack);
-  k_repack_movers<<<148 * 4, 256, 0, c->stream>>>(c->g, c->mov, c->mov_placed, c->mov_count, c->alt,
-                                                  c->seg_start_alt, c->fill, c->repack);
-  k_repack_copy_back<<<small, 256, 0, c->stream>>>(view(c), c->alt, c->seg_start_alt, c->fill,
-                                                   c->repack);
-  k_repack_finish<<<small, 256, 0, c->stream>>>(nb, c->seg_start_alt, c->cap_alt, c->seg_start,
-                                                 c->cap, c->repack, c->heap_top);
-  k_repack_clear<<<1, 1, 0, c->stream>>>(c->repack, c->flags, c->diag, c->mov_count);
-  k_ovf_reset<<<1, 256, 0, c->stream>>>(c->ovf_list, c->ovf_count, c->ovf_state);
-  return cudaGetLastError();
+  RebinTail t;
+  t.v = view(c);
+  t.alt = c->alt, t.mov = c->mov;
+  t.seg_start = c->seg_start, t.cap = c->cap;
+  t.start_alt = c->seg_start_alt, t.cap_alt = c->cap_alt, t.fill = c->fill;
+  t.placed = c->mov_placed, t.mov_count = c->mov_count;
+  t.list = c->ovf_list, t.nlist = c->ovf_count, t.state = c->ovf_state;
+  t.heap_top = c->heap_top, t.capacity = c->capacity;
+  t.repack = c->repack, t.flags = c->flags, t.diag = c->diag;
+  void* args[] = {&t};
+  c->launches += 1;
+  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&k_rebin_tail), dim3(c->num_sms),
+                                     dim3(TAIL_THREADS), args, 0, c->stream);
 }
 
 }  // namespace lf2
