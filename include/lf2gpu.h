@@ -471,6 +471,29 @@ lf2_status lf2_pm_kick_drift(lf2_ctx* ctx, int64_t np, int32_t* cell,
 lf2_status lf2_pm_step(lf2_ctx* ctx, int64_t np, int32_t* cell, float* off3,
                        float* vel3, const float* F4, double dt_kick,
                        double dt_drift);
+/* the same into other arrays; the state before the step stays. */
+lf2_status lf2_pm_step_to(lf2_ctx* ctx, int64_t np, const int32_t* cell,
+                          const float* off3, const float* vel3,
+                          const float* F4, double dt_kick, double dt_drift,
+                          int32_t* cell_out, float* off3_out,
+                          float* vel3_out);
+/* adjoint of a step at its state (cell, off3): g_vel3 += dt_drift / res *
+ * g_off3 (the drift), then the gather's adjoint for the gradient dt_kick *
+ * g_vel3 of the gathered force, into g_F4 (+=) and g_off3 (+=). */
+lf2_status lf2_pm_step_adjoint(lf2_ctx* ctx, int64_t np, const int32_t* cell,
+                               const float* off3, const float* F4,
+                               double dt_kick, double dt_drift,
+                               float* g_vel3, float* g_off3, float* g_F4);
+/* the chain's loss sum_g w(g) rho(g) (FP64, fixed order, to the device), and
+ * its adjoint at the last state, which starts a backward pass: for g_rho =
+ * g_loss * w the gradients of lf2_pm_deposit_adjoint are written (not added),
+ * and g_vel3 is set to zero. */
+lf2_status lf2_pm_loss(lf2_ctx* ctx, const float* w, const float* rho,
+                       double* loss);
+lf2_status lf2_pm_loss_adjoint(lf2_ctx* ctx, int64_t np, const int32_t* cell,
+                               const float* off3, const float* mass,
+                               const float* w, double g_loss, float* g_off3,
+                               float* g_mass, float* g_vel3);
 lf2_status lf2_pm_deposit_adjoint(lf2_ctx* ctx, int64_t np,
                                   const int32_t* cell, const float* off3,
                                   const float* mass, double gmass,

@@ -131,6 +131,24 @@ class _Ops:
                                                          _p(m), 0.0, _p(g_rho), _p(g_off),
                                                          _p(g_m)), "pm_deposit_adjoint")
 
+    def loss(self, w, rho):
+        """sum_g w_g rho_g in FP64."""
+        if w.device != rho.device or w.numel() != rho.numel():
+            raise RuntimeError(f"the loss weights need {rho.numel()} values on {rho.device} "
+                               f"(got {w.numel()} on {w.device})")
+        out = torch.empty((), dtype=torch.float64, device=rho.device)
+        _check(self.ctx, self.lib.lf2_pm_loss(self.ctx.h, _p(w), _p(rho), _p(out)), "pm_loss")
+        return out
+
+    def loss_adj(self, cell, off, m, w, g_loss):
+        """gradients of the loss at its state: offsets, velocities (zero),
+        masses."""
+        g_off, g_v, g_m = torch.empty_like(off), torch.empty_like(off), torch.empty_like(m)
+        _check(self.ctx, self.lib.lf2_pm_loss_adjoint(self.ctx.h, cell.numel(), _p(cell), _p(off),
+                                                      _p(m), _p(w), g_loss, _p(g_off), _p(g_m),
+                                                      _p(g_v)), "pm_loss_adjoint")
+        return g_off, g_v, g_m
+
     def gather_adj(self, cell, off, F, g_G, g_F, g_off):
         _check(self.ctx, self.lib.lf2_pm_gather_adjoint(self.ctx.h, cell.numel(), _p(cell), _p(off),
                                                         _p(F), _p(g_G), _p(g_F), _p(g_off)),
@@ -161,9 +179,23 @@ class _Ops:
         return rho, F
 
     def step(self, cell, off, vel, F, dt):
-        """gather, kick and drift in one pass (lf2_pm_step)."""
+        """gather, kick and drift in one pass (lf2_pm_step), in place."""
         _check(self.ctx, self.lib.lf2_pm_step(self.ctx.h, cell.numel(), _p(cell), _p(off), _p(vel),
                                               _p(F), dt, dt), "pm_step")
+
+    def next_state(self, cell, off, vel, F, dt):
+        """the same (lf2_pm_step_to): the state after the step, in new
+        tensors."""
+        out = torch.empty_like(cell), torch.empty_like(off), torch.empty_like(vel)
+        _check(self.ctx, self.lib.lf2_pm_step_to(self.ctx.h, cell.numel(), _p(cell), _p(off), _p(vel),
+                                                 _p(F), dt, dt, *(_p(t) for t in out)), "pm_step_to")
+        return out
+
+    def step_adj(self, cell, off, F, dt, g_v, g_off, g_F):
+        """adjoint of the drift, the kick and the gather of a step."""
+        _check(self.ctx, self.lib.lf2_pm_step_adjoint(self.ctx.h, cell.numel(), _p(cell), _p(off),
+                                                      _p(F), dt, dt, _p(g_v), _p(g_off), _p(g_F)),
+               "pm_step_adjoint")
 
 
 class PMChain(torch.autograd.Function):
@@ -190,14 +222,14 @@ class PMChain(torch.autograd.Function):
         ckpts, rhos, Fs = {}, [], []
         for k in range(steps):
             if k % checkpoint_every == 0:
-                ckpts[k] = (cell.clone(), off.clone(), vel.clone())
+                ckpts[k] = (cell, off, vel)
             rho, F = ops.fields(cell, off, m, S32, coupling)
             rhos.append(rho)
             Fs.append(F)
-            ops.step(cell, off, vel, F, dt)
+            cell, off, vel = ops.next_state(cell, off, vel, F, dt)
         rhoK = torch.zeros(lf2ctx.nsites, dtype=torch.float32, device=cell.device)
         ops.deposit(cell, off, m, rhoK)
-        loss = torch.dot(w32.to(torch.float64), rhoK.to(torch.float64))
+        loss = ops.loss(w32, rhoK)
         fctx.lf2 = (lf2ctx, steps, dt, checkpoint_every, ckpts, rhos, Fs, coupling)
         fctx.save_for_backward(cell, off, m, S32, w32, rhoK, order)
         fctx.pos_dtype = pos0.dtype
@@ -211,13 +243,9 @@ class PMChain(torch.autograd.Function):
         ops = _Ops(lf2ctx)
         dev = cellK.device
         res = lf2ctx.res
-        npart = cellK.numel()
         g = float(gloss)
-        g_off = torch.zeros(npart, 3, dtype=torch.float32, device=dev)
-        g_v = torch.zeros(npart, 3, dtype=torch.float32, device=dev)
-        g_m = torch.zeros(npart, dtype=torch.float32, device=dev)
         g_S = torch.zeros(81, dtype=torch.float32, device=dev)
-        ops.deposit_adj(cellK, offK, m, (w32 * g).contiguous(), g_off, g_m)
+        g_off, g_v, g_m = ops.loss_adj(cellK, offK, m, w32, g)
         seg = {}
         for k in range(steps - 1, -1, -1):
             k0 = (k // every) * every
@@ -231,16 +259,14 @@ class PMChain(torch.autograd.Function):
                                        "consumed (call backward once per forward)")
                 c, o, v = ckpts.pop(k0)
                 for j in range(k0, k + 1):
-                    seg[j] = (c.clone(), o.clone()) if j < k else (c, o)
+                    seg[j] = (c, o)
                     if j < k:
-                        ops.step(c, o, v, Fs[j], dt)
+                        c, o, v = ops.next_state(c, o, v, Fs[j], dt)
             cell_k, off_k = seg[k]
-            # drift x_{k+1} = x_k + dt v_{k+1} (cell units: off += dt/res v)
-            g_v += (dt / res) * g_off
-            # kick v_{k+1} = v_k + dt G_k
-            g_G = (dt * g_v).contiguous()
+            # drift x_{k+1} = x_k + dt v_{k+1} (cell units: off += dt/res v),
+            # kick v_{k+1} = v_k + dt G_k, gather G_k = sum W F
             g_F = torch.zeros(4 * lf2ctx.nsites, dtype=torch.float32, device=dev)
-            ops.gather_adj(cell_k, off_k, Fs[k], g_G, g_F, g_off)
+            ops.step_adj(cell_k, off_k, Fs[k], dt, g_v, g_off, g_F)
             g_rho = torch.zeros(lf2ctx.nsites, dtype=torch.float32, device=dev)
             if coupling is None:
                 ops.stencil_adj(rhos[k], S32, g_F, g_rho, g_S)

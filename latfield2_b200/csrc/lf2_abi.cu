@@ -381,11 +381,11 @@ lf2_status lf2_destroy(lf2_ctx* c)
   cudaFree(c->stats);
   cudaFree(c->mig);
   cudaFree(c->work);
-  cudaFree(c->flags);
-  cudaFree(c->vmax_bits);
   cudaFree(c->move_list);
   cudaFree(c->f_rows);
   cudaFree(c->move_mark);
+  cudaFree(c->flags);
+  cudaFree(c->vmax_bits);
   cudaFree(c->redep);
   cudaFree(c->repack);
   cudaFree(c->diag);
@@ -398,6 +398,7 @@ lf2_status lf2_destroy(lf2_ctx* c)
   cudaFree(c->part_head);
   cudaFree(c->part_mark);
   cudaFree(c->stencil_partial);
+  cudaFree(c->loss_part);
   cudaFree(c->pm_acc);
   fft_release(c);
   cudaFreeHost(c->h_stats);
@@ -1240,7 +1241,36 @@ lf2_status lf2_pm_step(lf2_ctx* c, int64_t np, int32_t* cell, float* off3, float
   if (!c || np < 0 || !F4 || !f4_ok(F4) || (np > 0 && (!cell || !off3 || !vel3))) return LF2_ERR_ARG;
   if (np == 0) return LF2_OK;
   PhaseScope ps(c, PH_OTHER);
-  LF2_CUDA(c, launch_pm_step(c, np, cell, off3, vel3, F4, (float)dt_kick, (float)(dt_drift / c->res)));
+  LF2_CUDA(c, launch_pm_step(c, np, cell, off3, vel3, F4, (float)dt_kick, (float)(dt_drift / c->res),
+                             cell, off3, vel3));
+  return LF2_OK;
+}
+
+lf2_status lf2_pm_step_to(lf2_ctx* c, int64_t np, const int32_t* cell, const float* off3,
+                          const float* vel3, const float* F4, double dt_kick, double dt_drift,
+                          int32_t* cell_out, float* off3_out, float* vel3_out)
+{
+  if (!c || np < 0 || !F4 || !f4_ok(F4) ||
+      (np > 0 && (!cell || !off3 || !vel3 || !cell_out || !off3_out || !vel3_out)))
+    return LF2_ERR_ARG;
+  if (np == 0) return LF2_OK;
+  PhaseScope ps(c, PH_OTHER);
+  LF2_CUDA(c, launch_pm_step(c, np, cell, off3, vel3, F4, (float)dt_kick, (float)(dt_drift / c->res),
+                             cell_out, off3_out, vel3_out));
+  return LF2_OK;
+}
+
+lf2_status lf2_pm_step_adjoint(lf2_ctx* c, int64_t np, const int32_t* cell, const float* off3,
+                               const float* F4, double dt_kick, double dt_drift, float* g_vel3,
+                               float* g_off3, float* g_F4)
+{
+  if (!c || np < 0 || !F4 || !f4_ok(F4) || !g_F4 || !f4_ok(g_F4) ||
+      (np > 0 && (!cell || !off3 || !g_vel3 || !g_off3)))
+    return LF2_ERR_ARG;
+  if (np == 0) return LF2_OK;
+  PhaseScope ps(c, PH_OTHER);
+  LF2_CUDA(c, launch_pm_step_adjoint(c, np, cell, off3, F4, g_vel3, g_off3, g_F4, (float)dt_kick,
+                                     (float)(dt_drift / c->res)));
   return LF2_OK;
 }
 
@@ -1251,6 +1281,31 @@ lf2_status lf2_pm_deposit_adjoint(lf2_ctx* c, int64_t np, const int32_t* cell, c
   if (!cell || !off3 || !g_rho) return LF2_ERR_ARG;
   return pm_call(c, 3, np, cell, off3, mass, gmass, g_rho, nullptr, g_off3, g_mass, 0, 0, nullptr,
                  nullptr, nullptr);
+}
+
+lf2_status lf2_pm_loss(lf2_ctx* c, const float* w, const float* rho, double* loss)
+{
+  if (!c || !w || !rho || !loss) return LF2_ERR_ARG;
+  PhaseScope ps(c, PH_OTHER);
+  if (!c->loss_part && cudaMalloc(&c->loss_part, sizeof(double) * loss_ctas(c)) != cudaSuccess) {
+    cudaGetLastError();
+    c->loss_part = nullptr;
+    return fail(c, LF2_ERR_NOMEM, "cannot allocate the loss's partial sums");
+  }
+  LF2_CUDA(c, launch_pm_loss(c, w, rho, loss));
+  return LF2_OK;
+}
+
+lf2_status lf2_pm_loss_adjoint(lf2_ctx* c, int64_t np, const int32_t* cell, const float* off3,
+                               const float* mass, const float* w, double g_loss, float* g_off3,
+                               float* g_mass, float* g_vel3)
+{
+  if (!c || np < 0 || !w || (np > 0 && (!cell || !off3 || !mass || !g_off3 || !g_mass || !g_vel3)))
+    return LF2_ERR_ARG;
+  if (np == 0) return LF2_OK;
+  PhaseScope ps(c, PH_OTHER);
+  LF2_CUDA(c, launch_pm_loss_adjoint(c, np, cell, off3, mass, w, (float)g_loss, g_off3, g_mass, g_vel3));
+  return LF2_OK;
 }
 
 lf2_status lf2_pm_gather_adjoint(lf2_ctx* c, int64_t np, const int32_t* cell, const float* off3,

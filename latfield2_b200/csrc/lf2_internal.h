@@ -99,6 +99,7 @@ struct lf2_ctx {
   uint32_t* vmax_bits = nullptr;     // device: largest |v_i| (float bits), fixed-point deposits
   uint32_t* redep = nullptr;         // device: the fused deposit must be redone by the tile pass
   float* stencil_partial = nullptr;  // per-CTA partial sums of the stencil weight gradient
+  double* loss_part = nullptr;       // partial sums of the chain's loss
   unsigned long long* pm_acc = nullptr; // chain's fixed-point deposit: [nsites] sums + max mass word
   size_t spill_slots = 0;
   // parts of heavy bricks (deposit tile passes, lf2_deposit_common.cuh)
@@ -178,8 +179,8 @@ cudaError_t launch_maxv_to_device(lf2_ctx* c, double* dst);
 // fixed-point scalar deposit fused in; its rim store is c->spill,
 // rim_store_slots(c) slots).  A kick needs move_pipe_eligible.
 bool move_pipe_eligible(const lf2_ctx* c, const float* F);
-bool move_dep_eligible(const lf2_ctx* c, const float* F);
 bool move_pipe_auto(lf2_ctx* c, const float* F);
+bool move_dep_eligible(const lf2_ctx* c, const float* F);
 size_t rim_store_slots(const lf2_ctx* c);
 cudaError_t launch_move_pipe(lf2_ctx* c, const float* F, bool kick, bool drift, MoveParams mp,
                              float* rho);
@@ -198,6 +199,8 @@ DepositParams deposit_params(const lf2_ctx* c);
 struct PartView;
 cudaError_t launch_part_plan(lf2_ctx* c, size_t smem, int threads, size_t tile_slots, int cap,
                              PartView* pv);
+// largest |v_i| of the store into c->vmax_bits (fixed-point momentum/stress)
+cudaError_t launch_vmax(lf2_ctx* c, const PartView& pv);
 
 // lf2_exchange.cu (slab decomposition): particles with cell z outside
 // [zlo, zhi] counted (below, above, more than one plane outside: 3 counters)
@@ -205,8 +208,6 @@ cudaError_t launch_part_plan(lf2_ctx* c, size_t smem, int threads, size_t tile_s
 cudaError_t launch_count_outside(lf2_ctx* c, int zlo, int zhi, unsigned long long* n,
                                  bool max_v = false);
 cudaError_t launch_extract_outside(lf2_ctx* c, int zlo, int zhi, int32_t* cell, float* off3,
-// largest |v_i| of the store into c->vmax_bits (fixed-point momentum/stress)
-cudaError_t launch_vmax(lf2_ctx* c, const PartView& pv);
                                    float* vel3, float* mass, int64_t* id,
                                    unsigned long long* out_count);
 cudaError_t launch_pack_movers(lf2_ctx* c, int64_t n, const int32_t* cell, const float* off3,
@@ -242,8 +243,17 @@ cudaError_t launch_pm_deposit(lf2_ctx* c, int64_t np, const int64_t* brick_start
 // the chain's particle state: sort keys and 32-byte records in the caller's
 // order, the state in a given order, the bricks' first slots; gradients back
 // to the caller's order through the same records
-cudaError_t launch_pm_step(lf2_ctx* c, int64_t np, int32_t* cell, float* off3, float* vel3,
-                           const float* F4, float dtk, float dtn);
+cudaError_t launch_pm_step(lf2_ctx* c, int64_t np, const int32_t* cell, const float* off3,
+                           const float* vel3, const float* F4, float dtk, float dtn, int32_t* cell_out,
+                           float* off_out, float* vel_out);
+cudaError_t launch_pm_step_adjoint(lf2_ctx* c, int64_t np, const int32_t* cell, const float* off3,
+                                   const float* F4, float* g_vel3, float* g_off3, float* gF4, float dtk,
+                                   float dtn);
+cudaError_t launch_pm_loss_adjoint(lf2_ctx* c, int64_t np, const int32_t* cell, const float* off3,
+                                   const float* mass, const float* w, float scale, float* g_off3,
+                                   float* g_mass, float* g_vel3);
+int loss_ctas(const lf2_ctx* c);
+cudaError_t launch_pm_loss(lf2_ctx* c, const float* w, const float* rho, double* loss);
 cudaError_t launch_pm_pack(lf2_ctx* c, int64_t np, const double* pos, const double* vel,
                            const double* mass, double inv_res, int32_t* key, void* rec);
 cudaError_t launch_pm_unpack(lf2_ctx* c, int64_t np, const int64_t* order, const void* rec,

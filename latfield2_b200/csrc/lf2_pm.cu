@@ -25,6 +25,8 @@
 // that a corner is one 16-byte load and one vector atomic.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "lf2_deposit_common.cuh"
 #include "lf2_internal.h"
 
@@ -42,7 +44,7 @@ inline int grid_for(int64_t n, int threads)
 }
 
 struct Corners {
-  int64_t site[8];
+  int32_t site[8];  // (a lattice has fewer than 2^31 sites)
   float w[8];
   float dw[8][3];
 };
@@ -50,7 +52,8 @@ struct Corners {
 __device__ __forceinline__ void corners(const Geom& g, int32_t c, const float* off3, int64_t p,
                                         Corners& k)
 {
-  const int x = c % g.n[0], y = (c / g.n[0]) % g.n[1], z = c / (g.n[0] * g.n[1]);
+  int x, y, z;
+  cell_xyz(g, c, x, y, z);
   const int xs[2] = {x, x + 1 < g.n[0] ? x + 1 : 0};
   const int ys[2] = {y, y + 1 < g.n[1] ? y + 1 : 0};
   const int zs[2] = {z, z + 1 < g.n[2] ? z + 1 : 0};
@@ -60,7 +63,7 @@ __device__ __forceinline__ void corners(const Geom& g, int32_t c, const float* o
   for (int q = 0; q < 8; q++) {
     const int bx = (q >> 2) & 1, by = (q >> 1) & 1, bz = q & 1;
     const float wx = bx ? f[0] : h[0], wy = by ? f[1] : h[1], wz = bz ? f[2] : h[2];
-    k.site[q] = site_index(g, xs[bx], ys[by], zs[bz]);
+    k.site[q] = (int32_t)site_index(g, xs[bx], ys[by], zs[bz]);
     k.w[q] = wx * wy * wz;
     k.dw[q][0] = (bx ? 1.0f : -1.0f) * wy * wz;
     k.dw[q][1] = (by ? 1.0f : -1.0f) * wx * wz;
@@ -91,11 +94,13 @@ __global__ void k_pm_deposit(Geom g, int64_t np, const int32_t* __restrict__ cel
 __global__ void k_pm_mass_max(int64_t np, const float* __restrict__ mass, uint32_t* mmax)
 {
   uint32_t m = 0u;
+#pragma unroll 8
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < np;
        p += (int64_t)gridDim.x * blockDim.x)
     m = max(m, __float_as_uint(fmaxf(mass[p], 0.0f)));  // non-negative floats order as integers
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m) atomicMax(mmax, m);
+  m = __reduce_max_sync(0xffffffffu, m);
+  // (most warps find the maximum there already: no queue at one address)
+  if ((threadIdx.x & 31) == 0 && m > *reinterpret_cast<volatile uint32_t*>(mmax)) atomicMax(mmax, m);
 }
 
 __global__ void k_pm_deposit_fixed(Geom g, int64_t np, const int32_t* __restrict__ cell,
@@ -106,7 +111,8 @@ __global__ void k_pm_deposit_fixed(Geom g, int64_t np, const int32_t* __restrict
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < np;
        p += (int64_t)gridDim.x * blockDim.x) {
     const int32_t c = cell[p];
-    const int x = c % g.n[0], y = (c / g.n[0]) % g.n[1], z = c / (g.n[0] * g.n[1]);
+    int x, y, z;
+    cell_xyz(g, c, x, y, z);
     const int xs[2] = {x, x + 1 < g.n[0] ? x + 1 : 0};
     const int ys[2] = {y, y + 1 < g.n[1] ? y + 1 : 0};
     const int zs[2] = {z, z + 1 < g.n[2] ? z + 1 : 0};
@@ -126,14 +132,23 @@ __global__ void k_pm_deposit_fixed(Geom g, int64_t np, const int32_t* __restrict
 // Brick-tiled forms of the two deposits, for particles grouped by brick
 // (brick_start[b] .. brick_start[b+1] hold the particles that were in brick
 // b when the chain sorted its state; a particle that has since drifted out
-// of the brick goes straight to the global sums).  One CTA per brick: its
-// particles add their corner weights into the brick's (BRICK+1)^3 vertex
-// tile in shared memory, then the tile's non-zero sums go to the global
-// field with one atomic each: 4913 global atomics per brick instead of 8 per
-// particle.  The fixed-point tile keeps a low word whose carry goes to a high
-// word (the order of the additions does not change the sums); the FP32 tile
-// adds floats, so its roundings depend on the order, as the global atomics'
-// do.
+// of the brick goes straight to the global sums).  A CTA adds its particles'
+// corner weights into the brick's (BRICK+1)^3 vertex tile in shared memory,
+// then the tile's non-zero sums go to the global field with one atomic each:
+// 4913 global atomics per tile instead of 8 per particle.  Both keep integer
+// sums, a low word whose carry goes to a high word: the fixed-point weights,
+// or the FP32 products in units of 2^-48 of the largest (add_comp_int; a
+// floating-point shared atomic is a compare-and-swap loop).  The CTA of a
+// brick takes its first `part` particles; what a brick holds beyond those is
+// shared out among CTAs by their slots, since each adds to the field on its
+// own (one CTA took 1.4 ms for a brick of 131k particles at 256^3).
+//
+// Particles sorted by cell put whole warps into dense cells, whose lanes
+// would add to the same words one after the other: a warp whose lanes lie in
+// at most DENSE_RUNS runs of one cell sums each run with warp reductions
+// first.
+constexpr int DENSE_RUNS = 3;
+
 __device__ __forceinline__ bool in_brick(int x, int y, int z, int x0, int y0, int z0)
 {
   return (unsigned)(x - x0) < (unsigned)BRICK && (unsigned)(y - y0) < (unsigned)BRICK &&
@@ -158,101 +173,168 @@ __device__ __forceinline__ int64_t tile_site(const Geom& g, int t, int x0, int y
   return site_index(g, x, y, z);
 }
 
-__global__ void __launch_bounds__(256)
-    k_pm_deposit_fixed_tile(Geom g, int64_t np, const int64_t* __restrict__ brick_start,
-                            const int32_t* __restrict__ cell, const float* __restrict__ off3,
-                            const float* __restrict__ mass, const uint32_t* __restrict__ mmax,
-                            unsigned long long* __restrict__ acc)
+// Brick of slot p: the last b with brick_start[b] <= p.
+__device__ __forceinline__ int64_t brick_of_slot(const int64_t* brick_start, int64_t nb, int64_t p)
 {
-  __shared__ uint32_t lo[TILE3], hi[TILE3];
-  for (int t = threadIdx.x; t < TILE3; t += blockDim.x) lo[t] = hi[t] = 0u;
-  __syncthreads();
-  const int64_t b = blockIdx.x;
-  int bx, by, bz;
-  brick_coords(g, b, bx, by, bz);
-  const int x0 = bx * BRICK, y0 = by * BRICK, z0 = bz * BRICK;
-  const float inv_m = mass ? 1.0f / __uint_as_float(*mmax) : 0.0f;
-  int64_t p0, p1;
-  group_range(brick_start, b, np, p0, p1);
-  for (int64_t p = p0 + threadIdx.x; p < p1; p += blockDim.x) {
-    const int32_t c = cell[p];
-    const int x = c % g.n[0], y = (c / g.n[0]) % g.n[1], z = c / (g.n[0] * g.n[1]);
-    const uint32_t ux = weight_q(off3[3 * p]), uy = weight_q(off3[3 * p + 1]), uz = weight_q(off3[3 * p + 2]);
-    const uint32_t qx[2] = {(1u << 31) - ux, ux}, qy[2] = {(1u << 31) - uy, uy}, qz[2] = {(1u << 31) - uz, uz};
-    const uint64_t mq = mass ? (uint64_t)__float2uint_rn(fminf(__fmul_rn(mass[p], inv_m), 1.0f) * 16777216.0f) : 0;
-    if (in_brick(x, y, z, x0, y0, z0)) {
-      const int t0 = (x - x0) + TILE * ((y - y0) + TILE * (z - z0));
-#pragma unroll
-      for (int q = 0; q < 8; q++) {
-        const int cx = (q >> 2) & 1, cy = (q >> 1) & 1, cz = q & 1;
-        uint64_t w = fixed_corner(qx[cx], qy[cy], qz[cz]);
-        if (mass) w = (w * mq + (1ull << 23)) >> 24;
-        const int t = t0 + cx + TILE * (cy + TILE * cz);
-        const uint32_t wl = (uint32_t)w;
-        const uint32_t old = atomicAdd(&lo[t], wl);
-        const uint32_t up = (uint32_t)(w >> 32) + ((uint32_t)(old + wl) < old ? 1u : 0u);
-        if (up) atomicAdd(&hi[t], up);
-      }
-    } else {  // drifted out of the brick since the sort
-      const int xs[2] = {x, x + 1 < g.n[0] ? x + 1 : 0};
-      const int ys[2] = {y, y + 1 < g.n[1] ? y + 1 : 0};
-      const int zs[2] = {z, z + 1 < g.n[2] ? z + 1 : 0};
-#pragma unroll
-      for (int q = 0; q < 8; q++) {
-        const int cx = (q >> 2) & 1, cy = (q >> 1) & 1, cz = q & 1;
-        uint64_t w = fixed_corner(qx[cx], qy[cy], qz[cz]);
-        if (mass) w = (w * mq + (1ull << 23)) >> 24;
-        atomicAdd(&acc[site_index(g, xs[cx], ys[cy], zs[cz])], (unsigned long long)w);
-      }
-    }
+  int64_t lo = 0, hi = nb - 1;
+  while (lo < hi) {
+    const int64_t mid = lo + ((hi - lo + 1) >> 1);
+    if (brick_start[mid] <= p) lo = mid;
+    else hi = mid - 1;
   }
-  __syncthreads();
-  for (int t = threadIdx.x; t < TILE3; t += blockDim.x) {
-    const unsigned long long v = ((unsigned long long)hi[t] << 32) | lo[t];
-    if (v) atomicAdd(&acc[tile_site(g, t, x0, y0, z0)], v);
-  }
+  return lo;
 }
 
-__global__ void __launch_bounds__(256)
-    k_pm_deposit_tile(Geom g, int64_t np, const int64_t* __restrict__ brick_start,
-                      const int32_t* __restrict__ cell, const float* __restrict__ off3,
-                      const float* __restrict__ mass, float gmass, float inv_vol,
-                      float* __restrict__ rho)
+// Adds the integer w (below 2^33, or any signed 64-bit value) of every lane
+// to the tile's words at t.
+__device__ __forceinline__ void tile_add(uint32_t* lo, uint32_t* hi, int t, long long w)
 {
-  __shared__ float tile[TILE3];
-  for (int t = threadIdx.x; t < TILE3; t += blockDim.x) tile[t] = 0.0f;
-  __syncthreads();
-  const int64_t b = blockIdx.x;
-  int bx, by, bz;
-  brick_coords(g, b, bx, by, bz);
-  const int x0 = bx * BRICK, y0 = by * BRICK, z0 = bz * BRICK;
-  int64_t p0, p1;
-  group_range(brick_start, b, np, p0, p1);
-  for (int64_t p = p0 + threadIdx.x; p < p1; p += blockDim.x) {
-    const int32_t c = cell[p];
-    const int x = c % g.n[0], y = (c / g.n[0]) % g.n[1], z = c / (g.n[0] * g.n[1]);
-    const float m = (mass ? mass[p] : gmass) * inv_vol;
-    if (in_brick(x, y, z, x0, y0, z0)) {
-      const float f[3] = {off3[3 * p], off3[3 * p + 1], off3[3 * p + 2]};
-      const float h[3] = {1.0f - f[0], 1.0f - f[1], 1.0f - f[2]};
-      const int t0 = (x - x0) + TILE * ((y - y0) + TILE * (z - z0));
-#pragma unroll
-      for (int q = 0; q < 8; q++) {
-        const int cx = (q >> 2) & 1, cy = (q >> 1) & 1, cz = q & 1;
-        const float w = (cx ? f[0] : h[0]) * (cy ? f[1] : h[1]) * (cz ? f[2] : h[2]);
-        atomicAdd(&tile[t0 + cx + TILE * (cy + TILE * cz)], w * m);
-      }
-    } else {  // drifted out of the brick since the sort
-      Corners k;
-      corners(g, c, off3, p, k);
-#pragma unroll
-      for (int q = 0; q < 8; q++) atomicAdd(&rho[k.site[q]], k.w[q] * m);
+  const uint32_t wl = (uint32_t)(unsigned long long)w;
+  const uint32_t old = atomicAdd(&lo[t], wl);
+  const int up = (int)(w >> 32) + ((uint32_t)(old + wl) < old ? 1 : 0);
+  if (up) atomicAdd(reinterpret_cast<int*>(&hi[t]), up);
+}
+
+// FIXED: acc += integer weights (times the masses relative to *mmax);
+// otherwise rho += FP32 products.  CTA u < nbricks: brick u's first `part`
+// particles; CTA nbricks + r: what the slots [r part, (r + 1) part) hold of
+// bricks beyond their first `part` particles (at most two such bricks reach a
+// range of that length: those at its ends).
+template <bool FIXED>
+__global__ void __launch_bounds__(256)
+    k_pm_deposit_tile(Geom g, int64_t np, const int64_t* __restrict__ brick_start, int part,
+                      const int32_t* __restrict__ cell, const float* __restrict__ off3,
+                      const float* __restrict__ mass, const uint32_t* __restrict__ mmax, float gmass,
+                      float inv_vol, unsigned long long* __restrict__ acc, float* __restrict__ rho)
+{
+  __shared__ uint32_t lo[TILE3], hi[TILE3];
+  __shared__ unsigned s_max[2];
+  const float inv_m = FIXED && mass ? 1.0f / __uint_as_float(*mmax) : 0.0f;
+  const int lane = threadIdx.x & 31;
+  for (int half = 0; half < 2; half++) {
+    int64_t b, p0, p1;
+    if (blockIdx.x < g.nbricks) {
+      if (half) return;
+      b = blockIdx.x;
+      group_range(brick_start, b, np, p0, p1);
+      p1 = min(p1, p0 + part);
+    } else {
+      const int64_t r0 = ((int64_t)blockIdx.x - g.nbricks) * part, r1 = min(r0 + part, np);
+      b = brick_of_slot(brick_start, g.nbricks, half ? r1 - 1 : r0);
+      if (half && brick_start[b] <= r0) return;  // the same brick as at the other end
+      group_range(brick_start, b, np, p0, p1);
+      p0 = max(p0 + part, r0);
+      p1 = min(p1, r1);
+      if (p0 >= p1) continue;
     }
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < TILE3; t += blockDim.x) {
-    const float v = tile[t];
-    if (v != 0.0f) atomicAdd(&rho[tile_site(g, t, x0, y0, z0)], v);
+    if (half) __syncthreads();  // the tile before is flushed
+    for (int t = threadIdx.x; t < TILE3; t += blockDim.x) lo[t] = hi[t] = 0u;
+    CompUnit cu{0, true};
+    if (!FIXED)  // (slots may exceed 32 bits)
+      cu = comp_unit<0>(mass ? mass + p0 : nullptr, inv_vol, gmass * inv_vol, nullptr, nullptr, nullptr,
+                        0u, (int)(p1 - p0), s_max);
+    const float unit = !FIXED && cu.ok ? ldexpf(1.0f, 16 - cu.e) : 1.0f;
+    __syncthreads();
+    int bx, by, bz;
+    brick_coords(g, b, bx, by, bz);
+    const int x0 = bx * BRICK, y0 = by * BRICK, z0 = bz * BRICK;
+    // the next trip's particle is read while this one's is added
+    int32_t c_next = 0;
+    float f_next[3] = {0.f, 0.f, 0.f}, m_next = gmass;
+    auto fetch = [&](int64_t p) {
+      if (p >= p1) return;
+      c_next = cell[p];
+      f_next[0] = off3[3 * p], f_next[1] = off3[3 * p + 1], f_next[2] = off3[3 * p + 2];
+      if (mass) m_next = mass[p];
+    };
+    fetch(p0 + threadIdx.x);
+    for (int64_t q0 = p0; q0 < p1; q0 += blockDim.x) {
+      const int64_t p = q0 + threadIdx.x;
+      const bool on = p < p1;
+      int x, y, z;
+      cell_xyz(g, c_next, x, y, z);
+      const float f[3] = {f_next[0], f_next[1], f_next[2]};
+      float m = m_next;
+      fetch(p + blockDim.x);
+      uint32_t qx[2], qy[2], qz[2];
+      uint64_t mq = 0;
+      if (FIXED) {
+        qx[1] = weight_q(f[0]), qy[1] = weight_q(f[1]), qz[1] = weight_q(f[2]);
+        qx[0] = (1u << 31) - qx[1], qy[0] = (1u << 31) - qy[1], qz[0] = (1u << 31) - qz[1];
+        if (mass) mq = (uint64_t)__float2uint_rn(fminf(__fmul_rn(m, inv_m), 1.0f) * 16777216.0f);
+      } else {
+        m *= inv_vol;
+      }
+      // corner q's integer contribution
+      auto weight = [&](int q) -> long long {
+        const int cx = (q >> 2) & 1, cy = (q >> 1) & 1, cz = q & 1;
+        if (FIXED) {
+          uint64_t w = fixed_corner(qx[cx], qy[cy], qz[cz]);
+          if (mass) w = (w * mq + (1ull << 23)) >> 24;
+          return (long long)w;
+        }
+        const float w = (cx ? f[0] : 1.0f - f[0]) * (cy ? f[1] : 1.0f - f[1]) * (cz ? f[2] : 1.0f - f[2]);
+        const float v = w * (m * unit);  // |v| < 2^16
+        const float h = __fadd_rn(v, 12582912.0f);
+        const float r = __fsub_rn(v, __fsub_rn(h, 12582912.0f));
+        return ((long long)(__float_as_int(h) - 0x4B400000) << 32) +
+               (long long)__float2int_rn(__fmul_rn(r, 4294967296.0f));
+      };
+      const bool tiled = on && cu.ok && in_brick(x, y, z, x0, y0, z0);
+      const int t0 = (x - x0) + TILE * ((y - y0) + TILE * (z - z0));
+      // runs of lanes in one cell
+      const int key = tiled ? t0 : -1 - lane;
+      const int before = __shfl_up_sync(0xffffffffu, key, 1);
+      const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || key != before);
+      if (__popc(heads) <= DENSE_RUNS) {
+        for (unsigned rest = heads; rest; rest &= rest - 1) {
+          const int first = __ffs(rest) - 1, next = __ffs(rest & (rest - 1));
+          const bool mine = lane >= first && (next == 0 || lane < next - 1);
+          const int t = __shfl_sync(0xffffffffu, key, first);
+          if (t < 0) continue;  // a lane that is not in the tile: below
+#pragma unroll
+          for (int q = 0; q < 8; q++) {
+            const long long w = mine ? weight(q) : 0ll;
+            // 32 values below 2^48: the sums of 20-bit pieces stay below 2^31
+            const long long sum =
+                (long long)__reduce_add_sync(0xffffffffu, (unsigned)(w & 0xfffff)) +
+                ((long long)__reduce_add_sync(0xffffffffu, (unsigned)((w >> 20) & 0xfffff)) << 20) +
+                ((long long)__reduce_add_sync(0xffffffffu, (int)(w >> 40)) << 40);
+            if (lane == q)
+              tile_add(lo, hi, t + ((q >> 2) & 1) + TILE * (((q >> 1) & 1) + TILE * (q & 1)), sum);
+          }
+        }
+      } else if (tiled) {
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+          tile_add(lo, hi, t0 + ((q >> 2) & 1) + TILE * (((q >> 1) & 1) + TILE * (q & 1)), weight(q));
+      }
+      if (on && !tiled) {  // drifted out of the brick since the sort, or no common unit
+        const int xs[2] = {x, x + 1 < g.n[0] ? x + 1 : 0};
+        const int ys[2] = {y, y + 1 < g.n[1] ? y + 1 : 0};
+        const int zs[2] = {z, z + 1 < g.n[2] ? z + 1 : 0};
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+          const int cx = (q >> 2) & 1, cy = (q >> 1) & 1, cz = q & 1;
+          const int64_t site = site_index(g, xs[cx], ys[cy], zs[cz]);
+          if (FIXED) {
+            atomicAdd(&acc[site], (unsigned long long)weight(q));
+          } else {
+            const float w = (cx ? f[0] : 1.0f - f[0]) * (cy ? f[1] : 1.0f - f[1]) * (cz ? f[2] : 1.0f - f[2]);
+            atomicAdd(&rho[site], w * m);
+          }
+        }
+      }
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < TILE3; t += blockDim.x) {
+      const unsigned long long v = ((unsigned long long)hi[t] << 32) | lo[t];
+      if (!v) continue;
+      if (FIXED)
+        atomicAdd(&acc[tile_site(g, t, x0, y0, z0)], v);
+      else
+        atomicAdd(&rho[tile_site(g, t, x0, y0, z0)], ldexpf(__ll2float_rn((long long)v), cu.e - 48));
+    }
   }
 }
 
@@ -300,7 +382,8 @@ __global__ void k_pm_kick_drift(Geom g, int64_t np, int32_t* __restrict__ cell, 
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < np;
        p += (int64_t)gridDim.x * blockDim.x) {
     const int32_t c = cell[p];
-    int xyz[3] = {c % g.n[0], (c / g.n[0]) % g.n[1], c / (g.n[0] * g.n[1])};
+    int xyz[3];
+    cell_xyz(g, c, xyz[0], xyz[1], xyz[2]);
     for (int d = 0; d < 3; d++) {
       float v = vel3[3 * p + d];
       if (G3) v = __fmaf_rn(dtk, G3[3 * p + d], v);
@@ -326,17 +409,20 @@ __global__ void k_pm_kick_drift(Geom g, int64_t np, int32_t* __restrict__ cell, 
 
 // The gather, the kick and the drift of one chain step in one pass, with
 // the arithmetic of k_pm_gather and k_pm_kick_drift (the same results bit
-// for bit) and no gathered field written in between.
-__global__ void k_pm_gather_kick_drift(Geom g, int64_t np, int32_t* __restrict__ cell,
-                                       float* __restrict__ off3, float* __restrict__ vel3,
-                                       const float4* __restrict__ F4, float dtk, float dtn,
+// for bit) and no gathered field written in between.  The new state may go
+// to other arrays, so that the old one stays as a checkpoint without a copy.
+__global__ void k_pm_gather_kick_drift(Geom g, int64_t np, const int32_t* cell, const float* off3,
+                                       const float* vel3, const float4* __restrict__ F4, float dtk,
+                                       float dtn, int32_t* cell_out, float* off_out, float* vel_out,
                                        uint32_t* flags)
 {
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < np;
        p += (int64_t)gridDim.x * blockDim.x) {
     const int32_t c = cell[p];
+    const float o3[3] = {off3[3 * p], off3[3 * p + 1], off3[3 * p + 2]};
+    const float v3[3] = {vel3[3 * p], vel3[3 * p + 1], vel3[3 * p + 2]};
     Corners k;
-    corners(g, c, off3, p, k);
+    corners(g, c, o3, 0, k);
     float a[3] = {0.f, 0.f, 0.f};
 #pragma unroll
     for (int q = 0; q < 8; q++) {
@@ -345,13 +431,16 @@ __global__ void k_pm_gather_kick_drift(Geom g, int64_t np, int32_t* __restrict__
       a[1] = fmaf(k.w[q], f.y, a[1]);
       a[2] = fmaf(k.w[q], f.z, a[2]);
     }
-    int xyz[3] = {c % g.n[0], (c / g.n[0]) % g.n[1], c / (g.n[0] * g.n[1])};
+    int xyz[3];
+    cell_xyz(g, c, xyz[0], xyz[1], xyz[2]);
+#pragma unroll
     for (int d = 0; d < 3; d++) {
-      float v = __fmaf_rn(dtk, a[d], vel3[3 * p + d]);
-      vel3[3 * p + d] = v;
-      float o = __fmaf_rn(dtn, v, off3[3 * p + d]);
+      const float v = __fmaf_rn(dtk, a[d], v3[d]);
+      vel_out[3 * p + d] = v;
+      float o = __fmaf_rn(dtn, v, o3[d]);
       if (!isfinite(o)) {
         set_flag(flags, ERR_NONFINITE);
+        off_out[3 * p + d] = o3[d];
         continue;
       }
       const float fl = floorf(o);
@@ -361,17 +450,22 @@ __global__ void k_pm_gather_kick_drift(Geom g, int64_t np, int32_t* __restrict__
         o = 0.0f;
         carry += 1;
       }
-      off3[3 * p + d] = o;
+      off_out[3 * p + d] = o;
       xyz[d] = wrap_add(xyz[d], carry, g.n[d]);
     }
-    cell[p] = (int32_t)site_index(g, xyz[0], xyz[1], xyz[2]);
+    cell_out[p] = (int32_t)site_index(g, xyz[0], xyz[1], xyz[2]);
   }
 }
 
+// FIRST: the adjoint of the loss, the first of a backward pass: g_rho is the
+// loss weights, scaled by `scale`, and the gradients are written (g_vel3
+// zero) instead of added to.
+template <bool FIRST>
 __global__ void k_pm_deposit_adj(Geom g, int64_t np, const int32_t* __restrict__ cell,
                                  const float* __restrict__ off3, const float* __restrict__ mass,
-                                 float gmass, float inv_vol, const float* __restrict__ g_rho,
-                                 float* __restrict__ g_off3, float* __restrict__ g_mass)
+                                 float gmass, float inv_vol, const float* __restrict__ g_rho, float scale,
+                                 float* __restrict__ g_off3, float* __restrict__ g_mass,
+                                 float* __restrict__ g_vel3)
 {
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < np;
        p += (int64_t)gridDim.x * blockDim.x) {
@@ -380,39 +474,154 @@ __global__ void k_pm_deposit_adj(Geom g, int64_t np, const int32_t* __restrict__
     float s = 0.f, d[3] = {0.f, 0.f, 0.f};
 #pragma unroll
     for (int q = 0; q < 8; q++) {
-      const float gr = __ldg(g_rho + k.site[q]);
+      float gr = __ldg(g_rho + k.site[q]);
+      if (FIRST) gr = __fmul_rn(gr, scale);
       s = fmaf(k.w[q], gr, s);
       for (int c = 0; c < 3; c++) d[c] = fmaf(k.dw[q][c], gr, d[c]);
     }
     const float m = (mass ? mass[p] : gmass) * inv_vol;
-    if (g_mass) g_mass[p] += s * inv_vol;
+    if (g_mass) g_mass[p] = FIRST ? s * inv_vol : g_mass[p] + s * inv_vol;
     if (g_off3)
-      for (int c = 0; c < 3; c++) g_off3[3 * p + c] += m * d[c];
+      for (int c = 0; c < 3; c++) g_off3[3 * p + c] = FIRST ? m * d[c] : g_off3[3 * p + c] + m * d[c];
+    if (FIRST)
+      for (int c = 0; c < 3; c++) g_vel3[3 * p + c] = 0.0f;
   }
 }
 
-__global__ void k_pm_gather_adj(Geom g, int64_t np, const int32_t* __restrict__ cell,
-                                const float* __restrict__ off3, const float4* __restrict__ F4,
-                                const float* __restrict__ gG3, float4* __restrict__ gF4,
-                                float* __restrict__ g_off3)
+// sum_i w[i] rho[i] in FP64, in a fixed order: a partial sum per CTA, then
+// one CTA.
+constexpr int LOSS_THREADS = 256;
+
+__device__ __forceinline__ double block_sum(double v, double* sh)
 {
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < np;
-       p += (int64_t)gridDim.x * blockDim.x) {
-    Corners k;
-    corners(g, cell[p], off3, p, k);
-    const float gg[3] = {gG3[3 * p], gG3[3 * p + 1], gG3[3 * p + 2]};
-    float d[3] = {0.f, 0.f, 0.f};
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = 0.0;
+  if (threadIdx.x == 0)
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++) v += sh[w];
+  return v;
+}
+
+__global__ void __launch_bounds__(LOSS_THREADS) k_pm_loss(int64_t n, const float* __restrict__ w,
+                                                          const float* __restrict__ rho, double* partial)
+{
+  __shared__ double sh[LOSS_THREADS / 32];
+  double v = 0.0;
+#pragma unroll 4
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    v = fma((double)__ldg(w + i), (double)__ldg(rho + i), v);
+  v = block_sum(v, sh);
+  if (threadIdx.x == 0) partial[blockIdx.x] = v;
+}
+
+__global__ void __launch_bounds__(LOSS_THREADS) k_pm_loss_sum(int n, const double* __restrict__ partial,
+                                                              double* loss)
+{
+  __shared__ double sh[LOSS_THREADS / 32];
+  double v = 0.0;
+  for (int i = threadIdx.x; i < n; i += LOSS_THREADS) v += partial[i];
+  v = block_sum(v, sh);
+  if (threadIdx.x == 0) *loss = v;
+}
+
+// Sum over the lanes of a warp of 24 values each: lane l < 24 returns the sum
+// of value l (recursive halving: 31 exchanges for up to 32 values).
+__device__ __forceinline__ float reduce24(float (&v)[32])
+{
+  const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int q = 0; q < 8; q++) {
-      if (gF4) atomicAdd(&gF4[k.site[q]], make_float4(k.w[q] * gg[0], k.w[q] * gg[1], k.w[q] * gg[2], 0.f));
-      if (g_off3) {
-        const float4 f = __ldg(F4 + k.site[q]);
-        const float dot = fmaf(gg[0], f.x, fmaf(gg[1], f.y, gg[2] * f.z));
-        for (int c = 0; c < 3; c++) d[c] = fmaf(k.dw[q][c], dot, d[c]);
+  for (int h = 16; h > 0; h >>= 1) {
+    const bool upper = lane & h;
+#pragma unroll
+    for (int i = 0; i < h; i++) {
+      const float give = upper ? v[i] : v[i + h], keep = upper ? v[i + h] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+    }
+  }
+  return v[0];
+}
+
+// Gather adjoint.  STEP: with the adjoint of the drift and the kick before it
+// (g_vel += dtn g_off, then the gradient of the gathered force is dtk g_vel),
+// otherwise that gradient is given (gG3).  Bound by the vector atomics on the
+// gradient field; the particles come sorted by cell, so a warp in a dense
+// region adds to a few vertices only: where its lanes lie in at most
+// DENSE_RUNS runs of one cell, each run's 24 sums are formed in the warp and
+// added once (at one particle per cell the same costs more than the atomics
+// it saves).
+template <bool STEP>
+__global__ void __launch_bounds__(PM_THREADS)
+    k_pm_gather_adj(Geom g, int64_t np, const int32_t* __restrict__ cell, const float* __restrict__ off3,
+                    const float4* __restrict__ F4, const float* __restrict__ gG3, float4* __restrict__ gF4,
+                    float* __restrict__ g_off3, float* __restrict__ g_vel3, float dtk, float dtn)
+{
+  const int lane = threadIdx.x & 31;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t p0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); p0 < np; p0 += stride) {
+    const int64_t p = min(p0 + lane, np - 1);
+    const bool on = p0 + lane < np;
+    Corners k;
+    const int32_t c = cell[p];
+    corners(g, c, off3, p, k);
+    float gg[3], go[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      if (STEP || g_off3) go[d] = g_off3[3 * p + d];
+      if (STEP) {
+        const float gv = __fadd_rn(g_vel3[3 * p + d], __fmul_rn(dtn, go[d]));
+        if (on) g_vel3[3 * p + d] = gv;
+        gg[d] = __fmul_rn(dtk, gv);
+      } else {
+        gg[d] = gG3[3 * p + d];
       }
     }
-    if (g_off3)
-      for (int c = 0; c < 3; c++) g_off3[3 * p + c] += d[c];
+    if (gF4) {
+      const int key = on ? c : -1;
+      const int before = __shfl_up_sync(0xffffffffu, key, 1);
+      const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || key != before);
+      if (__popc(heads) <= DENSE_RUNS) {
+        for (unsigned rest = heads; rest; rest &= rest - 1) {
+          const int first = __ffs(rest) - 1, next = __ffs(rest & (rest - 1));
+          const bool mine = on && lane >= first && (next == 0 || lane < next - 1);
+          float v[32];
+#pragma unroll
+          for (int q = 0; q < 8; q++) {
+            v[q] = mine ? k.w[q] * gg[0] : 0.f;
+            v[8 + q] = mine ? k.w[q] * gg[1] : 0.f;
+            v[16 + q] = mine ? k.w[q] * gg[2] : 0.f;
+            v[24 + q] = 0.f;
+          }
+          const float sum = reduce24(v);
+          const float sy = __shfl_down_sync(0xffffffffu, sum, 8), sz = __shfl_down_sync(0xffffffffu, sum, 16);
+          // the run's sites: corner q of its first lane
+          int32_t site = 0;
+#pragma unroll
+          for (int q = 0; q < 8; q++) {
+            const int32_t s = __shfl_sync(0xffffffffu, k.site[q], first);
+            if (lane == q) site = s;
+          }
+          if (lane < 8 && p0 + first < np)
+            atomicAdd(&gF4[site], make_float4(sum, sy, sz, 0.f));
+        }
+      } else if (on) {
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+          atomicAdd(&gF4[k.site[q]], make_float4(k.w[q] * gg[0], k.w[q] * gg[1], k.w[q] * gg[2], 0.f));
+      }
+    }
+    if (g_off3 && on) {
+      float d[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const float4 f = __ldg(F4 + k.site[q]);
+        const float dot = fmaf(gg[0], f.x, fmaf(gg[1], f.y, gg[2] * f.z));
+#pragma unroll
+        for (int i = 0; i < 3; i++) d[i] = fmaf(k.dw[q][i], dot, d[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < 3; i++) g_off3[3 * p + i] = go[i] + d[i];
+    }
   }
 }
 
@@ -434,118 +643,187 @@ __device__ inline Tile tile_of()
           (int)threadIdx.x / SX};
 }
 
-// halo site t of the tile (t < HX*HY*HZ) -> periodic global site index
-__device__ inline int64_t halo_site(const Geom& g, const Tile& T, int t)
+// The tile's input with its halo, one warp per row of HX sites; `put` takes
+// halo index and global site.  The wrapped coordinates are laid down once
+// (`w`), and the loop over a warp's rows is unrolled, so that their loads are
+// in flight together.
+constexpr int HALO_WRAP = HX + HY + HZ;
+
+template <typename Put>
+__device__ __forceinline__ void halo_rows(const Geom& g, int x0, int y0, int z0, int32_t* w, Put put)
 {
-  const int i = t % HX, j = (t / HX) % HY, k = t / (HX * HY);
-  return site_index(g, wrap_add(T.x0, i - 1, g.n[0]), wrap_add(T.y0, j - 1, g.n[1]),
-                    wrap_add(T.z0, k - 1, g.n[2]));
+  const int t = threadIdx.x, lane = t & 31;
+  if (t < HX) w[t] = wrap_add(x0, t - 1, g.n[0]);
+  else if (t < HX + HY) w[t] = g.n[0] * wrap_add(y0, t - HX - 1, g.n[1]);
+  else if (t < HALO_WRAP) w[t] = g.n[0] * g.n[1] * wrap_add(z0, t - HX - HY - 1, g.n[2]);
+  __syncthreads();
+  const int xa = w[lane], xb = w[32 + (lane < HX - 32 ? lane : 0)];
+#pragma unroll
+  for (int it = 0; it < (HY * HZ + STENCIL_THREADS / 32 - 1) / (STENCIL_THREADS / 32); it++) {
+    const int row = (t >> 5) + it * (STENCIL_THREADS / 32);
+    if (row < HY * HZ) {
+      const int base = w[HX + row % HY] + w[HX + HY + row / HY];  // (fewer than 2^31 sites)
+      put(row * HX + lane, base + xa);
+      if (lane < HX - 32) put(row * HX + 32 + lane, base + xb);
+    }
+  }
+}
+
+// The three stencil kernels are bound by issue: 81 multiply-adds per site and
+// the loads of their operands.  A thread keeps the 81 weights (or sums) in
+// registers and walks its z column plane by plane: the 9 values of a plane
+// serve the three sites whose stencils touch it, so that a site costs 9
+// shared loads per input component instead of 27, and no weight is read again.
+
+// The weights into registers, by way of shared memory.  (Volatile loads: an
+// ordinary one would be repeated for every plane to save registers.)
+__device__ __forceinline__ void weights_to_registers(const float* S, float* sh, float (&s)[81])
+{
+  if (threadIdx.x < 81) sh[threadIdx.x] = __ldg(S + threadIdx.x);
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 81; q++) s[q] = reinterpret_cast<volatile float*>(sh)[q];
 }
 
 // F_c(g) = sum_o S[c][o] rho(g + o); o = (dz, dy, dx) in {-1,0,1}^3,
-// S index c*27 + (dz+1)*9 + (dy+1)*3 + (dx+1).
+// S index c*27 + (dz+1)*9 + (dy+1)*3 + (dx+1), added in ascending o.
 __global__ void __launch_bounds__(STENCIL_THREADS) k_stencil(Geom g, const float* __restrict__ rho,
                                                              const float* __restrict__ S,
                                                              float4* __restrict__ F4)
 {
-  __shared__ float s[81];
-  __shared__ float r[HZ][HY][HX];
+  __shared__ float r[HZ * HY * HX];
+  __shared__ int32_t wrap[HALO_WRAP];
   const Tile T = tile_of();
-  if (threadIdx.x < 81) s[threadIdx.x] = S[threadIdx.x];
-  for (int t = threadIdx.x; t < HX * HY * HZ; t += STENCIL_THREADS)
-    (&r[0][0][0])[t] = __ldg(rho + halo_site(g, T, t));
+  __shared__ float sh[81];
+  float s[81];
+  weights_to_registers(S, sh, s);
+  halo_rows(g, T.x0, T.y0, T.z0, wrap, [&](int t, int site) { r[t] = __ldg(rho + site); });
   __syncthreads();
   const int x = T.x0 + T.tx, y = T.y0 + T.ty;
   if (x >= g.n[0] || y >= g.n[1]) return;
-  for (int kz = 0; kz < SZ && T.z0 + kz < g.n[2]; kz++) {
-    float a[3] = {0.f, 0.f, 0.f};
+  // a[m]: the site one plane below (m = 0), at, or above the plane read
+  float a[3][3] = {};
+  const int64_t plane = (int64_t)g.n[0] * g.n[1];
+  int64_t site = site_index(g, x, y, T.z0) - plane;
 #pragma unroll
-    for (int o = 0; o < 27; o++) {
-      const float v = r[kz + o / 9][T.ty + (o / 3) % 3][T.tx + o % 3];
+  for (int k = 0; k < HZ; k++) {
+    float v[9];
 #pragma unroll
-      for (int c = 0; c < 3; c++) a[c] = fmaf(s[c * 27 + o], v, a[c]);
-    }
-    F4[site_index(g, x, y, T.z0 + kz)] = make_float4(a[0], a[1], a[2], 0.f);
+    for (int o = 0; o < 9; o++) v[o] = r[(k * HY + T.ty + o / 3) * HX + T.tx + o % 3];
+#pragma unroll
+    for (int m = 0; m < 3; m++)  // the site's plane k sits at dz = 1 - m
+#pragma unroll
+      for (int o = 0; o < 9; o++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) a[m][c] = fmaf(s[c * 27 + (2 - m) * 9 + o], v[o], a[m][c]);
+    if (k >= 2 && T.z0 + k - 2 < g.n[2])
+      F4[site] = make_float4(a[0][0], a[0][1], a[0][2], 0.f);
+    if (k >= 1) site += plane;
+#pragma unroll
+    for (int c = 0; c < 3; c++) a[0][c] = a[1][c], a[1][c] = a[2][c], a[2][c] = 0.f;
   }
 }
 
-// gR(h) = sum_c sum_o S[c][o] gF_c(h - o)
+// gR(h) = sum_c sum_o S[c][o] gF_c(h - o), added in ascending o: the planes
+// from the top of the column down.
 __global__ void __launch_bounds__(STENCIL_THREADS) k_stencil_adj_rho(Geom g,
                                                                      const float4* __restrict__ gF4,
                                                                      const float* __restrict__ S,
                                                                      float* __restrict__ g_rho)
 {
-  __shared__ float s[81];
-  __shared__ float f[3][HZ][HY][HX];
+  __shared__ float f[3][HZ * HY * HX];
+  __shared__ int32_t wrap[HALO_WRAP];
   const Tile T = tile_of();
-  if (threadIdx.x < 81) s[threadIdx.x] = S[threadIdx.x];
-  for (int t = threadIdx.x; t < HX * HY * HZ; t += STENCIL_THREADS) {
-    const float4 v = __ldg(gF4 + halo_site(g, T, t));
-    (&f[0][0][0][0])[t] = v.x;
-    (&f[1][0][0][0])[t] = v.y;
-    (&f[2][0][0][0])[t] = v.z;
-  }
+  __shared__ float sh[81];
+  float s[81];
+  weights_to_registers(S, sh, s);
+  halo_rows(g, T.x0, T.y0, T.z0, wrap, [&](int t, int site) {
+    const float4 v = __ldg(gF4 + site);
+    f[0][t] = v.x;
+    f[1][t] = v.y;
+    f[2][t] = v.z;
+  });
   __syncthreads();
   const int x = T.x0 + T.tx, y = T.y0 + T.ty;
   if (x >= g.n[0] || y >= g.n[1]) return;
-  for (int kz = 0; kz < SZ && T.z0 + kz < g.n[2]; kz++) {
-    float a = 0.f;
+  float a[3] = {};  // the site above, at, or below the plane read
+  const int64_t plane = (int64_t)g.n[0] * g.n[1];
 #pragma unroll
-    for (int o = 0; o < 27; o++) {
-      // h - o for o = (dz, dy, dx): halo offset (1 - d) per axis
-      const int k = kz + 2 - o / 9, j = T.ty + 2 - (o / 3) % 3, i = T.tx + 2 - o % 3;
+  for (int k = HZ - 1; k >= 0; k--) {
 #pragma unroll
-      for (int c = 0; c < 3; c++) a = fmaf(s[c * 27 + o], f[c][k][j][i], a);
+    for (int o = 0; o < 9; o++) {
+      // h - o: halo offset (1 - d) per axis
+      const int t = (k * HY + T.ty + 2 - o / 3) * HX + T.tx + 2 - o % 3;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const float v = f[c][t];
+        // plane k is h - dz with dz = -1 for the site below it, 0, 1
+        a[2] = fmaf(s[c * 27 + o], v, a[2]);
+        a[1] = fmaf(s[c * 27 + 9 + o], v, a[1]);
+        a[0] = fmaf(s[c * 27 + 18 + o], v, a[0]);
+      }
     }
-    g_rho[site_index(g, x, y, T.z0 + kz)] += a;
+    const int z = T.z0 + k;  // the site above plane k is complete
+    if (k < SZ && z < g.n[2]) g_rho[site_index(g, x, y, T.z0) + plane * k] += a[0];
+    a[0] = a[1], a[1] = a[2], a[2] = 0.f;
   }
 }
 
-// gS[c][o] = sum_g gF_c(g) rho(g + o).  Every thread keeps the 81 sums of
-// its z-column in registers; the warps reduce them with shuffles, the CTA
-// adds its 8 warps in order and writes one row of `partial` per tile;
-// k_stencil_adj_S_sum adds the rows in a fixed order.
-__global__ void __launch_bounds__(STENCIL_THREADS) k_stencil_adj_S(Geom g,
-                                                                   const float4* __restrict__ gF4,
-                                                                   const float* __restrict__ rho,
-                                                                   float* __restrict__ partial)
+// gS[c][o] = sum_g gF_c(g) rho(g + o).  A CTA takes one component c
+// (blockIdx.y); every thread keeps its 27 sums in registers over the z-columns
+// of the CTA's tiles (a few CTAs per SM); the warps then reduce them with
+// shuffles, the CTA adds its 8 warps in order and writes its third of a row
+// of `partial`; k_stencil_adj_S_sum adds the rows in a fixed order.  (All 81
+// sums in one thread leave 16 warps per SM: no faster than one tile per CTA.)
+__global__ void __launch_bounds__(STENCIL_THREADS, 3) k_stencil_adj_S(Geom g, int ntx, int nty, int ntiles,
+                                                                      const float4* __restrict__ gF4,
+                                                                      const float* __restrict__ rho,
+                                                                      float* __restrict__ partial)
 {
-  __shared__ float r[HZ][HY][HX];
-  __shared__ float red[STENCIL_THREADS / 32][81];
-  const Tile T = tile_of();
-  for (int t = threadIdx.x; t < HX * HY * HZ; t += STENCIL_THREADS)
-    (&r[0][0][0])[t] = __ldg(rho + halo_site(g, T, t));
-  __syncthreads();
-  float acc[81];
+  __shared__ float r[HZ * HY * HX];
+  __shared__ int32_t wrap[HALO_WRAP];
+  __shared__ float red[STENCIL_THREADS / 32][27];
+  const int tx = threadIdx.x % SX, ty = threadIdx.x / SX;
+  const float* gF = reinterpret_cast<const float*>(gF4) + blockIdx.y;
+  float acc[27];
 #pragma unroll
-  for (int q = 0; q < 81; q++) acc[q] = 0.f;
-  const int x = T.x0 + T.tx, y = T.y0 + T.ty;
-  if (x < g.n[0] && y < g.n[1]) {
-    for (int kz = 0; kz < SZ && T.z0 + kz < g.n[2]; kz++) {
-      const float4 q = __ldg(gF4 + site_index(g, x, y, T.z0 + kz));
+  for (int q = 0; q < 27; q++) acc[q] = 0.f;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int x0 = (tile % ntx) * SX, y0 = (tile / ntx % nty) * SY, z0 = tile / (ntx * nty) * SZ;
+    __syncthreads();  // the tile before is read
+    halo_rows(g, x0, y0, z0, wrap, [&](int t, int site) { r[t] = __ldg(rho + site); });
+    const int x = x0 + tx, y = y0 + ty;
+    const bool on = x < g.n[0] && y < g.n[1];
+    float q[SZ];
+    const int64_t site = on ? site_index(g, x, y, z0) : 0, plane = (int64_t)g.n[0] * g.n[1];
 #pragma unroll
-      for (int o = 0; o < 27; o++) {
-        const float v = r[kz + o / 9][T.ty + (o / 3) % 3][T.tx + o % 3];
-        acc[o] = fmaf(q.x, v, acc[o]);
-        acc[27 + o] = fmaf(q.y, v, acc[27 + o]);
-        acc[54 + o] = fmaf(q.z, v, acc[54 + o]);
+    for (int k = 0; k < SZ; k++) q[k] = on && z0 + k < g.n[2] ? __ldg(gF + 4 * (site + plane * k)) : 0.f;
+    __syncthreads();
+    // plane k of the halo lies above site k - 2, at site k - 1 and below site k
+#pragma unroll
+    for (int k = 0; k < HZ; k++) {
+#pragma unroll
+      for (int o = 0; o < 9; o++) {
+        const float v = r[(k * HY + ty + o / 3) * HX + tx + o % 3];
+#pragma unroll
+        for (int m = 0; m < 3; m++)
+          if (k - m >= 0 && k - m < SZ) acc[9 * m + o] = fmaf(q[k - m], v, acc[9 * m + o]);
       }
     }
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int q = 0; q < 81; q++) {
+  for (int q = 0; q < 27; q++) {
     float v = acc[q];
 #pragma unroll
     for (int m = 16; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
     if (lane == 0) red[warp][q] = v;
   }
   __syncthreads();
-  if (threadIdx.x < 81) {
-    const int64_t tile = blockIdx.x + (int64_t)gridDim.x * (blockIdx.y + (int64_t)gridDim.y * blockIdx.z);
+  if (threadIdx.x < 27) {
     float v = 0.f;
     for (int w = 0; w < STENCIL_THREADS / 32; w++) v += red[w][threadIdx.x];
-    partial[tile * 81 + threadIdx.x] = v;
+    partial[(size_t)blockIdx.x * 81 + blockIdx.y * 27 + threadIdx.x] = v;
   }
 }
 
@@ -594,14 +872,57 @@ __device__ __forceinline__ int32_t pos_state(const Geom& g, const double* p, dou
 // so that sorted particles come grouped by brick and by cell inside it.
 __device__ __forceinline__ int32_t brick_key(const Geom& g, int32_t c)
 {
-  const int x = c % g.n[0], y = (c / g.n[0]) % g.n[1], z = c / (g.n[0] * g.n[1]);
+  int x, y, z;
+  cell_xyz(g, c, x, y, z);
   const int64_t b = brick_of(g, x, y, z);
   return (int32_t)(b * (BRICK * BRICK * BRICK) + (x % BRICK) + BRICK * ((y % BRICK) + BRICK * (z % BRICK)));
 }
 
+// A particle's 32-byte record: one 32-byte access where the array starts on
+// such a boundary (WIDE), so that the permutations' random accesses touch
+// their sector once; two of 16 bytes otherwise.
+struct Record {
+  uint32_t w[8];
+};
+
+template <bool WIDE>
+__device__ __forceinline__ Record load_record(const uint4* rec, int64_t i)
+{
+  Record r;
+  const uint4* p = rec + 2 * i;
+  if (WIDE) {
+    asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]), "=r"(r.w[4]), "=r"(r.w[5]),
+                   "=r"(r.w[6]), "=r"(r.w[7])
+                 : "l"(p));
+  } else {
+    const uint4 a = p[0], b = p[1];
+    r.w[0] = a.x, r.w[1] = a.y, r.w[2] = a.z, r.w[3] = a.w;
+    r.w[4] = b.x, r.w[5] = b.y, r.w[6] = b.z, r.w[7] = b.w;
+  }
+  return r;
+}
+
+template <bool WIDE>
+__device__ __forceinline__ void store_record(uint4* rec, int64_t i, const Record& r)
+{
+  uint4* p = rec + 2 * i;
+  if (WIDE) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(r.w[0]), "r"(r.w[1]),
+                 "r"(r.w[2]), "r"(r.w[3]), "r"(r.w[4]), "r"(r.w[5]), "r"(r.w[6]), "r"(r.w[7])
+                 : "memory");
+  } else {
+    p[0] = make_uint4(r.w[0], r.w[1], r.w[2], r.w[3]);
+    p[1] = make_uint4(r.w[4], r.w[5], r.w[6], r.w[7]);
+  }
+}
+
+inline bool wide_records(const void* rec) { return (reinterpret_cast<uintptr_t>(rec) & 31) == 0; }
+
 // Caller order, coalesced: the sort key of every particle (brick_key) and
 // its 32-byte record (cell, offsets, FP32 velocity, FP32 mass), so that the
 // permutation reads one full sector per particle.
+template <bool WIDE>
 __global__ void k_pm_pack(Geom g, int64_t np, const double* __restrict__ pos,
                           const double* __restrict__ vel, const double* __restrict__ mass,
                           double inv_res, int32_t* __restrict__ key, uint4* __restrict__ rec)
@@ -612,29 +933,39 @@ __global__ void k_pm_pack(Geom g, int64_t np, const double* __restrict__ pos,
     const int32_t c = pos_state(g, pos + 3 * i, inv_res, o);
     key[i] = brick_key(g, c);
     const float m = mass ? __double2float_rn(mass[i]) : 0.0f;
-    rec[2 * i] = make_uint4((uint32_t)c, __float_as_uint(o[0]), __float_as_uint(o[1]),
-                            __float_as_uint(o[2]));
-    rec[2 * i + 1] = make_uint4(__float_as_uint(__double2float_rn(vel[3 * i])),
-                                __float_as_uint(__double2float_rn(vel[3 * i + 1])),
-                                __float_as_uint(__double2float_rn(vel[3 * i + 2])), __float_as_uint(m));
+    const Record r{{(uint32_t)c, __float_as_uint(o[0]), __float_as_uint(o[1]), __float_as_uint(o[2]),
+                    __float_as_uint(__double2float_rn(vel[3 * i])),
+                    __float_as_uint(__double2float_rn(vel[3 * i + 1])),
+                    __float_as_uint(__double2float_rn(vel[3 * i + 2])), __float_as_uint(m)}};
+    store_record<WIDE>(rec, i, r);
   }
 }
 
 // Slot i takes the record of particle order[i].
+template <bool WIDE>
 __global__ void k_pm_unpack(int64_t np, const int64_t* __restrict__ order, const uint4* __restrict__ rec,
                             int32_t* __restrict__ cell, float* __restrict__ off3,
                             float* __restrict__ vel3, float* __restrict__ m)
 {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t s = order[i];
-    const uint4 a = rec[2 * s], b = rec[2 * s + 1];
-    cell[i] = (int32_t)a.x;
-    off3[3 * i] = __uint_as_float(a.y), off3[3 * i + 1] = __uint_as_float(a.z);
-    off3[3 * i + 2] = __uint_as_float(a.w);
-    vel3[3 * i] = __uint_as_float(b.x), vel3[3 * i + 1] = __uint_as_float(b.y);
-    vel3[3 * i + 2] = __uint_as_float(b.z);
-    if (m) m[i] = __uint_as_float(b.w);
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  constexpr int U = 4;  // records in flight per thread
+  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i0 < np; i0 += U * stride) {
+    Record r[U];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (i0 + u * stride < np) r[u] = load_record<WIDE>(rec, order[i0 + u * stride]);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int64_t i = i0 + u * stride;
+      if (i >= np) continue;
+      cell[i] = (int32_t)r[u].w[0];
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        off3[3 * i + k] = __uint_as_float(r[u].w[1 + k]);
+        vel3[3 * i + k] = __uint_as_float(r[u].w[4 + k]);
+      }
+      if (m) m[i] = __uint_as_float(r[u].w[7]);
+    }
   }
 }
 
@@ -650,7 +981,8 @@ __global__ void k_pm_brick_start(Geom g, int64_t np, const int32_t* __restrict__
     while (lo < hi) {
       const int64_t mid = lo + ((hi - lo) >> 1);
       const int32_t c = cell[mid];
-      const int x = c % g.n[0], y = (c / g.n[0]) % g.n[1], z = c / (g.n[0] * g.n[1]);
+      int x, y, z;
+      cell_xyz(g, c, x, y, z);
       if (brick_of(g, x, y, z) < b) lo = mid + 1;
       else hi = mid;
     }
@@ -660,36 +992,37 @@ __global__ void k_pm_brick_start(Geom g, int64_t np, const int32_t* __restrict__
 
 // The gradients of slot i as the 32-byte record of particle order[i] (one
 // full sector written per particle; no partial-sector writes).
+template <bool WIDE>
 __global__ void k_pm_grads_scatter(int64_t np, const int64_t* __restrict__ order,
                                    const float* __restrict__ g_off3, const float* __restrict__ g_vel3,
                                    const float* __restrict__ g_m, uint4* __restrict__ rec)
 {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np;
        i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t s = order[i];
-    rec[2 * s] = make_uint4(__float_as_uint(g_off3[3 * i]), __float_as_uint(g_off3[3 * i + 1]),
-                            __float_as_uint(g_off3[3 * i + 2]), __float_as_uint(g_m[i]));
-    rec[2 * s + 1] = make_uint4(__float_as_uint(g_vel3[3 * i]), __float_as_uint(g_vel3[3 * i + 1]),
-                                __float_as_uint(g_vel3[3 * i + 2]), 0u);
+    const Record r{{__float_as_uint(g_off3[3 * i]), __float_as_uint(g_off3[3 * i + 1]),
+                    __float_as_uint(g_off3[3 * i + 2]), __float_as_uint(g_m[i]),
+                    __float_as_uint(g_vel3[3 * i]), __float_as_uint(g_vel3[3 * i + 1]),
+                    __float_as_uint(g_vel3[3 * i + 2]), 0u}};
+    store_record<WIDE>(rec, order[i], r);
   }
 }
 
 // Caller order, coalesced: the records into FP64 gradients (the offset
 // gradient times inv_res: per box unit).
+template <bool WIDE>
 __global__ void k_pm_grads_unpack(int64_t np, const uint4* __restrict__ rec, double inv_res,
                                   double* __restrict__ g_pos, double* __restrict__ g_vel,
                                   double* __restrict__ g_mass)
 {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np;
        i += (int64_t)gridDim.x * blockDim.x) {
-    const uint4 a = rec[2 * i], b = rec[2 * i + 1];
-    g_pos[3 * i] = __dmul_rn((double)__uint_as_float(a.x), inv_res);
-    g_pos[3 * i + 1] = __dmul_rn((double)__uint_as_float(a.y), inv_res);
-    g_pos[3 * i + 2] = __dmul_rn((double)__uint_as_float(a.z), inv_res);
-    g_mass[i] = (double)__uint_as_float(a.w);
-    g_vel[3 * i] = (double)__uint_as_float(b.x);
-    g_vel[3 * i + 1] = (double)__uint_as_float(b.y);
-    g_vel[3 * i + 2] = (double)__uint_as_float(b.z);
+    const Record r = load_record<WIDE>(rec, i);
+    g_mass[i] = (double)__uint_as_float(r.w[3]);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      g_pos[3 * i + k] = __dmul_rn((double)__uint_as_float(r.w[k]), inv_res);
+      g_vel[3 * i + k] = (double)__uint_as_float(r.w[4 + k]);
+    }
   }
 }
 
@@ -706,6 +1039,9 @@ inline int64_t stencil_tiles(const Geom& g)
   return (int64_t)d.x * d.y * d.z;
 }
 
+// Rows of partial sums of the weight gradient: three CTAs per SM, three to a row.
+inline int stencil_rows(const lf2_ctx* c) { return c->num_sms; }
+
 // The chain's deposit into rho (+=): per particle, or brick-tiled when
 // brick_start is given (particles grouped by brick, nbricks + 1 entries).
 cudaError_t launch_pm_deposit(lf2_ctx* c, int64_t np, const int64_t* brick_start, const int32_t* cell,
@@ -715,6 +1051,11 @@ cudaError_t launch_pm_deposit(lf2_ctx* c, int64_t np, const int64_t* brick_start
   const float inv_vol = (float)(1.0 / vol);
   const Geom g = c->g;
   const unsigned nb = (unsigned)g.nbricks;
+  // particles of one CTA: twice a brick's at one per cell, fewer where that
+  // would leave SMs without two CTAs
+  const int part = (int)std::max<int64_t>(1024, std::min<int64_t>(2 * BRICK * BRICK * BRICK,
+                                                                  np / (2 * c->num_sms)));
+  const unsigned extra = (unsigned)((np + part - 1) / part);
   if (c->mode == LF2_DEPOSIT_FIXED64) {
     // integer sums in the context's scratch (zero between calls)
     if (!c->pm_acc) {
@@ -728,12 +1069,13 @@ cudaError_t launch_pm_deposit(lf2_ctx* c, int64_t np, const int64_t* brick_start
       cudaError_t e = cudaMemsetAsync(mmax, 0, sizeof(uint32_t), c->stream);
       if (e != cudaSuccess) return e;
       c->launches += 1;
-      k_pm_mass_max<<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(np, mass, mmax);
+      k_pm_mass_max<<<grid_for((np + 7) / 8, PM_THREADS), PM_THREADS, 0, c->stream>>>(np, mass, mmax);
     }
     c->launches += 2;
     if (brick_start)
-      k_pm_deposit_fixed_tile<<<nb, 256, 0, c->stream>>>(g, np, brick_start, cell, off3, mass, mmax,
-                                                          c->pm_acc);
+      k_pm_deposit_tile<true><<<nb + extra, 256, 0, c->stream>>>(g, np, brick_start, part, cell,
+                                                                off3, mass, mmax, gmass, inv_vol, c->pm_acc,
+                                                                nullptr);
     else
       k_pm_deposit_fixed<<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(g, np, cell, off3,
                                                                                 mass, mmax, c->pm_acc);
@@ -743,8 +1085,9 @@ cudaError_t launch_pm_deposit(lf2_ctx* c, int64_t np, const int64_t* brick_start
   }
   c->launches += 1;
   if (brick_start)
-    k_pm_deposit_tile<<<nb, 256, 0, c->stream>>>(g, np, brick_start, cell, off3, mass, gmass, inv_vol,
-                                                 rho);
+    k_pm_deposit_tile<false><<<nb + extra, 256, 0, c->stream>>>(g, np, brick_start, part, cell,
+                                                               off3, mass, nullptr, gmass, inv_vol,
+                                                               nullptr, rho);
   else
     k_pm_deposit<<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(g, np, cell, off3, mass,
                                                                           gmass, inv_vol, rho);
@@ -774,14 +1117,14 @@ cudaError_t launch_pm(lf2_ctx* c, int op, int64_t np, const int32_t* cell, const
       break;
     case 3:  // deposit adjoint: in_a = g_rho; out_a = g_off (+=), out_b = g_mass (+=)
       c->launches += 1;
-      k_pm_deposit_adj<<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(
-          g, np, cell, off3, mass, gmass, inv_vol, in_a, out_a, out_b);
+      k_pm_deposit_adj<false><<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(
+          g, np, cell, off3, mass, gmass, inv_vol, in_a, 1.0f, out_a, out_b, nullptr);
       break;
     case 4:  // gather adjoint: in_a = F4, in_b = gG; out_a = gF4 (+=), out_b = g_off (+=)
       c->launches += 1;
-      k_pm_gather_adj<<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(
+      k_pm_gather_adj<false><<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(
           g, np, cell, off3, reinterpret_cast<const float4*>(in_a), in_b,
-          reinterpret_cast<float4*>(out_a), out_b);
+          reinterpret_cast<float4*>(out_a), out_b, nullptr, 0.0f, 0.0f);
       break;
     default:
       return cudaErrorInvalidValue;
@@ -803,22 +1146,63 @@ cudaError_t launch_stencil(lf2_ctx* c, int op, const float* a, const float* S, f
         g, reinterpret_cast<const float4*>(a), S, out);
   } else {  // a = gF4, S = rho -> out = gS (+=)
     c->launches += 2;
-    k_stencil_adj_S<<<grid, STENCIL_THREADS, 0, c->stream>>>(
-        g, reinterpret_cast<const float4*>(a), S, partial);
-    k_stencil_adj_S_sum<<<1, 352, 0, c->stream>>>((int)stencil_tiles(g), partial, out);
+    const int ntiles = (int)stencil_tiles(g), ctas = std::min(ntiles, stencil_rows(c));
+    k_stencil_adj_S<<<dim3(ctas, 3), STENCIL_THREADS, 0, c->stream>>>(
+        g, (int)grid.x, (int)grid.y, ntiles, reinterpret_cast<const float4*>(a), S, partial);
+    k_stencil_adj_S_sum<<<1, 352, 0, c->stream>>>(ctas, partial, out);
   }
   return cudaGetLastError();
 }
 
-size_t stencil_partial_floats(const lf2_ctx* c) { return (size_t)stencil_tiles(c->g) * 81; }
+size_t stencil_partial_floats(const lf2_ctx* c)
+{
+  return (size_t)std::min<int64_t>(stencil_tiles(c->g), stencil_rows(c)) * 81;
+}
 
-cudaError_t launch_pm_step(lf2_ctx* c, int64_t np, int32_t* cell, float* off3, float* vel3,
-                           const float* F4, float dtk, float dtn)
+cudaError_t launch_pm_step(lf2_ctx* c, int64_t np, const int32_t* cell, const float* off3,
+                           const float* vel3, const float* F4, float dtk, float dtn, int32_t* cell_out,
+                           float* off_out, float* vel_out)
 {
   if (np == 0) return cudaSuccess;
   c->launches += 1;
   k_pm_gather_kick_drift<<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(
-      c->g, np, cell, off3, vel3, reinterpret_cast<const float4*>(F4), dtk, dtn, c->flags);
+      c->g, np, cell, off3, vel3, reinterpret_cast<const float4*>(F4), dtk, dtn, cell_out, off_out,
+      vel_out, c->flags);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_pm_step_adjoint(lf2_ctx* c, int64_t np, const int32_t* cell, const float* off3,
+                                   const float* F4, float* g_vel3, float* g_off3, float* gF4, float dtk,
+                                   float dtn)
+{
+  if (np == 0) return cudaSuccess;
+  c->launches += 1;
+  k_pm_gather_adj<true><<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(
+      c->g, np, cell, off3, reinterpret_cast<const float4*>(F4), nullptr, reinterpret_cast<float4*>(gF4),
+      g_off3, g_vel3, dtk, dtn);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_pm_loss_adjoint(lf2_ctx* c, int64_t np, const int32_t* cell, const float* off3,
+                                   const float* mass, const float* w, float scale, float* g_off3,
+                                   float* g_mass, float* g_vel3)
+{
+  if (np == 0) return cudaSuccess;
+  c->launches += 1;
+  k_pm_deposit_adj<true><<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(
+      c->g, np, cell, off3, mass, 0.0f, (float)(1.0 / (c->res * c->res * c->res)), w, scale, g_off3, g_mass,
+      g_vel3);
+  return cudaGetLastError();
+}
+
+// Partial sums of the loss (c->loss_part): four CTAs per SM.
+int loss_ctas(const lf2_ctx* c) { return 4 * c->num_sms; }
+
+cudaError_t launch_pm_loss(lf2_ctx* c, const float* w, const float* rho, double* loss)
+{
+  c->launches += 2;
+  k_pm_loss<<<loss_ctas(c), LOSS_THREADS, 0, c->stream>>>(c->g.nsites, w, rho, c->loss_part);
+  k_pm_loss_sum<<<1, LOSS_THREADS, 0, c->stream>>>(loss_ctas(c), c->loss_part, loss);
   return cudaGetLastError();
 }
 
@@ -827,7 +1211,8 @@ cudaError_t launch_pm_pack(lf2_ctx* c, int64_t np, const double* pos, const doub
 {
   if (np == 0) return cudaSuccess;
   c->launches += 1;
-  k_pm_pack<<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(
+  const auto kern = wide_records(rec) ? k_pm_pack<true> : k_pm_pack<false>;
+  kern<<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(
       c->g, np, pos, vel, mass, inv_res, key, reinterpret_cast<uint4*>(rec));
   return cudaGetLastError();
 }
@@ -837,7 +1222,8 @@ cudaError_t launch_pm_unpack(lf2_ctx* c, int64_t np, const int64_t* order, const
 {
   if (np == 0) return cudaSuccess;
   c->launches += 1;
-  k_pm_unpack<<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(
+  const auto kern = wide_records(rec) ? k_pm_unpack<true> : k_pm_unpack<false>;
+  kern<<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(
       np, order, reinterpret_cast<const uint4*>(rec), cell, off3, vel3, m);
   return cudaGetLastError();
 }
@@ -856,9 +1242,12 @@ cudaError_t launch_pm_grads_back(lf2_ctx* c, int64_t np, const int64_t* order, c
 {
   if (np == 0) return cudaSuccess;
   c->launches += 2;
-  k_pm_grads_scatter<<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(
+  const bool wide = wide_records(rec);
+  const auto scatter = wide ? k_pm_grads_scatter<true> : k_pm_grads_scatter<false>;
+  const auto unpack = wide ? k_pm_grads_unpack<true> : k_pm_grads_unpack<false>;
+  scatter<<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(
       np, order, g_off3, g_vel3, g_m, reinterpret_cast<uint4*>(rec));
-  k_pm_grads_unpack<<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(
+  unpack<<<grid_for(np, PM_THREADS), PM_THREADS, 0, c->stream>>>(
       np, reinterpret_cast<const uint4*>(rec), inv_res, g_pos, g_vel, g_mass);
   return cudaGetLastError();
 }
