@@ -120,3 +120,35 @@ def test_loss_and_its_adjoint(cuda):
     for bad in (w[:-1].contiguous(), w.cpu()):
         with pytest.raises(RuntimeError):
             ops.loss(bad, rho)
+
+
+def test_records_off_the_32_byte_boundary(cuda):
+    """32-byte records at an address that is a multiple of 16 only: the packed
+    state and the unordered gradients are the same bits as at one of 32."""
+    import torch
+    from latfield2_b200.autodiff import _check, _p
+    n, npart = 32, 5001
+    ctx, ops = _sorted_case(n, "fp32")[:2]
+    g = torch.Generator(device="cpu").manual_seed(8)
+    pos, vel = (torch.rand(npart, 3, generator=g, dtype=torch.float64).cuda() for _ in range(2))
+    m = torch.rand(npart, generator=g, dtype=torch.float64).cuda()
+    key, rec = ops.state_pack(pos, vel, m, float(n))
+    order = torch.argsort(key)
+    want = ops.state_unpack(order, rec)
+    room = torch.empty(npart * 8 + 8, dtype=torch.int32, device="cuda")
+    off16 = room[4 if room.data_ptr() % 32 == 0 else 0:][:npart * 8]
+    assert off16.data_ptr() % 32 == 16
+    key2 = torch.empty_like(key)
+    _check(ctx, ops.lib.lf2_pm_state_pack(ctx.h, npart, _p(pos), _p(vel), _p(m), float(n), _p(key2),
+                                          _p(off16)), "pack")
+    assert torch.equal(key, key2) and torch.equal(rec, off16)
+    for x, y in zip(ops.state_unpack(order, off16), want):
+        assert torch.equal(x, y)
+    g_off, g_v = torch.randn(npart, 3, generator=g).cuda(), torch.randn(npart, 3, generator=g).cuda()
+    g_m = torch.randn(npart, generator=g).cuda()
+    ref = ops.grads_unorder(order, g_off, g_v, g_m, float(n))
+    out = [torch.empty_like(x) for x in ref]
+    _check(ctx, ops.lib.lf2_pm_grads_unorder(ctx.h, npart, _p(order), _p(g_off), _p(g_v), _p(g_m),
+                                             float(n), _p(off16), *[_p(x) for x in out]), "grads")
+    for x, y in zip(out, ref):
+        assert torch.equal(x, y)
