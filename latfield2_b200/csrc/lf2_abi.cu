@@ -330,12 +330,11 @@ lf2_status lf2_create(lf2_ctx** out, int device, const int n[3], const double bo
   ok = ok && cudaMallocHost(&c->h_stats, sizeof(double) * 8) == cudaSuccess;
   ok = ok && cudaMallocHost(&c->h_flags, sizeof(uint32_t)) == cudaSuccess;
   ok = ok && cudaMallocHost(&c->h_i64, sizeof(int64_t) * 4) == cudaSuccess;
-  ok = ok && cudaMalloc(&c->work, 2 * sizeof(int) + sizeof(unsigned long long)) == cudaSuccess;
-  c->mov_count = reinterpret_cast<unsigned long long*>(c->work + 2);
+  ok = ok && cudaMalloc(&c->head, sizeof(PassHead)) == cudaSuccess;
+  c->mov_count = &c->head->mov_count;
   ok = ok && cudaMalloc(&c->move_list, sizeof(int32_t) * nb) == cudaSuccess;
   ok = ok && cudaMalloc(&c->move_mark, (size_t)nb) == cudaSuccess;
   ok = ok && cudaMalloc(&c->part_item, sizeof(int4) * (PART_ITEMS + PART_TILES)) == cudaSuccess;
-  ok = ok && cudaMalloc(&c->part_head, sizeof(int32_t) * 3) == cudaSuccess;
   ok = ok && cudaMalloc(&c->part_mark, (size_t)nb) == cudaSuccess;
   ok = ok && cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess;
   if (ok) {
@@ -348,7 +347,7 @@ lf2_status lf2_create(lf2_ctx** out, int device, const int n[3], const double bo
          cudaMemsetAsync(c->ovf_count, 0, sizeof(int32_t), c->stream) == cudaSuccess &&
          cudaMemsetAsync(c->ovf_state, 0, sizeof(int32_t) * nb, c->stream) == cudaSuccess &&
          cudaMemsetAsync(c->heap_top, 0, sizeof(unsigned long long), c->stream) == cudaSuccess &&
-         cudaMemsetAsync(c->mov_count, 0, sizeof(unsigned long long), c->stream) == cudaSuccess &&
+         cudaMemsetAsync(c->head, 0, sizeof(PassHead), c->stream) == cudaSuccess &&
          cudaMemsetAsync(c->brick_maxv2, 0, sizeof(float) * nb, c->stream) == cudaSuccess &&
          cudaStreamSynchronize(c->stream) == cudaSuccess;
   }
@@ -380,7 +379,7 @@ lf2_status lf2_destroy(lf2_ctx* c)
   cudaFree(c->brick_sums);
   cudaFree(c->stats);
   cudaFree(c->mig);
-  cudaFree(c->work);
+  cudaFree(c->head);
   cudaFree(c->move_list);
   cudaFree(c->f_rows);
   cudaFree(c->move_mark);
@@ -395,7 +394,6 @@ lf2_status lf2_destroy(lf2_ctx* c)
   cudaFree(c->ovf_state);
   cudaFree(c->spill);
   cudaFree(c->part_item);
-  cudaFree(c->part_head);
   cudaFree(c->part_mark);
   cudaFree(c->stencil_partial);
   cudaFree(c->loss_part);
@@ -495,7 +493,7 @@ lf2_status lf2_particles_set_pos(lf2_ctx* c, int64_t n, const void* pos3, const 
 #define LF2_FUSED_AUTO 0
 #endif
 
-static lf2_status rebin_tail(lf2_ctx* c);
+static lf2_status rebin_tail(lf2_ctx* c, const PartPlan* plan = nullptr);
 
 lf2_status lf2_particles_extract_z(lf2_ctx* c, int z_lo, int z_hi, int64_t capacity,
                                    int32_t* cell, float* off3, float* vel3, float* mass,
@@ -944,7 +942,7 @@ lf2_status lf2_halo_fill(lf2_ctx* c, void* data, int comps, int halo, int real_b
   return LF2_OK;
 }
 
-static lf2_status deposit(lf2_ctx* c, lf2_field f, int kind, int comps)
+static lf2_status deposit(lf2_ctx* c, lf2_field f, int kind, int comps, bool planned = false)
 {
   if (!valid_field(c, f)) return LF2_ERR_ARG;
   if (f->comps != comps) return fail(c, LF2_ERR_ARG, "field has the wrong number of components");
@@ -953,7 +951,7 @@ static lf2_status deposit(lf2_ctx* c, lf2_field f, int kind, int comps)
   {
     PhaseScope ps(c, PH_DEPOSIT);
     LF2_CUDA(c, kind >= 3 ? launch_deposit_full(c, kind, f->data, 0)
-                          : launch_deposit(c, kind, f->data, 0));
+                          : launch_deposit(c, kind, f->data, 0, nullptr, planned));
   }
   {
     PhaseScope ps(c, PH_FIXUP);
@@ -975,11 +973,12 @@ lf2_status lf2_deposit_vecvec_cic(lf2_ctx* c, lf2_field t) { return deposit(c, t
 #define LF2_FUSED_AUTO 0
 #endif
 
-static lf2_status rebin_tail(lf2_ctx* c)
+// plan: of the deposit that follows at once
+static lf2_status rebin_tail(lf2_ctx* c, const PartPlan* plan)
 {
   PhaseScope ps(c, PH_INSERT);
   LF2_CUDA(c, launch_insert(c));
-  LF2_CUDA(c, launch_repack(c));
+  LF2_CUDA(c, launch_repack(c, plan));
   return LF2_OK;
 }
 
@@ -1010,8 +1009,8 @@ lf2_status lf2_drift_rebin(lf2_ctx* c, double dtau)
 {
   if (!c) return LF2_ERR_ARG;
   MoveParams mp{0.0f, (float)(dtau / c->res)};
-  if (c->move_kernel == 1)  // the pipelined pass resets the counter itself
-    LF2_CUDA(c, cudaMemsetAsync(c->mov_count, 0, sizeof(unsigned long long), c->stream));
+  if (c->move_kernel == 1)  // the pipelined pass clears the counters itself
+    LF2_CUDA(c, cudaMemsetAsync(c->head, 0, sizeof(PassHead), c->stream));
   {
     PhaseScope ps(c, PH_MOVE);
     LF2_CUDA(c, c->move_kernel != 1 ? launch_move_pipe(c, nullptr, false, true, mp, nullptr)
@@ -1031,8 +1030,8 @@ lf2_status lf2_step(lf2_ctx* c, lf2_field F, double dtau_kick, double dtau_drift
     return fail(c, LF2_ERR_UNSUPPORTED, "the fused deposit needs the fixed-point mode and room "
                                         "for its tile");
   const bool pipe = c->move_kernel >= 2 || (c->move_kernel == 0 && move_pipe_auto(c, F->data));
-  if (!pipe)  // the pipelined pass resets the counter itself
-    LF2_CUDA(c, cudaMemsetAsync(c->mov_count, 0, sizeof(unsigned long long), c->stream));
+  if (!pipe)  // the pipelined pass clears the counters itself
+    LF2_CUDA(c, cudaMemsetAsync(c->head, 0, sizeof(PassHead), c->stream));
   // the fixed-point scalar deposit fused into the pipelined pass (automatic
   // when eligible, or kernel 3), finished by the movers' rim atomics and the
   // rim fix-up; redone by the tile pass if a mover went past the rim
@@ -1046,9 +1045,10 @@ lf2_status lf2_step(lf2_ctx* c, lf2_field F, double dtau_kick, double dtau_drift
       LF2_CUDA(c, pipe ? launch_move_pipe(c, F->data, true, true, mp, nullptr)
                        : launch_move(c, F->data, true, true, mp));
     }
-    LF2_TRY(rebin_tail(c));
-    if (rho) LF2_TRY(deposit(c, rho, 0, 1));
-    return LF2_OK;
+    if (!rho) return rebin_tail(c);
+    const PartPlan plan = scalar_plan(c);
+    LF2_TRY(rebin_tail(c, &plan));
+    return deposit(c, rho, 0, 1, true);
   }
   LF2_TRY(ensure_spill(c, std::max(rim_store_slots(c), deposit_spill_slots(c, 1))));
   LF2_CUDA(c, cudaMemsetAsync(c->redep, 0, sizeof(uint32_t), c->stream));

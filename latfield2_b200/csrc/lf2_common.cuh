@@ -203,4 +203,44 @@ __device__ inline int block_exclusive_scan(int v, int* warp_tot, int* total)
   return r;
 }
 
+// Counters of a pass over the store, cleared together before it.
+struct PassHead {
+  unsigned long long mov_count;  // particles in the mover buffer
+  int work;                      // next brick of the pipelined move
+  int heavy;                     // bricks of the move's list
+  int32_t items, splits, tiles;  // of the plan of heavy bricks
+  int32_t pad;
+};
+
+// What a plan of heavy bricks (lf2_deposit.cu) lists, and where.
+struct PartPlan {
+  int P, split, first;       // particles per part; counts above which a brick is split, is an item
+  int max_items, max_tiles;  // 0 items: nothing is listed
+  int4* item;
+  int4* split_list;
+  uint8_t* mark;
+  PassHead* head;
+};
+
+// Lists brick b of c particles: a brick above `split` makes ceil(c / P)
+// parts while there are scratch tiles, one above `first` a single item.
+__device__ __forceinline__ void part_plan_brick(const PartPlan& pl, int b, int c)
+{
+  bool listed = false;
+  if (c > pl.first) {
+    int parts = 1, t0 = 0;
+    if (c > pl.split) {
+      parts = (int)(((unsigned)c + (unsigned)pl.P - 1u) / (unsigned)pl.P);
+      t0 = atomicAdd(&pl.head->tiles, parts);
+      if (t0 + parts > pl.max_tiles) parts = 1;
+    }
+    const int i0 = atomicAdd(&pl.head->items, parts);
+    listed = i0 + parts <= pl.max_items;
+    for (int k = 0; k < parts && i0 + k < pl.max_items; k++)
+      pl.item[i0 + k] = make_int4(listed ? b : -1, k, parts, t0);
+    if (listed && parts > 1) pl.split_list[atomicAdd(&pl.head->splits, 1)] = make_int4(b, parts, t0, 0);
+  }
+  pl.mark[b] = listed;
+}
+
 }  // namespace lf2

@@ -126,14 +126,14 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
   const int ex = brick_extent(g.n[0], bx), ey = brick_extent(g.n[1], by),
             ez = brick_extent(g.n[2], bz);
   const int x0 = bx * BRICK, y0 = by * BRICK, z0 = bz * BRICK;
-  const int64_t base = v.seg_start[b] + part.first;
+  const uint32_t base = (uint32_t)(v.seg_start[b] + part.first);  // slots fit in 32 bits
   const int cnt = part.cnt;
   const int mass_bound =
-      FIXED && dp.has_mass ? part_mass_bound(v.a.mass, (uint32_t)base, cnt, dp.inv_unit, s_max) : 1;
+      FIXED && dp.has_mass ? part_mass_bound(v.a.mass, base, cnt, dp.inv_unit, s_max) : 1;
   CompUnit cu{0, false};
   if (ACC == ACC_COMP)
     cu = comp_unit<KIND>(dp.has_mass ? v.a.mass : nullptr, dp.inv_vol, dp.mf, v.a.vx, v.a.vy, v.a.vz,
-                         (uint32_t)base, cnt, s_max);
+                         base, cnt, s_max);
   // two integer words per vertex, or the sums that hold anything
   const bool ints = FIXED ? cnt <= split_max<SIGNED>(mass_bound) : cu.ok;
   TileRef<TILE3> tr{smem_raw, ints};
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
       for (int j = 0; j < ITEMS; j++) {
         const int i = c0 + j * T + threadIdx.x;
         if (i < cnt) {
-          const uint32_t p = (uint32_t)base + (uint32_t)i;  // slots fit in 32 bits
+          const uint32_t p = base + (uint32_t)i;
           key[j] = v.a.key[p];
           fx[j] = v.a.ox[p];
           fy[j] = v.a.oy[p];
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
     else particles(std::false_type{}, std::false_type{});
   }
   __syncthreads();
-  if (uint64_t* scratch = part_tile(pv, P::NC * TILE3)) {  // k_part_finish sums the parts and writes the vertices
+  if (uint64_t* scratch = part_tile(pv, NC * TILE3)) {  // k_part_finish writes the vertices
     part_store<ACC, SIGNED, NC, TILE3>(scratch, tr, cu.e);
     return;
   }
@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(FINISH_CHUNK) k_part_finish(Geom g, PartView p
   using P = Pass<KIND, PASS, ACC>;
   constexpr int C = Comps<KIND>::value;
   constexpr int CHUNKS = (TILE3 + FINISH_CHUNK - 1) / FINISH_CHUNK;
-  const int units = pv.head[1] * CHUNKS;
+  const int units = pv.head->splits * CHUNKS;
   if ((int)blockIdx.x >= units) return;
   const int vexp = ACC == ACC_FIXED && KIND != 0 ? vexp_of(*vmax_bits) : 0;
   const float conv = ldexpf(fixed_scale, (KIND == 1 ? vexp : 2 * vexp) - (KIND != 0 ? 16 : 0));
@@ -624,36 +624,28 @@ __global__ void __launch_bounds__(256) k_vmax(StoreView v, uint32_t* vmax_bits, 
   if (m > *reinterpret_cast<volatile uint32_t*>(vmax_bits)) atomicMax(vmax_bits, m);
 }
 
-// Items of the bricks above `first` particles: a brick above `split` makes
-// ceil(count / P) parts while there are scratch tiles, the others one.  One
-// CTA (which clears the counters head[0..2]), or several after they have
-// been cleared.
+// The plan, where no rebin has made it.  One CTA (which clears the counters),
+// or several after they have been cleared.
 __global__ void __launch_bounds__(1024) k_part_plan(int nb, const int32_t* __restrict__ count,
-                                                    const int32_t* __restrict__ cap, int P, int split,
-                                                    int first, int max_items, int max_tiles, int4* item,
-                                                    int4* split_list, uint8_t* mark, int32_t* head)
+                                                    const int32_t* __restrict__ cap, PartPlan pl)
 {
   if (gridDim.x == 1) {
-    if (threadIdx.x < 3) head[threadIdx.x] = 0;
+    if (threadIdx.x == 0) pl.head->items = pl.head->splits = pl.head->tiles = 0;
     __syncthreads();
   }
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-    const int c = min(count[b], cap[b]);
-    bool listed = false;
-    if (c > first) {
-      int parts = 1, t0 = 0;
-      if (c > split) {
-        parts = (int)(((unsigned)c + (unsigned)P - 1u) / (unsigned)P);
-        t0 = atomicAdd(&head[2], parts);
-        if (t0 + parts > max_tiles) parts = 1;
-      }
-      const int i0 = atomicAdd(&head[0], parts);
-      listed = i0 + parts <= max_items;
-      for (int k = 0; k < parts && i0 + k < max_items; k++)
-        item[i0 + k] = make_int4(listed ? b : -1, k, parts, t0);
-      if (listed && parts > 1) split_list[atomicAdd(&head[1], 1)] = make_int4(b, parts, t0, 0);
+  constexpr int U = 4;  // bricks in flight per thread
+  for (int b0 = blockIdx.x * blockDim.x + threadIdx.x; b0 < nb; b0 += U * gridDim.x * blockDim.x) {
+    int c[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int b = b0 + u * gridDim.x * blockDim.x;
+      c[u] = b < nb ? min(count[b], cap[b]) : 0;
     }
-    mark[b] = listed;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int b = b0 + u * gridDim.x * blockDim.x;
+      if (b < nb) part_plan_brick(pl, b, c[u]);
+    }
   }
 }
 
@@ -677,19 +669,27 @@ cudaError_t tile_pass(lf2_ctx* c, float* out, const DepositParams& dp, const uin
 }
 
 template <int KIND, int ACC>
-cudaError_t run(lf2_ctx* c, float* out, const DepositParams& dp, int stage, const uint32_t* gate)
+PartPlan tile_plan(lf2_ctx* c)
+{
+  using P = Pass<KIND, 0, ACC>;
+  return part_plan(c, P::smem(), P::THREADS, (size_t)P::NC * TILE3,
+                   ACC == ACC_FIXED  ? split_max<KIND != 0>(c->has_mass ? 2 : 1)
+                   : ACC == ACC_COMP ? split_max<true>(1)
+                                     : 0);
+}
+
+template <int KIND, int ACC>
+cudaError_t run(lf2_ctx* c, float* out, const DepositParams& dp, int stage, const uint32_t* gate,
+                bool planned)
 {
   const unsigned nb = (unsigned)c->g.nbricks;
   if (stage == 0) {
-    using P = Pass<KIND, 0, ACC>;
-    PartView pv;
-    const cudaError_t ep = launch_part_plan(
-        c, P::smem(), P::THREADS, (size_t)P::NC * TILE3,
-        ACC == ACC_FIXED  ? split_max<KIND != 0>(c->has_mass ? 2 : 1)
-        : ACC == ACC_COMP ? split_max<true>(1)
-                          : 0,
-        &pv);
-    if (ep != cudaSuccess) return ep;
+    const PartPlan pl = tile_plan<KIND, ACC>(c);
+    const PartView pv = part_view(c, pl, (size_t)Pass<KIND, 0, ACC>::NC * TILE3);
+    if (!planned) {
+      const cudaError_t ep = launch_part_plan(c, pl);
+      if (ep != cudaSuccess) return ep;
+    }
     if (ACC == ACC_FIXED && KIND != 0) {
       cudaError_t e = launch_vmax(c, pv);
       if (e != cudaSuccess) return e;
@@ -707,11 +707,12 @@ cudaError_t run(lf2_ctx* c, float* out, const DepositParams& dp, int stage, cons
 }
 
 template <int KIND>
-cudaError_t run_mode(lf2_ctx* c, float* out, const DepositParams& dp, int stage, const uint32_t* gate)
+cudaError_t run_mode(lf2_ctx* c, float* out, const DepositParams& dp, int stage, const uint32_t* gate,
+                     bool planned)
 {
-  if (c->mode == LF2_DEPOSIT_FIXED64) return run<KIND, ACC_FIXED>(c, out, dp, stage, gate);
-  if (c->mode == LF2_DEPOSIT_FP32_PLAIN) return run<KIND, ACC_PLAIN>(c, out, dp, stage, gate);
-  return run<KIND, ACC_COMP>(c, out, dp, stage, gate);
+  if (c->mode == LF2_DEPOSIT_FIXED64) return run<KIND, ACC_FIXED>(c, out, dp, stage, gate, planned);
+  if (c->mode == LF2_DEPOSIT_FP32_PLAIN) return run<KIND, ACC_PLAIN>(c, out, dp, stage, gate, planned);
+  return run<KIND, ACC_COMP>(c, out, dp, stage, gate, planned);
 }
 
 }  // namespace
@@ -725,40 +726,58 @@ cudaError_t run_mode(lf2_ctx* c, float* out, const DepositParams& dp, int stage,
 // of 1024 took 41 us for 64 uniform bricks of 4096 against 35 unsplit).
 // `cap` bounds what a split fixed-point tile sums.  The scratch tiles lie in
 // the repack scratch (c->alt), which nothing uses between the rebins.
-cudaError_t launch_part_plan(lf2_ctx* c, size_t smem, int threads, size_t tile_slots, int cap,
-                             PartView* pv)
+PartPlan part_plan(lf2_ctx* c, size_t smem, int threads, size_t tile_slots, int cap)
 {
-  *pv = PartView{};
-  if (c->np == 0) return cudaSuccess;
+  PartPlan pl{};
+  pl.item = c->part_item;
+  pl.split_list = c->part_item + PART_ITEMS;
+  pl.mark = c->part_mark;
+  pl.head = c->head;
+  if (c->np == 0) return pl;
   const int per_sm = std::max(1, std::min((int)(227 * 1024 / (smem + 1024)), 2048 / threads));
   const int64_t share = c->np / ((int64_t)c->num_sms * per_sm);
   if (cap <= 0) cap = 1 << 28;
   const int64_t P = std::min<int64_t>(std::max<int64_t>(share / 2, LF2_PART_MIN), cap - cap / 16);
   const int64_t split = std::min<int64_t>(P + P / 2, cap);
   const int64_t first = std::min(split, std::max(share / 4, 3 * (c->np / c->g.nbricks)));
+  pl.P = (int)P, pl.split = (int)split, pl.first = (int)first;
   // np particles make at most 3/2 np / P parts and np / first items
-  const int64_t most = std::min<int64_t>(PART_ITEMS, c->np * 3 / (2 * P) + c->np / first);
-  if (most == 0) return cudaSuccess;
+  pl.max_items = (int)std::min<int64_t>(PART_ITEMS, c->np * 3 / (2 * P) + c->np / first);
+  pl.max_tiles = (int)std::min<int64_t>(7 * (c->capacity / 2 / (int64_t)tile_slots), PART_TILES);
+  return pl;
+}
+
+PartView part_view(const lf2_ctx* c, const PartPlan& pl, size_t tile_slots)
+{
+  PartView pv{};
+  pv.item = pl.item, pv.split = pl.split_list, pv.mark = pl.mark, pv.head = pl.head;
   float* const banks[7] = {reinterpret_cast<float*>(c->alt.key), c->alt.ox, c->alt.oy, c->alt.oz,
                            c->alt.vx, c->alt.vy, c->alt.vz};
-  for (int i = 0; i < 7; i++) pv->bank[i] = reinterpret_cast<uint64_t*>(banks[i]);
-  pv->bank_tiles = (int)std::min<int64_t>(c->capacity / 2 / (int64_t)tile_slots, PART_TILES);
-  pv->item = c->part_item;
-  pv->split = c->part_item + PART_ITEMS;
-  pv->mark = c->part_mark;
-  pv->head = c->part_head;
-  pv->max_items = (int)most;
-  const int nb = (int)c->g.nbricks;
-  if (nb > 4096) {
-    const cudaError_t e = cudaMemsetAsync(c->part_head, 0, 3 * sizeof(int32_t), c->stream);
+  for (int i = 0; i < 7; i++) pv.bank[i] = reinterpret_cast<uint64_t*>(banks[i]);
+  pv.bank_tiles = (int)std::min<int64_t>(c->capacity / 2 / (int64_t)tile_slots, PART_TILES);
+  pv.max_items = pl.max_items;
+  return pv;
+}
+
+cudaError_t launch_part_plan(lf2_ctx* c, const PartPlan& pl)
+{
+  if (!pl.max_items) return cudaSuccess;
+  const int nb = (int)c->g.nbricks, ctas = (nb + 4095) / 4096;
+  if (ctas > 1) {
+    const cudaError_t e = cudaMemsetAsync(&c->head->items, 0, 3 * sizeof(int32_t), c->stream);
     if (e != cudaSuccess) return e;
   }
   c->launches += 1;
-  k_part_plan<<<nb > 4096 ? (nb + 1023) / 1024 : 1, 1024, 0, c->stream>>>(
-      nb, c->count, c->cap, (int)P, (int)split, (int)first, (int)most,
-      std::min(7 * pv->bank_tiles, PART_TILES), c->part_item, c->part_item + PART_ITEMS, c->part_mark,
-      c->part_head);
+  k_part_plan<<<ctas, 1024, 0, c->stream>>>(nb, c->count, c->cap, pl);
   return cudaGetLastError();
+}
+
+// The plan of the scalar deposit that follows a rebin.
+PartPlan scalar_plan(lf2_ctx* c)
+{
+  if (c->mode == LF2_DEPOSIT_FIXED64) return tile_plan<0, ACC_FIXED>(c);
+  if (c->mode == LF2_DEPOSIT_FP32_PLAIN) return tile_plan<0, ACC_PLAIN>(c);
+  return tile_plan<0, ACC_COMP>(c);
 }
 
 // Shell-store slots (8 bytes each) a deposit of `comps` components needs.
@@ -789,12 +808,12 @@ DepositParams deposit_params(const lf2_ctx* c)
   return dp;
 }
 
-cudaError_t launch_deposit(lf2_ctx* c, int kind, float* out, int stage, const uint32_t* gate)
+cudaError_t launch_deposit(lf2_ctx* c, int kind, float* out, int stage, const uint32_t* gate, bool planned)
 {
   const DepositParams dp = deposit_params(c);
-  if (kind == 0) return run_mode<0>(c, out, dp, stage, gate);
-  if (kind == 1) return run_mode<1>(c, out, dp, stage, gate);
-  return run_mode<2>(c, out, dp, stage, gate);
+  if (kind == 0) return run_mode<0>(c, out, dp, stage, gate, planned);
+  if (kind == 1) return run_mode<1>(c, out, dp, stage, gate, false);
+  return run_mode<2>(c, out, dp, stage, gate, false);
 }
 
 }  // namespace lf2

@@ -355,17 +355,18 @@ __host__ __device__ inline int vexp_of(uint32_t bits)
 
 // --------------------------------------------------- parts of heavy bricks
 // A brick that holds far more particles than the others would keep one CTA
-// busy long after the rest of the chip is done.  k_part_plan lists the heavy
-// bricks (lf2_deposit.cu says which) as items that the first CTAs of a tile
-// pass take, the heaviest of them split into parts of equal particle counts.
-// A part's CTA writes its whole tile to the scratch; a finishing kernel sums
-// the parts of each split brick in part order and writes the brick's vertices
-// as the tile pass does for a brick in one part.
+// busy long after the rest of the chip is done.  A plan (PartPlan) lists the
+// heavy bricks as items that the first CTAs of a tile pass take, the heaviest
+// of them split into parts of equal particle counts.  A part's CTA writes its
+// whole tile to the scratch; a finishing kernel sums the parts of each split
+// brick in part order and writes the brick's vertices as the tile pass does
+// for a brick in one part.  (Finishing in the CTA of the last part cost the
+// particle loops registers: 1591 us against 1364 at 512^3.)
 struct PartView {
   const int4* item;       // brick (-1: none), part, parts of the brick, tile of part 0
   const int4* split;      // brick, parts, tile of part 0
   const uint8_t* mark;    // per brick: 1 when it is an item
-  const int32_t* head;    // items, split bricks
+  const PassHead* head;
   uint64_t* bank[7];      // scratch tiles, NC * N 8-byte slots each,
   int bank_tiles;         // so many to a bank
   int max_items;          // what the plan may list
@@ -382,7 +383,7 @@ __device__ __forceinline__ uint64_t* scratch_tile(const PartView& pv, int i, int
 
 __device__ __forceinline__ int part_items(const PartView& pv)
 {
-  return pv.max_items ? min(pv.head[0], pv.max_items) : 0;
+  return pv.max_items ? min(pv.head->items, pv.max_items) : 0;
 }
 
 // One unit of work of a tile pass: particles [first, first + cnt) of a brick.

@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(FINISH_CHUNK)
 {
   constexpr int CT = FullPass<PASS>::total;
   constexpr int CHUNKS = (FT3 + FINISH_CHUNK - 1) / FINISH_CHUNK;
-  const int units = pv.head[1] * CHUNKS;
+  const int units = pv.head->splits * CHUNKS;
   if ((int)blockIdx.x >= units) return;
   const int vexp = ACC == ACC_FIXED ? vexp_of(*vmax_bits) : 0;
   const float conv = ldexpf(fixed_scale, (PASS == 0 ? vexp : 2 * vexp) - 16);
@@ -834,9 +834,10 @@ cudaError_t run2(lf2_ctx* c, int kind, float* out, const DepositParams& dp, int 
 {
   const unsigned nb = (unsigned)c->g.nbricks;
   if (stage == 0) {
-    PartView pv;
-    cudaError_t e = launch_part_plan(c, FULL2_SMEM, FULL2_THREADS, (size_t)3 * FT3,
-                                     split_max<true>(ACC == ACC_FIXED && c->has_mass ? 2 : 1), &pv);
+    const PartPlan pl = part_plan(c, FULL2_SMEM, FULL2_THREADS, (size_t)3 * FT3,
+                                  split_max<true>(ACC == ACC_FIXED && c->has_mass ? 2 : 1));
+    const PartView pv = part_view(c, pl, (size_t)3 * FT3);
+    cudaError_t e = launch_part_plan(c, pl);
     if (e != cudaSuccess) return e;
     if (ACC == ACC_FIXED) e = launch_vmax(c, pv);
     if (e != cudaSuccess) return e;
@@ -882,8 +883,9 @@ cudaError_t launch_deposit_full(lf2_ctx* c, int kind, float* out, int stage)
   const unsigned nb = (unsigned)c->g.nbricks;
   float* outer = reinterpret_cast<float*>(c->spill);
   if (stage == 0) {
-    PartView pv;
-    cudaError_t e = launch_part_plan(c, FULL_SMEM, FULL_THREADS, (size_t)3 * FT3, 0, &pv);
+    const PartPlan pl = part_plan(c, FULL_SMEM, FULL_THREADS, (size_t)3 * FT3, 0);
+    const PartView pv = part_view(c, pl, (size_t)3 * FT3);
+    cudaError_t e = launch_part_plan(c, pl);
     if (e != cudaSuccess) return e;
     if (kind == 3) return tile_pass<0>(c, out, dp, pv);
     e = tile_pass<1>(c, out, dp, pv);

@@ -83,7 +83,7 @@ struct lf2_ctx {
   int32_t* cap = nullptr;            // [nbricks]
   int32_t* cap_alt = nullptr;        // [nbricks]
   int32_t* fill = nullptr;           // [nbricks] scratch
-  unsigned long long* mov_count = nullptr;
+  unsigned long long* mov_count = nullptr;  // head->mov_count
   unsigned long long* mig = nullptr;  // device [4]: slab migration counters
   uint32_t* flags = nullptr;         // device error bits
   int32_t* repack = nullptr;         // device: 1 when the whole store must be repacked
@@ -104,7 +104,6 @@ struct lf2_ctx {
   size_t spill_slots = 0;
   // parts of heavy bricks (deposit tile passes, lf2_deposit_common.cuh)
   int4* part_item = nullptr;         // [PART_ITEMS] items, [PART_TILES] split bricks
-  int32_t* part_head = nullptr;      // device [3]: items, split bricks, tiles
   uint8_t* part_mark = nullptr;      // [nbricks] 1 when the brick is an item
   double* h_stats = nullptr;         // pinned [8]
   uint32_t* h_flags = nullptr;       // pinned
@@ -114,7 +113,7 @@ struct lf2_ctx {
   int num_sms = 0;
   int move_kernel = 0;               // 0 auto, 1 per-brick k_move, 2 pipelined
   int last_move_kernel = 0;          // kernel of the last kick-drift pass (1 or 2)
-  int* work = nullptr;               // device [2]: brick counter, bricks of move_list; then mov_count
+  lf2::PassHead* head = nullptr;     // device: counters of the pass
   int32_t* move_list = nullptr;      // [nbricks] bricks taken first
   uint8_t* move_mark = nullptr;      // [nbricks] 1 for those
   float* f_rows = nullptr;           // F with rows on 16-byte boundaries (other row lengths)
@@ -166,7 +165,9 @@ cudaError_t launch_state_to_pos(lf2_ctx* c, int64_t n, const int32_t* cell, cons
                                 void* pos3, int real_bytes);
 cudaError_t launch_cell_counts(lf2_ctx* c, int32_t* counts);
 cudaError_t launch_scan_counts(lf2_ctx* c, int64_t* out_start);
-cudaError_t launch_repack(lf2_ctx* c);
+// after launch_insert: relocations, repack; then the plan, if one is given
+// (c->head cleared before the pass)
+cudaError_t launch_repack(lf2_ctx* c, const PartPlan* plan = nullptr);
 cudaError_t launch_heap_reset(lf2_ctx* c);
 
 // lf2_move.cu
@@ -189,16 +190,19 @@ cudaError_t launch_fixup_rim(lf2_ctx* c, float* rho);
 
 // lf2_deposit.cu
 // stage 0: tile pass (k_deposit), stage 1: face fix-up (k_fixup)
+// (planned: the plan of the store as it is was made by launch_repack)
 cudaError_t launch_deposit(lf2_ctx* c, int kind, float* out, int stage,
-                           const uint32_t* gate = nullptr);
+                           const uint32_t* gate = nullptr, bool planned = false);
 DepositParams deposit_params(const lf2_ctx* c);
 // The plan of heavy bricks for a tile pass of `smem` bytes and `threads`
 // threads per CTA, tiles of tile_slots 8-byte values and at most `cap`
-// particles summed in one split tile (0: no such bound); enqueues the plan
-// kernel and fills *pv.
+// particles summed in one split tile (0: no such bound); its view for the
+// kernels; the plan kernel, where no rebin makes the plan.
 struct PartView;
-cudaError_t launch_part_plan(lf2_ctx* c, size_t smem, int threads, size_t tile_slots, int cap,
-                             PartView* pv);
+PartPlan part_plan(lf2_ctx* c, size_t smem, int threads, size_t tile_slots, int cap);
+PartView part_view(const lf2_ctx* c, const PartPlan& pl, size_t tile_slots);
+cudaError_t launch_part_plan(lf2_ctx* c, const PartPlan& pl);
+PartPlan scalar_plan(lf2_ctx* c);
 // largest |v_i| of the store into c->vmax_bits (fixed-point momentum/stress)
 cudaError_t launch_vmax(lf2_ctx* c, const PartView& pv);
 

@@ -418,13 +418,10 @@ cudaError_t launch_move(lf2_ctx* c, const float* F, bool kick, bool drift, MoveP
   return cudaGetLastError();
 }
 
-#ifndef LF2_INS
-#define LF2_INS 8
-#endif
 cudaError_t launch_insert(lf2_ctx* c)
 {
   c->launches += 1;
-  k_insert<<<LF2_INS * 148, 256, 0, c->stream>>>(view(c), c->mov, c->mov_count, c->mov_placed,
+  k_insert<<<148 * 4, 256, 0, c->stream>>>(view(c), c->mov, c->mov_count, c->mov_placed,
                                            c->ovf_list, c->ovf_count, c->ovf_state, c->flags);
   return cudaGetLastError();
 }

@@ -266,10 +266,10 @@ struct DepOut {
   int split_max;     // bricks up to this count accumulate in two 32-bit words
 };
 
-// Order of work of the bricks: head[0] is the counter, head[1] the number of
-// bricks of `list`, which come first; mark[b] tells them from the others.
+// Order of work of the bricks: head->work is the counter; the head->heavy
+// bricks of `list` come first, and mark[b] tells them from the others.
 struct MoveOrder {
-  int* head;
+  PassHead* head;
   const int32_t* list;
   const uint8_t* mark;
 };
@@ -364,10 +364,10 @@ __global__ void __launch_bounds__(WARPS * 32 + 64, 1)
         if (tl_busy[f]) mbar_wait(&tma_f[f], tl_par[f], flags, WAIT_CYCLES);
     };
     // the bricks in their order of work: the listed ones, then the others
-    const int nheavy = order.head[1];
+    const int nheavy = order.head->heavy;
     auto take = [&]() -> long long {
       for (;;) {
-        const long long i = atomicAdd(&order.head[0], 1);
+        const long long i = atomicAdd(&order.head->work, 1);
         if (i < nheavy) return order.list[i];
         if (i - nheavy >= g.nbricks || nheavy == 0 || !order.mark[i - nheavy]) return i - nheavy;
       }
@@ -826,25 +826,16 @@ __global__ void __launch_bounds__(WARPS * 32 + 64, 1)
 }
 
 // The order of work: bricks above `first` particles before the others, so
-// that none of them is left to one SM at the end.  One CTA (which resets the
-// counters of the pass), or several after they have been.
-__global__ void __launch_bounds__(1024) k_move_order(int nb, const int32_t* __restrict__ count,
-                                                     const int32_t* __restrict__ cap, int first,
-                                                     int32_t* list, uint8_t* mark, int* head,
-                                                     unsigned long long* mov_count)
+// that none of them is left to one SM at the end.  The counters are clear.
+__global__ void __launch_bounds__(256) k_move_order(int nb, const int32_t* __restrict__ count,
+                                                    const int32_t* __restrict__ cap, int first,
+                                                    int32_t* list, uint8_t* mark, PassHead* head)
 {
-  if (gridDim.x == 1) {
-    if (threadIdx.x == 0) {
-      head[0] = head[1] = 0;
-      *mov_count = 0ull;
-    }
-    __syncthreads();
-  }
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-    const bool heavy = min(count[b], cap[b]) > first;
-    mark[b] = heavy;
-    if (heavy) list[atomicAdd(&head[1], 1)] = (int32_t)b;
-  }
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= nb) return;
+  const bool heavy = min(count[b], cap[b]) > first;
+  mark[b] = heavy;
+  if (heavy) list[atomicAdd(&head->heavy, 1)] = (int32_t)b;
 }
 
 // `rows` rows of n floats to rows of `pitch` floats, a warp per row.
@@ -1146,20 +1137,22 @@ cudaError_t launch_move_pipe(lf2_ctx* c, const float* F, bool kick, bool drift, 
   // distribution in its order
   const int64_t share = c->np / c->num_sms;
   const int64_t first = std::max(share / 4, 3 * (c->np / c->g.nbricks));
+  e = cudaMemsetAsync(c->head, 0, sizeof(PassHead), c->stream);
+  if (e != cudaSuccess) return e;
+  c->launches += 1;
+  // (no more bricks than SMs: each has its own, whatever the order)
   const int nb = (int)c->g.nbricks;
-  if (nb > 4096) {
-    e = cudaMemsetAsync(c->work, 0, 2 * sizeof(int) + sizeof(unsigned long long), c->stream);
+  if (nb > c->num_sms) {
+    c->launches += 1;
+    k_move_order<<<(nb + 255) / 256, 256, 0, c->stream>>>(nb, c->count, c->cap,
+                                                          (int)std::min<int64_t>(first, INT32_MAX),
+                                                          c->move_list, c->move_mark, c->head);
+    e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
-  c->launches += 2;
-  k_move_order<<<nb > 4096 ? (nb + 1023) / 1024 : 1, 1024, 0, c->stream>>>(
-      nb, c->count, c->cap, (int)std::min<int64_t>(first, INT32_MAX), c->move_list, c->move_mark,
-      c->work, c->mov_count);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
   kern<<<c->num_sms, warps * 32 + 64, smem, c->stream>>>(
       *map, view(c), F, mp, c->mov, c->mov_count, c->brick_maxv2, c->flags,
-      MoveOrder{c->work, c->move_list, c->move_mark}, nst, (int)sb,
+      MoveOrder{c->head, c->move_list, c->move_mark}, nst, (int)sb,
       c->wait_cycles > 0 ? (long long)c->wait_cycles : WAIT_CYCLES, c->wait_stall, d);
   return cudaGetLastError();
 }

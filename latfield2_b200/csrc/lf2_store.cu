@@ -317,6 +317,7 @@ struct RebinTail {
   int32_t* repack;
   uint32_t* flags;
   unsigned long long* diag;
+  PartPlan plan;        // of the deposit that follows (0 items: none)
 };
 
 constexpr int TAIL_THREADS = 1024;
@@ -355,15 +356,21 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) k_rebin_tail(RebinTail t)
   __shared__ int64_t sh[TAIL_THREADS];
   __shared__ long long s_new;
   const int n = *t.nlist;
+  const Geom& g = t.v.g;
+  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  auto plan = [&]() {
+    if (t.plan.max_items)
+      for (int64_t b = i0; b < g.nbricks; b += stride)
+        part_plan_brick(t.plan, (int)b, min(t.v.count[b], t.cap[b]));
+  };
   if (n == 0) {
+    plan();
     if (blockIdx.x == 0 && threadIdx.x == 0) t.diag[1] = *t.mov_count;
     return;
   }
   cooperative_groups::grid_group grid = cooperative_groups::this_grid();
-  const Geom& g = t.v.g;
   const int64_t nm = (int64_t)*t.mov_count;
-  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
 
   // full bricks into new segments
   for (int i = blockIdx.x; i < n; i += gridDim.x) {
@@ -438,6 +445,7 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) k_rebin_tail(RebinTail t)
     }
   }
   grid.sync();
+  plan();
   if (blockIdx.x != 0) return;
   for (int i = threadIdx.x; i < n; i += blockDim.x) t.state[t.list[i]] = 0;
   if (threadIdx.x == 0) {
@@ -566,9 +574,10 @@ cudaError_t launch_heap_reset(lf2_ctx* c)
                          cudaMemcpyDeviceToDevice, c->stream);
 }
 
-cudaError_t launch_repack(lf2_ctx* c)
+cudaError_t launch_repack(lf2_ctx* c, const PartPlan* plan)
 {
   RebinTail t;
+  t.plan = plan ? *plan : PartPlan{};
   t.v = view(c);
   t.alt = c->alt, t.mov = c->mov;
   t.seg_start = c->seg_start, t.cap = c->cap;
