@@ -99,7 +99,9 @@ struct Pass {
 __device__ __forceinline__ float sel(int b, float up, float dn) { return b ? up : dn; }
 
 // ------------------------------------------------------------- tile pass
-template <int KIND, int PASS, int ACC>
+// HM: per-particle masses, or a global one (a kernel each: 1332 us against
+// 1353 for both in one at 512^3).
+template <int KIND, int PASS, int ACC, bool HM>
 __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PASS, ACC>::CTAS)
     k_deposit(StoreView v, DepositParams dp, float* __restrict__ out, uint64_t* __restrict__ spill,
               const uint32_t* __restrict__ vmax_bits, uint32_t* flags, const uint32_t* gate,
@@ -116,10 +118,12 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
   extern __shared__ __align__(16) unsigned char smem_raw[];
 
   __shared__ unsigned s_max[2];
+  __shared__ int s_tile;  // (not a register of the particle loop)
 
   const Geom& g = v.g;
   Part part;
   if (!part_take(pv, g.nbricks, v.count, v.cap, part)) return;
+  if (threadIdx.x == 0) s_tile = part.tile;
   const int64_t b = part.b;
   int bx, by, bz;
   brick_coords(g, b, bx, by, bz);
@@ -128,11 +132,10 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
   const int x0 = bx * BRICK, y0 = by * BRICK, z0 = bz * BRICK;
   const uint32_t base = (uint32_t)(v.seg_start[b] + part.first);  // slots fit in 32 bits
   const int cnt = part.cnt;
-  const int mass_bound =
-      FIXED && dp.has_mass ? part_mass_bound(v.a.mass, base, cnt, dp.inv_unit, s_max) : 1;
+  const int mass_bound = FIXED && HM ? part_mass_bound(v.a.mass, base, cnt, dp.inv_unit, s_max) : 1;
   CompUnit cu{0, false};
   if (ACC == ACC_COMP)
-    cu = comp_unit<KIND>(dp.has_mass ? v.a.mass : nullptr, dp.inv_vol, dp.mf, v.a.vx, v.a.vy, v.a.vz,
+    cu = comp_unit<KIND>(HM ? v.a.mass : nullptr, dp.inv_vol, dp.mf, v.a.vx, v.a.vy, v.a.vz,
                          base, cnt, s_max);
   // two integer words per vertex, or the sums that hold anything
   const bool ints = FIXED ? cnt <= split_max<SIGNED>(mass_bound) : cu.ok;
@@ -155,12 +158,11 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
   }
   __syncthreads();
 
-  // The particle loop, instantiated for the split fixed-point tile (or not)
-  // and for per-particle masses (or a global mass), chosen once per CTA.
+  // The particle loop, instantiated for the tile of two integer words per
+  // vertex or the other one, chosen once per CTA.
   constexpr int ITEMS = P::ITEMS;
-  auto particles = [&](auto split_c, auto hm_c) {
+  auto particles = [&](auto split_c) {
     constexpr bool SPLIT = decltype(split_c)::value;
-    constexpr bool HM = decltype(hm_c)::value;
     for (int c0 = 0; c0 < cnt; c0 += ITEMS * T) {
       uint32_t key[ITEMS];
       float fx[ITEMS], fy[ITEMS], fz[ITEMS], m[ITEMS];
@@ -337,17 +339,12 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
       }
     }
   };
-  const bool hm_rt = dp.has_mass != 0;
-  if (ACC != ACC_PLAIN && tr.split) {
-    if (hm_rt) particles(std::true_type{}, std::true_type{});
-    else particles(std::true_type{}, std::false_type{});
-  } else {
-    if (hm_rt) particles(std::false_type{}, std::true_type{});
-    else particles(std::false_type{}, std::false_type{});
-  }
+  
+  if (ACC != ACC_PLAIN && tr.split) particles(std::true_type{});
+  else particles(std::false_type{});
   __syncthreads();
-  if (uint64_t* scratch = part_tile(pv, NC * TILE3)) {  // k_part_finish writes the vertices
-    part_store<ACC, SIGNED, NC, TILE3>(scratch, tr, cu.e);
+  if (s_tile >= 0) {  // k_part_finish writes the vertices
+    part_store<ACC, SIGNED, NC, TILE3>(scratch_tile(pv, s_tile, NC * TILE3), tr, cu.e);
     return;
   }
 
@@ -503,10 +500,14 @@ struct ShellSum {
 };
 
 constexpr int FIX_FACE = (BRICK - 1) * (BRICK - 1), FIX_EDGE = 3 * (BRICK - 1);
+// CTAs per SM: with more of them (their registers cut to 32) the scalar pass is
+// faster where the L2 holds the shell store (256^3: 30 us against 33) and
+// slower where it does not (512^3: 278 us against 252).
+constexpr int FIX_CTAS = 4;
 constexpr int FIX_THREADS = (FIX_FACE + FIX_EDGE + 1 + 31) & ~31;
 
 template <int KIND, int ACC>
-__global__ void __launch_bounds__(FIX_THREADS)
+__global__ void __launch_bounds__(FIX_THREADS, KIND == 0 ? FIX_CTAS : 1)
     k_fixup(Geom g, const uint64_t* __restrict__ spill, float fixed_scale,
             const uint32_t* __restrict__ vmax_bits, float* __restrict__ out, uint32_t* flags,
             const uint32_t* gate)
@@ -514,7 +515,8 @@ __global__ void __launch_bounds__(FIX_THREADS)
   if (gate && *gate == 0u) return;
   constexpr int CT = Comps<KIND>::value, C = CT < 3 ? CT : 3;  // of the field, of this CTA
   const int c0 = C * blockIdx.y;
-  const int64_t b = blockIdx.x;
+  // the bricks in descending order: the L2 still holds what the tile pass wrote last
+  const int64_t b = gridDim.x - 1 - blockIdx.x;
   int bx, by, bz;
   brick_coords(g, b, bx, by, bz);
   const int e[3] = {brick_extent(g.n[0], bx), brick_extent(g.n[1], by), brick_extent(g.n[2], bz)};
@@ -655,11 +657,11 @@ cudaError_t tile_pass(lf2_ctx* c, float* out, const DepositParams& dp, const uin
 {
   using P = Pass<KIND, PASS, ACC>;
   const size_t smem = P::smem();
-  cudaError_t e = cudaFuncSetAttribute(k_deposit<KIND, PASS, ACC>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const auto kern = dp.has_mass ? k_deposit<KIND, PASS, ACC, true> : k_deposit<KIND, PASS, ACC, false>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   c->launches += 1;
-  k_deposit<KIND, PASS, ACC><<<(unsigned)(c->g.nbricks + pv.max_items), P::THREADS, smem, c->stream>>>(
+  kern<<<(unsigned)(c->g.nbricks + pv.max_items), P::THREADS, smem, c->stream>>>(
       view(c), dp, out, c->spill, c->vmax_bits, c->flags, gate, pv);
   if (!pv.max_items) return cudaGetLastError();
   c->launches += 1;

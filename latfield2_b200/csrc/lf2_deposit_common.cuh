@@ -390,37 +390,39 @@ __device__ __forceinline__ int part_items(const PartView& pv)
 struct Part {
   int64_t b;
   int first, cnt;
+  int tile;  // scratch tile of a part of a split brick, or -1
 };
 
 // The unit of this CTA in a grid of nbricks + max_items: the items, then the
 // bricks in their order; false where there is none or the brick is an item.
+// The brick's counts are read with the number of items, as if there were
+// none, so that a plan without items (the ordinary one) costs a CTA one trip
+// to memory and not two.
 __device__ __forceinline__ bool part_take(const PartView& pv, int64_t nbricks, const int32_t* count,
                                           const int32_t* cap, Part& p)
 {
-  const int i = (int)blockIdx.x, items = part_items(pv);
-  p.first = 0;
+  const int i = (int)blockIdx.x;
+  p.first = 0, p.tile = -1;
+  p.cnt = i < nbricks ? min(count[i], cap[i]) : 0;
+  const int items = part_items(pv);
+  p.b = i - items;
   if (i >= items) {
-    p.b = i - items;
-    if (p.b >= nbricks || (items && pv.mark[p.b])) return false;
-    p.cnt = min(count[p.b], cap[p.b]);
+    if (p.b >= nbricks) return false;
+    if (items) {
+      if (pv.mark[p.b]) return false;
+      p.cnt = min(count[p.b], cap[p.b]);
+    }
     return true;
   }
   const int4 w = pv.item[i];
   p.b = w.x;
   if (w.x < 0) return false;
   const int64_t n = min(count[p.b], cap[p.b]);
-  p.first = (int)(n * w.y / w.z) & ~3;  // parts start on 16-byte boundaries
-  p.cnt = (w.y + 1 == w.z ? (int)n : (int)(n * (w.y + 1) / w.z) & ~3) - p.first;
+  const int k = w.y;
+  p.first = (int)(n * k / w.z) & ~3;  // parts start on 16-byte boundaries
+  p.cnt = (k + 1 == w.z ? (int)n : (int)(n * (k + 1) / w.z) & ~3) - p.first;
+  if (w.z > 1) p.tile = w.w + k;
   return true;
-}
-
-// The scratch tile of this CTA's unit when that is a part of a split brick
-// (read again here, so that the particle loop keeps no register for it).
-__device__ __forceinline__ uint64_t* part_tile(const PartView& pv, int slots)
-{
-  if ((int)blockIdx.x >= part_items(pv)) return nullptr;
-  const int4 w = pv.item[blockIdx.x];
-  return w.z > 1 ? scratch_tile(pv, w.w + w.y, slots) : nullptr;
 }
 
 // A part's tile to the scratch: 8-byte values, component j of vertex t at

@@ -122,10 +122,12 @@ __global__ void __launch_bounds__(FULL_THREADS)
 {
   constexpr int CT = FullPass<PASS>::total;
   extern __shared__ __align__(16) float tile[];
+  __shared__ int s_tile;
 
   const Geom& g = v.g;
   Part part;
   if (!part_take(pv, g.nbricks, v.count, v.cap, part)) return;
+  if (threadIdx.x == 0) s_tile = part.tile;
   const int64_t b = part.b;
   int bx, by, bz;
   brick_coords(g, b, bx, by, bz);
@@ -219,9 +221,9 @@ __global__ void __launch_bounds__(FULL_THREADS)
     }
   }
   __syncthreads();
-  if (uint64_t* scratch = part_tile(pv, 3 * FT3)) {  // k_part_finish_full sums the parts and writes the vertices
-    part_store<ACC_PLAIN, true, 3, FT3>(
-        scratch, TileRef<FT3>{reinterpret_cast<unsigned char*>(tile), false}, 0);
+  if (s_tile >= 0) {  // k_part_finish_full writes the vertices
+    part_store<ACC_PLAIN, true, 3, FT3>(scratch_tile(pv, s_tile, 3 * FT3),
+                                        TileRef<FT3>{reinterpret_cast<unsigned char*>(tile), false}, 0);
     return;
   }
 
@@ -334,8 +336,9 @@ __global__ void __launch_bounds__(256, 4)
 #endif
 constexpr int FULL2_THREADS = LF2_FULL2_THREADS;
 
-template <int PASS, int ACC>
-__global__ void __launch_bounds__(FULL2_THREADS)
+// HM: per-particle masses, or a global one.
+template <int PASS, int ACC, bool HM>
+__global__ void __launch_bounds__(FULL2_THREADS, 1)
     k_deposit_full2(StoreView v, DepositParams dp, float* __restrict__ out,
                     uint64_t* __restrict__ store, const uint32_t* __restrict__ vmax_bits,
                     uint32_t* flags, PartView pv)
@@ -344,23 +347,21 @@ __global__ void __launch_bounds__(FULL2_THREADS)
   constexpr bool FIXED = ACC == ACC_FIXED;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned s_max[2];
+  __shared__ int s_brick, s_tile;  // (so that the particle loop keeps no register for them)
 
   const Geom& g = v.g;
   Part part;
   if (!part_take(pv, g.nbricks, v.count, v.cap, part)) return;
-  const int64_t b = part.b;
+  if (threadIdx.x == 0) s_brick = (int)part.b, s_tile = part.tile;
   int bx, by, bz;
-  brick_coords(g, b, bx, by, bz);
-  const int e[3] = {brick_extent(g.n[0], bx), brick_extent(g.n[1], by),
-                    brick_extent(g.n[2], bz)};
+  brick_coords(g, part.b, bx, by, bz);
   const int x0 = bx * BRICK, y0 = by * BRICK, z0 = bz * BRICK;
-  const int64_t base = v.seg_start[b] + part.first;
+  const int64_t base = v.seg_start[part.b] + part.first;
   const int cnt = part.cnt;
-  const int mass_bound =
-      FIXED && dp.has_mass ? part_mass_bound(v.a.mass, (uint32_t)base, cnt, dp.inv_unit, s_max) : 1;
+  const int mass_bound = FIXED && HM ? part_mass_bound(v.a.mass, (uint32_t)base, cnt, dp.inv_unit, s_max) : 1;
   CompUnit cu{0, false};
   if (!FIXED)
-    cu = comp_unit<PASS == 0 ? 1 : 2>(dp.has_mass ? v.a.mass : nullptr, dp.inv_vol, dp.mf, v.a.vx, v.a.vy,
+    cu = comp_unit<PASS == 0 ? 1 : 2>(HM ? v.a.mass : nullptr, dp.inv_vol, dp.mf, v.a.vx, v.a.vy,
                                       v.a.vz, (uint32_t)base, cnt, s_max);
   TileRef<FT3> tr{smem_raw, FIXED ? cnt <= split_max<true>(mass_bound) : cu.ok};
   const float unit = !FIXED && cu.ok ? ldexpf(1.0f, 16 - cu.e) : 1.0f;
@@ -368,7 +369,7 @@ __global__ void __launch_bounds__(FULL2_THREADS)
   if (FIXED) vexp = vexp_of(*vmax_bits);
   const float vscale = vel_scale(vexp);
   const float conv = FIXED ? ldexpf(dp.fixed_scale, (PASS == 0 ? vexp : 2 * vexp) - 16) : 0.0f;
-  if (FIXED && threadIdx.x == 0 && b == 0 && !(conv > 0.0f && conv <= 3.402823466e38f))
+  if (FIXED && threadIdx.x == 0 && part.b == 0 && !(conv > 0.0f && conv <= 3.402823466e38f))
     set_flag(flags, ERR_FIXED_OVERFLOW);
 
   {
@@ -378,11 +379,9 @@ __global__ void __launch_bounds__(FULL2_THREADS)
   __syncthreads();
 
   constexpr int pa[3] = {0, 0, 1}, pb[3] = {1, 2, 2};
-  // the particle loop, instantiated per CTA for the split tile (or not) and
-  // for per-particle masses (or a global mass)
-  auto particles = [&](auto split_c, auto hm_c) {
+  // the particle loop, instantiated per CTA for the split tile (or not)
+  auto particles = [&](auto split_c) {
     constexpr bool SPLIT = decltype(split_c)::value;
-    constexpr bool HM = decltype(hm_c)::value;
     for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
       const uint32_t p = (uint32_t)base + (uint32_t)i;  // slots fit in 32 bits
       int x, y, z;
@@ -527,20 +526,18 @@ __global__ void __launch_bounds__(FULL2_THREADS)
       }
     }
   };
-  const bool hm_rt = dp.has_mass != 0;
-  if (tr.split) {
-    if (hm_rt) particles(std::true_type{}, std::true_type{});
-    else particles(std::true_type{}, std::false_type{});
-  } else {
-    if (hm_rt) particles(std::false_type{}, std::true_type{});
-    else particles(std::false_type{}, std::false_type{});
-  }
+  if (tr.split) particles(std::true_type{});
+  else particles(std::false_type{});
   __syncthreads();
-  if (uint64_t* scratch = part_tile(pv, 3 * FT3)) {
-    part_store<ACC, true, 3, FT3>(scratch, tr, cu.e);
+  if (s_tile >= 0) {
+    part_store<ACC, true, 3, FT3>(scratch_tile(pv, s_tile, 3 * FT3), tr, cu.e);
     return;
   }
 
+  const int64_t b = s_brick;
+  brick_coords(g, b, bx, by, bz);
+  const int e[3] = {brick_extent(g.n[0], bx), brick_extent(g.n[1], by),
+                    brick_extent(g.n[2], bz)};
   // Flush: private vertices (every tile coordinate in [2, e-1]) to the field,
   // the thick shell to the store.
   uint64_t* st = store + (size_t)b * CT * FSHELL;
@@ -549,7 +546,8 @@ __global__ void __launch_bounds__(FULL2_THREADS)
     if (t0 > e[0] + 1 || t1 > e[1] + 1 || t2 > e[2] + 1) continue;
     const bool priv = t0 >= 2 && t0 < e[0] && t1 >= 2 && t1 < e[1] && t2 >= 2 && t2 < e[2];
     const int si = priv ? 0 : thick_index(canon(t0, e[0]), canon(t1, e[1]), canon(t2, e[2]));
-    const int64_t site = priv ? site_index(g, x0 + t0 - 1, y0 + t1 - 1, z0 + t2 - 1) : 0;
+    const int64_t site =
+        priv ? site_index(g, bx * BRICK + t0 - 1, by * BRICK + t1 - 1, bz * BRICK + t2 - 1) : 0;
 #pragma unroll
     for (int j = 0; j < 3; j++) {
       const int c = FullPass<PASS>::comp(j);
@@ -819,13 +817,12 @@ template <int PASS, int ACC>
 cudaError_t tile_pass2(lf2_ctx* c, float* out, const DepositParams& dp, const PartView& pv)
 {
   constexpr size_t smem = FULL2_SMEM;
-  cudaError_t e = cudaFuncSetAttribute(k_deposit_full2<PASS, ACC>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const auto kern = dp.has_mass ? k_deposit_full2<PASS, ACC, true> : k_deposit_full2<PASS, ACC, false>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   c->launches += 1;
-  k_deposit_full2<PASS, ACC>
-      <<<(unsigned)(c->g.nbricks + pv.max_items), FULL2_THREADS, smem, c->stream>>>(
-          view(c), dp, out, c->spill, c->vmax_bits, c->flags, pv);
+  kern<<<(unsigned)(c->g.nbricks + pv.max_items), FULL2_THREADS, smem, c->stream>>>(
+      view(c), dp, out, c->spill, c->vmax_bits, c->flags, pv);
   return finish<PASS, ACC>(c, out, dp, pv);
 }
 

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from tests.helpers import precision, small_case
+from tests.helpers import by_id, precision, small_case
 from tests.test_gpu_precision import KINDS, _ctx, _deposit, _fp64
 
 pytestmark = pytest.mark.gpu
@@ -130,4 +130,40 @@ def test_compensated_sums_with_a_wide_range_of_masses(cuda):
     sel = ref > 1e-9 * 8000
     # three FP32 products and the rounding of the sum: 4 ulp of 2^-24
     assert np.max(np.abs(got[sel] - ref[sel]) / ref[sel]) < 4 * 2.0 ** -24 + 8 * 2.0 ** -48 / 1e-9
+    ctx.close()
+
+
+def test_more_bricks_than_a_load_counts_in_shared_memory(cuda):
+    """51,201 bricks: the load counts in global memory, the plan of heavy bricks
+    and the move's order take several CTAs, and the rebin tail plans the scalar
+    deposit.  Bit-exact against the oracle before and after a step."""
+    import torch
+    n = (2, 2, 16 * 51201)
+    rng = np.random.default_rng(6)
+    z = np.concatenate([rng.integers(0, n[2], 20000), 16 * 40000 + rng.integers(0, 16, 15000),
+                        16 * 51200 + rng.integers(0, 16, 5000)])
+    npart = z.size
+    cell = (rng.integers(0, 2, npart) + 2 * (rng.integers(0, 2, npart) + 2 * z)).astype(np.int32)
+    off = (rng.random((npart, 3)) * (1 - 2.0 ** -23)).astype(np.float32)
+    vel = (0.2 * rng.standard_normal((npart, 3))).astype(np.float32)
+    gm = 1.0 / npart
+    ctx = _ctx(n, 1)
+    ctx.set_particles(cell, off, vel, ids=np.arange(npart, dtype=np.int64), global_mass=gm)
+    scale = np.float32(2.0 ** -32 * gm / 0.5 ** 3)
+    f, v = ctx.field(1), ctx.field(3)
+
+    def check(field, c, o):
+        np.testing.assert_array_equal(field.export_internal().reshape(-1),
+                                      O.fixed_to_f32(O.state_deposit_fixed(n, c, o), scale))
+    ctx.deposit_scalar(f)
+    check(f, cell, off)
+    ctx.deposit_vector(v)
+    acc, e = O.state_deposit_fixed_kind(1, n, cell, off, vel)
+    np.testing.assert_array_equal(v.export_internal(), O.fixed_kind_to_f32(acc, 1, e, gm, 0.5))
+    F = torch.from_numpy(rng.standard_normal((3, n[2], n[1], n[0])).astype(np.float32)).cuda()
+    ctx.step(ctx.field(3, F), 0.05, 0.3, f)
+    s = ctx.get_particles(ids=True)
+    assert not np.array_equal(by_id(s)["cell"], cell)
+    check(f, s["cell"], s["off"])
+    assert ctx.flags() & ~0x8 == 0
     ctx.close()
