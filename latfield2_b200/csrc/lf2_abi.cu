@@ -337,6 +337,7 @@ lf2_status lf2_create(lf2_ctx** out, int device, const int n[3], const double bo
   ok = ok && cudaMalloc(&c->part_item, sizeof(int4) * (PART_ITEMS + PART_TILES)) == cudaSuccess;
   ok = ok && cudaMalloc(&c->part_mark, (size_t)nb) == cudaSuccess;
   ok = ok && cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess;
+  ok = ok && cudaMalloc(&c->loss_part, sizeof(double) * loss_ctas(c)) == cudaSuccess;
   if (ok) {
     ok = cudaMemsetAsync(c->count, 0, sizeof(int32_t) * nb, c->stream) == cudaSuccess &&
          cudaMemsetAsync(c->cap, 0, sizeof(int32_t) * nb, c->stream) == cudaSuccess &&
@@ -1287,11 +1288,6 @@ lf2_status lf2_pm_loss(lf2_ctx* c, const float* w, const float* rho, double* los
 {
   if (!c || !w || !rho || !loss) return LF2_ERR_ARG;
   PhaseScope ps(c, PH_OTHER);
-  if (!c->loss_part && cudaMalloc(&c->loss_part, sizeof(double) * loss_ctas(c)) != cudaSuccess) {
-    cudaGetLastError();
-    c->loss_part = nullptr;
-    return fail(c, LF2_ERR_NOMEM, "cannot allocate the loss's partial sums");
-  }
   LF2_CUDA(c, launch_pm_loss(c, w, rho, loss));
   return LF2_OK;
 }

@@ -1053,6 +1053,9 @@ bool move_pipe_auto(lf2_ctx* c, const float* F)
     if (c->g.n[d] < 2 * BRICK) return false;
   if (!encode_fn() || 3 * c->np < c->g.nsites) return false;
   if (!c->f_rows) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
+      return false;  // no allocation under capture
     const size_t floats = (size_t)3 * padded_row(c) * c->g.n[1] * c->g.n[2];
     if (cudaMalloc(&c->f_rows, floats * sizeof(float)) != cudaSuccess) {
       cudaGetLastError();

@@ -89,3 +89,44 @@ def test_field_off_the_16_byte_boundary_and_sparse_stores(cuda):
     F2 = torch.zeros(3, 40, 36, 33, device="cuda")
     c.step(c.field(3, F2), 0.05, 0.3)
     assert c.last_move_kernel() == 1
+
+
+@pytest.mark.parametrize("warm", [False, True])
+def test_kick_drift_and_deposit_under_capture(cuda, warm):
+    """Captured calls allocate nothing: the first kick of a context on padded
+    rows keeps the per-brick kernel, a later one takes the pipelined one.  The
+    replayed graph moves the particles as the same calls outside one."""
+    import torch
+    import latfield2_b200 as L
+    n, npart = (50, 32, 48), 60000
+    cell, off, vel = small_case(n, npart, seed=19, vel_sigma=0.05, clustered=True)
+    F = torch.from_numpy(np.random.default_rng(5).standard_normal((3, n[2], n[1], n[0])).astype(np.float32)).cuda()
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    ctxs = []
+    for stream in (None, s.cuda_stream):
+        ctx = L.Context(n, box=tuple(v / n[0] for v in n), mode=1, stream=stream)
+        ctx.set_particles(cell, off, vel, ids=np.arange(npart, dtype=np.int64), global_mass=1.0 / npart)
+        f, rho = ctx.field(3, F), ctx.field(1)
+        ctx.deposit_scalar(rho)  # (its scratch)
+
+        def passes(ctx=ctx, f=f, rho=rho):
+            ctx.gather_kick(f, 0.05)
+            ctx.drift_rebin(0.3)
+            ctx.deposit_scalar(rho)
+        if warm:
+            passes()
+        ctxs.append((ctx, passes, rho))
+    (a, pass_a, rho_a), (b, pass_b, rho_b) = ctxs
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        pass_b()
+    for _ in range(3):
+        pass_a()
+        with torch.cuda.stream(s):
+            graph.replay()
+    torch.cuda.synchronize()
+    _same(a, b, False)
+    np.testing.assert_array_equal(rho_a.export_internal(), rho_b.export_internal())
+    assert a.flags() & ~0x8 == 0 and b.flags() & ~0x8 == 0
