@@ -959,10 +959,11 @@ def main():
     ms, value = replica_throughput(ms, npart, args.steps, pg, device)
     ms_step = ms / args.steps
 
-    # dominant kernel and its roofline (algorithmic bytes per launch / mean launch time)
+    # dominant kernel and its roofline (algorithmic bytes per launch / mean time of its phase,
+    # which has one launch of it per step and the small ones that prepare or finish it)
     peak, peak_kind = peaks()
     dom = max(("move", "deposit_tile"), key=lambda p: phases[p][0])
-    per_launch_ms = phases[dom][0] / max(1, phases[dom][1])
+    per_launch_ms = phases[dom][0] / args.steps
     mk = ctx.last_move_kernel()
     if dom == "move":
         ab = alg_bytes_move(npart, nsites)
