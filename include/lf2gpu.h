@@ -59,10 +59,10 @@ typedef int lf2_status;
 #define LF2_ERR_NOMEM (-4)       /* device allocation failed */
 #define LF2_ERR_UNSUPPORTED (-5) /* combination not provided */
 
-/* Deposit modes (lf2_create).  FP32: FP32 atomics whose rounding errors are
- * recovered exactly and carried in a second FP32 word, so every vertex sum
- * is within about 1e-7 of exact whatever the order (not bit-identical run to
- * run).  FIXED64: int64 fixed point, bit-exact run to run; quantum 2^-32 of
+/* Deposit modes (lf2_create).  FP32: FP32 terms in a compensated sum (wide
+ * integers, or FP32 additions whose rounding errors are recovered exactly and
+ * carried in a second FP32 word), so every vertex sum is within about 1e-7 of
+ * exact whatever the order (not bit-identical run to run).  FIXED64: int64 fixed point, bit-exact run to run; quantum 2^-32 of
  * a unit mass (the global particle mass, or the mean of per-particle
  * masses) for the density, 2^-48 of a unit mass times V for momentum and
  * times V^2 for stress, V the smallest power of two above every |v_i| of the

@@ -16,7 +16,7 @@ LF2_ERR_STATE = -3
 LF2_ERR_NOMEM = -4
 LF2_ERR_UNSUPPORTED = -5
 
-DEPOSIT_FP32 = 0        # FP32 atomics with compensated (TwoSum) rounding errors
+DEPOSIT_FP32 = 0        # FP32 terms, compensated sums
 DEPOSIT_FIXED64 = 1     # int64 fixed point, bit-exact run to run
 DEPOSIT_FP32_PLAIN = 2  # FP32 atomics without compensation (the speed reference)
 FFT_FORWARD = 1

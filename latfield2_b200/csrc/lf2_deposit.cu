@@ -18,12 +18,15 @@
 // atomics are used.
 //
 // Three accumulation modes (the context's deposit mode):
-//   LF2_DEPOSIT_FP32        FP32 shared atomics with compensation: each add
-//                           returns the value it replaced, the rounding error
-//                           of that add is recovered exactly (TwoSum) and
-//                           accumulated in a second FP32 word.  hi + lo is the
-//                           sum to within the rounding of the terms (about
-//                           1e-7 relative), whatever the order.
+//   LF2_DEPOSIT_FP32        the reference's FP32 terms, their sum compensated:
+//                           integers in a unit set by the part's largest term
+//                           (add_comp_int), or, where that range does not
+//                           hold, FP32 atomics that return the value they
+//                           replaced, the rounding error of each recovered
+//                           exactly (TwoSum) and accumulated in a second FP32
+//                           word.  hi + lo is the sum to within the rounding
+//                           of the terms (about 1e-7 relative), whatever the
+//                           order.
 //   LF2_DEPOSIT_FIXED64     int64 fixed point: every contribution is rounded
 //                           once, deterministically, to an integer quantum;
 //                           the integer sums do not depend on the order, so
@@ -49,22 +52,12 @@ namespace lf2 {
 
 namespace {
 
-#ifndef LF2_DEP_THREADS
-#define LF2_DEP_THREADS 256
-#endif
-constexpr int DEP_THREADS = LF2_DEP_THREADS;
-// ... and of a tile that leaves room for one CTA per SM
-#ifndef LF2_DEP_BIG
-#define LF2_DEP_BIG 1024
-#endif
-#ifndef LF2_DEP_BIG_ITEMS
-#define LF2_DEP_BIG_ITEMS 2
-#endif
+// Threads of a tile pass, and of one whose tile leaves room for one CTA per SM
+//.
+constexpr int DEP_THREADS = 256, DEP_BIG_THREADS = 1024;
 
 // Fewest particles of a part of a split brick.
-#ifndef LF2_PART_MIN
-#define LF2_PART_MIN 4096
-#endif
+constexpr int64_t PART_MIN = 4096;
 
 // Components of the field of a kind.
 template <int KIND>
@@ -88,10 +81,9 @@ struct Pass {
                                          : (j == 0 ? 1 : j == 1 ? 2 : 4);
   }
   static constexpr size_t smem() { return (size_t)NC * WORDS * TILE3 * 4; }
-  // threads per CTA: a tile above 100 KB leaves room for one CTA per SM, so
-  // it gets twice the warps
-  static constexpr int THREADS = smem() > 100 * 1024 ? LF2_DEP_BIG : DEP_THREADS;
-  static constexpr int ITEMS = smem() > 100 * 1024 ? LF2_DEP_BIG_ITEMS : 4;  // particles in flight per thread
+  // a tile above 100 KB leaves room for one CTA per SM
+  static constexpr int THREADS = smem() > 100 * 1024 ? DEP_BIG_THREADS : DEP_THREADS;
+  static constexpr int ITEMS = smem() > 100 * 1024 ? 2 : 4;  // particles in flight per thread
   // CTAs per SM that the registers leave room for: those whose tiles fit
   static constexpr int CTAS = smem() > 100 * 1024 ? 1 : smem() > 50 * 1024 ? 3 : 5;
 };
@@ -122,7 +114,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
 
   const Geom& g = v.g;
   Part part;
-  if (!part_take(pv, g.nbricks, v.count, v.cap, part)) return;
+  if (!part_take(pv, g.nbricks, v.count, v.cap, v.seg_start, part)) return;
   if (threadIdx.x == 0) s_tile = part.tile;
   const int64_t b = part.b;
   int bx, by, bz;
@@ -130,7 +122,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
   const int ex = brick_extent(g.n[0], bx), ey = brick_extent(g.n[1], by),
             ez = brick_extent(g.n[2], bz);
   const int x0 = bx * BRICK, y0 = by * BRICK, z0 = bz * BRICK;
-  const uint32_t base = (uint32_t)(v.seg_start[b] + part.first);  // slots fit in 32 bits
+  const uint32_t base = (uint32_t)(part.start + part.first);  // slots fit in 32 bits
   const int cnt = part.cnt;
   const int mass_bound = FIXED && HM ? part_mass_bound(v.a.mass, base, cnt, dp.inv_unit, s_max) : 1;
   CompUnit cu{0, false};
@@ -474,7 +466,9 @@ __global__ void __launch_bounds__(FINISH_CHUNK) k_part_finish(Geom g, PartView p
 // runs in that fixed order: exact integers (fixed point), a compensated FP32
 // sum of the hi and lo words, or plain FP32 additions.
 //
-// The pass is bound by the latency of its scattered reads.  675 of the 721
+// The pass is bound by its scattered reads and the partial sectors it writes:
+// at 512^3 about 1.1 GB of traffic (160 us) in 252 us (263 with two vertices
+// of any kind per thread), at 256^3 33 us (41).  675 of the 721
 // vertices lie inside one of the three faces and have one neighbour: thread
 // t < 225 takes vertex t of each face, so that all its reads (two per face
 // and component, at fixed offsets from one another) are in flight together;
@@ -604,9 +598,9 @@ __global__ void __launch_bounds__(FIX_THREADS, KIND == 0 ? FIX_CTAS : 1)
 __global__ void __launch_bounds__(256) k_vmax(StoreView v, uint32_t* vmax_bits, uint32_t* flags, PartView pv)
 {
   Part part;  // the tile passes' units, so that no CTA reads a heavy brick alone
-  if (!part_take(pv, v.g.nbricks, v.count, v.cap, part)) return;
+  if (!part_take(pv, v.g.nbricks, v.count, v.cap, v.seg_start, part)) return;
   // four slots per load: segments and parts start on multiples of four
-  const int64_t base = v.seg_start[part.b] + part.first;
+  const int64_t base = part.start + part.first;
   const float* const comp[3] = {v.a.vx + base, v.a.vy + base, v.a.vz + base};
   uint32_t m = 0u;
 #pragma unroll 4
@@ -703,8 +697,8 @@ cudaError_t run(lf2_ctx* c, float* out, const DepositParams& dp, int stage, cons
     return e;
   }
   c->launches += 1;
-  k_fixup<KIND, ACC><<<dim3(nb, KIND == 2 ? 2 : 1), FIX_THREADS, 0, c->stream>>>(c->g, c->spill, dp.fixed_scale, c->vmax_bits, out,
-                                                c->flags, gate);
+  k_fixup<KIND, ACC><<<dim3(nb, KIND == 2 ? 2 : 1), FIX_THREADS, 0, c->stream>>>(
+      c->g, c->spill, dp.fixed_scale, c->vmax_bits, out, c->flags, gate);
   return cudaGetLastError();
 }
 
@@ -724,7 +718,7 @@ cudaError_t run_mode(lf2_ctx* c, float* out, const DepositParams& dp, int stage,
 // share (a brick that starts last then ends with the others) and three times
 // the mean count (an even distribution has no items).  It is split above 3/2 P
 // with P half the share, so that no CTA is left with more than that, but parts
-// hold at least LF2_PART_MIN particles: each clears and writes its tile (parts
+// hold at least PART_MIN particles: each clears and writes its tile (parts
 // of 1024 took 41 us for 64 uniform bricks of 4096 against 35 unsplit).
 // `cap` bounds what a split fixed-point tile sums.  The scratch tiles lie in
 // the repack scratch (c->alt), which nothing uses between the rebins.
@@ -739,7 +733,7 @@ PartPlan part_plan(lf2_ctx* c, size_t smem, int threads, size_t tile_slots, int 
   const int per_sm = std::max(1, std::min((int)(227 * 1024 / (smem + 1024)), 2048 / threads));
   const int64_t share = c->np / ((int64_t)c->num_sms * per_sm);
   if (cap <= 0) cap = 1 << 28;
-  const int64_t P = std::min<int64_t>(std::max<int64_t>(share / 2, LF2_PART_MIN), cap - cap / 16);
+  const int64_t P = std::min<int64_t>(std::max<int64_t>(share / 2, PART_MIN), cap - cap / 16);
   const int64_t split = std::min<int64_t>(P + P / 2, cap);
   const int64_t first = std::min(split, std::max(share / 4, 3 * (c->np / c->g.nbricks)));
   pl.P = (int)P, pl.split = (int)split, pl.first = (int)first;

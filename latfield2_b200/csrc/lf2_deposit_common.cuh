@@ -388,22 +388,23 @@ __device__ __forceinline__ int part_items(const PartView& pv)
 
 // One unit of work of a tile pass: particles [first, first + cnt) of a brick.
 struct Part {
-  int64_t b;
+  int64_t b, start;  // the brick, and its first slot
   int first, cnt;
   int tile;  // scratch tile of a part of a split brick, or -1
 };
 
 // The unit of this CTA in a grid of nbricks + max_items: the items, then the
 // bricks in their order; false where there is none or the brick is an item.
-// The brick's counts are read with the number of items, as if there were
-// none, so that a plan without items (the ordinary one) costs a CTA one trip
-// to memory and not two.
+// The brick's counts and first slot are read with the number of items, as if
+// there were none, so that a plan without items (the ordinary one) costs a CTA
+// one trip to memory and not three.
 __device__ __forceinline__ bool part_take(const PartView& pv, int64_t nbricks, const int32_t* count,
-                                          const int32_t* cap, Part& p)
+                                          const int32_t* cap, const int64_t* seg_start, Part& p)
 {
   const int i = (int)blockIdx.x;
   p.first = 0, p.tile = -1;
   p.cnt = i < nbricks ? min(count[i], cap[i]) : 0;
+  p.start = i < nbricks ? seg_start[i] : 0;
   const int items = part_items(pv);
   p.b = i - items;
   if (i >= items) {
@@ -411,6 +412,7 @@ __device__ __forceinline__ bool part_take(const PartView& pv, int64_t nbricks, c
     if (items) {
       if (pv.mark[p.b]) return false;
       p.cnt = min(count[p.b], cap[p.b]);
+      p.start = seg_start[p.b];
     }
     return true;
   }
@@ -418,6 +420,7 @@ __device__ __forceinline__ bool part_take(const PartView& pv, int64_t nbricks, c
   p.b = w.x;
   if (w.x < 0) return false;
   const int64_t n = min(count[p.b], cap[p.b]);
+  p.start = seg_start[p.b];
   const int k = w.y;
   p.first = (int)(n * k / w.z) & ~3;  // parts start on 16-byte boundaries
   p.cnt = (k + 1 == w.z ? (int)n : (int)(n * (k + 1) / w.z) & ~3) - p.first;

@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(FULL_THREADS)
 
   const Geom& g = v.g;
   Part part;
-  if (!part_take(pv, g.nbricks, v.count, v.cap, part)) return;
+  if (!part_take(pv, g.nbricks, v.count, v.cap, v.seg_start, part)) return;
   if (threadIdx.x == 0) s_tile = part.tile;
   const int64_t b = part.b;
   int bx, by, bz;
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(FULL_THREADS)
   const int e[3] = {brick_extent(g.n[0], bx), brick_extent(g.n[1], by),
                     brick_extent(g.n[2], bz)};
   const int x0 = bx * BRICK, y0 = by * BRICK, z0 = bz * BRICK;
-  const int64_t base = v.seg_start[b] + part.first;
+  const int64_t base = part.start + part.first;
   const int cnt = part.cnt;
 
   for (int t = threadIdx.x; t < 3 * FT3; t += blockDim.x) tile[t] = 0.0f;
@@ -329,12 +329,11 @@ __global__ void __launch_bounds__(256, 4)
 
 // Compensated FP32 and fixed-point tile pass: the same weights and vertices
 // as k_deposit_full, two words per vertex (140 KB for three components, one
-// CTA per SM with 512 threads), and every vertex another brick can reach goes
-// to the thick-shell store.
-#ifndef LF2_FULL2_THREADS
-#define LF2_FULL2_THREADS 1024
-#endif
-constexpr int FULL2_THREADS = LF2_FULL2_THREADS;
+// CTA per SM), and every vertex another brick can reach goes to the
+// thick-shell store.  The three passes of the compensated mode at 256^3 took
+// 9.96 ms with FP32 atomics (their compare-and-swap loops: 26% issue) and one
+// CTA per brick; with the integer sums and split bricks 2.68 ms.
+constexpr int FULL2_THREADS = 1024;
 
 // HM: per-particle masses, or a global one.
 template <int PASS, int ACC, bool HM>
@@ -351,12 +350,12 @@ __global__ void __launch_bounds__(FULL2_THREADS, 1)
 
   const Geom& g = v.g;
   Part part;
-  if (!part_take(pv, g.nbricks, v.count, v.cap, part)) return;
+  if (!part_take(pv, g.nbricks, v.count, v.cap, v.seg_start, part)) return;
   if (threadIdx.x == 0) s_brick = (int)part.b, s_tile = part.tile;
   int bx, by, bz;
   brick_coords(g, part.b, bx, by, bz);
   const int x0 = bx * BRICK, y0 = by * BRICK, z0 = bz * BRICK;
-  const int64_t base = v.seg_start[part.b] + part.first;
+  const int64_t base = part.start + part.first;
   const int cnt = part.cnt;
   const int mass_bound = FIXED && HM ? part_mass_bound(v.a.mass, (uint32_t)base, cnt, dp.inv_unit, s_max) : 1;
   CompUnit cu{0, false};
