@@ -56,8 +56,9 @@ namespace {
 //.
 constexpr int DEP_THREADS = 256, DEP_BIG_THREADS = 1024;
 
-// Fewest particles of a part of a split brick.
-constexpr int64_t PART_MIN = 4096;
+// Fewest particles of a part of a split brick, and of any item (a brick below
+// that ends soon wherever it starts: four trips of a CTA's threads at most).
+constexpr int64_t PART_MIN = 4096, ITEM_MIN = 1024;
 
 // Components of the field of a kind.
 template <int KIND>
@@ -715,11 +716,13 @@ cudaError_t run_mode(lf2_ctx* c, float* out, const DepositParams& dp, int stage,
 
 // What is heavy depends on the chip's share of the particles per CTA that runs
 // at once (`share`).  A brick is an item, taken first, above a quarter of the
-// share (a brick that starts last then ends with the others) and three times
-// the mean count (an even distribution has no items).  It is split above 3/2 P
-// with P half the share, so that no CTA is left with more than that, but parts
-// hold at least PART_MIN particles: each clears and writes its tile (parts
-// of 1024 took 41 us for 64 uniform bricks of 4096 against 35 unsplit).
+// share (a brick that starts last then ends with the others), three times
+// the mean count (an even distribution has no items) and ITEM_MIN (the others
+// are 0 for stores with fewer particles than bricks and CTAs).  It is split
+// above 3/2 P with P half the share, so that no CTA is left with more than
+// that, but parts hold at least PART_MIN particles: each clears and writes its
+// tile (parts of 1024 took 41 us for 64 uniform bricks of 4096 against 35
+// unsplit).
 // `cap` bounds what a split fixed-point tile sums.  The scratch tiles lie in
 // the repack scratch (c->alt), which nothing uses between the rebins.
 PartPlan part_plan(lf2_ctx* c, size_t smem, int threads, size_t tile_slots, int cap)
@@ -735,7 +738,8 @@ PartPlan part_plan(lf2_ctx* c, size_t smem, int threads, size_t tile_slots, int 
   if (cap <= 0) cap = 1 << 28;
   const int64_t P = std::min<int64_t>(std::max<int64_t>(share / 2, PART_MIN), cap - cap / 16);
   const int64_t split = std::min<int64_t>(P + P / 2, cap);
-  const int64_t first = std::min(split, std::max(share / 4, 3 * (c->np / c->g.nbricks)));
+  const int64_t first =
+      std::min(split, std::max({ITEM_MIN, share / 4, 3 * (c->np / c->g.nbricks)}));
   pl.P = (int)P, pl.split = (int)split, pl.first = (int)first;
   // np particles make at most 3/2 np / P parts and np / first items
   pl.max_items = (int)std::min<int64_t>(PART_ITEMS, c->np * 3 / (2 * P) + c->np / first);
