@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
   constexpr int T = P::THREADS;
   extern __shared__ __align__(16) unsigned char smem_raw[];
 
-  __shared__ unsigned s_max[2];
+  __shared__ unsigned s_max;
   __shared__ int s_tile;  // (not a register of the particle loop)
 
   const Geom& g = v.g;
@@ -125,16 +125,14 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
   const int x0 = bx * BRICK, y0 = by * BRICK, z0 = bz * BRICK;
   const uint32_t base = (uint32_t)(part.start + part.first);  // slots fit in 32 bits
   const int cnt = part.cnt;
-  const int mass_bound = FIXED && HM ? part_mass_bound(v.a.mass, base, cnt, dp.inv_unit, s_max) : 1;
-  CompUnit cu{0, false};
+  const int mass_bound = FIXED && HM ? part_mass_bound(v.a.mass, base, cnt, dp.inv_unit, &s_max) : 1;
+  CompUnit cu{0, 1.0f, false};
   if (ACC == ACC_COMP)
     cu = comp_unit<KIND>(HM ? v.a.mass : nullptr, dp.inv_vol, dp.mf, v.a.vx, v.a.vy, v.a.vz,
-                         base, cnt, s_max);
+                         base, cnt, &s_max);
   // two integer words per vertex, or the sums that hold anything
   const bool ints = FIXED ? cnt <= split_max<SIGNED>(mass_bound) : cu.ok;
   TileRef<TILE3> tr{smem_raw, ints};
-  // unit of the FP32 terms that the integer sums take (add_comp_int)
-  const float unit = ACC == ACC_COMP && ints ? ldexpf(1.0f, 16 - cu.e) : 1.0f;
   // fixed point: velocity quantum and conversion scale for this field
   int vexp = 0;
   if (FIXED && KIND != 0) vexp = vexp_of(*vmax_bits);
@@ -267,33 +265,32 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
         const float gx = __fsub_rn(1.0f, fx[j]), gy = __fsub_rn(1.0f, fy[j]),
                     gz = __fsub_rn(1.0f, fz[j]);
         const float ox = fx[j], oy = fy[j], oz = fz[j];
-        float mf = HM ? __fmul_rn(m[j], dp.inv_vol) : dp.mf;
-        if (ACC == ACC_COMP && SPLIT) mf = __fmul_rn(mf, unit);
+        const float mf = HM ? __fmul_rn(m[j], dp.inv_vol) : dp.mf;
         if (KIND == 0) {
   #pragma unroll
           for (int k = 0; k < 8; k++) {
             const int cx = (k >> 2) & 1, cy = (k >> 1) & 1, cz = k & 1;
             const float w = __fmul_rn(
                 __fmul_rn(__fmul_rn(sel(cx, ox, gx), sel(cy, oy, gy)), sel(cz, oz, gz)), mf);
-            add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0 + cx + cy * TY + cz * TZ, w);
+            add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0 + cx + cy * TY + cz * TZ, w, cu.unit);
           }
         } else if (KIND == 1) {
           // projections.hpp:501-544: component i is NGP along i, CIC across.
           const float vxm = __fmul_rn(mf, vx[j]);
           const float vym = __fmul_rn(mf, vy[j]);
           const float vzm = __fmul_rn(mf, vz[j]);
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0, __fmul_rn(__fmul_rn(vxm, gy), gz));
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0 + TY, __fmul_rn(__fmul_rn(vxm, oy), gz));
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0 + TZ, __fmul_rn(__fmul_rn(vxm, gy), oz));
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0 + TY + TZ, __fmul_rn(__fmul_rn(vxm, oy), oz));
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 1, t0, __fmul_rn(__fmul_rn(vym, gx), gz));
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 1, t0 + 1, __fmul_rn(__fmul_rn(vym, ox), gz));
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 1, t0 + TZ, __fmul_rn(__fmul_rn(vym, gx), oz));
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 1, t0 + 1 + TZ, __fmul_rn(__fmul_rn(vym, ox), oz));
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 2, t0, __fmul_rn(__fmul_rn(vzm, gx), gy));
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 2, t0 + 1, __fmul_rn(__fmul_rn(vzm, ox), gy));
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 2, t0 + TY, __fmul_rn(__fmul_rn(vzm, gx), oy));
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 2, t0 + 1 + TY, __fmul_rn(__fmul_rn(vzm, ox), oy));
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0, __fmul_rn(__fmul_rn(vxm, gy), gz), cu.unit);
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0 + TY, __fmul_rn(__fmul_rn(vxm, oy), gz), cu.unit);
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0 + TZ, __fmul_rn(__fmul_rn(vxm, gy), oz), cu.unit);
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0 + TY + TZ, __fmul_rn(__fmul_rn(vxm, oy), oz), cu.unit);
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 1, t0, __fmul_rn(__fmul_rn(vym, gx), gz), cu.unit);
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 1, t0 + 1, __fmul_rn(__fmul_rn(vym, ox), gz), cu.unit);
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 1, t0 + TZ, __fmul_rn(__fmul_rn(vym, gx), oz), cu.unit);
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 1, t0 + 1 + TZ, __fmul_rn(__fmul_rn(vym, ox), oz), cu.unit);
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 2, t0, __fmul_rn(__fmul_rn(vzm, gx), gy), cu.unit);
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 2, t0 + 1, __fmul_rn(__fmul_rn(vzm, ox), gy), cu.unit);
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 2, t0 + TY, __fmul_rn(__fmul_rn(vzm, gx), oy), cu.unit);
+          add_float<ACC, SPLIT, TILE3>(smem_raw, 2, t0 + 1 + TY, __fmul_rn(__fmul_rn(vzm, ox), oy), cu.unit);
         } else {
           // projections.hpp:786-843: T_ii at the 8 vertices, T_ij on plaquettes.
           const float vv[3] = {vx[j], vy[j], vz[j]};
@@ -311,7 +308,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
                 const int cx = (k >> 2) & 1, cy = (k >> 1) & 1, cz = k & 1;
                 const float w = __fmul_rn(
                     __fmul_rn(__fmul_rn(mv2, sel(cx, ox, gx)), sel(cy, oy, gy)), sel(cz, oz, gz));
-                add_float<ACC, SPLIT, TILE3>(smem_raw, jd, t0 + cx + cy * TY + cz * TZ, w);
+                add_float<ACC, SPLIT, TILE3>(smem_raw, jd, t0 + cx + cy * TY + cz * TZ, w, cu.unit);
               }
             }
           }
@@ -321,12 +318,12 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
             const float m01 = __fmul_rn(__fmul_rn(mf, vv[0]), vv[1]);
             const float m02 = __fmul_rn(__fmul_rn(mf, vv[0]), vv[2]);
             const float m12 = __fmul_rn(__fmul_rn(mf, vv[1]), vv[2]);
-            add_float<ACC, SPLIT, TILE3>(smem_raw, j01, t0, __fmul_rn(m01, gz));
-            add_float<ACC, SPLIT, TILE3>(smem_raw, j01, t0 + TZ, __fmul_rn(m01, oz));
-            add_float<ACC, SPLIT, TILE3>(smem_raw, j02, t0, __fmul_rn(m02, gy));
-            add_float<ACC, SPLIT, TILE3>(smem_raw, j02, t0 + TY, __fmul_rn(m02, oy));
-            add_float<ACC, SPLIT, TILE3>(smem_raw, j12, t0, __fmul_rn(m12, gx));
-            add_float<ACC, SPLIT, TILE3>(smem_raw, j12, t0 + 1, __fmul_rn(m12, ox));
+            add_float<ACC, SPLIT, TILE3>(smem_raw, j01, t0, __fmul_rn(m01, gz), cu.unit);
+            add_float<ACC, SPLIT, TILE3>(smem_raw, j01, t0 + TZ, __fmul_rn(m01, oz), cu.unit);
+            add_float<ACC, SPLIT, TILE3>(smem_raw, j02, t0, __fmul_rn(m02, gy), cu.unit);
+            add_float<ACC, SPLIT, TILE3>(smem_raw, j02, t0 + TY, __fmul_rn(m02, oy), cu.unit);
+            add_float<ACC, SPLIT, TILE3>(smem_raw, j12, t0, __fmul_rn(m12, gx), cu.unit);
+            add_float<ACC, SPLIT, TILE3>(smem_raw, j12, t0 + 1, __fmul_rn(m12, ox), cu.unit);
           }
         }
       }
@@ -337,7 +334,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
   else particles(std::false_type{});
   __syncthreads();
   if (s_tile >= 0) {  // k_part_finish writes the vertices
-    part_store<ACC, SIGNED, NC, TILE3>(scratch_tile(pv, s_tile, NC * TILE3), tr, cu.e);
+    part_store<ACC, SIGNED, NC, TILE3>(scratch_tile(pv, s_tile, NC * TILE3), tr, cu.q);
     return;
   }
 
@@ -364,7 +361,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
         if (!SIGNED && q < 0) set_flag(flags, ERR_FIXED_OVERFLOW);
         out[(size_t)c * g.nsites + s] = __fmul_rn(__ll2float_rn(q), conv);
       } else if (ACC == ACC_COMP) {
-        const float2 p = comp_pair(tr, j, t, cu.e);
+        const float2 p = comp_pair(tr, j, t, cu.q);
         out[(size_t)c * g.nsites + s] = __fadd_rn(p.x, p.y);
       } else {
         out[(size_t)c * g.nsites + s] = facc[(size_t)j * TILE3 + t];
@@ -400,7 +397,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
       if (FIXED) {
         sp[(size_t)c * SHELL + f] = (uint64_t)tile_fixed<SIGNED>(tr, j, t);
       } else if (ACC == ACC_COMP) {
-        reinterpret_cast<float2*>(sp)[(size_t)c * SHELL + f] = comp_pair(tr, j, t, cu.e);
+        reinterpret_cast<float2*>(sp)[(size_t)c * SHELL + f] = comp_pair(tr, j, t, cu.q);
       } else {
         reinterpret_cast<float*>(sp)[(size_t)c * SHELL + f] = facc[(size_t)j * TILE3 + t];
       }

@@ -140,73 +140,82 @@ __device__ __forceinline__ void add_comp_int(unsigned char* smem, int j, int t, 
   atomicAdd(reinterpret_cast<int*>(&w[N + t]), hi + (lo >> 31) + carry);
 }
 
-// One FP32 term of either mode; SPLIT: the integer sums of the compensated one.
+// One FP32 term of either mode; SPLIT: the integer sums of the compensated one
+// (unit: CompUnit).
 template <int ACC, bool SPLIT, int N>
-__device__ __forceinline__ void add_float(unsigned char* smem, int j, int t, float w)
+__device__ __forceinline__ void add_float(unsigned char* smem, int j, int t, float w, float unit)
 {
   float* f = reinterpret_cast<float*>(smem);
   if (ACC == ACC_PLAIN)
     atomicAdd(&f[(size_t)j * N + t], w);
   else if (SPLIT)
-    add_comp_int<N>(smem, j, t, w);
+    add_comp_int<N>(smem, j, t, __fmul_rn(w, unit));
   else
     add_comp(&f[(size_t)j * 2 * N + t], &f[(size_t)j * 2 * N + N + t], w);
 }
 
-// The unit of a CTA's terms: e with 2^(e - 1) above every |factor| (the FP32
-// rounding of a term's products stays below 2^e).  ok: the scaled factors
-// are in range.
+// The unit of a CTA's terms, from the largest bound M of any of its particles:
+// 2^q is the quantum of the integer sums, `unit` = 2^(-32 - q) takes a term to
+// what add_comp_int adds.  ok: M is in the range where both are normal FP32
+// numbers with room to spare, and the particles are few enough.
 struct CompUnit {
-  int e;
+  int q;
+  float unit;
   bool ok;
 };
 
-// Largest |mass / volume| (mf for a global mass) and, for NV = 3, |v_i| of
-// the particles, to the power P: the bound of the factors |mf v_i v_j|.
+__device__ __forceinline__ CompUnit comp_unit_of(unsigned bits, int cnt)
+{
+  const int e = (int)(bits >> 23) - 126;  // M < 2^e for a normal number
+  CompUnit r;
+  r.ok = e >= -90 && e <= 127 && cnt <= split_max<true>(1);
+  r.q = e - 48;
+  r.unit = r.ok ? ldexpf(1.0f, 16 - e) : 1.0f;
+  return r;
+}
+
+// M: the product of |mass / volume| (mf for a global mass) and P times the
+// largest |v_i| of a particle, rounded as the terms' products are: rounding is
+// monotonic and the weights are at most 1, so no |term| is above it, and a
+// particle whose product leaves the FP32 range shows in it (infinity, or NaN,
+// whose bits order above it).
 template <int P>
 __device__ __forceinline__ CompUnit comp_unit(const float* mass, float inv_vol, float mf,
                                               const float* vx, const float* vy, const float* vz,
                                               uint32_t p0, int cnt, unsigned* s_max)
 {
-  unsigned m = mass ? 0u : __float_as_uint(mf) & 0x7fffffffu, u = 0u;
-  if (mass || P > 0) {
-    if (threadIdx.x < 2) s_max[threadIdx.x] = 0u;
-    __syncthreads();
-    for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
-      const uint32_t p = p0 + (uint32_t)i;
-      if (mass) m = max(m, __float_as_uint(__fmul_rn(mass[p], inv_vol)) & 0x7fffffffu);
-      if (P > 0)
-        u = max(max(u, __float_as_uint(vx[p]) & 0x7fffffffu),
-                max(__float_as_uint(vy[p]) & 0x7fffffffu, __float_as_uint(vz[p]) & 0x7fffffffu));
+  if (!mass && P == 0) return comp_unit_of(__float_as_uint(mf) & 0x7fffffffu, cnt);
+  if (threadIdx.x == 0) *s_max = 0u;
+  __syncthreads();
+  unsigned m = 0u;
+  for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
+    const uint32_t p = p0 + (uint32_t)i;
+    float f = mass ? __fmul_rn(mass[p], inv_vol) : mf;
+    if (P > 0) {
+      const float v = __uint_as_float(max(max(__float_as_uint(vx[p]) & 0x7fffffffu,
+                                              __float_as_uint(vy[p]) & 0x7fffffffu),
+                                          __float_as_uint(vz[p]) & 0x7fffffffu));
+      f = __fmul_rn(f, v);
+      if (P > 1) f = __fmul_rn(f, v);
     }
-    m = __reduce_max_sync(0xffffffffu, m);  // bits of |x| order as integers, NaN above infinity
-    u = __reduce_max_sync(0xffffffffu, u);
-    if ((threadIdx.x & 31) == 0) {
-      atomicMax(&s_max[0], m);
-      if (P > 0) atomicMax(&s_max[1], u);
-    }
-    __syncthreads();
-    m = s_max[0];
-    u = s_max[1];
+    m = max(m, __float_as_uint(f) & 0x7fffffffu);
   }
-  // exponents: |x| < 2^(bits - 126) for a normal number
-  const int em = (int)(m >> 23) - 126, eu = P > 0 ? (int)(u >> 23) - 126 : 0;
-  CompUnit r;
-  r.e = em + P * eu + 1;
-  r.ok = m != 0u && em >= -90 && em <= 90 && (P == 0 || (u != 0u && eu >= -40 && eu <= 40)) &&
-         cnt <= split_max<true>(1);
-  return r;
+  m = __reduce_max_sync(0xffffffffu, m);  // bits of |x| order as integers
+  if ((threadIdx.x & 31) == 0) atomicMax(s_max, m);
+  __syncthreads();
+  return comp_unit_of(*s_max, cnt);
 }
 
-// hi/lo pair of a compensated vertex sum, from the integers or the floats.
+// hi/lo pair of a compensated vertex sum, from the integers (quantum 2^q) or
+// the floats.
 template <int N>
-__device__ __forceinline__ float2 comp_pair(const TileRef<N>& tr, int j, int t, int e)
+__device__ __forceinline__ float2 comp_pair(const TileRef<N>& tr, int j, int t, int q)
 {
   const uint32_t* w = reinterpret_cast<const uint32_t*>(tr.smem) + (size_t)j * 2 * N;
   if (!tr.split) return make_float2(__uint_as_float(w[t]), __uint_as_float(w[N + t]));
-  const long long q = (long long)(int32_t)w[N + t] * 4294967296ll + (long long)w[t];
-  const float hi = __ll2float_rn(q), lo = __ll2float_rn(q - (long long)hi);
-  return make_float2(ldexpf(hi, e - 48), ldexpf(lo, e - 48));
+  const long long s = (long long)(int32_t)w[N + t] * 4294967296ll + (long long)w[t];
+  const float hi = __ll2float_rn(s), lo = __ll2float_rn(s - (long long)hi);
+  return make_float2(ldexpf(hi, q), ldexpf(lo, q));
 }
 
 // Integer vertex sum of component j: the scalar's split (lo + hi 2^16) or
@@ -429,10 +438,10 @@ __device__ __forceinline__ bool part_take(const PartView& pv, int64_t nbricks, c
 }
 
 // A part's tile to the scratch: 8-byte values, component j of vertex t at
-// j * N + t (the integer sum, the hi/lo pair or the float).  e: the unit of
-// the compensated mode's terms.
+// j * N + t (the integer sum, the hi/lo pair or the float).  cq: the quantum of
+// the compensated mode's integers (CompUnit).
 template <int ACC, bool SIGNED, int NC, int N>
-__device__ __forceinline__ void part_store(uint64_t* dst, const TileRef<N>& tr, int e)
+__device__ __forceinline__ void part_store(uint64_t* dst, const TileRef<N>& tr, int cq)
 {
   const uint32_t* w = reinterpret_cast<const uint32_t*>(tr.smem);
   for (int t = threadIdx.x; t < N; t += blockDim.x) {
@@ -442,7 +451,7 @@ __device__ __forceinline__ void part_store(uint64_t* dst, const TileRef<N>& tr, 
       if (ACC == ACC_FIXED) {
         q = (uint64_t)tile_fixed<SIGNED>(tr, j, t);
       } else if (ACC == ACC_COMP) {
-        const float2 v = comp_pair(tr, j, t, e);
+        const float2 v = comp_pair(tr, j, t, cq);
         q = (uint64_t)__float_as_uint(v.x) | ((uint64_t)__float_as_uint(v.y) << 32);
       } else {
         q = w[(size_t)j * N + t];

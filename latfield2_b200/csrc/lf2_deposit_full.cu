@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(FULL2_THREADS, 1)
   constexpr int CT = FullPass<PASS>::total;
   constexpr bool FIXED = ACC == ACC_FIXED;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ unsigned s_max[2];
+  __shared__ unsigned s_max;
   __shared__ int s_brick, s_tile;  // (so that the particle loop keeps no register for them)
 
   const Geom& g = v.g;
@@ -357,13 +357,12 @@ __global__ void __launch_bounds__(FULL2_THREADS, 1)
   const int x0 = bx * BRICK, y0 = by * BRICK, z0 = bz * BRICK;
   const int64_t base = part.start + part.first;
   const int cnt = part.cnt;
-  const int mass_bound = FIXED && HM ? part_mass_bound(v.a.mass, (uint32_t)base, cnt, dp.inv_unit, s_max) : 1;
-  CompUnit cu{0, false};
+  const int mass_bound = FIXED && HM ? part_mass_bound(v.a.mass, (uint32_t)base, cnt, dp.inv_unit, &s_max) : 1;
+  CompUnit cu{0, 1.0f, false};
   if (!FIXED)
     cu = comp_unit<PASS == 0 ? 1 : 2>(HM ? v.a.mass : nullptr, dp.inv_vol, dp.mf, v.a.vx, v.a.vy,
-                                      v.a.vz, (uint32_t)base, cnt, s_max);
+                                      v.a.vz, (uint32_t)base, cnt, &s_max);
   TileRef<FT3> tr{smem_raw, FIXED ? cnt <= split_max<true>(mass_bound) : cu.ok};
-  const float unit = !FIXED && cu.ok ? ldexpf(1.0f, 16 - cu.e) : 1.0f;
   int vexp = 0;
   if (FIXED) vexp = vexp_of(*vmax_bits);
   const float vscale = vel_scale(vexp);
@@ -462,8 +461,7 @@ __global__ void __launch_bounds__(FULL2_THREADS, 1)
         continue;
       }
       // compensated FP32: the arithmetic of k_deposit_full
-      float mf = HM ? __fmul_rn(v.a.mass[p], dp.inv_vol) : dp.mf;
-      if (SPLIT) mf = __fmul_rn(mf, unit);
+      const float mf = HM ? __fmul_rn(v.a.mass[p], dp.inv_vol) : dp.mf;
       float sw[3][2], tw[3][2];
   #pragma unroll
       for (int d = 0; d < 3; d++) {
@@ -489,7 +487,8 @@ __global__ void __launch_bounds__(FULL2_THREADS, 1)
             const float w2 = c == 2 ? tw[2][b2] : sw[2][b2];
             const int t = tile_at((c == 0 ? lt[0] : ls[0]) + b0, (c == 1 ? lt[1] : ls[1]) + b1,
                                   (c == 2 ? lt[2] : ls[2]) + b2);
-            add_float<ACC, SPLIT, FT3>(smem_raw, c, t, __fmul_rn(__fmul_rn(__fmul_rn(mv, w0), w1), w2));
+            add_float<ACC, SPLIT, FT3>(smem_raw, c, t, __fmul_rn(__fmul_rn(__fmul_rn(mv, w0), w1), w2),
+                                    cu.unit);
           }
         }
       } else if (PASS == 1) {
@@ -500,7 +499,7 @@ __global__ void __launch_bounds__(FULL2_THREADS, 1)
           for (int k = 0; k < 8; k++) {
             const int b0 = (k >> 2) & 1, b1 = (k >> 1) & 1, b2 = k & 1;
             add_float<ACC, SPLIT, FT3>(smem_raw, i2, tile_at(ls[0] + b0, ls[1] + b1, ls[2] + b2),
-                           __fmul_rn(__fmul_rn(__fmul_rn(m2, sw[0][b0]), sw[1][b1]), sw[2][b2]));
+                           __fmul_rn(__fmul_rn(__fmul_rn(m2, sw[0][b0]), sw[1][b1]), sw[2][b2]), cu.unit);
           }
         }
       } else {
@@ -519,7 +518,7 @@ __global__ void __launch_bounds__(FULL2_THREADS, 1)
               t[d] = (st ? lt[d] : ls[d]) + bb[d];
             }
             add_float<ACC, SPLIT, FT3>(smem_raw, q, tile_at(t[0], t[1], t[2]),
-                           __fmul_rn(__fmul_rn(__fmul_rn(mm, w[0]), w[1]), w[2]));
+                           __fmul_rn(__fmul_rn(__fmul_rn(mm, w[0]), w[1]), w[2]), cu.unit);
           }
         }
       }
@@ -529,7 +528,7 @@ __global__ void __launch_bounds__(FULL2_THREADS, 1)
   else particles(std::false_type{});
   __syncthreads();
   if (s_tile >= 0) {
-    part_store<ACC, true, 3, FT3>(scratch_tile(pv, s_tile, 3 * FT3), tr, cu.e);
+    part_store<ACC, true, 3, FT3>(scratch_tile(pv, s_tile, 3 * FT3), tr, cu.q);
     return;
   }
 
@@ -555,7 +554,7 @@ __global__ void __launch_bounds__(FULL2_THREADS, 1)
         if (priv) out[(size_t)c * g.nsites + site] = __fmul_rn(__ll2float_rn(q), conv);
         else st[(size_t)c * FSHELL + si] = (uint64_t)q;
       } else {
-        const float2 p = comp_pair(tr, j, t, cu.e);
+        const float2 p = comp_pair(tr, j, t, cu.q);
         if (priv) out[(size_t)c * g.nsites + site] = __fadd_rn(p.x, p.y);
         else reinterpret_cast<float2*>(st)[(size_t)c * FSHELL + si] = p;
       }

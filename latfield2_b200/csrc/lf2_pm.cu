@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(256)
                       float inv_vol, unsigned long long* __restrict__ acc, float* __restrict__ rho)
 {
   __shared__ uint32_t lo[TILE3], hi[TILE3];
-  __shared__ unsigned s_max[2];
+  __shared__ unsigned s_max;
   const float inv_m = FIXED && mass ? 1.0f / __uint_as_float(*mmax) : 0.0f;
   const int lane = threadIdx.x & 31;
   for (int half = 0; half < 2; half++) {
@@ -229,11 +229,10 @@ __global__ void __launch_bounds__(256)
     }
     if (half) __syncthreads();  // the tile before is flushed
     for (int t = threadIdx.x; t < TILE3; t += blockDim.x) lo[t] = hi[t] = 0u;
-    CompUnit cu{0, true};
+    CompUnit cu{0, 1.0f, true};
     if (!FIXED)  // (slots may exceed 32 bits)
       cu = comp_unit<0>(mass ? mass + p0 : nullptr, inv_vol, gmass * inv_vol, nullptr, nullptr, nullptr,
-                        0u, (int)(p1 - p0), s_max);
-    const float unit = !FIXED && cu.ok ? ldexpf(1.0f, 16 - cu.e) : 1.0f;
+                        0u, (int)(p1 - p0), &s_max);
     __syncthreads();
     int bx, by, bz;
     brick_coords(g, b, bx, by, bz);
@@ -274,7 +273,7 @@ __global__ void __launch_bounds__(256)
           return (long long)w;
         }
         const float w = (cx ? f[0] : 1.0f - f[0]) * (cy ? f[1] : 1.0f - f[1]) * (cz ? f[2] : 1.0f - f[2]);
-        const float v = w * (m * unit);  // |v| < 2^16
+        const float v = w * m * cu.unit;  // |v| < 2^16
         const float h = __fadd_rn(v, 12582912.0f);
         const float r = __fsub_rn(v, __fsub_rn(h, 12582912.0f));
         return ((long long)(__float_as_int(h) - 0x4B400000) << 32) +
@@ -333,7 +332,7 @@ __global__ void __launch_bounds__(256)
       if (FIXED)
         atomicAdd(&acc[tile_site(g, t, x0, y0, z0)], v);
       else
-        atomicAdd(&rho[tile_site(g, t, x0, y0, z0)], ldexpf(__ll2float_rn((long long)v), cu.e - 48));
+        atomicAdd(&rho[tile_site(g, t, x0, y0, z0)], ldexpf(__ll2float_rn((long long)v), cu.q));
     }
   }
 }

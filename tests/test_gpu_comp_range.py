@@ -1,0 +1,69 @@
+"""The compensated FP32 mode over the range of units: masses and velocities
+scaled by powers of two give the field scaled by the product's power, wherever
+the terms are normal FP32 numbers, whether the sums are integers in a common
+unit or the FP32 pairs that hold anything."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from tests.helpers import positions, precision
+from tests.test_gpu_precision import KINDS, _fp64
+
+pytestmark = pytest.mark.gpu
+
+N = (8, 8, 8)
+NPART = 400
+
+
+def _case():
+    """Offsets in [1/4, 3/4], masses and |v_i| in [1/2, 1): a term is at least
+    2^-9 of the largest."""
+    rng = np.random.default_rng(3)
+    cell = rng.integers(0, 512, NPART).astype(np.int32)
+    off = (0.25 + 0.5 * rng.random((NPART, 3))).astype(np.float32)
+    vel = ((0.5 + 0.49 * rng.random((NPART, 3))) * rng.choice([-1, 1], (NPART, 3))).astype(np.float32)
+    mass = (0.5 + 0.49 * rng.random(NPART)).astype(np.float32)
+    return cell, off, vel, mass
+
+
+@pytest.mark.parametrize("individual", [False, True])
+@pytest.mark.parametrize("kind", [0, 1, 2, 3, 4])
+def test_units_of_mass_and_velocity(cuda, kind, individual):
+    import latfield2_b200 as L
+    cell, off, vel, mass = _case()
+    power = (0, 1, 2, 1, 2)[kind]
+    if individual:  # FP64 reference: the projection of the masses' multiples
+        cs, order = O.lists_from_insertion(N, cell)
+        pos = positions(N, 1.0, cell, off)[order]
+        if kind == 0:
+            ref = O.state_deposit_f64(N, cell, off, 1.0, mass=mass).reshape(1, *N)
+            mag = ref
+        else:
+            ref, mag = (O.interior(KINDS[kind][2](N, 1, 1.0, cs, pos, v.astype(np.float64)[order],
+                                                  pmass=mass.astype(np.float64)[order]), N, 1)
+                        for v in (vel, np.abs(vel)))
+    else:
+        ref, mag = _fp64(N, kind, cell, off, vel, 8.0 ** -3)
+    ctx = L.Context(N, box=8.0 if individual else 1.0, mode=L.DEPOSIT_FP32)
+    name, comps = ("deposit_scalar", 1) if kind == 0 else KINDS[kind][:2]
+    f = ctx.field(comps)
+    tried = 0
+    for em in list(range(-100, 101, 20)) + [-83, -44, -91, 91]:
+        for ev in (-45, -41, -35, -34, -17, 0, 17, 39, 41, 45) if power else (0,):
+            k = em + power * ev
+            # every term and every partial product a normal number, the sums finite
+            if not (-117 <= k <= 110 and -117 <= em + ev <= 110):
+                continue
+            s = 2.0 ** em
+            ctx.set_particles(cell, off, np.ldexp(vel, ev).astype(np.float32),
+                              mass=(mass * np.float32(s)) if individual else None,
+                              global_mass=0.0 if individual else s * 8.0 ** -3)
+            getattr(ctx, name)(f)
+            got = np.ldexp(f.export_internal().astype(np.float64), -k)
+            for c in range(comps):
+                p = precision(got[c], ref[c], mag[c])
+                assert p["norm_max"] <= 1e-6 and p["cell_max"] <= 1e-6, (em, ev, c, p)
+            tried += 1
+    assert tried >= (11 if power == 0 else 40)
+    assert ctx.flags() == 0
+    ctx.close()
