@@ -20,11 +20,11 @@
 // Three accumulation modes (the context's deposit mode):
 //   LF2_DEPOSIT_FP32        the reference's FP32 terms, their sum compensated:
 //                           integers in a unit set by the part's largest term
-//                           (add_comp_int), or, where that range does not
-//                           hold, FP32 atomics that return the value they
-//                           replaced, the rounding error of each recovered
-//                           exactly (TwoSum) and accumulated in a second FP32
-//                           word.  hi + lo is the sum to within the rounding
+//                           (add_comp_int) with what small terms leave below
+//                           it (add_rest), or, where that range does not hold,
+//                           FP32 atomics that return the value they replaced,
+//                           the rounding error of each recovered exactly
+//                           (TwoSum) and accumulated in a second FP32 word.  hi + lo is the sum to within the rounding
 //                           of the terms (about 1e-7 relative), whatever the
 //                           order.
 //   LF2_DEPOSIT_FIXED64     int64 fixed point: every contribution is rounded
@@ -82,6 +82,12 @@ struct Pass {
                                          : (j == 0 ? 1 : j == 1 ? 2 : 4);
   }
   static constexpr size_t smem() { return (size_t)NC * WORDS * TILE3 * 4; }
+  // after the tile, what the compensated mode keeps of small terms: notes
+  // (Rests) and listed particles (RestList: all of a part, or what five CTAs
+  // per SM leave room for)
+  static constexpr int NOTES = ACC != ACC_COMP ? 0 : smem() > 100 * 1024 ? 2048 : 128;
+  static constexpr int RESTS = ACC != ACC_COMP ? 0 : smem() > 100 * 1024 ? 32768 : 1536;
+  static constexpr size_t dyn() { return smem() + NOTES * sizeof(uint2) + RESTS * sizeof(uint16_t); }
   // a tile above 100 KB leaves room for one CTA per SM
   static constexpr int THREADS = smem() > 100 * 1024 ? DEP_BIG_THREADS : DEP_THREADS;
   static constexpr int ITEMS = smem() > 100 * 1024 ? 2 : 4;  // particles in flight per thread
@@ -112,6 +118,9 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
 
   __shared__ unsigned s_max;
   __shared__ int s_tile;  // (not a register of the particle loop)
+  __shared__ int s_rests, s_notes;
+  __shared__ uint32_t s_marks[ACC == ACC_COMP ? (NC * TILE3 + 31) / 32 : 1];
+  __shared__ float s_quantum;
 
   const Geom& g = v.g;
   Part part;
@@ -126,13 +135,13 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
   const uint32_t base = (uint32_t)(part.start + part.first);  // slots fit in 32 bits
   const int cnt = part.cnt;
   const int mass_bound = FIXED && HM ? part_mass_bound(v.a.mass, base, cnt, dp.inv_unit, &s_max) : 1;
-  CompUnit cu{0, 1.0f, false};
+  CompUnit cu{1.0f, 1.0f, false};
   if (ACC == ACC_COMP)
     cu = comp_unit<KIND>(HM ? v.a.mass : nullptr, dp.inv_vol, dp.mf, v.a.vx, v.a.vy, v.a.vz,
                          base, cnt, &s_max);
   // two integer words per vertex, or the sums that hold anything
   const bool ints = FIXED ? cnt <= split_max<SIGNED>(mass_bound) : cu.ok;
-  TileRef<TILE3> tr{smem_raw, ints};
+  TileRef<TILE3> tr{smem_raw, ints, nullptr};
   // fixed point: velocity quantum and conversion scale for this field
   int vexp = 0;
   if (FIXED && KIND != 0) vexp = vexp_of(*vmax_bits);
@@ -146,14 +155,22 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
     uint32_t* z = reinterpret_cast<uint32_t*>(smem_raw);
     constexpr int words = NC * P::WORDS * TILE3;
     for (int t = threadIdx.x; t < words; t += blockDim.x) z[t] = 0u;
+    if (ACC == ACC_COMP)
+      for (int t = threadIdx.x; t < (NC * TILE3 + 31) / 32; t += blockDim.x) s_marks[t] = 0u;
+    if (threadIdx.x == 0) s_rests = 0, s_notes = 0, s_quantum = cu.quantum;
   }
   __syncthreads();
+  uint2* const notes = reinterpret_cast<uint2*>(smem_raw + P::smem());
+  const RestList rl{reinterpret_cast<uint16_t*>(notes + P::NOTES), &s_rests, P::RESTS};
 
   // The particle loop, instantiated for the tile of two integer words per
-  // vertex or the other one, chosen once per CTA.
+  // vertex or the other one, chosen once per CTA, and for the listed particles'
+  // rests.
   constexpr int ITEMS = P::ITEMS;
-  auto particles = [&](auto split_c) {
-    constexpr bool SPLIT = decltype(split_c)::value;
+  Rests rs{0, false, cu.quantum, s_marks, notes, &s_notes, P::NOTES};
+  auto particles = [&](auto sum_c, int cnt) {
+    constexpr int SUM = decltype(sum_c)::value;
+    constexpr bool SPLIT = SUM == SUM_INT;
     for (int c0 = 0; c0 < cnt; c0 += ITEMS * T) {
       uint32_t key[ITEMS];
       float fx[ITEMS], fy[ITEMS], fz[ITEMS], m[ITEMS];
@@ -162,7 +179,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
       for (int j = 0; j < ITEMS; j++) {
         const int i = c0 + j * T + threadIdx.x;
         if (i < cnt) {
-          const uint32_t p = base + (uint32_t)i;
+          const uint32_t p = base + (uint32_t)(SUM == SUM_REST ? rl.entry[i] : i);
           key[j] = v.a.key[p];
           fx[j] = v.a.ox[p];
           fy[j] = v.a.oy[p];
@@ -266,31 +283,45 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
                     gz = __fsub_rn(1.0f, fz[j]);
         const float ox = fx[j], oy = fy[j], oz = fz[j];
         const float mf = HM ? __fmul_rn(m[j], dp.inv_vol) : dp.mf;
+        if (ACC == ACC_COMP && SPLIT) {  // the particle's smallest term, or a bound below it
+          auto least3 = [](float a, float b, float c) { return fminf(fminf(fabsf(a), fabsf(b)), fabsf(c)); };
+          const float mx = __fmul_rn(mf, vx[j]), my = __fmul_rn(mf, vy[j]), mz = __fmul_rn(mf, vz[j]);
+          float f = KIND == 0 ? fabsf(mf) : least3(mx, my, mz);
+          if (KIND == 2)
+            f = PASS == 0 ? least3(__fmul_rn(mx, vx[j]), __fmul_rn(my, vy[j]), __fmul_rn(mz, vz[j]))
+                          : least3(__fmul_rn(mx, vy[j]), __fmul_rn(mx, vz[j]), __fmul_rn(my, vz[j]));
+          const float ux = fminf(ox, gx), uy = fminf(oy, gy), uz = fminf(oz, gz);
+          if (KIND == 2 && PASS == 1)  // one weight to a term
+            f = __fmul_rn(f, fminf(fminf(ux, uy), uz));
+          else
+            f = __fmul_rn(__fmul_rn(__fmul_rn(f, ux), uy), uz);
+          if (has_rest(__fmul_rn(f, cu.unit))) rl.add(i);
+        }
         if (KIND == 0) {
   #pragma unroll
           for (int k = 0; k < 8; k++) {
             const int cx = (k >> 2) & 1, cy = (k >> 1) & 1, cz = k & 1;
             const float w = __fmul_rn(
                 __fmul_rn(__fmul_rn(sel(cx, ox, gx), sel(cy, oy, gy)), sel(cz, oz, gz)), mf);
-            add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0 + cx + cy * TY + cz * TZ, w, cu.unit);
+            add_float<ACC, SUM, TILE3>(smem_raw, 0, t0 + cx + cy * TY + cz * TZ, w, cu.unit, rs);
           }
         } else if (KIND == 1) {
           // projections.hpp:501-544: component i is NGP along i, CIC across.
           const float vxm = __fmul_rn(mf, vx[j]);
           const float vym = __fmul_rn(mf, vy[j]);
           const float vzm = __fmul_rn(mf, vz[j]);
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0, __fmul_rn(__fmul_rn(vxm, gy), gz), cu.unit);
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0 + TY, __fmul_rn(__fmul_rn(vxm, oy), gz), cu.unit);
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0 + TZ, __fmul_rn(__fmul_rn(vxm, gy), oz), cu.unit);
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 0, t0 + TY + TZ, __fmul_rn(__fmul_rn(vxm, oy), oz), cu.unit);
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 1, t0, __fmul_rn(__fmul_rn(vym, gx), gz), cu.unit);
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 1, t0 + 1, __fmul_rn(__fmul_rn(vym, ox), gz), cu.unit);
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 1, t0 + TZ, __fmul_rn(__fmul_rn(vym, gx), oz), cu.unit);
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 1, t0 + 1 + TZ, __fmul_rn(__fmul_rn(vym, ox), oz), cu.unit);
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 2, t0, __fmul_rn(__fmul_rn(vzm, gx), gy), cu.unit);
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 2, t0 + 1, __fmul_rn(__fmul_rn(vzm, ox), gy), cu.unit);
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 2, t0 + TY, __fmul_rn(__fmul_rn(vzm, gx), oy), cu.unit);
-          add_float<ACC, SPLIT, TILE3>(smem_raw, 2, t0 + 1 + TY, __fmul_rn(__fmul_rn(vzm, ox), oy), cu.unit);
+          add_float<ACC, SUM, TILE3>(smem_raw, 0, t0, __fmul_rn(__fmul_rn(vxm, gy), gz), cu.unit, rs);
+          add_float<ACC, SUM, TILE3>(smem_raw, 0, t0 + TY, __fmul_rn(__fmul_rn(vxm, oy), gz), cu.unit, rs);
+          add_float<ACC, SUM, TILE3>(smem_raw, 0, t0 + TZ, __fmul_rn(__fmul_rn(vxm, gy), oz), cu.unit, rs);
+          add_float<ACC, SUM, TILE3>(smem_raw, 0, t0 + TY + TZ, __fmul_rn(__fmul_rn(vxm, oy), oz), cu.unit, rs);
+          add_float<ACC, SUM, TILE3>(smem_raw, 1, t0, __fmul_rn(__fmul_rn(vym, gx), gz), cu.unit, rs);
+          add_float<ACC, SUM, TILE3>(smem_raw, 1, t0 + 1, __fmul_rn(__fmul_rn(vym, ox), gz), cu.unit, rs);
+          add_float<ACC, SUM, TILE3>(smem_raw, 1, t0 + TZ, __fmul_rn(__fmul_rn(vym, gx), oz), cu.unit, rs);
+          add_float<ACC, SUM, TILE3>(smem_raw, 1, t0 + 1 + TZ, __fmul_rn(__fmul_rn(vym, ox), oz), cu.unit, rs);
+          add_float<ACC, SUM, TILE3>(smem_raw, 2, t0, __fmul_rn(__fmul_rn(vzm, gx), gy), cu.unit, rs);
+          add_float<ACC, SUM, TILE3>(smem_raw, 2, t0 + 1, __fmul_rn(__fmul_rn(vzm, ox), gy), cu.unit, rs);
+          add_float<ACC, SUM, TILE3>(smem_raw, 2, t0 + TY, __fmul_rn(__fmul_rn(vzm, gx), oy), cu.unit, rs);
+          add_float<ACC, SUM, TILE3>(smem_raw, 2, t0 + 1 + TY, __fmul_rn(__fmul_rn(vzm, ox), oy), cu.unit, rs);
         } else {
           // projections.hpp:786-843: T_ii at the 8 vertices, T_ij on plaquettes.
           const float vv[3] = {vx[j], vy[j], vz[j]};
@@ -308,7 +339,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
                 const int cx = (k >> 2) & 1, cy = (k >> 1) & 1, cz = k & 1;
                 const float w = __fmul_rn(
                     __fmul_rn(__fmul_rn(mv2, sel(cx, ox, gx)), sel(cy, oy, gy)), sel(cz, oz, gz));
-                add_float<ACC, SPLIT, TILE3>(smem_raw, jd, t0 + cx + cy * TY + cz * TZ, w, cu.unit);
+                add_float<ACC, SUM, TILE3>(smem_raw, jd, t0 + cx + cy * TY + cz * TZ, w, cu.unit, rs);
               }
             }
           }
@@ -318,23 +349,47 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
             const float m01 = __fmul_rn(__fmul_rn(mf, vv[0]), vv[1]);
             const float m02 = __fmul_rn(__fmul_rn(mf, vv[0]), vv[2]);
             const float m12 = __fmul_rn(__fmul_rn(mf, vv[1]), vv[2]);
-            add_float<ACC, SPLIT, TILE3>(smem_raw, j01, t0, __fmul_rn(m01, gz), cu.unit);
-            add_float<ACC, SPLIT, TILE3>(smem_raw, j01, t0 + TZ, __fmul_rn(m01, oz), cu.unit);
-            add_float<ACC, SPLIT, TILE3>(smem_raw, j02, t0, __fmul_rn(m02, gy), cu.unit);
-            add_float<ACC, SPLIT, TILE3>(smem_raw, j02, t0 + TY, __fmul_rn(m02, oy), cu.unit);
-            add_float<ACC, SPLIT, TILE3>(smem_raw, j12, t0, __fmul_rn(m12, gx), cu.unit);
-            add_float<ACC, SPLIT, TILE3>(smem_raw, j12, t0 + 1, __fmul_rn(m12, ox), cu.unit);
+            add_float<ACC, SUM, TILE3>(smem_raw, j01, t0, __fmul_rn(m01, gz), cu.unit, rs);
+            add_float<ACC, SUM, TILE3>(smem_raw, j01, t0 + TZ, __fmul_rn(m01, oz), cu.unit, rs);
+            add_float<ACC, SUM, TILE3>(smem_raw, j02, t0, __fmul_rn(m02, gy), cu.unit, rs);
+            add_float<ACC, SUM, TILE3>(smem_raw, j02, t0 + TY, __fmul_rn(m02, oy), cu.unit, rs);
+            add_float<ACC, SUM, TILE3>(smem_raw, j12, t0, __fmul_rn(m12, gx), cu.unit, rs);
+            add_float<ACC, SUM, TILE3>(smem_raw, j12, t0 + 1, __fmul_rn(m12, ox), cu.unit, rs);
           }
         }
       }
     }
   };
   
-  if (ACC != ACC_PLAIN && tr.split) particles(std::true_type{});
-  else particles(std::false_type{});
+  using std::integral_constant;
+  bool pairs = ACC == ACC_PLAIN || !tr.split;
+  if constexpr (ACC != ACC_PLAIN) {
+    if (!pairs) particles(integral_constant<int, SUM_INT>{}, cnt);
+  }
+  if constexpr (ACC == ACC_COMP) {
+    __syncthreads();
+    rs.count = s_rests;
+    if (rs.count > P::RESTS) {  // more than the list holds: again, with the FP32 pairs
+      uint32_t* z = reinterpret_cast<uint32_t*>(smem_raw);
+      for (int t = threadIdx.x; t < NC * P::WORDS * TILE3; t += blockDim.x) z[t] = 0u;
+      tr.split = false;
+      pairs = true;
+      __syncthreads();
+    } else if (rs.count) {
+      for (int pass = 0; pass < 2; pass++) {
+        particles(integral_constant<int, SUM_REST>{}, rs.count);
+        __syncthreads();
+        if (rs.apply || !s_notes) break;
+        tr.marks = s_marks;
+        if (take_notes<TILE3>(smem_raw, NC, rs)) break;
+        rs.apply = true;
+      }
+    }
+  }
+  if (pairs) particles(integral_constant<int, SUM_PAIR>{}, cnt);
   __syncthreads();
   if (s_tile >= 0) {  // k_part_finish writes the vertices
-    part_store<ACC, SIGNED, NC, TILE3>(scratch_tile(pv, s_tile, NC * TILE3), tr, cu.q);
+    part_store<ACC, SIGNED, NC, TILE3>(scratch_tile(pv, s_tile, NC * TILE3), tr, s_quantum);
     return;
   }
 
@@ -361,7 +416,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
         if (!SIGNED && q < 0) set_flag(flags, ERR_FIXED_OVERFLOW);
         out[(size_t)c * g.nsites + s] = __fmul_rn(__ll2float_rn(q), conv);
       } else if (ACC == ACC_COMP) {
-        const float2 p = comp_pair(tr, j, t, cu.q);
+        const float2 p = comp_pair(tr, j, t, s_quantum);
         out[(size_t)c * g.nsites + s] = __fadd_rn(p.x, p.y);
       } else {
         out[(size_t)c * g.nsites + s] = facc[(size_t)j * TILE3 + t];
@@ -397,7 +452,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
       if (FIXED) {
         sp[(size_t)c * SHELL + f] = (uint64_t)tile_fixed<SIGNED>(tr, j, t);
       } else if (ACC == ACC_COMP) {
-        reinterpret_cast<float2*>(sp)[(size_t)c * SHELL + f] = comp_pair(tr, j, t, cu.q);
+        reinterpret_cast<float2*>(sp)[(size_t)c * SHELL + f] = comp_pair(tr, j, t, s_quantum);
       } else {
         reinterpret_cast<float*>(sp)[(size_t)c * SHELL + f] = facc[(size_t)j * TILE3 + t];
       }
@@ -648,7 +703,7 @@ cudaError_t tile_pass(lf2_ctx* c, float* out, const DepositParams& dp, const uin
                       const PartView& pv)
 {
   using P = Pass<KIND, PASS, ACC>;
-  const size_t smem = P::smem();
+  const size_t smem = P::dyn();
   const auto kern = dp.has_mass ? k_deposit<KIND, PASS, ACC, true> : k_deposit<KIND, PASS, ACC, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -666,7 +721,7 @@ template <int KIND, int ACC>
 PartPlan tile_plan(lf2_ctx* c)
 {
   using P = Pass<KIND, 0, ACC>;
-  return part_plan(c, P::smem(), P::THREADS, (size_t)P::NC * TILE3,
+  return part_plan(c, P::dyn(), P::THREADS, (size_t)P::NC * TILE3,
                    ACC == ACC_FIXED  ? split_max<KIND != 0>(c->has_mass ? 2 : 1)
                    : ACC == ACC_COMP ? split_max<true>(1)
                                      : 0);

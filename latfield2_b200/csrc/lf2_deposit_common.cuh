@@ -38,10 +38,17 @@ __host__ __device__ inline int split_max(int mass_bound)
 // A tile of N vertices per component in shared memory: component j occupies
 // words [2 j N, 2 (j + 1) N) (two 32-bit words per vertex), or [j N, (j+1) N)
 // in the plain mode.
+// marks: a bit per component and vertex (j N + t) whose words are the FP32 pair
+// although the tile is split (compensated mode), or null.
 template <int N>
 struct TileRef {
   unsigned char* smem;
   bool split;
+  const uint32_t* marks;
+  __device__ __forceinline__ bool pair(int i) const
+  {
+    return !split || (marks && (marks[i >> 5] >> (i & 31) & 1u));
+  }
 };
 
 template <int N>
@@ -117,60 +124,129 @@ __device__ __forceinline__ void add_fixed48_t(unsigned char* smem, int j, int t,
 
 // Compensated FP32 mode.  The terms are the FP32 products of the reference's
 // arithmetic; their sum is kept, as in the signed fixed-point kinds, as a
-// 64-bit integer in two 32-bit words, in units of 2^-48 of a power of two
-// 2^e above every |term| of the CTA's particles.  A term is added exactly
-// when it is at least 2^-24 of 2^e, and otherwise to 2^-49 of it; the sum is
-// exact.  (An FP32 shared atomic compiles to a compare-and-swap loop: the
-// TwoSum pair of add_comp takes 3.4 times the shared wavefronts of the two
-// integer words.)  add_comp stays for what the integers cannot hold: terms
-// that are not finite or out of range, and more than split_max particles.
-//
-// x: the term in units of 2^(e - 16), |x| < 2^16.  x = hi + lo 2^-32 with hi
-// the nearest integer (the sum with 1.5 * 2^23 rounds there) and lo signed.
+// 64-bit integer in two 32-bit words, in units of a quantum set by the largest
+// term of the CTA's particles (CompUnit).  A term at or above 2^23 quanta is a
+// whole number of them.  A particle that may have a smaller one (one in a
+// thousand for the density, 7% for the diagonal stress of Gaussian velocities)
+// is listed, and what its terms leave below the quantum joins the sums at the
+// end (add_rest) where it can be told from their rounding, so that every term
+// counts in full whatever stands beside it.
+// (An FP32 shared atomic compiles to a compare-and-swap loop: the TwoSum pair
+// of add_comp takes 3.4 times the shared wavefronts of the two integer words.)
+// add_comp stays for what the integers cannot hold: terms that are not finite
+// or out of range, more than split_max particles, and more listed ones than
+// the list takes.  The two full-CIC calls at 256^3 in clumps take 3.25 ms, of
+// which 0.37 are the rests; the densities of 64^3 and 256^3 show no difference.
+enum : int { SUM_PAIR, SUM_INT, SUM_REST };  // what a run over the particles does
+
+struct RestList {
+  uint16_t* entry;  // listed particles of the CTA
+  int* count;       // how many were to be listed
+  int room;
+  __device__ __forceinline__ void add(int i) const
+  {
+    const int k = atomicAdd(count, 1);
+    if (k < room) entry[k] = (uint16_t)i;
+  }
+};
+
+// The run over the listed particles takes a component to a warp (a chain of
+// the terms of all three is long for the few warps that have one): items
+// [c R, c R + count) with R = list_stride(count) are component c's.
+__host__ __device__ inline int list_stride(int count) { return (count + 31) & ~31; }
+
+// A particle whose smallest term, `least` in units of 2^31 quanta, has fewer
+// than 2^23 of them (2^24: with room for the rounding of the bound) is listed.
+__device__ __forceinline__ bool has_rest(float least) { return least < 0x1p-7f; }
+
+// w: the term; x = w in units of 2^31 quanta, |x| < 2^21.  x = hi + lo 2^-31
+// with hi the nearest integer (the sum with 1.5 * 2^23 rounds there) and lo
+// the nearest integer to the remainder, |lo| <= 2^30.  The words hold
+// hi 2^31 + lo: a carry or borrow of the low word is worth 2 of the high one.
 template <int N>
-__device__ __forceinline__ void add_comp_int(unsigned char* smem, int j, int t, float x)
+__device__ __forceinline__ void add_comp_int(unsigned char* smem, int j, int t, float w, float unit)
 {
-  uint32_t* w = reinterpret_cast<uint32_t*>(smem) + (size_t)j * 2 * N;
+  uint32_t* words = reinterpret_cast<uint32_t*>(smem) + (size_t)j * 2 * N;
+  const float x = __fmul_rn(w, unit);
   const float h = __fadd_rn(x, 12582912.0f);
   const int hi = __float_as_int(h) - 0x4B400000;
   const float r = __fsub_rn(x, __fsub_rn(h, 12582912.0f));  // exact, |r| <= 1/2
-  const int lo = __float2int_rn(__fmul_rn(r, 4294967296.0f));  // 2^31 - 1 at r = 1/2
-  const uint32_t old = atomicAdd(&w[t], (uint32_t)lo);
+  const int lo = __float2int_rn(__fmul_rn(r, 2147483648.0f));
+  const uint32_t old = atomicAdd(&words[t], (uint32_t)lo);
   const int carry = old + (uint32_t)lo < old ? 1 : 0;
-  atomicAdd(reinterpret_cast<int*>(&w[N + t]), hi + (lo >> 31) + carry);
+  atomicAdd(reinterpret_cast<int*>(&words[N + t]), hi + 2 * ((lo >> 31) + carry));
 }
 
-// One FP32 term of either mode; SPLIT: the integer sums of the compensated one
-// (unit: CompUnit).
-template <int ACC, bool SPLIT, int N>
-__device__ __forceinline__ void add_float(unsigned char* smem, int j, int t, float w, float unit)
+// What add_comp_int left of a listed particle's term below its quantum.  First
+// it is only asked whether it matters: half a quantum from each of `rests`
+// particles is under 2^-28 of a vertex sum of 2^27 `rests` quanta, a sixteenth
+// of the last rounding.  A smaller sum with a rest is marked, and the rest
+// noted; the marked sums become FP32 pairs (to_pairs) and then take their
+// rests, from the notes, or in another run (apply) where those ran out of room.
+struct Rests {
+  int count;
+  bool apply;
+  float quantum;
+  uint32_t* marks;  // TileRef
+  uint2* note;      // word of the vertex in the tile, bits of the rest
+  int* notes;       // how many were to be noted
+  int room;
+};
+
+template <int N>
+__device__ __forceinline__ void add_rest(unsigned char* smem, int j, int t, float w, float unit,
+                                         const Rests& rs)
+{
+  const float x = __fmul_rn(w, unit);
+  if (!(fabsf(x) < 0x1p-8f)) return;  // a whole number of quanta
+  const float lo = __int2float_rn(__float2int_rn(__fmul_rn(x, 2147483648.0f)));
+  const float rest = __fmaf_rn(-lo, rs.quantum, w);  // exact
+  if (rest == 0.0f) return;
+  float* f = reinterpret_cast<float*>(smem) + (size_t)j * 2 * N + t;
+  const int i = j * N + t;
+  if (rs.apply) {
+    if (rs.marks[i >> 5] >> (i & 31) & 1u) add_comp(f, f + N, rest);
+  } else if (rs.count > 16 * (abs(__float_as_int(f[N])) - 2)) {  // (high word: units of 2^31 quanta)
+    atomicOr(&rs.marks[i >> 5], 1u << (i & 31));
+    const int k = atomicAdd(rs.notes, 1);
+    if (k < rs.room) rs.note[k] = make_uint2((uint32_t)(j * 2 * N + t), __float_as_uint(rest));
+  }
+}
+
+// One FP32 term of either mode.
+template <int ACC, int SUM, int N>
+__device__ __forceinline__ void add_float(unsigned char* smem, int j, int t, float w, float unit,
+                                          const Rests& rs)
 {
   float* f = reinterpret_cast<float*>(smem);
   if (ACC == ACC_PLAIN)
     atomicAdd(&f[(size_t)j * N + t], w);
-  else if (SPLIT)
-    add_comp_int<N>(smem, j, t, __fmul_rn(w, unit));
+  else if (SUM == SUM_INT)
+    add_comp_int<N>(smem, j, t, w, unit);
+  else if (SUM == SUM_REST)
+    add_rest<N>(smem, j, t, w, unit, rs);
   else
     add_comp(&f[(size_t)j * 2 * N + t], &f[(size_t)j * 2 * N + N + t], w);
 }
 
 // The unit of a CTA's terms, from the largest bound M of any of its particles:
-// 2^q is the quantum of the integer sums, `unit` = 2^(-32 - q) takes a term to
-// what add_comp_int adds.  ok: M is in the range where both are normal FP32
-// numbers with room to spare, and the particles are few enough.
+// 2^q is the quantum of the integer sums, `unit` = 2^(-32 - q).  With M < 2^e
+// and fewer than 2^k particles the high words stay within int32 for
+// |x| <= 2^(31 - k).  ok: both powers and every whole number of quanta are
+// normal FP32 numbers, and the particles are few enough for 16 bits of x.
 struct CompUnit {
-  int q;
-  float unit;
+  float quantum, unit;
   bool ok;
 };
 
 __device__ __forceinline__ CompUnit comp_unit_of(unsigned bits, int cnt)
 {
   const int e = (int)(bits >> 23) - 126;  // M < 2^e for a normal number
+  const int s = min(21, __clz(cnt) - 1);
   CompUnit r;
-  r.ok = e >= -90 && e <= 127 && cnt <= split_max<true>(1);
-  r.q = e - 48;
-  r.unit = r.ok ? ldexpf(1.0f, 16 - e) : 1.0f;
+  r.ok = e >= -70 && e <= 127 && cnt <= split_max<true>(1);
+  r.unit = r.ok ? ldexpf(1.0f, s - e) : 1.0f;
+  r.quantum = r.ok ? ldexpf(1.0f, e - s - 31) : 1.0f;
   return r;
 }
 
@@ -206,16 +282,42 @@ __device__ __forceinline__ CompUnit comp_unit(const float* mass, float inv_vol, 
   return comp_unit_of(*s_max, cnt);
 }
 
-// hi/lo pair of a compensated vertex sum, from the integers (quantum 2^q) or
-// the floats.
+// hi/lo pair of a compensated vertex sum, from the integers or the floats.
 template <int N>
-__device__ __forceinline__ float2 comp_pair(const TileRef<N>& tr, int j, int t, int q)
+__device__ __forceinline__ float2 comp_pair(const TileRef<N>& tr, int j, int t, float quantum)
 {
   const uint32_t* w = reinterpret_cast<const uint32_t*>(tr.smem) + (size_t)j * 2 * N;
-  if (!tr.split) return make_float2(__uint_as_float(w[t]), __uint_as_float(w[N + t]));
-  const long long s = (long long)(int32_t)w[N + t] * 4294967296ll + (long long)w[t];
+  if (tr.pair(j * N + t)) return make_float2(__uint_as_float(w[t]), __uint_as_float(w[N + t]));
+  const long long s = (long long)(int32_t)w[N + t] * 2147483648ll + (long long)w[t];
   const float hi = __ll2float_rn(s), lo = __ll2float_rn(s - (long long)hi);
-  return make_float2(ldexpf(hi, q), ldexpf(lo, q));
+  return make_float2(__fmul_rn(hi, quantum), __fmul_rn(lo, quantum));
+}
+
+// After the first run over the listed particles, by the whole CTA: the marked
+// vertex sums as FP32 pairs, and the noted rests.  False where another run has
+// to add the rests.  (With all sums as pairs in every CTA that has a mark, and
+// the second run instead of notes, the calls above took 3.67 ms.)
+template <int N>
+__device__ __forceinline__ bool take_notes(unsigned char* smem, int comps, const Rests& rs)
+{
+  uint32_t* w = reinterpret_cast<uint32_t*>(smem);
+  float* f = reinterpret_cast<float*>(smem);
+  const TileRef<N> ints{smem, true, nullptr};
+  for (int k = threadIdx.x; k < (comps * N + 31) / 32; k += blockDim.x) {
+    for (uint32_t m = rs.marks[k]; m; m &= m - 1) {
+      const int i = 32 * k + __ffs(m) - 1, j = i / N, t = i % N, at = j * 2 * N + t;
+      const float2 p = comp_pair(ints, j, t, rs.quantum);
+      w[at] = __float_as_uint(p.x);
+      w[at + N] = __float_as_uint(p.y);
+    }
+  }
+  __syncthreads();
+  const int n = *rs.notes;
+  if (n > rs.room) return false;
+  for (int k = threadIdx.x; k < n; k += blockDim.x)
+    add_comp(&f[rs.note[k].x], &f[rs.note[k].x + N], __uint_as_float(rs.note[k].y));
+  __syncthreads();
+  return true;
 }
 
 // Integer vertex sum of component j: the scalar's split (lo + hi 2^16) or
@@ -438,10 +540,9 @@ __device__ __forceinline__ bool part_take(const PartView& pv, int64_t nbricks, c
 }
 
 // A part's tile to the scratch: 8-byte values, component j of vertex t at
-// j * N + t (the integer sum, the hi/lo pair or the float).  cq: the quantum of
-// the compensated mode's integers (CompUnit).
+// j * N + t (the integer sum, the hi/lo pair or the float); quantum: CompUnit.
 template <int ACC, bool SIGNED, int NC, int N>
-__device__ __forceinline__ void part_store(uint64_t* dst, const TileRef<N>& tr, int cq)
+__device__ __forceinline__ void part_store(uint64_t* dst, const TileRef<N>& tr, float quantum)
 {
   const uint32_t* w = reinterpret_cast<const uint32_t*>(tr.smem);
   for (int t = threadIdx.x; t < N; t += blockDim.x) {
@@ -451,7 +552,7 @@ __device__ __forceinline__ void part_store(uint64_t* dst, const TileRef<N>& tr, 
       if (ACC == ACC_FIXED) {
         q = (uint64_t)tile_fixed<SIGNED>(tr, j, t);
       } else if (ACC == ACC_COMP) {
-        const float2 v = comp_pair(tr, j, t, cq);
+        const float2 v = comp_pair(tr, j, t, quantum);
         q = (uint64_t)__float_as_uint(v.x) | ((uint64_t)__float_as_uint(v.y) << 32);
       } else {
         q = w[(size_t)j * N + t];

@@ -137,7 +137,7 @@ __global__ void k_pm_deposit_fixed(Geom g, int64_t np, const int32_t* __restrict
 // then the tile's non-zero sums go to the global field with one atomic each:
 // 4913 global atomics per tile instead of 8 per particle.  Both keep integer
 // sums, a low word whose carry goes to a high word: the fixed-point weights,
-// or the FP32 products in units of 2^-48 of the largest (add_comp_int; a
+// or the FP32 products in a unit set by the largest (CompUnit; a
 // floating-point shared atomic is a compare-and-swap loop).  The CTA of a
 // brick takes its first `part` particles; what a brick holds beyond those is
 // shared out among CTAs by their slots, since each adds to the field on its
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(256)
     }
     if (half) __syncthreads();  // the tile before is flushed
     for (int t = threadIdx.x; t < TILE3; t += blockDim.x) lo[t] = hi[t] = 0u;
-    CompUnit cu{0, 1.0f, true};
+    CompUnit cu{1.0f, 1.0f, true};
     if (!FIXED)  // (slots may exceed 32 bits)
       cu = comp_unit<0>(mass ? mass + p0 : nullptr, inv_vol, gmass * inv_vol, nullptr, nullptr, nullptr,
                         0u, (int)(p1 - p0), &s_max);
@@ -273,11 +273,11 @@ __global__ void __launch_bounds__(256)
           return (long long)w;
         }
         const float w = (cx ? f[0] : 1.0f - f[0]) * (cy ? f[1] : 1.0f - f[1]) * (cz ? f[2] : 1.0f - f[2]);
-        const float v = w * m * cu.unit;  // |v| < 2^16
+        const float v = w * m * cu.unit;  // |v| < 2^21, in units of 2^31 quanta
         const float h = __fadd_rn(v, 12582912.0f);
         const float r = __fsub_rn(v, __fsub_rn(h, 12582912.0f));
-        return ((long long)(__float_as_int(h) - 0x4B400000) << 32) +
-               (long long)__float2int_rn(__fmul_rn(r, 4294967296.0f));
+        return ((long long)(__float_as_int(h) - 0x4B400000) << 31) +
+               (long long)__float2int_rn(__fmul_rn(r, 2147483648.0f));
       };
       const bool tiled = on && cu.ok && in_brick(x, y, z, x0, y0, z0);
       const int t0 = (x - x0) + TILE * ((y - y0) + TILE * (z - z0));
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
           for (int q = 0; q < 8; q++) {
             const long long w = mine ? weight(q) : 0ll;
-            // 32 values below 2^48: the sums of 20-bit pieces stay below 2^31
+            // 32 values below 2^52: the sums of 20-bit pieces stay below 2^31
             const long long sum =
                 (long long)__reduce_add_sync(0xffffffffu, (unsigned)(w & 0xfffff)) +
                 ((long long)__reduce_add_sync(0xffffffffu, (unsigned)((w >> 20) & 0xfffff)) << 20) +
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(256)
       if (FIXED)
         atomicAdd(&acc[tile_site(g, t, x0, y0, z0)], v);
       else
-        atomicAdd(&rho[tile_site(g, t, x0, y0, z0)], ldexpf(__ll2float_rn((long long)v), cu.q));
+        atomicAdd(&rho[tile_site(g, t, x0, y0, z0)], __ll2float_rn((long long)v) * cu.quantum);
     }
   }
 }

@@ -67,3 +67,77 @@ def test_units_of_mass_and_velocity(cuda, kind, individual):
     assert tried >= (11 if power == 0 else 40)
     assert ctx.flags() == 0
     ctx.close()
+
+
+def _wide_case(name, npart=6000, n=(20, 20, 20)):
+    """Terms far below the largest of their brick, whole vertices among them."""
+    rng = np.random.default_rng(11)
+    cell = rng.integers(0, n[0] * n[1] * n[2], npart).astype(np.int32)
+    off = (rng.random((npart, 3)) * (1 - 2.0 ** -23)).astype(np.float32)
+    vel = rng.standard_normal((npart, 3)).astype(np.float32)
+    mass = np.full(npart, 1.0 / npart, np.float32)
+    few = rng.choice(npart, 60, replace=False)
+    if name == "fast one":  # a slow population beside one fast particle per brick
+        vel *= np.float32(1e-6)
+        vel[few[:8]] = (0.9, -0.7, 0.8)
+    elif name == "slow few":  # few enough for the list of rests
+        vel[few] *= np.float32(1e-9)
+    elif name == "planar":  # every T_i2 term far below T_00
+        vel[:, 2] *= np.float32(1e-9)
+    elif name == "light few":
+        mass[few] *= np.float32(1e-20)
+        cell[few] = np.arange(60) * 133
+    else:
+        assert name == "light"
+        mass = (10.0 ** rng.uniform(-25, 0, npart)).astype(np.float32)
+    return n, cell, off, vel, mass
+
+
+@pytest.mark.parametrize("name", ["fast one", "slow few", "planar", "light few", "light"])
+@pytest.mark.parametrize("kind", [0, 1, 2, 3, 4])
+def test_small_terms_beside_large_ones(cuda, kind, name):
+    """Every vertex that a particle touches, however small its sum beside the
+    others': within 1e-6 of the sum of its |terms| (six FP32 roundings of
+    2^-24 at most, the sum being exact)."""
+    import latfield2_b200 as L
+    n, cell, off, vel, mass = _wide_case(name)
+    res = 1.0 / n[0]
+    if kind == 0:
+        ref = O.state_deposit_f64(n, cell, off, res, mass=mass).reshape(1, *n)
+        mag = ref
+    else:
+        cs, order = O.lists_from_insertion(n, cell)
+        pos = positions(n, res, cell, off)[order]
+        ref, mag = (O.interior(KINDS[kind][2](n, 1, res, cs, pos, v.astype(np.float64)[order],
+                                              pmass=mass.astype(np.float64)[order]), n, 1)
+                    for v in (vel, np.abs(vel)))
+    ctx = L.Context(n, box=1.0, mode=L.DEPOSIT_FP32)
+    ctx.set_particles(cell, off, vel, mass=mass)
+    f = ctx.field(ref.shape[0])
+    getattr(ctx, ("deposit_scalar" if kind == 0 else KINDS[kind][0]))(f)
+    got = f.export_internal()
+    for c in range(ref.shape[0]):
+        some = mag[c] > 0
+        err = np.abs(got[c].astype(np.float64) - ref[c])[some] / mag[c][some]
+        assert err.max() <= 1e-6, (c, err.max())
+        assert not got[c][~some].any()
+    ctx.close()
+
+
+def test_single_terms_are_exact(cuda):
+    """A vertex that one term reaches holds that term, at every power of two
+    below the brick's largest and for values of 24 bits."""
+    import latfield2_b200 as L
+    n = (32, 32, 32)
+    k = np.arange(120)
+    cell = np.array([(2 * i % 16) + 32 * ((2 * i // 16 * 2) % 16) + 1024 * (2 * (i // 64)) for i in k],
+                    np.int32)
+    assert len(set(cell)) == 120
+    mass = (np.ldexp(1.0, -(k // 2)) * np.where(k % 2, 1.0, 1.0 - 2.0 ** -24)).astype(np.float32)
+    ctx = L.Context(n, box=32.0, mode=L.DEPOSIT_FP32)
+    ctx.set_particles(cell, np.zeros((120, 3), np.float32), np.zeros((120, 3), np.float32), mass=mass)
+    f = ctx.field(1)
+    ctx.deposit_scalar(f)
+    got = f.export_internal().reshape(-1)
+    np.testing.assert_array_equal(got[cell], mass)
+    ctx.close()
