@@ -193,14 +193,18 @@ struct Rests {
   int room;
 };
 
+__device__ __forceinline__ float comp_rest(float w, float unit, float quantum)
+{
+  const float x = __fmul_rn(w, unit);
+  if (!(fabsf(x) < 0x1p-8f)) return 0.0f;  // a whole number of quanta
+  return __fmaf_rn(-__int2float_rn(__float2int_rn(__fmul_rn(x, 2147483648.0f))), quantum, w);  // exact
+}
+
 template <int N>
 __device__ __forceinline__ void add_rest(unsigned char* smem, int j, int t, float w, float unit,
                                          const Rests& rs)
 {
-  const float x = __fmul_rn(w, unit);
-  if (!(fabsf(x) < 0x1p-8f)) return;  // a whole number of quanta
-  const float lo = __int2float_rn(__float2int_rn(__fmul_rn(x, 2147483648.0f)));
-  const float rest = __fmaf_rn(-lo, rs.quantum, w);  // exact
+  const float rest = comp_rest(w, unit, rs.quantum);
   if (rest == 0.0f) return;
   float* f = reinterpret_cast<float*>(smem) + (size_t)j * 2 * N + t;
   const int i = j * N + t;

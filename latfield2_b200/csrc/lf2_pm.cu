@@ -138,7 +138,8 @@ __global__ void k_pm_deposit_fixed(Geom g, int64_t np, const int32_t* __restrict
 // 4913 global atomics per tile instead of 8 per particle.  Both keep integer
 // sums, a low word whose carry goes to a high word: the fixed-point weights,
 // or the FP32 products in a unit set by the largest (CompUnit; a
-// floating-point shared atomic is a compare-and-swap loop).  The CTA of a
+// floating-point shared atomic is a compare-and-swap loop), a small product's
+// rest below the unit going straight to the field.  The CTA of a
 // brick takes its first `part` particles; what a brick holds beyond those is
 // shared out among CTAs by their slots, since each adds to the field on its
 // own (one CTA took 1.4 ms for a brick of 131k particles at 256^3).
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__(256)
           return (long long)w;
         }
         const float w = (cx ? f[0] : 1.0f - f[0]) * (cy ? f[1] : 1.0f - f[1]) * (cz ? f[2] : 1.0f - f[2]);
-        const float v = w * m * cu.unit;  // |v| < 2^21, in units of 2^31 quanta
+        const float term = w * m, v = __fmul_rn(term, cu.unit);  // |v| < 2^21, in units of 2^31 quanta
         const float h = __fadd_rn(v, 12582912.0f);
         const float r = __fsub_rn(v, __fsub_rn(h, 12582912.0f));
         return ((long long)(__float_as_int(h) - 0x4B400000) << 31) +
@@ -281,6 +282,20 @@ __global__ void __launch_bounds__(256)
       };
       const bool tiled = on && cu.ok && in_brick(x, y, z, x0, y0, z0);
       const int t0 = (x - x0) + TILE * ((y - y0) + TILE * (z - z0));
+      if (!FIXED && tiled) {  // terms that are no whole number of quanta: their rests to the field
+        const float least = fminf(f[0], 1.0f - f[0]) * fminf(f[1], 1.0f - f[1]) * fminf(f[2], 1.0f - f[2]) *
+                            fabsf(m);
+        if (has_rest(__fmul_rn(least, cu.unit))) {
+#pragma unroll 1
+          for (int q = 0; q < 8; q++) {
+            const int cx = (q >> 2) & 1, cy = (q >> 1) & 1, cz = q & 1;
+            const float w = (cx ? f[0] : 1.0f - f[0]) * (cy ? f[1] : 1.0f - f[1]) * (cz ? f[2] : 1.0f - f[2]);
+            const float rest = comp_rest(w * m, cu.unit, cu.quantum);
+            if (rest != 0.0f)
+              atomicAdd(&rho[tile_site(g, t0 + cx + TILE * (cy + TILE * cz), x0, y0, z0)], rest);
+          }
+        }
+      }
       // runs of lanes in one cell
       const int key = tiled ? t0 : -1 - lane;
       const int before = __shfl_up_sync(0xffffffffu, key, 1);

@@ -141,3 +141,30 @@ def test_single_terms_are_exact(cuda):
     got = f.export_internal().reshape(-1)
     np.testing.assert_array_equal(got[cell], mass)
     ctx.close()
+
+
+@pytest.mark.parametrize("name", ["light few", "light"])
+def test_chain_deposit_of_light_particles(cuda, name):
+    """The brick-tiled deposit of the chain: every vertex within the roundings
+    of its terms (three each) and of the FP32 additions to the field (a rest or
+    a brick's sum each, under 30 here), 2^-24 of the sum apiece."""
+    import torch
+    import latfield2_b200 as L
+    from latfield2_b200.autodiff import _Ops
+    n, cell, off, _, mass = _wide_case(name)
+    xyz = np.stack([cell % n[0], cell // n[0] % n[1], cell // (n[0] * n[1])], 1)
+    nb = [(m + 15) // 16 for m in n]
+    brick = xyz[:, 0] // 16 + nb[0] * (xyz[:, 1] // 16 + nb[1] * (xyz[:, 2] // 16))
+    order = np.lexsort((cell, brick))
+    c, o, m = (torch.from_numpy(a[order]).cuda() for a in (cell, off, mass))
+    ctx = L.Context(n, box=1.0, mode=L.DEPOSIT_FP32)
+    ops = _Ops(ctx)
+    ops.bricks = ops.brick_start(c)
+    rho = torch.zeros(n[0] * n[1] * n[2], device="cuda")
+    ops.deposit(c, o, m, rho)
+    ref = O.state_deposit_f64(n, cell, off, 1.0 / n[0], mass=mass)
+    some = ref > 0
+    got = rho.cpu().numpy()
+    assert (np.abs(got.astype(np.float64) - ref)[some] / ref[some]).max() <= 33 * 2.0 ** -24
+    assert not got[~some].any()
+    ctx.close()
