@@ -199,8 +199,8 @@ __device__ __forceinline__ void tile_add(uint32_t* lo, uint32_t* hi, int t, long
 // FIXED: acc += integer weights (times the masses relative to *mmax);
 // otherwise rho += FP32 products.  CTA u < nbricks: brick u's first `part`
 // particles; CTA nbricks + r: what the slots [r part, (r + 1) part) hold of
-// bricks beyond their first `part` particles (at most two such bricks reach a
-// range of that length: those at its ends).
+// bricks beyond their first `part` particles (only the brick of the first slot
+// can: one that starts later has no more than its first ones in the range).
 template <bool FIXED>
 __global__ void __launch_bounds__(256)
     k_pm_deposit_tile(Geom g, int64_t np, const int64_t* __restrict__ brick_start, int part,
@@ -212,143 +212,138 @@ __global__ void __launch_bounds__(256)
   __shared__ unsigned s_max;
   const float inv_m = FIXED && mass ? 1.0f / __uint_as_float(*mmax) : 0.0f;
   const int lane = threadIdx.x & 31;
-  for (int half = 0; half < 2; half++) {
-    int64_t b, p0, p1;
-    if (blockIdx.x < g.nbricks) {
-      if (half) return;
-      b = blockIdx.x;
-      group_range(brick_start, b, np, p0, p1);
-      p1 = min(p1, p0 + part);
+  int64_t b, p0, p1;
+  if (blockIdx.x < g.nbricks) {
+    b = blockIdx.x;
+    group_range(brick_start, b, np, p0, p1);
+    p1 = min(p1, p0 + part);
+  } else {
+    const int64_t r0 = ((int64_t)blockIdx.x - g.nbricks) * part, r1 = min(r0 + part, np);
+    b = brick_of_slot(brick_start, g.nbricks, r0);
+    group_range(brick_start, b, np, p0, p1);
+    p0 = max(p0 + part, r0);
+    p1 = min(p1, r1);
+    if (p0 >= p1) return;
+  }
+  for (int t = threadIdx.x; t < TILE3; t += blockDim.x) lo[t] = hi[t] = 0u;
+  CompUnit cu{1.0f, 1.0f, true};
+  if (!FIXED)  // (slots may exceed 32 bits)
+    cu = comp_unit<0>(mass ? mass + p0 : nullptr, inv_vol, gmass * inv_vol, nullptr, nullptr, nullptr,
+                      0u, (int)(p1 - p0), &s_max);
+  __syncthreads();
+  int bx, by, bz;
+  brick_coords(g, b, bx, by, bz);
+  const int x0 = bx * BRICK, y0 = by * BRICK, z0 = bz * BRICK;
+  // the next trip's particle is read while this one's is added
+  int32_t c_next = 0;
+  float f_next[3] = {0.f, 0.f, 0.f}, m_next = gmass;
+  auto fetch = [&](int64_t p) {
+    if (p >= p1) return;
+    c_next = cell[p];
+    f_next[0] = off3[3 * p], f_next[1] = off3[3 * p + 1], f_next[2] = off3[3 * p + 2];
+    if (mass) m_next = mass[p];
+  };
+  fetch(p0 + threadIdx.x);
+  for (int64_t q0 = p0; q0 < p1; q0 += blockDim.x) {
+    const int64_t p = q0 + threadIdx.x;
+    const bool on = p < p1;
+    int x, y, z;
+    cell_xyz(g, c_next, x, y, z);
+    const float f[3] = {f_next[0], f_next[1], f_next[2]};
+    float m = m_next;
+    fetch(p + blockDim.x);
+    uint32_t qx[2], qy[2], qz[2];
+    uint64_t mq = 0;
+    if (FIXED) {
+      qx[1] = weight_q(f[0]), qy[1] = weight_q(f[1]), qz[1] = weight_q(f[2]);
+      qx[0] = (1u << 31) - qx[1], qy[0] = (1u << 31) - qy[1], qz[0] = (1u << 31) - qz[1];
+      if (mass) mq = (uint64_t)__float2uint_rn(fminf(__fmul_rn(m, inv_m), 1.0f) * 16777216.0f);
     } else {
-      const int64_t r0 = ((int64_t)blockIdx.x - g.nbricks) * part, r1 = min(r0 + part, np);
-      b = brick_of_slot(brick_start, g.nbricks, half ? r1 - 1 : r0);
-      if (half && brick_start[b] <= r0) return;  // the same brick as at the other end
-      group_range(brick_start, b, np, p0, p1);
-      p0 = max(p0 + part, r0);
-      p1 = min(p1, r1);
-      if (p0 >= p1) continue;
+      m *= inv_vol;
     }
-    if (half) __syncthreads();  // the tile before is flushed
-    for (int t = threadIdx.x; t < TILE3; t += blockDim.x) lo[t] = hi[t] = 0u;
-    CompUnit cu{1.0f, 1.0f, true};
-    if (!FIXED)  // (slots may exceed 32 bits)
-      cu = comp_unit<0>(mass ? mass + p0 : nullptr, inv_vol, gmass * inv_vol, nullptr, nullptr, nullptr,
-                        0u, (int)(p1 - p0), &s_max);
-    __syncthreads();
-    int bx, by, bz;
-    brick_coords(g, b, bx, by, bz);
-    const int x0 = bx * BRICK, y0 = by * BRICK, z0 = bz * BRICK;
-    // the next trip's particle is read while this one's is added
-    int32_t c_next = 0;
-    float f_next[3] = {0.f, 0.f, 0.f}, m_next = gmass;
-    auto fetch = [&](int64_t p) {
-      if (p >= p1) return;
-      c_next = cell[p];
-      f_next[0] = off3[3 * p], f_next[1] = off3[3 * p + 1], f_next[2] = off3[3 * p + 2];
-      if (mass) m_next = mass[p];
-    };
-    fetch(p0 + threadIdx.x);
-    for (int64_t q0 = p0; q0 < p1; q0 += blockDim.x) {
-      const int64_t p = q0 + threadIdx.x;
-      const bool on = p < p1;
-      int x, y, z;
-      cell_xyz(g, c_next, x, y, z);
-      const float f[3] = {f_next[0], f_next[1], f_next[2]};
-      float m = m_next;
-      fetch(p + blockDim.x);
-      uint32_t qx[2], qy[2], qz[2];
-      uint64_t mq = 0;
+    // corner q's integer contribution
+    auto weight = [&](int q) -> long long {
+      const int cx = (q >> 2) & 1, cy = (q >> 1) & 1, cz = q & 1;
       if (FIXED) {
-        qx[1] = weight_q(f[0]), qy[1] = weight_q(f[1]), qz[1] = weight_q(f[2]);
-        qx[0] = (1u << 31) - qx[1], qy[0] = (1u << 31) - qy[1], qz[0] = (1u << 31) - qz[1];
-        if (mass) mq = (uint64_t)__float2uint_rn(fminf(__fmul_rn(m, inv_m), 1.0f) * 16777216.0f);
-      } else {
-        m *= inv_vol;
+        uint64_t w = fixed_corner(qx[cx], qy[cy], qz[cz]);
+        if (mass) w = (w * mq + (1ull << 23)) >> 24;
+        return (long long)w;
       }
-      // corner q's integer contribution
-      auto weight = [&](int q) -> long long {
-        const int cx = (q >> 2) & 1, cy = (q >> 1) & 1, cz = q & 1;
-        if (FIXED) {
-          uint64_t w = fixed_corner(qx[cx], qy[cy], qz[cz]);
-          if (mass) w = (w * mq + (1ull << 23)) >> 24;
-          return (long long)w;
-        }
-        const float w = (cx ? f[0] : 1.0f - f[0]) * (cy ? f[1] : 1.0f - f[1]) * (cz ? f[2] : 1.0f - f[2]);
-        const float term = w * m, v = __fmul_rn(term, cu.unit);  // |v| < 2^21, in units of 2^31 quanta
-        const float h = __fadd_rn(v, 12582912.0f);
-        const float r = __fsub_rn(v, __fsub_rn(h, 12582912.0f));
-        return ((long long)(__float_as_int(h) - 0x4B400000) << 31) +
-               (long long)__float2int_rn(__fmul_rn(r, 2147483648.0f));
-      };
-      const bool tiled = on && cu.ok && in_brick(x, y, z, x0, y0, z0);
-      const int t0 = (x - x0) + TILE * ((y - y0) + TILE * (z - z0));
-      if (!FIXED && tiled) {  // terms that are no whole number of quanta: their rests to the field
-        const float least = fminf(f[0], 1.0f - f[0]) * fminf(f[1], 1.0f - f[1]) * fminf(f[2], 1.0f - f[2]) *
-                            fabsf(m);
-        if (has_rest(__fmul_rn(least, cu.unit))) {
+      const float w = (cx ? f[0] : 1.0f - f[0]) * (cy ? f[1] : 1.0f - f[1]) * (cz ? f[2] : 1.0f - f[2]);
+      const float term = w * m, v = __fmul_rn(term, cu.unit);  // |v| < 2^21, in units of 2^31 quanta
+      const float h = __fadd_rn(v, 12582912.0f);
+      const float r = __fsub_rn(v, __fsub_rn(h, 12582912.0f));
+      return ((long long)(__float_as_int(h) - 0x4B400000) << 31) +
+             (long long)__float2int_rn(__fmul_rn(r, 2147483648.0f));
+    };
+    const bool tiled = on && cu.ok && in_brick(x, y, z, x0, y0, z0);
+    const int t0 = (x - x0) + TILE * ((y - y0) + TILE * (z - z0));
+    if (!FIXED && tiled) {  // terms that are no whole number of quanta: their rests to the field
+      const float least = fminf(f[0], 1.0f - f[0]) * fminf(f[1], 1.0f - f[1]) * fminf(f[2], 1.0f - f[2]) *
+                          fabsf(m);
+      if (has_rest(__fmul_rn(least, cu.unit))) {
 #pragma unroll 1
-          for (int q = 0; q < 8; q++) {
-            const int cx = (q >> 2) & 1, cy = (q >> 1) & 1, cz = q & 1;
-            const float w = (cx ? f[0] : 1.0f - f[0]) * (cy ? f[1] : 1.0f - f[1]) * (cz ? f[2] : 1.0f - f[2]);
-            const float rest = comp_rest(w * m, cu.unit, cu.quantum);
-            if (rest != 0.0f)
-              atomicAdd(&rho[tile_site(g, t0 + cx + TILE * (cy + TILE * cz), x0, y0, z0)], rest);
-          }
-        }
-      }
-      // runs of lanes in one cell
-      const int key = tiled ? t0 : -1 - lane;
-      const int before = __shfl_up_sync(0xffffffffu, key, 1);
-      const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || key != before);
-      if (__popc(heads) <= DENSE_RUNS) {
-        for (unsigned rest = heads; rest; rest &= rest - 1) {
-          const int first = __ffs(rest) - 1, next = __ffs(rest & (rest - 1));
-          const bool mine = lane >= first && (next == 0 || lane < next - 1);
-          const int t = __shfl_sync(0xffffffffu, key, first);
-          if (t < 0) continue;  // a lane that is not in the tile: below
-#pragma unroll
-          for (int q = 0; q < 8; q++) {
-            const long long w = mine ? weight(q) : 0ll;
-            // 32 values below 2^52: the sums of 20-bit pieces stay below 2^31
-            const long long sum =
-                (long long)__reduce_add_sync(0xffffffffu, (unsigned)(w & 0xfffff)) +
-                ((long long)__reduce_add_sync(0xffffffffu, (unsigned)((w >> 20) & 0xfffff)) << 20) +
-                ((long long)__reduce_add_sync(0xffffffffu, (int)(w >> 40)) << 40);
-            if (lane == q)
-              tile_add(lo, hi, t + ((q >> 2) & 1) + TILE * (((q >> 1) & 1) + TILE * (q & 1)), sum);
-          }
-        }
-      } else if (tiled) {
-#pragma unroll
-        for (int q = 0; q < 8; q++)
-          tile_add(lo, hi, t0 + ((q >> 2) & 1) + TILE * (((q >> 1) & 1) + TILE * (q & 1)), weight(q));
-      }
-      if (on && !tiled) {  // drifted out of the brick since the sort, or no common unit
-        const int xs[2] = {x, x + 1 < g.n[0] ? x + 1 : 0};
-        const int ys[2] = {y, y + 1 < g.n[1] ? y + 1 : 0};
-        const int zs[2] = {z, z + 1 < g.n[2] ? z + 1 : 0};
-#pragma unroll
         for (int q = 0; q < 8; q++) {
           const int cx = (q >> 2) & 1, cy = (q >> 1) & 1, cz = q & 1;
-          const int64_t site = site_index(g, xs[cx], ys[cy], zs[cz]);
-          if (FIXED) {
-            atomicAdd(&acc[site], (unsigned long long)weight(q));
-          } else {
-            const float w = (cx ? f[0] : 1.0f - f[0]) * (cy ? f[1] : 1.0f - f[1]) * (cz ? f[2] : 1.0f - f[2]);
-            atomicAdd(&rho[site], w * m);
-          }
+          const float w = (cx ? f[0] : 1.0f - f[0]) * (cy ? f[1] : 1.0f - f[1]) * (cz ? f[2] : 1.0f - f[2]);
+          const float rest = comp_rest(w * m, cu.unit, cu.quantum);
+          if (rest != 0.0f)
+            atomicAdd(&rho[tile_site(g, t0 + cx + TILE * (cy + TILE * cz), x0, y0, z0)], rest);
         }
       }
     }
-    __syncthreads();
-    for (int t = threadIdx.x; t < TILE3; t += blockDim.x) {
-      const unsigned long long v = ((unsigned long long)hi[t] << 32) | lo[t];
-      if (!v) continue;
-      if (FIXED)
-        atomicAdd(&acc[tile_site(g, t, x0, y0, z0)], v);
-      else
-        atomicAdd(&rho[tile_site(g, t, x0, y0, z0)], __ll2float_rn((long long)v) * cu.quantum);
+    // runs of lanes in one cell
+    const int key = tiled ? t0 : -1 - lane;
+    const int before = __shfl_up_sync(0xffffffffu, key, 1);
+    const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || key != before);
+    if (__popc(heads) <= DENSE_RUNS) {
+      for (unsigned rest = heads; rest; rest &= rest - 1) {
+        const int first = __ffs(rest) - 1, next = __ffs(rest & (rest - 1));
+        const bool mine = lane >= first && (next == 0 || lane < next - 1);
+        const int t = __shfl_sync(0xffffffffu, key, first);
+        if (t < 0) continue;  // a lane that is not in the tile: below
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+          const long long w = mine ? weight(q) : 0ll;
+          // 32 values below 2^52: the sums of 20-bit pieces stay below 2^31
+          const long long sum =
+              (long long)__reduce_add_sync(0xffffffffu, (unsigned)(w & 0xfffff)) +
+              ((long long)__reduce_add_sync(0xffffffffu, (unsigned)((w >> 20) & 0xfffff)) << 20) +
+              ((long long)__reduce_add_sync(0xffffffffu, (int)(w >> 40)) << 40);
+          if (lane == q)
+            tile_add(lo, hi, t + ((q >> 2) & 1) + TILE * (((q >> 1) & 1) + TILE * (q & 1)), sum);
+        }
+      }
+    } else if (tiled) {
+#pragma unroll
+      for (int q = 0; q < 8; q++)
+        tile_add(lo, hi, t0 + ((q >> 2) & 1) + TILE * (((q >> 1) & 1) + TILE * (q & 1)), weight(q));
     }
+    if (on && !tiled) {  // drifted out of the brick since the sort, or no common unit
+      const int xs[2] = {x, x + 1 < g.n[0] ? x + 1 : 0};
+      const int ys[2] = {y, y + 1 < g.n[1] ? y + 1 : 0};
+      const int zs[2] = {z, z + 1 < g.n[2] ? z + 1 : 0};
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const int cx = (q >> 2) & 1, cy = (q >> 1) & 1, cz = q & 1;
+        const int64_t site = site_index(g, xs[cx], ys[cy], zs[cz]);
+        if (FIXED) {
+          atomicAdd(&acc[site], (unsigned long long)weight(q));
+        } else {
+          const float w = (cx ? f[0] : 1.0f - f[0]) * (cy ? f[1] : 1.0f - f[1]) * (cz ? f[2] : 1.0f - f[2]);
+          atomicAdd(&rho[site], w * m);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < TILE3; t += blockDim.x) {
+    const unsigned long long v = ((unsigned long long)hi[t] << 32) | lo[t];
+    if (!v) continue;
+    if (FIXED)
+      atomicAdd(&acc[tile_site(g, t, x0, y0, z0)], v);
+    else
+      atomicAdd(&rho[tile_site(g, t, x0, y0, z0)], __ll2float_rn((long long)v) * cu.quantum);
   }
 }
 
