@@ -470,10 +470,12 @@ inline int grid_for(int64_t n, int threads)
 
 // Brick counters of a load in a CTA's shared memory: bytes, or 0 where they
 // do not fit (above 51,200 bricks, lattices beyond 590^3).
+constexpr size_t LOAD_COUNTERS_MAX = 200 * 1024;
+
 static size_t load_counters(const lf2_ctx* c)
 {
   const size_t bytes = sizeof(int32_t) * (size_t)c->g.nbricks;
-  return bytes <= 200 * 1024 ? bytes : 0;
+  return bytes <= LOAD_COUNTERS_MAX ? bytes : 0;
 }
 
 // CTAs of a load: those that run at once, fewer when they would hold under 4096
@@ -489,8 +491,10 @@ cudaError_t launch_load_count(lf2_ctx* c, int64_t n, const int32_t* cell, const 
 {
   c->launches += 1;
   if (const size_t sh = load_counters(c)) {
+    // (the setting is the kernel's, not the call's: one value for all, since
+    // contexts of other sizes may load from other threads)
     const cudaError_t e = cudaFuncSetAttribute(k_load_count_sh, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)sh);
+                                               (int)LOAD_COUNTERS_MAX);
     if (e != cudaSuccess) return e;
     k_load_count_sh<<<load_ctas(c, n), LOAD_THREADS, sh, c->stream>>>(c->g, n, cell, off3, c->count, c->flags);
     return cudaGetLastError();
