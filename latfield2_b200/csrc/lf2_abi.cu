@@ -160,8 +160,12 @@ lf2_status ensure_spill(lf2_ctx* c, size_t need)
     c->spill = nullptr;
     c->spill_slots = 0;
   }
-  if (cudaMalloc(&c->spill, need * sizeof(uint64_t)) != cudaSuccess)
+  cudaError_t e = cudaMalloc(&c->spill, need * sizeof(uint64_t));
+  if (e != cudaSuccess && release_rows(c)) e = cudaMalloc(&c->spill, need * sizeof(uint64_t));
+  if (e != cudaSuccess) {
+    c->spill = nullptr;
     return fail(c, LF2_ERR_NOMEM, "cannot allocate the deposit shell store");
+  }
   c->spill_slots = need;
   return LF2_OK;
 }
@@ -198,6 +202,7 @@ lf2_status load_device(lf2_ctx* c, int64_t n, const int32_t* cell, const float* 
   if (need > c->capacity || has_mass != c->has_mass || has_id != c->has_id ||
       mov_need > c->mov_capacity) {
     LF2_CUDA(c, cudaStreamSynchronize(c->stream));
+    release_rows(c);  // the store comes first
     free_parts(c->cur);
     free_parts(c->alt);
     free_parts(c->mov);
@@ -240,6 +245,7 @@ lf2_status load_device(lf2_ctx* c, int64_t n, const int32_t* cell, const float* 
     LF2_CUDA(c, cudaStreamSynchronize(c->stream));
     c->m_unit = (n > 0 && c->h_stats[1] > 0) ? c->h_stats[1] / (double)n : 1.0;
   }
+  prepare_rows(c);
   return LF2_OK;
 }
 
@@ -571,6 +577,7 @@ lf2_status lf2_slab_insert(lf2_ctx* c, int64_t n_a, const uint32_t* a, int64_t n
     LF2_TRY(rebin_tail(c));
     LF2_CUDA(c, cudaMemsetAsync(c->mov_count, 0, sizeof(unsigned long long), c->stream));
     c->np = total;
+    prepare_rows(c);
     return LF2_OK;
   }
   // the store is too small: separate arrays, then the reloading add (it waits)
@@ -620,6 +627,7 @@ lf2_status lf2_particles_add(lf2_ctx* c, int64_t n, const int32_t* cell, const f
     LF2_TRY(rebin_tail(c));
     LF2_CUDA(c, cudaMemsetAsync(c->mov_count, 0, sizeof(unsigned long long), c->stream));
     c->np = total;
+    prepare_rows(c);
     return LF2_OK;
   }
   // the store is too small: reload the current particles and the new ones
@@ -857,6 +865,10 @@ lf2_status lf2_field_wrap(lf2_ctx* c, int comps, float* device_data, lf2_field* 
   f->data = device_data;
   f->owned = false;
   *out = f;
+  if (comps == 3 && (reinterpret_cast<uintptr_t>(device_data) & 15)) {
+    c->odd_field = true;
+    prepare_rows(c);
+  }
   return LF2_OK;
 }
 
@@ -1092,6 +1104,8 @@ lf2_status lf2_set_move_kernel(lf2_ctx* c, int which)
 {
   if (!c || which < 0 || which > 3) return LF2_ERR_ARG;
   c->move_kernel = which;
+  if (which == 1) release_rows(c);
+  else prepare_rows(c);
   return LF2_OK;
 }
 

@@ -116,7 +116,8 @@ struct lf2_ctx {
   lf2::PassHead* head = nullptr;     // device: counters of the pass
   int32_t* move_list = nullptr;      // [nbricks] bricks taken first
   uint8_t* move_mark = nullptr;      // [nbricks] 1 for those
-  float* f_rows = nullptr;           // F with rows on 16-byte boundaries (other row lengths)
+  float* f_rows = nullptr;           // F with rows on 16-byte boundaries (prepare_rows)
+  bool odd_field = false;            // a 3-component field off the 16-byte boundary was wrapped
   int64_t wait_cycles = 0;           // limit of its bounded waits (0: about 2 s)
   int wait_stall = 0;                // consumers first wait on a barrier nothing completes
   const float* tmap_src = nullptr;   // field the cached tensor map describes
@@ -180,7 +181,9 @@ cudaError_t launch_maxv_to_device(lf2_ctx* c, double* dst);
 // fixed-point scalar deposit fused in; its rim store is c->spill,
 // rim_store_slots(c) slots).  A kick needs move_pipe_eligible.
 bool move_pipe_eligible(const lf2_ctx* c, const float* F);
-bool move_pipe_auto(lf2_ctx* c, const float* F);
+bool move_pipe_auto(const lf2_ctx* c, const float* F);
+void prepare_rows(lf2_ctx* c);
+bool release_rows(lf2_ctx* c);
 bool move_dep_eligible(const lf2_ctx* c, const float* F);
 size_t rim_store_slots(const lf2_ctx* c);
 cudaError_t launch_move_pipe(lf2_ctx* c, const float* F, bool kick, bool drift, MoveParams mp,

@@ -1039,31 +1039,51 @@ bool move_pipe_eligible(const lf2_ctx* c, const float* F)
   return encode_fn() != nullptr;
 }
 
-// Whether a kick with F takes the pipelined kernel when the choice is
-// automatic: where it is eligible, and on lattices with other row lengths (or
-// an F off the 16-byte boundary) from a copy of F with aligned rows, kept in
-// the context.  The copy moves 24 bytes per site and the pipelined kernel
-// saves the per-brick one's time per particle, so sparse stores (fewer than a
-// third of a particle per site) and contexts without room for the copy keep
-// the per-brick kernel.
-bool move_pipe_auto(lf2_ctx* c, const float* F)
+// On lattices with other row lengths (or with an F off the 16-byte boundary) the
+// pipelined kick works from a copy of F with aligned rows.  The copy moves 24
+// bytes per site and the pipelined kernel saves the per-brick one's time per
+// particle, so sparse stores (fewer than a third of a particle per site) and
+// contexts without the copy's memory keep the per-brick kernel.
+static bool rows_pay(const lf2_ctx* c) { return 3 * c->np >= c->g.nsites; }
+
+// That memory is taken where a program expects an allocation: when particles
+// are loaded or such a field is wrapped (the first kick of a new context is then
+// as fast as the others, and none allocates), and given back with the per-brick
+// kernel's choice, or where another allocation of the context needs it.
+void prepare_rows(lf2_ctx* c)
+{
+  if (c->f_rows || c->move_kernel == 1 || !((c->g.n[0] & 3) || c->odd_field) || !rows_pay(c)) return;
+  for (int d = 0; d < 3; d++)
+    if (c->g.n[d] < 2 * BRICK) return;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (!encode_fn() || cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess ||
+      cap != cudaStreamCaptureStatusNone)
+    return;
+  const size_t floats = (size_t)3 * padded_row(c) * c->g.n[1] * c->g.n[2];
+  if (cudaMalloc(&c->f_rows, floats * sizeof(float)) != cudaSuccess) {
+    cudaGetLastError();
+    c->f_rows = nullptr;
+  }
+}
+
+// (nothing is freed under capture)
+bool release_rows(lf2_ctx* c)
+{
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (!c->f_rows || cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess ||
+      cap != cudaStreamCaptureStatusNone || cudaStreamSynchronize(c->stream) != cudaSuccess)
+    return false;
+  if (c->tmap_src == c->f_rows) c->tmap_src = nullptr;
+  cudaFree(c->f_rows);
+  c->f_rows = nullptr;
+  return true;
+}
+
+// Whether a kick with F takes the pipelined kernel when the choice is automatic.
+bool move_pipe_auto(const lf2_ctx* c, const float* F)
 {
   if (!F || rows_aligned(c, F)) return move_pipe_eligible(c, F);
-  for (int d = 0; d < 3; d++)
-    if (c->g.n[d] < 2 * BRICK) return false;
-  if (!encode_fn() || 3 * c->np < c->g.nsites) return false;
-  if (!c->f_rows) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
-      return false;  // no allocation under capture
-    const size_t floats = (size_t)3 * padded_row(c) * c->g.n[1] * c->g.n[2];
-    if (cudaMalloc(&c->f_rows, floats * sizeof(float)) != cudaSuccess) {
-      cudaGetLastError();
-      c->f_rows = nullptr;
-      return false;
-    }
-  }
-  return true;
+  return c->f_rows && rows_pay(c);
 }
 
 cudaError_t launch_move_pipe(lf2_ctx* c, const float* F, bool kick, bool drift, MoveParams mp,

@@ -93,9 +93,9 @@ def test_field_off_the_16_byte_boundary_and_sparse_stores(cuda):
 
 @pytest.mark.parametrize("warm", [False, True])
 def test_kick_drift_and_deposit_under_capture(cuda, warm):
-    """Captured calls allocate nothing: the first kick of a context on padded
-    rows keeps the per-brick kernel, a later one takes the pipelined one.  The
-    replayed graph moves the particles as the same calls outside one."""
+    """Captured calls allocate nothing (the padded rows come with the load),
+    whether the context has kicked before or not.  The replayed graph moves the
+    particles as the same calls outside one."""
     import torch
     import latfield2_b200 as L
     n, npart = (50, 32, 48), 60000
@@ -130,3 +130,39 @@ def test_kick_drift_and_deposit_under_capture(cuda, warm):
     _same(a, b, False)
     np.testing.assert_array_equal(rho_a.export_internal(), rho_b.export_internal())
     assert a.flags() & ~0x8 == 0 and b.flags() & ~0x8 == 0
+
+
+def test_the_first_kick_allocates_nothing(cuda):
+    """The padded rows (36 MB here) come with the load and go with the choice of
+    the per-brick kernel; the first step takes the pipelined kernel."""
+    import torch
+    import latfield2_b200 as L
+    n, npart = (150, 141, 142), 1100000
+    cell, off, vel = small_case(n, npart, seed=23, vel_sigma=0.05)
+    F = torch.zeros(3, n[2], n[1], n[0], device="cuda")
+    sites = F.numel() // 3
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    def fresh():
+        ctx = L.Context(n, box=tuple(v / n[0] for v in n), mode=1)
+        ctx.set_particles(cell, off, vel, global_mass=1.0 / npart)
+        return ctx, ctx.field(3, F)
+    warm, f = fresh()  # (kernels are loaded with their first launch)
+    warm.gather_kick(f, 0.1)
+    warm.step(f, 0.1, 0.1)
+    warm.set_move_kernel(1)
+    ctx, f = fresh()
+    before = free()
+    ctx.gather_kick(f, 0.1)
+    ctx.step(f, 0.1, 0.1)
+    assert ctx.last_move_kernel() == 2
+    assert abs(before - free()) < 6 * sites
+    ctx.set_move_kernel(1)
+    assert free() - before > 6 * sites
+    ctx.step(f, 0.1, 0.1)
+    assert ctx.last_move_kernel() == 1
+    ctx.close()
+    warm.close()
