@@ -476,7 +476,8 @@ lf2_status lf2_pm_kick_drift(lf2_ctx* ctx, int64_t np, int32_t* cell,
 lf2_status lf2_pm_step(lf2_ctx* ctx, int64_t np, int32_t* cell, float* off3,
                        float* vel3, const float* F4, double dt_kick,
                        double dt_drift);
-/* the same into other arrays; the state before the step stays. */
+/* the same into other arrays; the state before the step stays.  An output may
+ * also be the input it follows from. */
 lf2_status lf2_pm_step_to(lf2_ctx* ctx, int64_t np, const int32_t* cell,
                           const float* off3, const float* vel3,
                           const float* F4, double dt_kick, double dt_drift,

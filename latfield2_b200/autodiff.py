@@ -5,14 +5,17 @@ rebinning; the gradients come back in the caller's order):
     rho_k   = deposit(x_k, m)                    lf2_pm_deposit      (CIC, projections.hpp:75-184)
     F_k     = stencil27(rho_k, S)                lf2_stencil27       (the grid operator), or
     F_k     = pm_force(rho_k)                    lf2_pm_force4       (the FFT Poisson force)
-    G_k     = gather(x_k, F_k)                   lf2_pm_gather       (CIC gather of updateVel)
-    v_{k+1} = v_k + dt G_k ;  x_{k+1} = x_k + dt v_{k+1}             lf2_pm_kick_drift
-(the last two in one pass, lf2_pm_step)
-and finally rho_K = deposit(x_K, m), loss = sum_g w_g rho_K(g).
+    G_k     = gather(x_k, F_k)                   (CIC gather of updateVel)
+    v_{k+1} = v_k + dt G_k ;  x_{k+1} = x_k + dt v_{k+1}
+                                                 lf2_pm_step (the last two lines in one
+                                                 pass, in place) or, from a state that is
+                                                 kept, lf2_pm_step_to
+and finally rho_K = deposit(x_K, m), loss = sum_g w_g rho_K(g) (lf2_pm_loss).
 
 `PMChain` is a torch.autograd.Function whose backward runs the hand-written
-adjoint kernels (lf2_pm_*_adjoint, lf2_stencil27_adjoint,
-lf2_pm_force4_adjoint) in reverse.
+adjoint kernels (lf2_pm_loss_adjoint, then per step lf2_pm_step_adjoint,
+lf2_stencil27_adjoint or lf2_pm_force4_adjoint, lf2_pm_deposit_adjoint) in
+reverse.
 Particle states are checkpointed every `checkpoint_every` steps and the
 states in between are recomputed during the backward pass; the grid fields
 rho_k and F_k of every step are kept (4 floats per lattice site per step).
@@ -183,10 +186,10 @@ class _Ops:
         _check(self.ctx, self.lib.lf2_pm_step(self.ctx.h, cell.numel(), _p(cell), _p(off), _p(vel),
                                               _p(F), dt, dt), "pm_step")
 
-    def next_state(self, cell, off, vel, F, dt):
+    def next_state(self, cell, off, vel, F, dt, keep_vel=True):
         """the same (lf2_pm_step_to): the state after the step, in new
-        tensors."""
-        out = torch.empty_like(cell), torch.empty_like(off), torch.empty_like(vel)
+        tensors (the velocities in place without keep_vel)."""
+        out = torch.empty_like(cell), torch.empty_like(off), torch.empty_like(vel) if keep_vel else vel
         _check(self.ctx, self.lib.lf2_pm_step_to(self.ctx.h, cell.numel(), _p(cell), _p(off), _p(vel),
                                                  _p(F), dt, dt, *(_p(t) for t in out)), "pm_step_to")
         return out
@@ -226,7 +229,10 @@ class PMChain(torch.autograd.Function):
             rho, F = ops.fields(cell, off, m, S32, coupling)
             rhos.append(rho)
             Fs.append(F)
-            cell, off, vel = ops.next_state(cell, off, vel, F, dt)
+            if k in ckpts:
+                cell, off, vel = ops.next_state(cell, off, vel, F, dt)
+            else:
+                ops.step(cell, off, vel, F, dt)
         rhoK = torch.zeros(lf2ctx.nsites, dtype=torch.float32, device=cell.device)
         ops.deposit(cell, off, m, rhoK)
         loss = ops.loss(w32, rhoK)
@@ -261,7 +267,7 @@ class PMChain(torch.autograd.Function):
                 for j in range(k0, k + 1):
                     seg[j] = (c, o)
                     if j < k:
-                        c, o, v = ops.next_state(c, o, v, Fs[j], dt)
+                        c, o, v = ops.next_state(c, o, v, Fs[j], dt, keep_vel=False)
             cell_k, off_k = seg[k]
             # drift x_{k+1} = x_k + dt v_{k+1} (cell units: off += dt/res v),
             # kick v_{k+1} = v_k + dt G_k, gather G_k = sum W F

@@ -152,3 +152,39 @@ def test_records_off_the_32_byte_boundary(cuda):
                                              float(n), _p(off16), *[_p(x) for x in out]), "grads")
     for x, y in zip(out, ref):
         assert torch.equal(x, y)
+
+
+def test_chain_keeps_no_state_beside_its_checkpoints(cuda):
+    """Forward and backward with a checkpoint every 4 steps: between two of them
+    only the running state lives (28 bytes per particle), as its loss, the same
+    in fixed point whatever the interval, is reached in place."""
+    import torch
+    import latfield2_b200 as L
+    from latfield2_b200.autodiff import pm_chain_loss
+    n, npart = 32, 400000
+    g = torch.Generator(device="cpu").manual_seed(7)
+    ctx = L.Context((n, n, n), box=1.0, mode=L.DEPOSIT_FIXED64)
+    pos = torch.rand(npart, 3, generator=g, dtype=torch.float64).cuda()
+    vel = (0.02 * torch.randn(npart, 3, generator=g, dtype=torch.float64)).cuda()
+    m = torch.full((npart,), 1.0 / npart, dtype=torch.float64, device="cuda")
+    S = (0.02 * torch.randn(81, generator=g, dtype=torch.float64)).cuda()
+    w = torch.randn(n ** 3, generator=g, dtype=torch.float64).cuda()
+
+    def run(every):
+        leaves = [t.clone().requires_grad_(True) for t in (pos, vel, m, S, w)]
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        base = torch.cuda.memory_allocated()
+        loss = pm_chain_loss(ctx, *leaves, steps=8, dt=0.02, checkpoint_every=every)
+        peak = torch.cuda.max_memory_allocated() - base
+        return loss, torch.autograd.grad(loss, leaves), peak
+    run(4)
+    loss, grads, peak = run(4)
+    fields = 8 * 5 * 4 * n ** 3 + 3 * 4 * n ** 3
+    # order and masses, two checkpoints and the running state, with half a state to spare
+    assert peak <= (8 + 4 + 3.5 * 28) * npart + fields, peak / npart
+    loss1, grads1, _ = run(1)
+    assert torch.equal(loss.detach(), loss1.detach())
+    for a, b in zip(grads, grads1):
+        assert _rel(a, b) < 1e-5  # (FP32 atomics of the adjoints in two orders)
+    ctx.close()
