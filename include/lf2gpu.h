@@ -290,12 +290,14 @@ lf2_status lf2_step(lf2_ctx* ctx, lf2_field F, double dtau_kick,
  * n >= 32 and F 16-byte aligned; the fused deposit the fixed-point mode,
  * else LF2_ERR_UNSUPPORTED).  All give the same particles (the order of the
  * particles inside a brick may differ) and the same fixed-point density; no
- * reference counterpart.  The automatic choice also takes the pipelined kernel
- * for lf2_gather_kick, and on other row lengths or an unaligned F from a copy
- * of F with padded rows (12 bytes per site, rows rounded up to four sites),
- * which stores of a third of a particle per site or more get when particles
- * are loaded or added or such a field is wrapped; no kick allocates it, and
- * kernel 1 gives it back. */
+ * reference counterpart.  The choice also covers lf2_gather_kick and
+ * lf2_drift_rebin (automatic: where the store's size and clumping make the
+ * pipelined kernel the faster one).  On other row lengths or with an unaligned
+ * F the pipelined kernel works from a copy of F with padded rows (12 bytes per
+ * site, rows rounded up to four sites), which stores dense enough to gain from
+ * it (a third of a particle per site in clumps, three quarters otherwise) get
+ * when particles are loaded or added or such a field is wrapped; no kick
+ * allocates it, and kernel 1 gives it back. */
 lf2_status lf2_set_move_kernel(lf2_ctx* ctx, int which);
 /* Bounded waits of the pipelined kernel (no reference counterpart): every
  * wait on a copy or on another warp gives up after `cycles` SM clock cycles

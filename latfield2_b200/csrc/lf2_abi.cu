@@ -231,9 +231,13 @@ lf2_status load_device(lf2_ctx* c, int64_t n, const int32_t* cell, const float* 
   LF2_CUDA(c, cudaMemcpyAsync(c->count, c->fill, sizeof(int32_t) * nb, cudaMemcpyDeviceToDevice,
                               c->stream));
   LF2_CUDA(c, launch_heap_reset(c));
+  LF2_CUDA(c, cudaMemcpyAsync(c->h_stats, c->stats, sizeof(double) * 2, cudaMemcpyDeviceToHost,
+                              c->stream));  // the largest brick's count (check_flags waits)
   c->np = n;
-  if (check_flags(c) != LF2_OK) {
-    c->np = 0;
+  const lf2_status loaded = check_flags(c);
+  c->most = (int64_t)c->h_stats[1];
+  if (loaded != LF2_OK) {
+    c->np = c->most = 0;
     LF2_CUDA(c, cudaMemsetAsync(c->count, 0, sizeof(int32_t) * nb, c->stream));
     return fail(c, LF2_ERR_ARG, "particles_set: a cell index or offset is out of range");
   }
@@ -1002,18 +1006,17 @@ lf2_status lf2_gather_kick(lf2_ctx* c, lf2_field F, double dtau, double* max_v)
   MoveParams mp{(float)dtau, 0.0f};
   {
     PhaseScope ps(c, PH_MOVE);
-    // the pipelined kernel where it takes the field (lf2_set_move_kernel(1)
-    // keeps the per-brick one)
-    LF2_CUDA(c, c->move_kernel != 1 && move_pipe_auto(c, F->data)
+    LF2_CUDA(c, kick_pipe_auto(c, F->data)
                     ? launch_move_pipe(c, F->data, true, false, mp, nullptr)
                     : launch_move(c, F->data, true, false, mp));
   }
   if (max_v) {
     LF2_CUDA(c, launch_reduce_maxv(c));
-    LF2_CUDA(c, cudaMemcpyAsync(c->h_stats, c->stats, sizeof(double), cudaMemcpyDeviceToHost,
+    LF2_CUDA(c, cudaMemcpyAsync(c->h_stats, c->stats, sizeof(double) * 2, cudaMemcpyDeviceToHost,
                                 c->stream));
     LF2_CUDA(c, cudaStreamSynchronize(c->stream));
     *max_v = std::sqrt(c->h_stats[0]);
+    c->most = (int64_t)c->h_stats[1];
   }
   return LF2_OK;
 }
@@ -1022,12 +1025,13 @@ lf2_status lf2_drift_rebin(lf2_ctx* c, double dtau)
 {
   if (!c) return LF2_ERR_ARG;
   MoveParams mp{0.0f, (float)(dtau / c->res)};
-  if (c->move_kernel == 1)  // the pipelined pass clears the counters itself
+  const bool pipe = drift_pipe_auto(c);
+  if (!pipe)  // the pipelined pass clears the counters itself
     LF2_CUDA(c, cudaMemsetAsync(c->head, 0, sizeof(PassHead), c->stream));
   {
     PhaseScope ps(c, PH_MOVE);
-    LF2_CUDA(c, c->move_kernel != 1 ? launch_move_pipe(c, nullptr, false, true, mp, nullptr)
-                                    : launch_move(c, nullptr, false, true, mp));
+    LF2_CUDA(c, pipe ? launch_move_pipe(c, nullptr, false, true, mp, nullptr)
+                     : launch_move(c, nullptr, false, true, mp));
   }
   return rebin_tail(c);
 }
@@ -1117,9 +1121,10 @@ lf2_status lf2_last_max_velocity(lf2_ctx* c, double* max_v, int ptr_kind)
     return LF2_OK;
   }
   LF2_CUDA(c, launch_reduce_maxv(c));
-  LF2_CUDA(c, cudaMemcpyAsync(c->h_stats, c->stats, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  LF2_CUDA(c, cudaMemcpyAsync(c->h_stats, c->stats, sizeof(double) * 2, cudaMemcpyDeviceToHost, c->stream));
   LF2_CUDA(c, cudaStreamSynchronize(c->stream));
   *max_v = std::sqrt(c->h_stats[0]);
+  c->most = (int64_t)c->h_stats[1];
   return LF2_OK;
 }
 

@@ -69,6 +69,7 @@ struct lf2_ctx {
 
   // particle store
   int64_t np = 0;
+  int64_t most = 0;     // count of the largest brick, as last read by the host (kernel choice)
   bool has_mass = false;
   bool has_id = false;
   double gmass = 0.0;   // global particle mass (GLOBAL_MASS types)
@@ -182,6 +183,8 @@ cudaError_t launch_maxv_to_device(lf2_ctx* c, double* dst);
 // rim_store_slots(c) slots).  A kick needs move_pipe_eligible.
 bool move_pipe_eligible(const lf2_ctx* c, const float* F);
 bool move_pipe_auto(const lf2_ctx* c, const float* F);
+bool kick_pipe_auto(const lf2_ctx* c, const float* F);
+bool drift_pipe_auto(const lf2_ctx* c);
 void prepare_rows(lf2_ctx* c);
 bool release_rows(lf2_ctx* c);
 bool move_dep_eligible(const lf2_ctx* c, const float* F);

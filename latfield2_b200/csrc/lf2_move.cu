@@ -375,20 +375,29 @@ __global__ void k_insert(StoreView v, PartArrays mov, const unsigned long long* 
   }
 }
 
-// max over bricks of max |v|^2 -> stats[0] (one CTA, fixed order).
+// max over bricks of max |v|^2 -> stats[0], and of the counts -> stats[1] (one
+// CTA, fixed order).
 __global__ void __launch_bounds__(1024) k_reduce_maxv(int64_t nb, const float* __restrict__ bm,
-                                                      double* stats)
+                                                      const int32_t* __restrict__ count, double* stats)
 {
   __shared__ float sh[1024];
+  __shared__ int s_most;
+  if (threadIdx.x == 0) s_most = 0;
   float m = 0.0f;
-  for (int64_t b = threadIdx.x; b < nb; b += blockDim.x) m = fmaxf(m, bm[b]);
+  int most = 0;
+  for (int64_t b = threadIdx.x; b < nb; b += blockDim.x) {
+    m = fmaxf(m, bm[b]);
+    most = max(most, count[b]);
+  }
+  most = __reduce_max_sync(0xffffffffu, most);
   sh[threadIdx.x] = m;
   __syncthreads();
+  if ((threadIdx.x & 31) == 0) atomicMax(&s_most, most);
   for (int o = blockDim.x / 2; o > 0; o >>= 1) {
     if ((int)threadIdx.x < o) sh[threadIdx.x] = fmaxf(sh[threadIdx.x], sh[threadIdx.x + o]);
     __syncthreads();
   }
-  if (threadIdx.x == 0) stats[0] = (double)sh[0];
+  if (threadIdx.x == 0) stats[0] = (double)sh[0], stats[1] = (double)s_most;
 }
 
 }  // namespace
@@ -429,7 +438,7 @@ cudaError_t launch_insert(lf2_ctx* c)
 cudaError_t launch_reduce_maxv(lf2_ctx* c)
 {
   c->launches += 1;
-  k_reduce_maxv<<<1, 1024, 0, c->stream>>>(c->g.nbricks, c->brick_maxv2, c->stats);
+  k_reduce_maxv<<<1, 1024, 0, c->stream>>>(c->g.nbricks, c->brick_maxv2, c->count, c->stats);
   return cudaGetLastError();
 }
 

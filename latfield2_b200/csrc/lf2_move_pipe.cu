@@ -1039,12 +1039,28 @@ bool move_pipe_eligible(const lf2_ctx* c, const float* F)
   return encode_fn() != nullptr;
 }
 
+// The automatic choice of the kernel.  The pipelined one has about 3 us to a
+// brick on each SM whatever it holds; the per-brick one's time goes with the
+// particles, and a brick far above the others keeps its last CTA busy long
+// after the rest (the pipelined one takes it first).  Clumped: the largest
+// brick's count, as last read by the host (a load, a maximum velocity), is
+// above a quarter of an SM's share and three times what the mean density puts
+// into a whole brick.
+static bool clumped(const lf2_ctx* c)
+{
+  const double whole = (double)c->np / (double)c->g.nsites * BRICK * BRICK * BRICK;
+  return (double)c->most > std::max((double)c->np / (4.0 * c->num_sms), 3.0 * whole);
+}
+
 // On lattices with other row lengths (or with an F off the 16-byte boundary) the
-// pipelined kick works from a copy of F with aligned rows.  The copy moves 24
-// bytes per site and the pipelined kernel saves the per-brick one's time per
-// particle, so sparse stores (fewer than a third of a particle per site) and
-// contexts without the copy's memory keep the per-brick kernel.
-static bool rows_pay(const lf2_ctx* c) { return 3 * c->np >= c->g.nsites; }
+// pipelined kick works from a copy of F with aligned rows, 24 bytes of traffic
+// per site.  Steps per-brick / pipelined in us, 150 x 141 x 133 and 314^3: even,
+// 0.34 particles per site 58 / 83 and 504 / 496, 1.0 118 / 112 and 926 / 778;
+// clumps, 0.34 121 / 98 and 797 / 545, 1.0 262 / 160 and 1746 / 881.
+static bool rows_pay(const lf2_ctx* c)
+{
+  return clumped(c) ? 3 * c->np >= c->g.nsites : 4 * c->np >= 3 * c->g.nsites;
+}
 
 // That memory is taken where a program expects an allocation: when particles
 // are loaded or such a field is wrapped (the first kick of a new context is then
@@ -1079,11 +1095,40 @@ bool release_rows(lf2_ctx* c)
   return true;
 }
 
-// Whether a kick with F takes the pipelined kernel when the choice is automatic.
+// Whether a step with F takes the pipelined kernel when the choice is automatic.
 bool move_pipe_auto(const lf2_ctx* c, const float* F)
 {
   if (!F || rows_aligned(c, F)) return move_pipe_eligible(c, F);
   return c->f_rows && rows_pay(c);
+}
+
+// A kick alone leaves the pipelined kernel less to hide.  Aligned rows, even and
+// about one particle per site: 64^3 19 / 27 us, 128^3 44 / 59, 176^3 107 / 111,
+// 192^3 137 / 136, 256^3 296 / 270, 512^3 2214 / 1871; clumps 128^3 102 / 94,
+// 144^3 125 / 115, 160^3 203 / 163 (0.25 per site 58 / 63), 256^3 531 / 310; few
+// particles at 256^3: 0.1 per brick 24 / 40, 1 97 / 99, 4 140 / 117.  From padded
+// rows even stores never gain (210^3 181 / 219), clumps from 162^3 on (200 / 176;
+// 0.34 per site 76 / 99).
+bool kick_pipe_auto(const lf2_ctx* c, const float* F)
+{
+  if (c->move_kernel == 1) return false;
+  if (!rows_aligned(c, F))
+    return move_pipe_auto(c, F) && (c->move_kernel || (clumped(c) && 2 * c->np >= c->g.nsites &&
+                                                       c->g.nbricks >= 6 * c->num_sms));
+  const int per_sm = clumped(c) && 3 * c->np >= c->g.nsites ? 4 : 10;
+  return move_pipe_eligible(c, F) &&
+         (c->move_kernel || (c->np >= 4 * c->g.nbricks && c->g.nbricks >= per_sm * c->num_sms));
+}
+
+// A drift needs no field and takes any lattice.  Even, per-brick / pipelined with
+// the rebin: 256^3 at 0.25 particles per site 104 / 125 us, 0.5 197 / 152, 1
+// 364 / 223; 314^3 at 0.34 229 / 235; 512^3 at 0.004 213 / 632; clumps 256^3 at
+// 0.06 85 / 118, 0.125 169 / 124, 1 811 / 261, 512^3 at 0.125 712 / 896, 0.25
+// 1259 / 1051.
+bool drift_pipe_auto(const lf2_ctx* c)
+{
+  if (c->move_kernel) return c->move_kernel != 1;
+  return clumped(c) ? 5 * c->np >= c->g.nsites : 5 * c->np >= 2 * c->g.nsites;
 }
 
 cudaError_t launch_move_pipe(lf2_ctx* c, const float* F, bool kick, bool drift, MoveParams mp,

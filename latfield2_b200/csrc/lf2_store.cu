@@ -96,20 +96,26 @@ __global__ void __launch_bounds__(LOAD_THREADS) k_load_count_sh(Geom g, int64_t 
 // One CTA: cap[b] = count[b] + slack (when caps != nullptr), starts = exclusive
 // scan of caps (or of counts), starts[nb] = total.
 __global__ void __launch_bounds__(1024) k_caps_scan(int64_t nb, const int32_t* __restrict__ counts,
-                                                    int32_t* caps, int64_t* starts)
+                                                    int32_t* caps, int64_t* starts, double* most)
 {
   __shared__ int64_t sh[1024];
+  __shared__ int s_most;
   const int t = threadIdx.x;
   const int64_t per = (nb + blockDim.x - 1) / blockDim.x;
   const int64_t lo = t * per, hi = min(nb, lo + per);
   int64_t s = 0;
+  int m = 0;
   for (int64_t b = lo; b < hi; b++) {
-    const int32_t v = caps ? cap_of(counts[b]) : counts[b];
+    const int32_t c = counts[b], v = caps ? cap_of(c) : c;
     if (caps) caps[b] = v;
     s += v;
+    m = max(m, c);
   }
+  if (t == 0) s_most = 0;
   sh[t] = s;
   __syncthreads();
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((t & 31) == 0) atomicMax(&s_most, m);
   for (int o = 1; o < (int)blockDim.x; o <<= 1) {
     const int64_t add = t >= o ? sh[t - o] : 0;
     __syncthreads();
@@ -122,6 +128,7 @@ __global__ void __launch_bounds__(1024) k_caps_scan(int64_t nb, const int32_t* _
     run += caps ? caps[b] : counts[b];
   }
   if (t == blockDim.x - 1) starts[nb] = sh[t];
+  if (t == 0 && most) *most = (double)s_most;
 }
 
 __global__ void k_load_scatter(Geom g, int64_t n, const int32_t* __restrict__ cell,
@@ -507,14 +514,14 @@ cudaError_t launch_caps_and_scan(lf2_ctx* c, const int32_t* counts, int32_t* cap
                                  int64_t*)
 {
   c->launches += 1;
-  k_caps_scan<<<1, 1024, 0, c->stream>>>(c->g.nbricks, counts, caps, starts);
+  k_caps_scan<<<1, 1024, 0, c->stream>>>(c->g.nbricks, counts, caps, starts, c->stats + 1);
   return cudaGetLastError();
 }
 
 cudaError_t launch_scan_counts(lf2_ctx* c, int64_t* out_start)
 {
   c->launches += 1;
-  k_caps_scan<<<1, 1024, 0, c->stream>>>(c->g.nbricks, c->count, nullptr, out_start);
+  k_caps_scan<<<1, 1024, 0, c->stream>>>(c->g.nbricks, c->count, nullptr, out_start, nullptr);
   return cudaGetLastError();
 }
 

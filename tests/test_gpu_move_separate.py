@@ -137,7 +137,7 @@ def test_the_first_kick_allocates_nothing(cuda):
     the per-brick kernel; the first step takes the pipelined kernel."""
     import torch
     import latfield2_b200 as L
-    n, npart = (150, 141, 142), 1100000
+    n, npart = (150, 141, 142), 2300000
     cell, off, vel = small_case(n, npart, seed=23, vel_sigma=0.05)
     F = torch.zeros(3, n[2], n[1], n[0], device="cuda")
     sites = F.numel() // 3
@@ -166,3 +166,25 @@ def test_the_first_kick_allocates_nothing(cuda):
     assert ctx.last_move_kernel() == 1
     ctx.close()
     warm.close()
+
+
+@pytest.mark.parametrize("n,npart,clustered,with_mass",
+                         CASES + [((64, 48, 32), 40, False, False), ((64, 48, 32), 90000, True, True)])
+def test_both_kernels_of_the_separate_calls(cuda, n, npart, clustered, with_mass):
+    """The kernel that the sizes do not choose here: pipelined (2) against
+    per-brick (1), kick and drift each."""
+    import torch
+    cell, off, vel = small_case(n, npart, seed=29, vel_sigma=0.05, clustered=clustered)
+    rng = np.random.default_rng(4)
+    mass = ((1 + 0.1 * rng.random(npart)) / npart).astype(np.float32) if with_mass else None
+    a, b = _pair(n, cell, off, vel, mass, np.arange(npart, dtype=np.int64))
+    a.set_move_kernel(2)
+    F = torch.from_numpy(rng.standard_normal((3, n[2], n[1], n[0])).astype(np.float32)).cuda()
+    Fa, Fb = a.field(3, F), b.field(3, F)
+    for _ in range(3):
+        assert a.gather_kick(Fa, 0.05, want_max_v=True) == b.gather_kick(Fb, 0.05, want_max_v=True)
+        a.drift_rebin(0.3)
+        b.drift_rebin(0.3)
+        assert a.rebin_stats()[2] == b.rebin_stats()[2]
+    _same(a, b, with_mass)
+    assert a.flags() & ~0x8 == 0 and b.flags() & ~0x8 == 0
