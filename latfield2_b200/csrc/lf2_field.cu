@@ -28,13 +28,52 @@ __device__ inline int wrap_coord(int v, int n)
   return v < 0 ? v + n : v;
 }
 
-// Layout conversion, a warp per row of sites along x: the row's y and z are
-// divided out and wrapped once, and a lane takes elements e = x * comps + c of
-// the reference's row, so that its accesses are contiguous.  (A 64-bit division
-// chain per site bound the first form: 145 us for the 256^3 density to double
-// with a halo of 2, and 106 us for a 3-component import, against 31 and 91 us
-// for the bytes.)  COMPS 0: any number of components.
-// I: an integer that holds the elements of a row (int except for rows of 2^31).
+// Layout conversion, a warp per row of sites along x, or per chunk of a long
+// row: the row's y and z are divided out and wrapped once, and a lane takes
+// elements e = x * comps + c of the reference's row, so that its accesses are
+// contiguous.  Rows under ROW_MIN sites leave lanes idle and pay the divisions
+// for few of them: those go by sites.  In us, by sites / by rows: 256^3 to double
+// with a halo 138 / 52, its 3-component import 101 / 74; 33 x 200 x 200, 3
+// components 17 / 21; 20 x 20 x 20,000, 3 components to double 96 / 156; 7 x 9 x
+// 100,000, 3 components 62 / 172; 10^6 x 1 x 1 13 / 17 (6400 without chunks).
+constexpr int ROW_MIN = 48;
+
+struct RowUnits {
+  int64_t units;  // chunks of all rows
+  int chunks;     // of a row
+  int span;       // elements of a chunk
+};
+
+inline RowUnits row_units(int64_t rows, int64_t row_elements, int lane_elements)
+{
+  RowUnits u;
+  u.span = 32 * lane_elements;
+  u.chunks = (int)((row_elements + u.span - 1) / u.span);
+  u.units = rows * u.chunks;
+  return u;
+}
+
+// fn(row, first element of the lane, end) for the chunks of this warp.
+// I: an integer that holds the elements of a row and 32 more.
+template <typename I, typename Fn>
+__device__ __forceinline__ void for_rows(const RowUnits& ru, I row_elements, Fn fn)
+{
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t u = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); u < ru.units; u += warps) {
+    int64_t row = u;
+    I e0 = lane, end = row_elements;
+    if (ru.chunks > 1) {
+      row = u / ru.chunks;
+      const I first = (I)(u - row * ru.chunks) * ru.span, left = row_elements - first;
+      e0 += first;
+      end = first + (left < ru.span ? left : ru.span);
+    }
+    fn(row, e0, end);
+  }
+}
+
+// COMPS 0: any number of components.
 template <int COMPS, typename I>
 __device__ __forceinline__ void element(I e, int comps, int& x, int& c)
 {
@@ -50,14 +89,12 @@ __device__ __forceinline__ void element(I e, int comps, int& x, int& c)
 // Every gross site of the reference layout; halo sites either copy their
 // periodic image (Field::updateHalo, LATfield2_Field_decl.hpp:889-935) or are 0.
 template <typename T, int COMPS, typename I>
-__global__ void __launch_bounds__(256) k_export(Geom g, int comps, const float* __restrict__ src,
+__global__ void __launch_bounds__(256) k_export(Geom g, RowUnits ru, int comps, const float* __restrict__ src,
                                                 T* __restrict__ dst, int halo, int fill_halo)
 {
   const int G0 = g.n[0] + 2 * halo, G1 = g.n[1] + 2 * halo;
-  const int64_t rows = (int64_t)G1 * (g.n[2] + 2 * halo);
-  const int nc = COMPS ? COMPS : comps, lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t row = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += warps) {
+  const int nc = COMPS ? COMPS : comps;
+  for_rows<I>(ru, (I)G0 * nc, [&](int64_t row, I e0, I end) {
     int y = (int)(row % G1) - halo, z = (int)(row / G1) - halo;
     const bool inside = y >= 0 && y < g.n[1] && z >= 0 && z < g.n[2];
     y = wrap_coord(y, g.n[1]);
@@ -65,7 +102,7 @@ __global__ void __launch_bounds__(256) k_export(Geom g, int comps, const float* 
     const float* s = src + site_index(g, 0, y, z);
     T* d = dst + row * G0 * nc;
 #pragma unroll 4
-    for (I e = lane; e < (I)G0 * nc; e += 32) {
+    for (I e = e0; e < end; e += 32) {
       int x, c;
       element<COMPS, I>(e, comps, x, c);
       x -= halo;
@@ -73,27 +110,71 @@ __global__ void __launch_bounds__(256) k_export(Geom g, int comps, const float* 
       if (x < 0 || x >= g.n[0]) x = wrap_coord(x, g.n[0]);
       d[e] = in || fill_halo ? (T)__ldg(s + c * g.nsites + x) : (T)0;
     }
-  }
+  });
 }
 
+// By elements up to 3 components, by sites above: there the writes of one
+// component would be short runs (6 components at 256^3 by elements: 198 us).
+constexpr bool by_sites(int comps) { return comps == 0 || comps > 3; }
+
 template <typename T, int COMPS, typename I>
-__global__ void __launch_bounds__(256) k_import(Geom g, int comps, float* __restrict__ dst,
+__global__ void __launch_bounds__(256) k_import(Geom g, RowUnits ru, int comps, float* __restrict__ dst,
                                                 const T* __restrict__ src, int halo)
 {
   const int64_t G0 = g.n[0] + 2 * halo, G1 = g.n[1] + 2 * halo;
-  const int64_t rows = (int64_t)g.n[1] * g.n[2];
-  const int nc = COMPS ? COMPS : comps, lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t row = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += warps) {
+  const int nc = COMPS ? COMPS : comps;
+  constexpr bool SITES = by_sites(COMPS);
+  for_rows<I>(ru, (I)g.n[0] * (SITES ? 1 : nc), [&](int64_t row, I e0, I end) {
     const int y = (int)(row % g.n[1]), z = (int)(row / g.n[1]);
     const T* s = src + (halo + G0 * (y + halo + G1 * (z + halo))) * nc;
     float* d = dst + row * g.n[0];
+    if constexpr (SITES) {
+      for (I e = e0; e < end; e += 32) {
+#pragma unroll(COMPS ? COMPS : 4)
+        for (int c = 0; c < nc; c++) d[c * g.nsites + e] = (float)__ldg(s + (int64_t)e * nc + c);
+      }
+    } else {
 #pragma unroll 4
-    for (I e = lane; e < (I)g.n[0] * nc; e += 32) {
-      int x, c;
-      element<COMPS, I>(e, comps, x, c);
-      d[c * g.nsites + x] = (float)__ldg(s + e);
+      for (I e = e0; e < end; e += 32) {
+        int x, c;
+        element<COMPS, I>(e, comps, x, c);
+        d[c * g.nsites + x] = (float)__ldg(s + e);
+      }
     }
+  });
+}
+
+// The same by sites, for short rows.
+template <typename T>
+__global__ void __launch_bounds__(256) k_export_sites(Geom g, int comps, const float* __restrict__ src,
+                                                      T* __restrict__ dst, int halo, int fill_halo)
+{
+  const int64_t G0 = g.n[0] + 2 * halo, G1 = g.n[1] + 2 * halo, total = G0 * G1 * (g.n[2] + 2 * halo);
+  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
+       idx += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t row = idx / G0;
+    int x = (int)(idx - row * G0) - halo, y = (int)(row % G1) - halo, z = (int)(row / G1) - halo;
+    const bool inside = x >= 0 && x < g.n[0] && y >= 0 && y < g.n[1] && z >= 0 && z < g.n[2];
+    x = wrap_coord(x, g.n[0]);
+    y = wrap_coord(y, g.n[1]);
+    z = wrap_coord(z, g.n[2]);
+    const int64_t s = site_index(g, x, y, z);
+    for (int c = 0; c < comps; c++)
+      dst[idx * comps + c] = inside || fill_halo ? (T)src[c * g.nsites + s] : (T)0;
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_import_sites(Geom g, int comps, float* __restrict__ dst,
+                                                      const T* __restrict__ src, int halo)
+{
+  const int64_t G0 = g.n[0] + 2 * halo, G1 = g.n[1] + 2 * halo;
+  for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < g.nsites;
+       s += (int64_t)gridDim.x * blockDim.x) {
+    int x, y, z;
+    cell_xyz(g, (int32_t)s, x, y, z);
+    const int64_t idx = (x + halo) + G0 * ((y + halo) + G1 * (int64_t)(z + halo));
+    for (int c = 0; c < comps; c++) dst[c * g.nsites + s] = (float)src[idx * comps + c];
   }
 }
 
@@ -192,7 +273,7 @@ template <typename Fn>
 static void by_comps(int comps, int64_t row_elements, Fn fn)
 {
   using std::integral_constant;
-  if (row_elements > INT32_MAX) fn(integral_constant<int, 0>{}, int64_t{});
+  if (row_elements > INT32_MAX - 64) fn(integral_constant<int, 0>{}, int64_t{});
   else if (comps == 1) fn(integral_constant<int, 1>{}, int{});
   else if (comps == 3) fn(integral_constant<int, 3>{}, int{});
   else if (comps == 6) fn(integral_constant<int, 6>{}, int{});
@@ -204,14 +285,23 @@ cudaError_t launch_export(lf2_ctx* c, int comps, const float* src, void* dst, in
 {
   c->launches += 1;
   const int64_t G0 = (int64_t)c->g.n[0] + 2 * halo;
-  const int grid = grid_for((int64_t)(c->g.n[1] + 2 * halo) * (c->g.n[2] + 2 * halo) * 32, 256);
+  if (G0 < ROW_MIN) {
+    const int sites = grid_for(G0 * (c->g.n[1] + 2 * halo) * (c->g.n[2] + 2 * halo), 256);
+    if (real_bytes == 8)
+      k_export_sites<double><<<sites, 256, 0, c->stream>>>(c->g, comps, src, (double*)dst, halo, fill_halo);
+    else
+      k_export_sites<float><<<sites, 256, 0, c->stream>>>(c->g, comps, src, (float*)dst, halo, fill_halo);
+    return cudaGetLastError();
+  }
+  const RowUnits ru = row_units((int64_t)(c->g.n[1] + 2 * halo) * (c->g.n[2] + 2 * halo), G0 * comps, 64);
+  const int grid = grid_for(ru.units * 32, 256);
   by_comps(comps, G0 * comps, [&](auto k, auto i) {
     constexpr int K = decltype(k)::value;
     using I = decltype(i);
     if (real_bytes == 8)
-      k_export<double, K, I><<<grid, 256, 0, c->stream>>>(c->g, comps, src, (double*)dst, halo, fill_halo);
+      k_export<double, K, I><<<grid, 256, 0, c->stream>>>(c->g, ru, comps, src, (double*)dst, halo, fill_halo);
     else
-      k_export<float, K, I><<<grid, 256, 0, c->stream>>>(c->g, comps, src, (float*)dst, halo, fill_halo);
+      k_export<float, K, I><<<grid, 256, 0, c->stream>>>(c->g, ru, comps, src, (float*)dst, halo, fill_halo);
   });
   return cudaGetLastError();
 }
@@ -220,14 +310,25 @@ cudaError_t launch_import(lf2_ctx* c, int comps, float* dst, const void* src, in
                           int real_bytes)
 {
   c->launches += 1;
-  const int grid = grid_for((int64_t)c->g.n[1] * c->g.n[2] * 32, 256);
+  if (c->g.n[0] < ROW_MIN) {
+    const int sites = grid_for(c->g.nsites, 256);
+    if (real_bytes == 8)
+      k_import_sites<double><<<sites, 256, 0, c->stream>>>(c->g, comps, dst, (const double*)src, halo);
+    else
+      k_import_sites<float><<<sites, 256, 0, c->stream>>>(c->g, comps, dst, (const float*)src, halo);
+    return cudaGetLastError();
+  }
   by_comps(comps, (int64_t)c->g.n[0] * comps, [&](auto k, auto i) {
     constexpr int K = decltype(k)::value;
     using I = decltype(i);
+    const RowUnits ru =
+        row_units((int64_t)c->g.n[1] * c->g.n[2], (int64_t)c->g.n[0] * (by_sites(K) ? 1 : comps),
+                  by_sites(K) ? 16 : 64);
+    const int grid = grid_for(ru.units * 32, 256);
     if (real_bytes == 8)
-      k_import<double, K, I><<<grid, 256, 0, c->stream>>>(c->g, comps, dst, (const double*)src, halo);
+      k_import<double, K, I><<<grid, 256, 0, c->stream>>>(c->g, ru, comps, dst, (const double*)src, halo);
     else
-      k_import<float, K, I><<<grid, 256, 0, c->stream>>>(c->g, comps, dst, (const float*)src, halo);
+      k_import<float, K, I><<<grid, 256, 0, c->stream>>>(c->g, ru, comps, dst, (const float*)src, halo);
   });
   return cudaGetLastError();
 }

@@ -1,6 +1,6 @@
 """Field import and export in the reference's layout (interleaved components,
 halo) against numpy, for the component counts with kernels of their own and
-others, rows shorter and longer than a warp, and halos up to the lattice."""
+others, rows of one site to several chunks (by sites below 48, by rows above), and halos up to the lattice."""
 import numpy as np
 import pytest
 
@@ -10,7 +10,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,halo", [((5, 6, 7), 0), ((5, 6, 7), 5), ((33, 4, 9), 1), ((70, 3, 2), 2),
-                                    ((1, 1, 40), 1)])
+                                    ((1, 1, 40), 1), ((700, 1, 1), 0), ((513, 2, 1), 1),
+                                    ((2, 3, 50), 0), ((47, 3, 5), 0), ((16, 2, 2), 16),
+                                    ((5000, 1, 1), 0)])
 @pytest.mark.parametrize("comps", [1, 2, 3, 6, 7])
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 def test_import_and_export(cuda, n, halo, comps, dtype):
