@@ -763,34 +763,34 @@ __global__ void __launch_bounds__(FIX2_THREADS, 2)
     for (int c = 0; c < 3; c++) out[(c0 + c) * g.nsites + site] = r[c].value(conv);
   };
   // any owned boundary vertex, neighbours on both sides included: z outermost,
-  // below before own before above
-  auto general = [&](const int (&q)[3]) {
+  // below before own before above; one component (an absent neighbour adds 0,
+  // so that the reads do not wait for one another)
+  auto general = [&](const int (&q)[3], int c) {
     const int own[3] = {canon(q[0] + 1, e[0]), canon(q[1] + 1, e[1]), canon(q[2] + 1, e[2])};
     const int64_t site = site0 + q[0] * step[0] + q[1] * step[1] + q[2] * step[2];
-#pragma unroll 1
-    for (int c = 0; c < 3; c++) {
-      Sum r;
-#pragma unroll 1
-      for (int s = 0; s < 27; s++) {
-        int64_t nb = b;
-        int u[3], rest[3] = {s % 3, (s / 3) % 3, s / 9};
-        bool in = true;
+    Sum r;
+#pragma unroll 9
+    for (int s = 0; s < 27; s++) {
+      int64_t nb = b;
+      int u[3], rest[3] = {s % 3, (s / 3) % 3, s / 9};
+      bool in = true;
 #pragma unroll
-        for (int d = 0; d < 3; d++) {
-          in &= rest[d] == 1 || q[d] == (rest[d] ? e[d] - 1 : 0);
-          nb += rest[d] == 1 ? 0 : rest[d] ? nbr[d][1] : nbr[d][0];
-          u[d] = rest[d] == 1 ? own[d] : rest[d] ? 0 : FT - 1;
-        }
-        if (in) r.add(read(nb, c, thick_index(u[0], u[1], u[2])));
+      for (int d = 0; d < 3; d++) {
+        in &= rest[d] == 1 || q[d] == (rest[d] ? e[d] - 1 : 0);
+        nb += rest[d] == 1 ? 0 : rest[d] ? nbr[d][1] : nbr[d][0];
+        u[d] = rest[d] == 1 ? own[d] : rest[d] ? 0 : FT - 1;
       }
-      out[(c0 + c) * g.nsites + site] = r.value(conv);
+      r.add(in ? read(nb, c, thick_index(u[0], u[1], u[2])) : 0);
     }
+    out[(c0 + c) * g.nsites + site] = r.value(conv);
   };
   if (e[0] < 2 || e[1] < 2 || e[2] < 2) {
-    for (int v = threadIdx.x; v < e[0] * e[1] * e[2]; v += blockDim.x) {
+    const int vertices = e[0] * e[1] * e[2];
+    for (int i = threadIdx.x; i < 3 * vertices; i += blockDim.x) {
+      const int c = i / vertices, v = i % vertices;
       const int q[3] = {v % e[0], v / e[0] % e[1], v / (e[0] * e[1])};
       if (q[0] == 0 || q[1] == 0 || q[2] == 0 || q[0] == e[0] - 1 || q[1] == e[1] - 1 || q[2] == e[2] - 1)
-        general(q);
+        general(q, c);
     }
     return;
   }
