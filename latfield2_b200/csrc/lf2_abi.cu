@@ -236,6 +236,7 @@ lf2_status load_device(lf2_ctx* c, int64_t n, const int32_t* cell, const float* 
   c->np = n;
   const lf2_status loaded = check_flags(c);
   c->most = (int64_t)c->h_stats[1];
+  c->most_age = 0;
   if (loaded != LF2_OK) {
     c->np = c->most = 0;
     LF2_CUDA(c, cudaMemsetAsync(c->count, 0, sizeof(int32_t) * nb, c->stream));
@@ -581,6 +582,7 @@ lf2_status lf2_slab_insert(lf2_ctx* c, int64_t n_a, const uint32_t* a, int64_t n
     LF2_TRY(rebin_tail(c));
     LF2_CUDA(c, cudaMemsetAsync(c->mov_count, 0, sizeof(unsigned long long), c->stream));
     c->np = total;
+    c->most_age = INT32_MAX;  // (the host has not seen where they went)
     prepare_rows(c);
     return LF2_OK;
   }
@@ -631,6 +633,7 @@ lf2_status lf2_particles_add(lf2_ctx* c, int64_t n, const int32_t* cell, const f
     LF2_TRY(rebin_tail(c));
     LF2_CUDA(c, cudaMemsetAsync(c->mov_count, 0, sizeof(unsigned long long), c->stream));
     c->np = total;
+    c->most_age = INT32_MAX;  // (the host has not seen where they went)
     prepare_rows(c);
     return LF2_OK;
   }
@@ -1017,6 +1020,7 @@ lf2_status lf2_gather_kick(lf2_ctx* c, lf2_field F, double dtau, double* max_v)
     LF2_CUDA(c, cudaStreamSynchronize(c->stream));
     *max_v = std::sqrt(c->h_stats[0]);
     c->most = (int64_t)c->h_stats[1];
+    c->most_age = 0;
   }
   return LF2_OK;
 }
@@ -1025,6 +1029,7 @@ lf2_status lf2_drift_rebin(lf2_ctx* c, double dtau)
 {
   if (!c) return LF2_ERR_ARG;
   MoveParams mp{0.0f, (float)(dtau / c->res)};
+  c->most_age++;
   const bool pipe = drift_pipe_auto(c);
   if (!pipe)  // the pipelined pass clears the counters itself
     LF2_CUDA(c, cudaMemsetAsync(c->head, 0, sizeof(PassHead), c->stream));
@@ -1041,6 +1046,7 @@ lf2_status lf2_step(lf2_ctx* c, lf2_field F, double dtau_kick, double dtau_drift
   if (!valid_field(c, F)) return LF2_ERR_ARG;
   if (F->comps != 3) return fail(c, LF2_ERR_ARG, "the kick field needs 3 components");
   MoveParams mp{(float)dtau_kick, (float)(dtau_drift / c->res)};
+  c->most_age++;
   if ((c->move_kernel == 2 || c->move_kernel == 3) && !move_pipe_eligible(c, F->data))
     return fail(c, LF2_ERR_UNSUPPORTED, "pipelined move needs n0 % 4 == 0, n >= 32, aligned F");
   if (c->move_kernel == 3 && !move_dep_eligible(c, F->data))
@@ -1125,6 +1131,7 @@ lf2_status lf2_last_max_velocity(lf2_ctx* c, double* max_v, int ptr_kind)
   LF2_CUDA(c, cudaStreamSynchronize(c->stream));
   *max_v = std::sqrt(c->h_stats[0]);
   c->most = (int64_t)c->h_stats[1];
+  c->most_age = 0;
   return LF2_OK;
 }
 

@@ -52,8 +52,9 @@ namespace lf2 {
 
 namespace {
 
-// Threads of a tile pass, and of one whose tile leaves room for one CTA per SM
-//.
+// Threads of a tile pass, and of one whose tile leaves room for one CTA per SM.
+// (512 for stores with few particles per brick won 3% in fixed point and lost as
+// much with the FP32 sums: 128^3 at 0.02 per site, six components.)
 constexpr int DEP_THREADS = 256, DEP_BIG_THREADS = 1024;
 
 // Fewest particles of a part of a split brick, and of any item (a brick below
@@ -766,6 +767,19 @@ cudaError_t run_mode(lf2_ctx* c, float* out, const DepositParams& dp, int stage,
 
 }  // namespace
 
+// Whether the plan can be left out, with its launch and that of every pass's
+// finishing kernel (5 us each: an even 64^3 in fixed point, density 28 us against
+// 22): no brick can be split, or the host knows the store to be even, its largest
+// brick a quarter below an item and read a few rebins ago.  A captured call is
+// replayed on stores that the host has not seen.
+static bool no_heavy_brick(const lf2_ctx* c, int64_t split, int64_t first)
+{
+  if (c->np <= split) return true;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  return c->most_age <= 32 && c->most + c->most / 4 <= first &&
+         cudaStreamIsCapturing(c->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+}
+
 // What is heavy depends on the chip's share of the particles per CTA that runs
 // at once (`share`).  A brick is an item, taken first, above a quarter of the
 // share (a brick that starts last then ends with the others), three times
@@ -793,6 +807,7 @@ PartPlan part_plan(lf2_ctx* c, size_t smem, int threads, size_t tile_slots, int 
   const int64_t first =
       std::min(split, std::max({ITEM_MIN, share / 4, 3 * (c->np / c->g.nbricks)}));
   pl.P = (int)P, pl.split = (int)split, pl.first = (int)first;
+  if (no_heavy_brick(c, split, first)) return pl;
   // np particles make at most 3/2 np / P parts and np / first items
   pl.max_items = (int)std::min<int64_t>(PART_ITEMS, c->np * 3 / (2 * P) + c->np / first);
   pl.max_tiles = (int)std::min<int64_t>(7 * (c->capacity / 2 / (int64_t)tile_slots), PART_TILES);

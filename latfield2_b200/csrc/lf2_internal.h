@@ -69,7 +69,8 @@ struct lf2_ctx {
 
   // particle store
   int64_t np = 0;
-  int64_t most = 0;     // count of the largest brick, as last read by the host (kernel choice)
+  int64_t most = 0;     // count of the largest brick, as last read by the host
+  int64_t most_age = 0; // rebins since
   bool has_mass = false;
   bool has_id = false;
   double gmass = 0.0;   // global particle mass (GLOBAL_MASS types)

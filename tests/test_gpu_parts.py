@@ -167,3 +167,48 @@ def test_more_bricks_than_a_load_counts_in_shared_memory(cuda):
     check(f, s["cell"], s["off"])
     assert ctx.flags() & ~0x8 == 0
     ctx.close()
+
+
+def test_a_store_that_clumps_after_its_load(cuda):
+    """An even store deposits without a plan of heavy bricks; one that collapses
+    into a brick afterwards is bit-exact whether the host has read its counts
+    since (the maximum velocity) or not, after a few steps and after many."""
+    import torch
+    n = (64, 64, 64)
+    rng = np.random.default_rng(12)
+    npart = 60000
+    cell = rng.integers(0, 64 ** 3, npart).astype(np.int32)
+    off = (rng.random((npart, 3)) * (1 - 2.0 ** -23)).astype(np.float32)
+    xyz = np.stack([cell % 64, cell // 64 % 64, cell // 4096], 1) + off
+    gm = 1.0 / npart
+    ctx = _ctx(n, 1)
+    # towards the middle of brick (1, 1, 1): nearly all of them there after 8 steps
+    vel = ((24.0 - xyz) / 64.0).astype(np.float32)
+    ctx.set_particles(cell, off, vel, global_mass=gm)
+    F = ctx.field(3, torch.zeros(3, 64, 64, 64, device="cuda"))
+    rho, vec = ctx.field(1), ctx.field(3)
+
+    def check(stepped):
+        s = ctx.get_particles()
+        scale = np.float32(2.0 ** -32 * gm / (1.0 / n[0]) ** 3)
+        want = O.fixed_to_f32(O.state_deposit_fixed(n, s["cell"], s["off"]), scale)
+        if stepped:
+            np.testing.assert_array_equal(rho.export_internal().reshape(-1), want)
+        ctx.deposit_scalar(rho)
+        np.testing.assert_array_equal(rho.export_internal().reshape(-1), want)
+        ctx.deposit_vector(vec)
+        acc, e = O.state_deposit_fixed_kind(1, n, s["cell"], s["off"], s["vel"])
+        np.testing.assert_array_equal(vec.export_internal(), O.fixed_kind_to_f32(acc, 1, e, gm, 1.0 / n[0]))
+        return np.bincount(s["cell"] % 64 // 16 + 4 * (s["cell"] // 64 % 64 // 16)
+                           + 16 * (s["cell"] // 4096 // 16)).max()
+    assert check(False) < 1200
+    for _ in range(8):
+        ctx.step(F, 0.0, 0.11, rho)
+    assert check(True) > 40000
+    ctx.last_max_velocity()
+    check(True)
+    for _ in range(40):
+        ctx.step(F, 0.0, 0.0, rho)
+    check(True)
+    assert ctx.flags() & ~0x8 == 0
+    ctx.close()
