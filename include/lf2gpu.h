@@ -60,9 +60,12 @@ typedef int lf2_status;
 #define LF2_ERR_UNSUPPORTED (-5) /* combination not provided */
 
 /* Deposit modes (lf2_create).  FP32: FP32 terms in a compensated sum (wide
- * integers, or FP32 additions whose rounding errors are recovered exactly and
- * carried in a second FP32 word), so every vertex sum is within about 1e-7 of
- * exact whatever the order (not bit-identical run to run).  FIXED64: int64 fixed point, bit-exact run to run; quantum 2^-32 of
+ * integers with the rests of small terms, or FP32 additions whose rounding
+ * errors are recovered exactly and carried in a second FP32 word), so that
+ * every vertex sum is within about 1e-7 of the sum of its terms' magnitudes
+ * (their own roundings, 2^-24 each, and one of the result), whatever the order
+ * and however large the other terms of its brick are (not bit-identical run to
+ * run).  FIXED64: int64 fixed point, bit-exact run to run; quantum 2^-32 of
  * a unit mass (the global particle mass, or the mean of per-particle
  * masses) for the density, 2^-48 of a unit mass times V for momentum and
  * times V^2 for stress, V the smallest power of two above every |v_i| of the

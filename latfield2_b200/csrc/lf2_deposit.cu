@@ -24,15 +24,17 @@
 //                           it (add_rest), or, where that range does not hold,
 //                           FP32 atomics that return the value they replaced,
 //                           the rounding error of each recovered exactly
-//                           (TwoSum) and accumulated in a second FP32 word.  hi + lo is the sum to within the rounding
-//                           of the terms (about 1e-7 relative), whatever the
-//                           order.
+//                           (TwoSum) and accumulated in a second FP32 word.
+//                           hi + lo is the sum to within the rounding of the
+//                           terms (about 1e-7 of the sum of their magnitudes),
+//                           whatever the order and whatever else the brick
+//                           holds.
 //   LF2_DEPOSIT_FIXED64     int64 fixed point: every contribution is rounded
 //                           once, deterministically, to an integer quantum;
 //                           the integer sums do not depend on the order, so
 //                           the result is bit-exact run to run.  Scalar: 2^-32
 //                           of a unit mass.  Momentum and stress are signed:
-//                           2^-32 of a unit mass times V (momentum) or V^2
+//                           2^-48 of a unit mass times V (momentum) or V^2
 //                           (stress), V the smallest power of two above every
 //                           |v_i| of the particles (found on the device before
 //                           the deposit, k_vmax).

@@ -251,9 +251,8 @@ cudaError_t launch_pm(lf2_ctx* c, int op, int64_t np, const int32_t* cell, const
 // the chain's deposit, per particle or brick-tiled (brick_start given)
 cudaError_t launch_pm_deposit(lf2_ctx* c, int64_t np, const int64_t* brick_start, const int32_t* cell,
                               const float* off3, const float* mass, float gmass, float* rho);
-// the chain's particle state: sort keys and 32-byte records in the caller's
-// order, the state in a given order, the bricks' first slots; gradients back
-// to the caller's order through the same records
+// a step of the chain: gather, kick and drift (the outputs may be the inputs),
+// its adjoint; the loss and its adjoint
 cudaError_t launch_pm_step(lf2_ctx* c, int64_t np, const int32_t* cell, const float* off3,
                            const float* vel3, const float* F4, float dtk, float dtn, int32_t* cell_out,
                            float* off_out, float* vel_out);
@@ -265,6 +264,9 @@ cudaError_t launch_pm_loss_adjoint(lf2_ctx* c, int64_t np, const int32_t* cell, 
                                    float* g_mass, float* g_vel3);
 int loss_ctas(const lf2_ctx* c);
 cudaError_t launch_pm_loss(lf2_ctx* c, const float* w, const float* rho, double* loss);
+// the chain's particle state: sort keys and 32-byte records in the caller's
+// order, the state in a given order, the bricks' first slots; gradients back
+// to the caller's order through the same records
 cudaError_t launch_pm_pack(lf2_ctx* c, int64_t np, const double* pos, const double* vel,
                            const double* mass, double inv_res, int32_t* key, void* rec);
 cudaError_t launch_pm_unpack(lf2_ctx* c, int64_t np, const int64_t* order, const void* rec,

@@ -2,7 +2,7 @@
 VecVecProjectionCIC; projections.hpp:978-1814) against the CPU oracle,
 called through the C ABI.
 
-Every case runs in the three deposit modes: FP32 (compensated atomics) and
+Every case runs in the three deposit modes: FP32 (compensated sums) and
 fixed point within 1e-6 of the FP64 oracle, normalized by the field's
 maximum, plain FP32 within 1e-5.  The cases cover ragged
 bricks (n not a multiple of 16), lattices one or two bricks wide (a brick is

@@ -8,7 +8,7 @@ restatement (layer B), for every projection:
   kind 4  VecVecProjectionCIC
 
 Tolerances (tests.helpers.precision):
-  - FP32 mode (compensated atomics) and fixed-point mode: error <= 1e-6 of the
+  - FP32 mode (compensated sums) and fixed-point mode: error <= 1e-6 of the
     field maximum, and <= 1e-6 of the vertex's sum of |contributions| on every
     vertex where that sum exceeds 1e-2 of its mean (the relative error of a
     sum, defined where signed momenta cancel).
