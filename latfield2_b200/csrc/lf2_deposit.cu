@@ -85,12 +85,10 @@ struct Pass {
                                          : (j == 0 ? 1 : j == 1 ? 2 : 4);
   }
   static constexpr size_t smem() { return (size_t)NC * WORDS * TILE3 * 4; }
-  // after the tile, what the compensated mode keeps of small terms: notes
-  // (Rests) and listed particles (RestList: all of a part, or what five CTAs
-  // per SM leave room for)
-  static constexpr int NOTES = ACC != ACC_COMP ? 0 : smem() > 100 * 1024 ? 2048 : 128;
-  static constexpr int RESTS = ACC != ACC_COMP ? 0 : smem() > 100 * 1024 ? 32768 : 1536;
-  static constexpr size_t dyn() { return smem() + NOTES * sizeof(uint2) + RESTS * sizeof(uint16_t); }
+  // after the tile, the compensated mode's rests of small terms (Rests): room for
+  // what five CTAs per SM leave, or for 64 KB
+  static constexpr int RESTS = ACC != ACC_COMP ? 0 : smem() > 100 * 1024 ? 8192 : 512;
+  static constexpr size_t dyn() { return smem() + RESTS * sizeof(uint2); }
   // a tile above 100 KB leaves room for one CTA per SM
   static constexpr int THREADS = smem() > 100 * 1024 ? DEP_BIG_THREADS : DEP_THREADS;
   static constexpr int ITEMS = smem() > 100 * 1024 ? 2 : 4;  // particles in flight per thread
@@ -121,7 +119,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
 
   __shared__ unsigned s_max;
   __shared__ int s_tile;  // (not a register of the particle loop)
-  __shared__ int s_rests, s_notes;
+  __shared__ int s_rests, s_any;
   __shared__ uint32_t s_marks[ACC == ACC_COMP ? (NC * TILE3 + 31) / 32 : 1];
   __shared__ float s_quantum;
 
@@ -160,20 +158,16 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
     for (int t = threadIdx.x; t < words; t += blockDim.x) z[t] = 0u;
     if (ACC == ACC_COMP)
       for (int t = threadIdx.x; t < (NC * TILE3 + 31) / 32; t += blockDim.x) s_marks[t] = 0u;
-    if (threadIdx.x == 0) s_rests = 0, s_notes = 0, s_quantum = cu.quantum;
+    if (threadIdx.x == 0) s_rests = 0, s_any = 0, s_quantum = cu.quantum;
   }
   __syncthreads();
-  uint2* const notes = reinterpret_cast<uint2*>(smem_raw + P::smem());
-  const RestList rl{reinterpret_cast<uint16_t*>(notes + P::NOTES), &s_rests, P::RESTS};
+  const Rests rs{reinterpret_cast<uint2*>(smem_raw + P::smem()), &s_rests, P::RESTS, s_marks, &s_any, &s_quantum};
 
   // The particle loop, instantiated for the tile of two integer words per
-  // vertex or the other one, chosen once per CTA, and for the listed particles'
-  // rests.
+  // vertex or the other one, chosen once per CTA.
   constexpr int ITEMS = P::ITEMS;
-  Rests rs{0, false, cu.quantum, s_marks, notes, &s_notes, P::NOTES};
-  auto particles = [&](auto sum_c, int cnt) {
-    constexpr int SUM = decltype(sum_c)::value;
-    constexpr bool SPLIT = SUM == SUM_INT;
+  auto particles = [&](auto split_c) {
+    constexpr bool SPLIT = decltype(split_c)::value;
     for (int c0 = 0; c0 < cnt; c0 += ITEMS * T) {
       uint32_t key[ITEMS];
       float fx[ITEMS], fy[ITEMS], fz[ITEMS], m[ITEMS];
@@ -182,7 +176,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
       for (int j = 0; j < ITEMS; j++) {
         const int i = c0 + j * T + threadIdx.x;
         if (i < cnt) {
-          const uint32_t p = base + (uint32_t)(SUM == SUM_REST ? rl.entry[i] : i);
+          const uint32_t p = base + (uint32_t)i;
           key[j] = v.a.key[p];
           fx[j] = v.a.ox[p];
           fy[j] = v.a.oy[p];
@@ -286,45 +280,50 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
                     gz = __fsub_rn(1.0f, fz[j]);
         const float ox = fx[j], oy = fy[j], oz = fz[j];
         const float mf = HM ? __fmul_rn(m[j], dp.inv_vol) : dp.mf;
-        if (ACC == ACC_COMP && SPLIT) {  // the particle's smallest term, or a bound below it
-          auto least3 = [](float a, float b, float c) { return fminf(fminf(fabsf(a), fabsf(b)), fabsf(c)); };
-          const float mx = __fmul_rn(mf, vx[j]), my = __fmul_rn(mf, vy[j]), mz = __fmul_rn(mf, vz[j]);
-          float f = KIND == 0 ? fabsf(mf) : least3(mx, my, mz);
-          if (KIND == 2)
-            f = PASS == 0 ? least3(__fmul_rn(mx, vx[j]), __fmul_rn(my, vy[j]), __fmul_rn(mz, vz[j]))
-                          : least3(__fmul_rn(mx, vy[j]), __fmul_rn(mx, vz[j]), __fmul_rn(my, vz[j]));
-          const float ux = fminf(ox, gx), uy = fminf(oy, gy), uz = fminf(oz, gz);
-          if (KIND == 2 && PASS == 1)  // one weight to a term
-            f = __fmul_rn(f, fminf(fminf(ux, uy), uz));
-          else
-            f = __fmul_rn(__fmul_rn(__fmul_rn(f, ux), uy), uz);
-          if (has_rest(__fmul_rn(f, cu.unit))) rl.add(i);
-        }
         if (KIND == 0) {
   #pragma unroll
           for (int k = 0; k < 8; k++) {
             const int cx = (k >> 2) & 1, cy = (k >> 1) & 1, cz = k & 1;
             const float w = __fmul_rn(
                 __fmul_rn(__fmul_rn(sel(cx, ox, gx), sel(cy, oy, gy)), sel(cz, oz, gz)), mf);
-            add_float<ACC, SUM, TILE3>(smem_raw, 0, t0 + cx + cy * TY + cz * TZ, w, cu.unit, rs);
+            add_float<ACC, SPLIT, false, TILE3>(smem_raw, 0, t0 + cx + cy * TY + cz * TZ, w, cu.unit, rs);
+          }
+          // the rests, for a particle in a thousand (asked of every term: 269 us
+          // against 261 at 256^3), from its arrays again, so that the loop keeps
+          // no registers for them
+          if (ACC == ACC_COMP && SPLIT &&
+              may_have_rest(__fmul_rn(
+                  __fmul_rn(__fmul_rn(__fmul_rn(fminf(ox, gx), fminf(oy, gy)), fminf(oz, gz)), fabsf(mf)),
+                  cu.unit))) {
+            const uint32_t p = base + (uint32_t)i;
+            const float mass = HM ? __fmul_rn(v.a.mass[p], dp.inv_vol) : dp.mf;
+  #pragma unroll 1
+            for (int k = 0; k < 8; k++) {
+              const int cx = (k >> 2) & 1, cy = (k >> 1) & 1, cz = k & 1;
+              const float wx = cx ? v.a.ox[p] : __fsub_rn(1.0f, v.a.ox[p]);
+              const float wy = cy ? v.a.oy[p] : __fsub_rn(1.0f, v.a.oy[p]);
+              const float wz = cz ? v.a.oz[p] : __fsub_rn(1.0f, v.a.oz[p]);
+              const float rest = comp_rest(__fmul_rn(__fmul_rn(__fmul_rn(wx, wy), wz), mass), cu.unit, s_quantum);
+              if (rest != 0.0f) note_rest(rs, t0 + cx + cy * TY + cz * TZ, rest);
+            }
           }
         } else if (KIND == 1) {
           // projections.hpp:501-544: component i is NGP along i, CIC across.
           const float vxm = __fmul_rn(mf, vx[j]);
           const float vym = __fmul_rn(mf, vy[j]);
           const float vzm = __fmul_rn(mf, vz[j]);
-          add_float<ACC, SUM, TILE3>(smem_raw, 0, t0, __fmul_rn(__fmul_rn(vxm, gy), gz), cu.unit, rs);
-          add_float<ACC, SUM, TILE3>(smem_raw, 0, t0 + TY, __fmul_rn(__fmul_rn(vxm, oy), gz), cu.unit, rs);
-          add_float<ACC, SUM, TILE3>(smem_raw, 0, t0 + TZ, __fmul_rn(__fmul_rn(vxm, gy), oz), cu.unit, rs);
-          add_float<ACC, SUM, TILE3>(smem_raw, 0, t0 + TY + TZ, __fmul_rn(__fmul_rn(vxm, oy), oz), cu.unit, rs);
-          add_float<ACC, SUM, TILE3>(smem_raw, 1, t0, __fmul_rn(__fmul_rn(vym, gx), gz), cu.unit, rs);
-          add_float<ACC, SUM, TILE3>(smem_raw, 1, t0 + 1, __fmul_rn(__fmul_rn(vym, ox), gz), cu.unit, rs);
-          add_float<ACC, SUM, TILE3>(smem_raw, 1, t0 + TZ, __fmul_rn(__fmul_rn(vym, gx), oz), cu.unit, rs);
-          add_float<ACC, SUM, TILE3>(smem_raw, 1, t0 + 1 + TZ, __fmul_rn(__fmul_rn(vym, ox), oz), cu.unit, rs);
-          add_float<ACC, SUM, TILE3>(smem_raw, 2, t0, __fmul_rn(__fmul_rn(vzm, gx), gy), cu.unit, rs);
-          add_float<ACC, SUM, TILE3>(smem_raw, 2, t0 + 1, __fmul_rn(__fmul_rn(vzm, ox), gy), cu.unit, rs);
-          add_float<ACC, SUM, TILE3>(smem_raw, 2, t0 + TY, __fmul_rn(__fmul_rn(vzm, gx), oy), cu.unit, rs);
-          add_float<ACC, SUM, TILE3>(smem_raw, 2, t0 + 1 + TY, __fmul_rn(__fmul_rn(vzm, ox), oy), cu.unit, rs);
+          add_float<ACC, SPLIT, true, TILE3>(smem_raw, 0, t0, __fmul_rn(__fmul_rn(vxm, gy), gz), cu.unit, rs);
+          add_float<ACC, SPLIT, true, TILE3>(smem_raw, 0, t0 + TY, __fmul_rn(__fmul_rn(vxm, oy), gz), cu.unit, rs);
+          add_float<ACC, SPLIT, true, TILE3>(smem_raw, 0, t0 + TZ, __fmul_rn(__fmul_rn(vxm, gy), oz), cu.unit, rs);
+          add_float<ACC, SPLIT, true, TILE3>(smem_raw, 0, t0 + TY + TZ, __fmul_rn(__fmul_rn(vxm, oy), oz), cu.unit, rs);
+          add_float<ACC, SPLIT, true, TILE3>(smem_raw, 1, t0, __fmul_rn(__fmul_rn(vym, gx), gz), cu.unit, rs);
+          add_float<ACC, SPLIT, true, TILE3>(smem_raw, 1, t0 + 1, __fmul_rn(__fmul_rn(vym, ox), gz), cu.unit, rs);
+          add_float<ACC, SPLIT, true, TILE3>(smem_raw, 1, t0 + TZ, __fmul_rn(__fmul_rn(vym, gx), oz), cu.unit, rs);
+          add_float<ACC, SPLIT, true, TILE3>(smem_raw, 1, t0 + 1 + TZ, __fmul_rn(__fmul_rn(vym, ox), oz), cu.unit, rs);
+          add_float<ACC, SPLIT, true, TILE3>(smem_raw, 2, t0, __fmul_rn(__fmul_rn(vzm, gx), gy), cu.unit, rs);
+          add_float<ACC, SPLIT, true, TILE3>(smem_raw, 2, t0 + 1, __fmul_rn(__fmul_rn(vzm, ox), gy), cu.unit, rs);
+          add_float<ACC, SPLIT, true, TILE3>(smem_raw, 2, t0 + TY, __fmul_rn(__fmul_rn(vzm, gx), oy), cu.unit, rs);
+          add_float<ACC, SPLIT, true, TILE3>(smem_raw, 2, t0 + 1 + TY, __fmul_rn(__fmul_rn(vzm, ox), oy), cu.unit, rs);
         } else {
           // projections.hpp:786-843: T_ii at the 8 vertices, T_ij on plaquettes.
           const float vv[3] = {vx[j], vy[j], vz[j]};
@@ -342,7 +341,7 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
                 const int cx = (k >> 2) & 1, cy = (k >> 1) & 1, cz = k & 1;
                 const float w = __fmul_rn(
                     __fmul_rn(__fmul_rn(mv2, sel(cx, ox, gx)), sel(cy, oy, gy)), sel(cz, oz, gz));
-                add_float<ACC, SUM, TILE3>(smem_raw, jd, t0 + cx + cy * TY + cz * TZ, w, cu.unit, rs);
+                add_float<ACC, SPLIT, true, TILE3>(smem_raw, jd, t0 + cx + cy * TY + cz * TZ, w, cu.unit, rs);
               }
             }
           }
@@ -352,44 +351,27 @@ __global__ void __launch_bounds__(Pass<KIND, PASS, ACC>::THREADS, Pass<KIND, PAS
             const float m01 = __fmul_rn(__fmul_rn(mf, vv[0]), vv[1]);
             const float m02 = __fmul_rn(__fmul_rn(mf, vv[0]), vv[2]);
             const float m12 = __fmul_rn(__fmul_rn(mf, vv[1]), vv[2]);
-            add_float<ACC, SUM, TILE3>(smem_raw, j01, t0, __fmul_rn(m01, gz), cu.unit, rs);
-            add_float<ACC, SUM, TILE3>(smem_raw, j01, t0 + TZ, __fmul_rn(m01, oz), cu.unit, rs);
-            add_float<ACC, SUM, TILE3>(smem_raw, j02, t0, __fmul_rn(m02, gy), cu.unit, rs);
-            add_float<ACC, SUM, TILE3>(smem_raw, j02, t0 + TY, __fmul_rn(m02, oy), cu.unit, rs);
-            add_float<ACC, SUM, TILE3>(smem_raw, j12, t0, __fmul_rn(m12, gx), cu.unit, rs);
-            add_float<ACC, SUM, TILE3>(smem_raw, j12, t0 + 1, __fmul_rn(m12, ox), cu.unit, rs);
+            add_float<ACC, SPLIT, true, TILE3>(smem_raw, j01, t0, __fmul_rn(m01, gz), cu.unit, rs);
+            add_float<ACC, SPLIT, true, TILE3>(smem_raw, j01, t0 + TZ, __fmul_rn(m01, oz), cu.unit, rs);
+            add_float<ACC, SPLIT, true, TILE3>(smem_raw, j02, t0, __fmul_rn(m02, gy), cu.unit, rs);
+            add_float<ACC, SPLIT, true, TILE3>(smem_raw, j02, t0 + TY, __fmul_rn(m02, oy), cu.unit, rs);
+            add_float<ACC, SPLIT, true, TILE3>(smem_raw, j12, t0, __fmul_rn(m12, gx), cu.unit, rs);
+            add_float<ACC, SPLIT, true, TILE3>(smem_raw, j12, t0 + 1, __fmul_rn(m12, ox), cu.unit, rs);
           }
         }
       }
     }
   };
   
-  using std::integral_constant;
-  bool pairs = ACC == ACC_PLAIN || !tr.split;
+  bool split = ACC != ACC_PLAIN && tr.split;
   if constexpr (ACC != ACC_PLAIN) {
-    if (!pairs) particles(integral_constant<int, SUM_INT>{}, cnt);
+    if (split) particles(std::true_type{});
   }
   if constexpr (ACC == ACC_COMP) {
     __syncthreads();
-    rs.count = s_rests;
-    if (rs.count > P::RESTS) {  // more than the list holds: again, with the FP32 pairs
-      uint32_t* z = reinterpret_cast<uint32_t*>(smem_raw);
-      for (int t = threadIdx.x; t < NC * P::WORDS * TILE3; t += blockDim.x) z[t] = 0u;
-      tr.split = false;
-      pairs = true;
-      __syncthreads();
-    } else if (rs.count) {
-      for (int pass = 0; pass < 2; pass++) {
-        particles(integral_constant<int, SUM_REST>{}, rs.count);
-        __syncthreads();
-        if (rs.apply || !s_notes) break;
-        tr.marks = s_marks;
-        if (take_notes<TILE3>(smem_raw, NC, rs)) break;
-        rs.apply = true;
-      }
-    }
+    if (split) split = take_rests(tr, NC, rs);
   }
-  if (pairs) particles(integral_constant<int, SUM_PAIR>{}, cnt);
+  if (!split) particles(std::false_type{});
   __syncthreads();
   if (s_tile >= 0) {  // k_part_finish writes the vertices
     part_store<ACC, SIGNED, NC, TILE3>(scratch_tile(pv, s_tile, NC * TILE3), tr, s_quantum);

@@ -126,45 +126,52 @@ __device__ __forceinline__ void add_fixed48_t(unsigned char* smem, int j, int t,
 // arithmetic; their sum is kept, as in the signed fixed-point kinds, as a
 // 64-bit integer in two 32-bit words, in units of a quantum set by the largest
 // term of the CTA's particles (CompUnit).  A term at or above 2^23 quanta is a
-// whole number of them.  A particle that may have a smaller one (one in a
-// thousand for the density, 7% for the diagonal stress of Gaussian velocities)
-// is listed, and what its terms leave below the quantum joins the sums at the
-// end (add_rest) where it can be told from their rounding, so that every term
-// counts in full whatever stands beside it.
-// (An FP32 shared atomic compiles to a compare-and-swap loop: the TwoSum pair
-// of add_comp takes 3.4 times the shared wavefronts of the two integer words.)
-// add_comp stays for what the integers cannot hold: terms that are not finite
-// or out of range, more than split_max particles, and more listed ones than
-// the list takes.  The two full-CIC calls at 256^3 in clumps take 3.25 ms, of
-// which 0.37 are the rests; the densities of 64^3 and 256^3 show no difference.
-enum : int { SUM_PAIR, SUM_INT, SUM_REST };  // what a run over the particles does
-
-struct RestList {
-  uint16_t* entry;  // listed particles of the CTA
-  int* count;       // how many were to be listed
+// whole number of them.  What a smaller one (one in 10^5 of the density's, 0.3%
+// of the diagonal stress's for Gaussian velocities) leaves below the quantum is
+// noted, and joins its vertex at the end where that can tell it from its
+// rounding (take_rests), so that every term counts in full whatever stands
+// beside it.  (An FP32 shared atomic compiles to a compare-and-swap loop: the
+// TwoSum pair of add_comp takes 3.4 times the shared wavefronts of the two
+// integer words.)  add_comp stays for what the integers cannot hold: terms that
+// are not finite or out of range, more than split_max particles, and more rests
+// than there is room for.  The tile passes of the two full-CIC calls at 256^3 in
+// clumps take 2.54 ms, as they did with the rests dropped and ldexpf for the
+// powers of two (a list of particles that may have one, looked through after
+// the loop: 2.74).
+struct Rests {
+  uint2* note;      // word of the vertex in the tile, bits of the rest
+  int* count;       // how many were to be noted
   int room;
-  __device__ __forceinline__ void add(int i) const
-  {
-    const int k = atomicAdd(count, 1);
-    if (k < room) entry[k] = (uint16_t)i;
-  }
+  uint32_t* marks;  // TileRef
+  int* any;         // set with the first mark
+  const float* quantum;  // (in shared memory: the particle loop keeps no register for it)
 };
 
-// The run over the listed particles takes a component to a warp (a chain of
-// the terms of all three is long for the few warps that have one): items
-// [c R, c R + count) with R = list_stride(count) are component c's.
-__host__ __device__ inline int list_stride(int count) { return (count + 31) & ~31; }
+// What a term w leaves below the quantum (0: a whole number of them).
+__device__ __forceinline__ float comp_rest(float w, float unit, float quantum)
+{
+  const float x = __fmul_rn(w, unit);
+  if (!(fabsf(x) < 0x1p-8f)) return 0.0f;
+  return __fmaf_rn(-__int2float_rn(__float2int_rn(__fmul_rn(x, 2147483648.0f))), quantum, w);  // exact
+}
 
-// A particle whose smallest term, `least` in units of 2^31 quanta, has fewer
-// than 2^23 of them (2^24: with room for the rounding of the bound) is listed.
-__device__ __forceinline__ bool has_rest(float least) { return least < 0x1p-7f; }
+// For a particle's smallest term in units of 2^31 quanta (a factor of two for
+// the rounding of its product).
+__device__ __forceinline__ bool may_have_rest(float least) { return least < 0x1p-7f; }
+
+__device__ __forceinline__ void note_rest(const Rests& rs, int word, float rest)
+{
+  const int k = atomicAdd(rs.count, 1);
+  if (k < rs.room) rs.note[k] = make_uint2((uint32_t)word, __float_as_uint(rest));
+}
 
 // w: the term; x = w in units of 2^31 quanta, |x| < 2^21.  x = hi + lo 2^-31
 // with hi the nearest integer (the sum with 1.5 * 2^23 rounds there) and lo
 // the nearest integer to the remainder, |lo| <= 2^30.  The words hold
 // hi 2^31 + lo: a carry or borrow of the low word is worth 2 of the high one.
-template <int N>
-__device__ __forceinline__ void add_comp_int(unsigned char* smem, int j, int t, float w, float unit)
+template <int N, bool NOTE>
+__device__ __forceinline__ void add_comp_int(unsigned char* smem, int j, int t, float w, float unit,
+                                             const Rests& rs)
 {
   uint32_t* words = reinterpret_cast<uint32_t*>(smem) + (size_t)j * 2 * N;
   const float x = __fmul_rn(w, unit);
@@ -175,60 +182,23 @@ __device__ __forceinline__ void add_comp_int(unsigned char* smem, int j, int t, 
   const uint32_t old = atomicAdd(&words[t], (uint32_t)lo);
   const int carry = old + (uint32_t)lo < old ? 1 : 0;
   atomicAdd(reinterpret_cast<int*>(&words[N + t]), hi + 2 * ((lo >> 31) + carry));
-}
-
-// What add_comp_int left of a listed particle's term below its quantum.  First
-// it is only asked whether it matters: half a quantum from each of `rests`
-// particles is under 2^-28 of a vertex sum of 2^27 `rests` quanta, a sixteenth
-// of the last rounding.  A smaller sum with a rest is marked, and the rest
-// noted; the marked sums become FP32 pairs (to_pairs) and then take their
-// rests, from the notes, or in another run (apply) where those ran out of room.
-struct Rests {
-  int count;
-  bool apply;
-  float quantum;
-  uint32_t* marks;  // TileRef
-  uint2* note;      // word of the vertex in the tile, bits of the rest
-  int* notes;       // how many were to be noted
-  int room;
-};
-
-__device__ __forceinline__ float comp_rest(float w, float unit, float quantum)
-{
-  const float x = __fmul_rn(w, unit);
-  if (!(fabsf(x) < 0x1p-8f)) return 0.0f;  // a whole number of quanta
-  return __fmaf_rn(-__int2float_rn(__float2int_rn(__fmul_rn(x, 2147483648.0f))), quantum, w);  // exact
-}
-
-template <int N>
-__device__ __forceinline__ void add_rest(unsigned char* smem, int j, int t, float w, float unit,
-                                         const Rests& rs)
-{
-  const float rest = comp_rest(w, unit, rs.quantum);
-  if (rest == 0.0f) return;
-  float* f = reinterpret_cast<float*>(smem) + (size_t)j * 2 * N + t;
-  const int i = j * N + t;
-  if (rs.apply) {
-    if (rs.marks[i >> 5] >> (i & 31) & 1u) add_comp(f, f + N, rest);
-  } else if (rs.count > 16 * (abs(__float_as_int(f[N])) - 2)) {  // (high word: units of 2^31 quanta)
-    atomicOr(&rs.marks[i >> 5], 1u << (i & 31));
-    const int k = atomicAdd(rs.notes, 1);
-    if (k < rs.room) rs.note[k] = make_uint2((uint32_t)(j * 2 * N + t), __float_as_uint(rest));
+  if (NOTE && fabsf(x) < 0x1p-8f) {
+    const float rest = __fmaf_rn(-__int2float_rn(lo), *rs.quantum, w);  // as comp_rest: here hi = 0
+    if (rest != 0.0f) note_rest(rs, j * 2 * N + t, rest);
   }
 }
 
-// One FP32 term of either mode.
-template <int ACC, int SUM, int N>
+// One FP32 term of either mode; SPLIT: the integer sums of the compensated one
+// (NOTE: with their rests).
+template <int ACC, bool SPLIT, bool NOTE, int N>
 __device__ __forceinline__ void add_float(unsigned char* smem, int j, int t, float w, float unit,
                                           const Rests& rs)
 {
   float* f = reinterpret_cast<float*>(smem);
   if (ACC == ACC_PLAIN)
     atomicAdd(&f[(size_t)j * N + t], w);
-  else if (SUM == SUM_INT)
-    add_comp_int<N>(smem, j, t, w, unit);
-  else if (SUM == SUM_REST)
-    add_rest<N>(smem, j, t, w, unit, rs);
+  else if (SPLIT)
+    add_comp_int<N, NOTE>(smem, j, t, w, unit, rs);
   else
     add_comp(&f[(size_t)j * 2 * N + t], &f[(size_t)j * 2 * N + N + t], w);
 }
@@ -297,30 +267,48 @@ __device__ __forceinline__ float2 comp_pair(const TileRef<N>& tr, int j, int t, 
   return make_float2(__fmul_rn(hi, quantum), __fmul_rn(lo, quantum));
 }
 
-// After the first run over the listed particles, by the whole CTA: the marked
-// vertex sums as FP32 pairs, and the noted rests.  False where another run has
-// to add the rests.  (With all sums as pairs in every CTA that has a mark, and
-// the second run instead of notes, the calls above took 3.67 ms.)
+// After the particles, by the whole CTA: the noted rests into the sums.  Half a
+// quantum each of n rests is under 2^-28 of a vertex sum of 2^27 n quanta, a
+// sixteenth of the last rounding; a smaller sum with a rest is marked, becomes
+// an FP32 pair and takes its rests.  (All sums as pairs in every CTA with a rest
+// cost the full-CIC passes 15%.)  False, with the tile cleared for a run with
+// pairs, where there were more rests than room.
 template <int N>
-__device__ __forceinline__ bool take_notes(unsigned char* smem, int comps, const Rests& rs)
+__device__ __forceinline__ bool take_rests(TileRef<N>& tr, int comps, const Rests& rs)
 {
-  uint32_t* w = reinterpret_cast<uint32_t*>(smem);
-  float* f = reinterpret_cast<float*>(smem);
-  const TileRef<N> ints{smem, true, nullptr};
+  uint32_t* w = reinterpret_cast<uint32_t*>(tr.smem);
+  float* f = reinterpret_cast<float*>(tr.smem);
+  const int n = *rs.count;
+  if (n == 0) return true;
+  if (n > rs.room) {
+    for (int t = threadIdx.x; t < comps * 2 * N; t += blockDim.x) w[t] = 0u;
+    tr.split = false;
+    __syncthreads();
+    return false;
+  }
+  for (int k = threadIdx.x; k < n; k += blockDim.x) {
+    const int at = (int)rs.note[k].x, i = at - at / (2 * N) * N;
+    if (n > 16 * (abs((int)w[at + N]) - 2)) {  // (high word: units of 2^31 quanta)
+      atomicOr(&rs.marks[i >> 5], 1u << (i & 31));
+      *rs.any = 1;
+    } else {
+      rs.note[k].y = 0u;
+    }
+  }
+  __syncthreads();
+  if (!*rs.any) return true;
   for (int k = threadIdx.x; k < (comps * N + 31) / 32; k += blockDim.x) {
     for (uint32_t m = rs.marks[k]; m; m &= m - 1) {
       const int i = 32 * k + __ffs(m) - 1, j = i / N, t = i % N, at = j * 2 * N + t;
-      const float2 p = comp_pair(ints, j, t, rs.quantum);
+      const float2 p = comp_pair(tr, j, t, *rs.quantum);
       w[at] = __float_as_uint(p.x);
       w[at + N] = __float_as_uint(p.y);
     }
   }
+  tr.marks = rs.marks;
   __syncthreads();
-  const int n = *rs.notes;
-  if (n > rs.room) return false;
   for (int k = threadIdx.x; k < n; k += blockDim.x)
-    add_comp(&f[rs.note[k].x], &f[rs.note[k].x + N], __uint_as_float(rs.note[k].y));
-  __syncthreads();
+    if (rs.note[k].y) add_comp(&f[rs.note[k].x], &f[rs.note[k].x + N], __uint_as_float(rs.note[k].y));
   return true;
 }
 

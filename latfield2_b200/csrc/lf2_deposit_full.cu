@@ -332,17 +332,16 @@ __global__ void __launch_bounds__(256, 4)
 // CTA per SM), and every vertex another brick can reach goes to the
 // thick-shell store.  The three passes of the compensated mode at 256^3 took
 // 9.96 ms with FP32 atomics (their compare-and-swap loops: 26% issue) and one
-// CTA per brick; with the integer sums and split bricks 2.74 ms.
+// CTA per brick; with the integer sums and split bricks 2.54 ms.
 constexpr int FULL2_THREADS = 1024;
 
-// Shared memory of a plain tile, of one of two words per vertex, and the
-// notes and the list that the compensated mode keeps after that (Rests;
-// RestList: room for all particles of a part).
+// Shared memory of a plain tile, of one of two words per vertex, and the rests
+// that the compensated mode notes after that (Rests).
 constexpr size_t FULL_SMEM = (size_t)3 * FT3 * sizeof(float), FULL2_SMEM = 2 * FULL_SMEM;
-constexpr int FULL_RESTS = 32768, FULL_NOTES = 2048;
+constexpr int FULL_RESTS = 8192;
 
 template <int ACC>
-constexpr size_t full2_dyn() { return FULL2_SMEM + (ACC == ACC_COMP ? FULL_NOTES * sizeof(uint2) + FULL_RESTS * sizeof(uint16_t) : 0); }
+constexpr size_t full2_dyn() { return FULL2_SMEM + (ACC == ACC_COMP ? FULL_RESTS * sizeof(uint2) : 0); }
 
 // HM: per-particle masses, or a global one.
 template <int PASS, int ACC, bool HM>
@@ -355,7 +354,7 @@ __global__ void __launch_bounds__(FULL2_THREADS, 1)
   constexpr bool FIXED = ACC == ACC_FIXED;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ unsigned s_max;
-  __shared__ int s_rests, s_notes;
+  __shared__ int s_rests, s_any;
   __shared__ uint32_t s_marks[ACC == ACC_COMP ? (3 * FT3 + 31) / 32 : 1];
   __shared__ float s_quantum;
   __shared__ int s_brick, s_tile;  // (so that the particle loop keeps no register for them)
@@ -387,28 +386,18 @@ __global__ void __launch_bounds__(FULL2_THREADS, 1)
     for (int t = threadIdx.x; t < 3 * 2 * FT3; t += blockDim.x) zw[t] = 0u;
     if (ACC == ACC_COMP)
       for (int t = threadIdx.x; t < (3 * FT3 + 31) / 32; t += blockDim.x) s_marks[t] = 0u;
-    if (threadIdx.x == 0) s_rests = 0, s_notes = 0, s_quantum = cu.quantum;
+    if (threadIdx.x == 0) s_rests = 0, s_any = 0, s_quantum = cu.quantum;
   }
   __syncthreads();
-  uint2* const notes = reinterpret_cast<uint2*>(smem_raw + FULL2_SMEM);
-  const RestList rl{reinterpret_cast<uint16_t*>(notes + FULL_NOTES), &s_rests, FULL_RESTS};
+  const Rests rs{reinterpret_cast<uint2*>(smem_raw + FULL2_SMEM), &s_rests, FULL_RESTS, s_marks, &s_any,
+                 &s_quantum};
 
   constexpr int pa[3] = {0, 0, 1}, pb[3] = {1, 2, 2};
-  // the particle loop, instantiated per CTA for the split tile (or not), and
-  // for the listed particles' rests
-  Rests rs{0, false, cu.quantum, s_marks, notes, &s_notes, FULL_NOTES};
-  auto particles = [&](auto sum_c, int cnt) {
-    constexpr int SUM = decltype(sum_c)::value;
-    constexpr bool SPLIT = SUM == SUM_INT;
-    const int stride = list_stride(rs.count);
+  // the particle loop, instantiated per CTA for the split tile (or not)
+  auto particles = [&](auto split_c) {
+    constexpr bool SPLIT = decltype(split_c)::value;
     for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
-      int only = 0, at = i;  // component and particle (the rests)
-      if (SUM == SUM_REST) {
-        only = i / stride;
-        if (i % stride >= rs.count) continue;
-        at = rl.entry[i % stride];
-      }
-      const uint32_t p = (uint32_t)base + (uint32_t)at;  // slots fit in 32 bits
+      const uint32_t p = (uint32_t)base + (uint32_t)i;  // slots fit in 32 bits
       int x, y, z;
       unpack_key(g, v.a.key[p], x, y, z);
       const float o[3] = {v.a.ox[p], v.a.oy[p], v.a.oz[p]};
@@ -502,24 +491,9 @@ __global__ void __launch_bounds__(FULL2_THREADS, 1)
           tw[d][1] = __fsub_rn(1.0f, tw[d][0]);
         }
       }
-      if (!FIXED && SPLIT) {  // a bound below the particle's smallest term
-        float f = 3.402823466e38f;
-  #pragma unroll
-        for (int c = 0; c < 3; c++) {
-          const float mv = __fmul_rn(mf, vel[PASS == 2 ? pa[c] : c]);
-          f = fminf(f, fabsf(PASS == 0 ? mv : __fmul_rn(mv, vel[PASS == 2 ? pb[c] : c])));
-        }
-  #pragma unroll
-        for (int d = 0; d < 3; d++) {
-          const float u = fminf(sw[d][0], sw[d][1]);
-          f = __fmul_rn(f, PASS == 1 ? u : fminf(u, fminf(tw[d][0], tw[d][1])));
-        }
-        if (has_rest(__fmul_rn(f, cu.unit))) rl.add(i);
-      }
       if (PASS == 0) {
   #pragma unroll
         for (int c = 0; c < 3; c++) {
-          if (SUM == SUM_REST && c != only) continue;
           const float mv = __fmul_rn(mf, vel[c]);
   #pragma unroll
           for (int k = 0; k < 8; k++) {
@@ -529,26 +503,24 @@ __global__ void __launch_bounds__(FULL2_THREADS, 1)
             const float w2 = c == 2 ? tw[2][b2] : sw[2][b2];
             const int t = tile_at((c == 0 ? lt[0] : ls[0]) + b0, (c == 1 ? lt[1] : ls[1]) + b1,
                                   (c == 2 ? lt[2] : ls[2]) + b2);
-            add_float<ACC, SUM, FT3>(smem_raw, c, t, __fmul_rn(__fmul_rn(__fmul_rn(mv, w0), w1), w2),
+            add_float<ACC, SPLIT, true, FT3>(smem_raw, c, t, __fmul_rn(__fmul_rn(__fmul_rn(mv, w0), w1), w2),
                                     cu.unit, rs);
           }
         }
       } else if (PASS == 1) {
   #pragma unroll
         for (int i2 = 0; i2 < 3; i2++) {
-          if (SUM == SUM_REST && i2 != only) continue;
           const float m2 = __fmul_rn(__fmul_rn(mf, vel[i2]), vel[i2]);
   #pragma unroll
           for (int k = 0; k < 8; k++) {
             const int b0 = (k >> 2) & 1, b1 = (k >> 1) & 1, b2 = k & 1;
-            add_float<ACC, SUM, FT3>(smem_raw, i2, tile_at(ls[0] + b0, ls[1] + b1, ls[2] + b2),
+            add_float<ACC, SPLIT, true, FT3>(smem_raw, i2, tile_at(ls[0] + b0, ls[1] + b1, ls[2] + b2),
                            __fmul_rn(__fmul_rn(__fmul_rn(m2, sw[0][b0]), sw[1][b1]), sw[2][b2]), cu.unit, rs);
           }
         }
       } else {
   #pragma unroll
         for (int q = 0; q < 3; q++) {
-          if (SUM == SUM_REST && q != only) continue;
           const float mm = __fmul_rn(__fmul_rn(mf, vel[pa[q]]), vel[pb[q]]);
   #pragma unroll
           for (int k = 0; k < 8; k++) {
@@ -561,31 +533,20 @@ __global__ void __launch_bounds__(FULL2_THREADS, 1)
               w[d] = st ? tw[d][bb[d]] : sw[d][bb[d]];
               t[d] = (st ? lt[d] : ls[d]) + bb[d];
             }
-            add_float<ACC, SUM, FT3>(smem_raw, q, tile_at(t[0], t[1], t[2]),
+            add_float<ACC, SPLIT, true, FT3>(smem_raw, q, tile_at(t[0], t[1], t[2]),
                            __fmul_rn(__fmul_rn(__fmul_rn(mm, w[0]), w[1]), w[2]), cu.unit, rs);
           }
         }
       }
     }
   };
-  using std::integral_constant;
-  bool pairs = !tr.split;
-  if (!pairs) particles(integral_constant<int, SUM_INT>{}, cnt);
+  bool split = tr.split;
+  if (split) particles(std::true_type{});
   if constexpr (!FIXED) {
     __syncthreads();
-    rs.count = s_rests;
-    if (rs.count) {  // (the list holds every particle of a part)
-      for (int pass = 0; pass < 2; pass++) {
-        particles(integral_constant<int, SUM_REST>{}, 3 * list_stride(rs.count));
-        __syncthreads();
-        if (rs.apply || !s_notes) break;
-        tr.marks = s_marks;
-        if (take_notes<FT3>(smem_raw, 3, rs)) break;
-        rs.apply = true;
-      }
-    }
+    if (split) split = take_rests(tr, 3, rs);
   }
-  if (pairs) particles(integral_constant<int, SUM_PAIR>{}, cnt);
+  if (!split) particles(std::false_type{});
   __syncthreads();
   if (s_tile >= 0) {
     part_store<ACC, true, 3, FT3>(scratch_tile(pv, s_tile, 3 * FT3), tr, s_quantum);

@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(256)
     if (!FIXED && tiled) {  // terms that are no whole number of quanta: their rests to the field
       const float least = fminf(f[0], 1.0f - f[0]) * fminf(f[1], 1.0f - f[1]) * fminf(f[2], 1.0f - f[2]) *
                           fabsf(m);
-      if (has_rest(__fmul_rn(least, cu.unit))) {
+      if (may_have_rest(__fmul_rn(least, cu.unit))) {
 #pragma unroll 1
         for (int q = 0; q < 8; q++) {
           const int cx = (q >> 2) & 1, cy = (q >> 1) & 1, cz = q & 1;
