@@ -755,69 +755,71 @@ __global__ void __launch_bounds__(FIX2_THREADS, 2)
     }
     return;
   }
-  constexpr int I = BRICK - 2;
-  if (threadIdx.x < FIX2_FACE) {
-    const int u = 1 + threadIdx.x % I, w = 1 + threadIdx.x / I;
+  for (int v = threadIdx.x; v < FIX2_FACE + FIX2_EDGE; v += blockDim.x) {
+    constexpr int I = BRICK - 2;
+    if (v < FIX2_FACE) {
+      const int u = 1 + v % I, w = 1 + v / I;
 #pragma unroll 1
-    for (int side = 0; side < 2; side++) {  // the faces below, then those above
-      uint64_t r[3][3][2];
-      bool on[3];
-      constexpr int du[3] = {1, 0, 0}, dw[3] = {2, 2, 1};
-      // own tile coordinate of the face, and the neighbour's that reaches it
-      const int mine = side ? FT - 2 : 1, theirs = side ? 0 : FT - 1;
+      for (int side = 0; side < 2; side++) {  // the faces below, then those above
+        uint64_t r[3][3][2];
+        bool on[3];
+        constexpr int du[3] = {1, 0, 0}, dw[3] = {2, 2, 1};
+        // own tile coordinate of the face, and the neighbour's that reaches it
+        const int mine = side ? FT - 2 : 1, theirs = side ? 0 : FT - 1;
 #pragma unroll
-      for (int d = 0; d < 3; d++) {
-        on[d] = u < e[du[d]] - 1 && w < e[dw[d]] - 1;
-        const int so = d == 0 ? thick_index(mine, u + 1, w + 1)
-                       : d == 1 ? thick_index(u + 1, mine, w + 1) : thick_index(u + 1, w + 1, mine);
-        const int sn = d == 0 ? thick_index(theirs, u + 1, w + 1)
-                       : d == 1 ? thick_index(u + 1, theirs, w + 1) : thick_index(u + 1, w + 1, theirs);
-        const int64_t nb = b + (side ? nbr[d][1] : nbr[d][0]);
+        for (int d = 0; d < 3; d++) {
+          on[d] = u < e[du[d]] - 1 && w < e[dw[d]] - 1;
+          const int so = d == 0 ? thick_index(mine, u + 1, w + 1)
+                         : d == 1 ? thick_index(u + 1, mine, w + 1) : thick_index(u + 1, w + 1, mine);
+          const int sn = d == 0 ? thick_index(theirs, u + 1, w + 1)
+                         : d == 1 ? thick_index(u + 1, theirs, w + 1) : thick_index(u + 1, w + 1, theirs);
+          const int64_t nb = b + (side ? nbr[d][1] : nbr[d][0]);
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-          // the lower one is added first
-          r[d][c][0] = on[d] ? read(side ? b : nb, c, side ? so : sn) : 0;
-          r[d][c][1] = on[d] ? read(side ? nb : b, c, side ? sn : so) : 0;
+          for (int c = 0; c < 3; c++) {
+            // the lower one is added first
+            r[d][c][0] = on[d] ? read(side ? b : nb, c, side ? so : sn) : 0;
+            r[d][c][1] = on[d] ? read(side ? nb : b, c, side ? sn : so) : 0;
+          }
+        }
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          if (!on[d]) continue;
+          const int64_t site = site0 + u * step[du[d]] + w * step[dw[d]] + (side ? (e[d] - 1) * step[d] : 0);
+#pragma unroll
+          for (int c = 0; c < 3; c++) {
+            Sum s;
+            s.add(r[d][c][0]);
+            s.add(r[d][c][1]);
+            out[(c0 + c) * g.nsites + site] = s.value(conv);
+          }
         }
       }
+      continue;
+    }
+    // edges (two coordinates at an end, the third inside) and corners
+    const int ne[3] = {e[0] - 2, e[1] - 2, e[2] - 2};
+    const int edges = 4 * (ne[0] + ne[1] + ne[2]);
+    const int f = v - FIX2_FACE;
+    if (f >= edges + 8) continue;
+    int q[3], side[3], ends = 7;
+    if (f < edges) {
+      const int d = f < 4 * ne[0] ? 0 : f < 4 * (ne[0] + ne[1]) ? 1 : 2;
+      const int r = f - (d > 0 ? 4 * ne[0] : 0) - (d > 1 ? 4 * ne[1] : 0);
+      ends = 7 & ~(1 << d);
 #pragma unroll
-      for (int d = 0; d < 3; d++) {
-        if (!on[d]) continue;
-        const int64_t site = site0 + u * step[du[d]] + w * step[dw[d]] + (side ? (e[d] - 1) * step[d] : 0);
+      for (int k = 0; k < 3; k++) {
+        side[k] = k == (d == 0 ? 1 : 0) ? r & 1 : (r >> 1) & 1;
+        q[k] = k == d ? 1 + r / 4 : side[k] ? e[k] - 1 : 0;
+      }
+    } else {
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-          Sum s;
-          s.add(r[d][c][0]);
-          s.add(r[d][c][1]);
-          out[(c0 + c) * g.nsites + site] = s.value(conv);
-        }
+      for (int k = 0; k < 3; k++) {
+        side[k] = ((f - edges) >> k) & 1;
+        q[k] = side[k] ? e[k] - 1 : 0;
       }
     }
-    return;
+    corner(q, ends, side);
   }
-  // edges (two coordinates at an end, the third inside) and corners
-  const int ne[3] = {e[0] - 2, e[1] - 2, e[2] - 2};
-  const int edges = 4 * (ne[0] + ne[1] + ne[2]);
-  const int f = (int)threadIdx.x - FIX2_FACE;
-  if (f >= edges + 8) return;
-  int q[3], side[3], ends = 7;
-  if (f < edges) {
-    const int d = f < 4 * ne[0] ? 0 : f < 4 * (ne[0] + ne[1]) ? 1 : 2;
-    const int r = f - (d > 0 ? 4 * ne[0] : 0) - (d > 1 ? 4 * ne[1] : 0);
-    ends = 7 & ~(1 << d);
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      side[k] = k == (d == 0 ? 1 : 0) ? r & 1 : (r >> 1) & 1;
-      q[k] = k == d ? 1 + r / 4 : side[k] ? e[k] - 1 : 0;
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      side[k] = ((f - edges) >> k) & 1;
-      q[k] = side[k] ? e[k] - 1 : 0;
-    }
-  }
-  corner(q, ends, side);
 }
 
 template <int PASS, int ACC>
@@ -861,9 +863,9 @@ cudaError_t run2(lf2_ctx* c, int kind, float* out, const DepositParams& dp, int 
   }
   c->launches += 1;
   if (kind == 3)
-    k_fixup_full2<3, ACC><<<nb, FIX2_THREADS, 0, c->stream>>>(c->g, c->spill, dp.fixed_scale, c->vmax_bits, out);
+    k_fixup_full2<3, ACC><<<nb, fix_threads(c, FIX2_THREADS), 0, c->stream>>>(c->g, c->spill, dp.fixed_scale, c->vmax_bits, out);
   else
-    k_fixup_full2<6, ACC><<<dim3(nb, 2), FIX2_THREADS, 0, c->stream>>>(c->g, c->spill, dp.fixed_scale, c->vmax_bits, out);
+    k_fixup_full2<6, ACC><<<dim3(nb, 2), fix_threads(c, FIX2_THREADS), 0, c->stream>>>(c->g, c->spill, dp.fixed_scale, c->vmax_bits, out);
   return cudaGetLastError();
 }
 

@@ -210,6 +210,7 @@ PartPlan part_plan(lf2_ctx* c, size_t smem, int threads, size_t tile_slots, int 
 PartView part_view(const lf2_ctx* c, const PartPlan& pl, size_t tile_slots);
 cudaError_t launch_part_plan(lf2_ctx* c, const PartPlan& pl);
 PartPlan scalar_plan(lf2_ctx* c);
+int fix_threads(const lf2_ctx* c, int whole);
 // largest |v_i| of the store into c->vmax_bits (fixed-point momentum/stress)
 cudaError_t launch_vmax(lf2_ctx* c, const PartView& pv);
 
