@@ -250,6 +250,7 @@ lf2_status load_device(lf2_ctx* c, int64_t n, const int32_t* cell, const float* 
     LF2_CUDA(c, cudaStreamSynchronize(c->stream));
     c->m_unit = (n > 0 && c->h_stats[1] > 0) ? c->h_stats[1] / (double)n : 1.0;
   }
+  if (!rows_pay(c)) release_rows(c);  // of the store before
   prepare_rows(c);
   return LF2_OK;
 }

@@ -288,7 +288,7 @@ __device__ __forceinline__ bool take_rests(TileRef<N>& tr, int comps, const Rest
   }
   for (int k = threadIdx.x; k < n; k += blockDim.x) {
     const int at = (int)rs.note[k].x, i = at - at / (2 * N) * N;
-    if (n > 16 * (abs((int)w[at + N]) - 2)) {  // (high word: units of 2^31 quanta)
+    if (abs((int)w[at + N]) < n / 16 + 3) {  // (high word: units of 2^31 quanta, at least |h| - 2 of them)
       atomicOr(&rs.marks[i >> 5], 1u << (i & 31));
       *rs.any = 1;
     } else {

@@ -186,6 +186,7 @@ bool move_pipe_eligible(const lf2_ctx* c, const float* F);
 bool move_pipe_auto(const lf2_ctx* c, const float* F);
 bool kick_pipe_auto(const lf2_ctx* c, const float* F);
 bool drift_pipe_auto(const lf2_ctx* c);
+bool rows_pay(const lf2_ctx* c);
 void prepare_rows(lf2_ctx* c);
 bool release_rows(lf2_ctx* c);
 bool move_dep_eligible(const lf2_ctx* c, const float* F);

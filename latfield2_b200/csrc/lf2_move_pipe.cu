@@ -1057,7 +1057,7 @@ static bool clumped(const lf2_ctx* c)
 // per site.  Steps per-brick / pipelined in us, 150 x 141 x 133 and 314^3: even,
 // 0.34 particles per site 58 / 83 and 504 / 496, 1.0 118 / 112 and 926 / 778;
 // clumps, 0.34 121 / 98 and 797 / 545, 1.0 262 / 160 and 1746 / 881.
-static bool rows_pay(const lf2_ctx* c)
+bool rows_pay(const lf2_ctx* c)
 {
   return clumped(c) ? 3 * c->np >= c->g.nsites : 4 * c->np >= 3 * c->g.nsites;
 }

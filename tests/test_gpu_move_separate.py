@@ -134,7 +134,8 @@ def test_kick_drift_and_deposit_under_capture(cuda, warm):
 
 def test_the_first_kick_allocates_nothing(cuda):
     """The padded rows (36 MB here) come with the load and go with the choice of
-    the per-brick kernel; the first step takes the pipelined kernel."""
+    the per-brick kernel, or with a store for which they do not pay; the first
+    step takes the pipelined kernel."""
     import torch
     import latfield2_b200 as L
     n, npart = (150, 141, 142), 2300000
@@ -164,6 +165,10 @@ def test_the_first_kick_allocates_nothing(cuda):
     assert free() - before > 6 * sites
     ctx.step(f, 0.1, 0.1)
     assert ctx.last_move_kernel() == 1
+    ctx.set_move_kernel(0)
+    assert abs(before - free()) < 6 * sites
+    ctx.set_particles(cell[:1000], off[:1000], vel[:1000], global_mass=1.0)  # nor with a sparse store
+    assert free() - before > 6 * sites
     ctx.close()
     warm.close()
 
